@@ -317,7 +317,7 @@ def run(st):
         new.pagerank_pull(c["iters"], DAMPING, out=st.ranks)
         deg = new.out_degrees()
     st.store.drop_level()
-    return {"ranks": st.ranks, "degrees": deg.astype(np.int64)}
+    return {"ranks": st.ranks, "degrees": deg.view(np.int32)}
 
 
 def work(case):
