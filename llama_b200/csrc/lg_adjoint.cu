@@ -249,6 +249,7 @@ struct lg_adjoint {
 	double d = 0.85, tol = 1e-12;
 	int max_iter = 0;
 	DevBuf x, w;           // converged scores; the weights, out-adjacency order
+	explicit lg_adjoint(const std::shared_ptr<lg::CallPool>& pool) : x(pool), w(pool) {}
 };
 
 namespace {
@@ -258,7 +259,8 @@ lg_status build_maps(lg_snapshot* sn, lg_adjoint_maps* m) {
 	cudaStream_t st = s->stream;
 	const uint64_t V = sn->V;
 	const uint64_t E = m->E;
-	DevBuf out_pos, in_pos, dst, adj_off, p32, scan_tmp, badb, flag, at;
+	DevBuf out_pos(s->pool), in_pos(s->pool), dst(s->pool), adj_off(s->pool), p32(s->pool),
+			scan_tmp(s->pool), badb(s->pool), flag(s->pool), at(s->pool);
 	LG_TRY(out_pos.reserve(std::max<uint64_t>(sn->out.n_frag_slots, 1) * 4));
 	LG_TRY(in_pos.reserve(std::max<uint64_t>(sn->in.n_frag_slots, 1) * 4));
 	LG_TRY(m->src.reserve(std::max<uint64_t>(E, 1) * 4));
@@ -465,7 +467,7 @@ extern "C" lg_status lg_pagerank_fwd(lg_snapshot* sn, const double* weights,
 	LG_TRY(fixed_point(sn, m->fin, m->win.as<double>(), m->base.as<double>(), damping, tol,
 			max_iter, &it, &r, &res));
 	if (tape) {
-		lg_adjoint* t = new (std::nothrow) lg_adjoint();
+		lg_adjoint* t = new (std::nothrow) lg_adjoint(s->pool);
 		if (!t) return set_error(LG_ENOMEM, "host allocation");
 		t->snap = sn;
 		t->d = damping;
@@ -497,7 +499,7 @@ extern "C" lg_status lg_pagerank_bwd(lg_adjoint* t, const double* dldx, double* 
 	const uint64_t V = sn->V;
 	lg_adjoint_maps* m = sn->adj_maps;
 	const uint64_t E = m->E;
-	DevBuf outw, oute;
+	DevBuf outw(s->pool), oute(s->pool);
 	const double* g;
 	LG_TRY(stage_in(s, dldx, V, m->stage_g, &g));
 	LG_TRY(m->xa.reserve(V * 8));

@@ -231,7 +231,8 @@ extern "C" lg_status lg_bc(lg_snapshot* sn, const int64_t* sources, int n_source
 	LG_CUDA(cudaSetDevice(s->device), "cudaSetDevice");
 	cudaStream_t st = s->stream;
 	const uint64_t V = sn->V;
-	DevBuf level, sigma, delta, order, cnt, pos, scan_tmp, ctrb, bcb, heavy;
+	DevBuf level(s->pool), sigma(s->pool), delta(s->pool), order(s->pool), cnt(s->pool),
+			pos(s->pool), scan_tmp(s->pool), ctrb(s->pool), bcb(s->pool), heavy(s->pool);
 	LG_TRY(level.reserve(V * 4));
 	LG_TRY(sigma.reserve(V * 8));
 	LG_TRY(delta.reserve(V * 8));

@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <memory>
 #include <utility>
 #include <vector>
 
@@ -136,19 +137,41 @@ __device__ __forceinline__ double warp_segsum(double v, uint32_t key, bool* tail
 // Host-side objects
 // ---------------------------------------------------------------------------
 
-// Device allocation owned by a host object.
+// A store's stream-ordered memory pool for the temporaries of one call.
+// Memory given back to it is handed out again without a driver call that
+// waits for the GPU; up to kPoolKeep bytes stay with the pool between calls,
+// the rest goes back to the device at the next synchronisation, and all of it
+// when the store is destroyed or when any allocation of the process fails
+// (trim_pools).  stream becomes null when the store is destroyed; a buffer
+// that outlives its store is then freed with cudaFree.
+struct CallPool {
+	cudaMemPool_t pool = nullptr;
+	cudaStream_t stream = nullptr;
+	CallPool() = default;
+	CallPool(const CallPool&) = delete;
+	CallPool& operator=(const CallPool&) = delete;
+	~CallPool();
+};
+constexpr uint64_t kPoolKeep = 1ull << 30;
+// A pool on `device` whose allocations and frees are ordered by `stream`.
+lg_status make_pool(int device, cudaStream_t stream, std::shared_ptr<CallPool>* out);
+
+// Device allocation owned by a host object: cudaMalloc / cudaFree, or, given
+// a pool, the pool's stream-ordered memory (used on the pool's stream only).
 struct DevBuf {
 	void* p = nullptr;
 	size_t bytes = 0;
+	std::shared_ptr<CallPool> from;
 	DevBuf() = default;
+	explicit DevBuf(const std::shared_ptr<CallPool>& pool) : from(pool) {}
 	DevBuf(const DevBuf&) = delete;
 	DevBuf& operator=(const DevBuf&) = delete;
 	~DevBuf() { release(); }
-	void release() { if (p) cudaFree(p); p = nullptr; bytes = 0; }
+	void release();
 	// (Re)allocate to at least n bytes; contents are not preserved.
 	lg_status reserve(size_t n);
 	template <class T> T* as() const { return static_cast<T*>(p); }
-	void swap(DevBuf& o) { std::swap(p, o.p); std::swap(bytes, o.bytes); }
+	void swap(DevBuf& o) { std::swap(p, o.p); std::swap(bytes, o.bytes); from.swap(o.from); }
 };
 
 struct DevLevel {
@@ -220,6 +243,8 @@ struct lg_store {
 	cudaEvent_t staged[2] = {nullptr, nullptr};
 	// scratch shared by the analytics calls of this store
 	lg::DevBuf scratch[12];
+	// temporaries of single calls (lg::DevBuf x(s->pool))
+	std::shared_ptr<lg::CallPool> pool;
 	int open_snapshots = 0;
 	uint64_t launches = 0;      // kernels launched by this store
 	uint64_t h2d_bytes = 0;     // host -> device bytes copied by this store

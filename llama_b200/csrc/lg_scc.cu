@@ -187,7 +187,9 @@ extern "C" lg_status lg_scc(lg_snapshot* sn, int64_t* labels, lg_scc_result* res
 	LG_CUDA(cudaSetDevice(s->device), "cudaSetDevice");
 	cudaStream_t st = s->stream;
 	const uint64_t V = sn->V;
-	DevBuf label, color, mark, stamp, rem, rem2, wl, wl2, cnt, pos, scan_tmp, ctrb, outb;
+	DevBuf label(s->pool), color(s->pool), mark(s->pool), stamp(s->pool), rem(s->pool),
+			rem2(s->pool), wl(s->pool), wl2(s->pool), cnt(s->pool), pos(s->pool),
+			scan_tmp(s->pool), ctrb(s->pool), outb(s->pool);
 	for (DevBuf* b : {&label, &color, &mark, &stamp, &rem, &rem2, &wl, &wl2, &cnt})
 		LG_TRY(b->reserve(V * 4));
 	LG_TRY(pos.reserve((V + 1) * 4));

@@ -37,15 +37,73 @@ lg_status cuda_status(cudaError_t e, const char* what) {
 	return set_error(LG_ECUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
+// Pools of every live store, to give their idle memory back when an
+// allocation fails.
+static std::mutex g_pools_mu;
+static std::vector<CallPool*> g_pools;
+
+CallPool::~CallPool() {
+	{
+		std::lock_guard<std::mutex> lk(g_pools_mu);
+		g_pools.erase(std::remove(g_pools.begin(), g_pools.end(), this), g_pools.end());
+	}
+	if (pool) cudaMemPoolDestroy(pool);
+}
+
+lg_status make_pool(int device, cudaStream_t stream, std::shared_ptr<CallPool>* out) {
+	std::shared_ptr<CallPool> c;
+	try {
+		c = std::make_shared<CallPool>();
+		std::lock_guard<std::mutex> lk(g_pools_mu);
+		g_pools.push_back(c.get());
+	} catch (const std::bad_alloc&) {
+		return set_error(LG_ENOMEM, "host allocation");
+	}
+	cudaMemPoolProps props;
+	std::memset(&props, 0, sizeof(props));
+	props.allocType = cudaMemAllocationTypePinned;
+	props.location.type = cudaMemLocationTypeDevice;
+	props.location.id = device;
+	LG_CUDA(cudaMemPoolCreate(&c->pool, &props), "memory pool");
+	uint64_t keep = kPoolKeep;
+	LG_CUDA(cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep),
+			"memory pool");
+	c->stream = stream;
+	*out = c;
+	return LG_OK;
+}
+
+// Gives the memory no buffer holds back to the device.
+static void trim_pools() {
+	cudaDeviceSynchronize();        // frees queued on the pools' streams have happened
+	std::lock_guard<std::mutex> lk(g_pools_mu);
+	for (CallPool* c : g_pools) if (c->pool) cudaMemPoolTrimTo(c->pool, 0);
+}
+
+void DevBuf::release() {
+	if (p) {
+		if (from && from->stream) cudaFreeAsync(p, from->stream);
+		else cudaFree(p);
+	}
+	p = nullptr;
+	bytes = 0;
+}
+
 lg_status DevBuf::reserve(size_t n) {
 	if (n <= bytes && p) return LG_OK;
 	release();
 	if (n == 0) n = 16;
-	cudaError_t e = cudaMalloc(&p, n);
+	cudaError_t e = cudaSuccess;
+	for (int attempt = 0; attempt < 2; attempt++) {
+		e = from ? cudaMallocFromPoolAsync(&p, n, from->pool, from->stream) : cudaMalloc(&p, n);
+		if (e != cudaErrorMemoryAllocation || attempt) break;
+		(void)cudaGetLastError();
+		trim_pools();
+	}
 	if (e != cudaSuccess) {
 		p = nullptr;
 		(void)cudaGetLastError();
-		return cuda_status(e, "cudaMalloc");
+		return cuda_status(e, from ? "cudaMallocFromPoolAsync" : "cudaMalloc");
 	}
 	bytes = n;
 	return LG_OK;
@@ -772,6 +830,12 @@ lg_status lg_store_create(lg_store** out, const lg_store_opts* opts) {
 		if (e != cudaSuccess) { delete s; return cuda_status(e, "stream"); }
 		s->own_stream = true;
 	}
+	const lg_status ps = make_pool(dev, s->stream, &s->pool);
+	if (ps) {
+		if (s->own_stream) cudaStreamDestroy(s->stream);
+		delete s;
+		return ps;
+	}
 	*out = s;
 	return LG_OK;
 }
@@ -800,6 +864,8 @@ lg_status lg_store_destroy(lg_store* s) {
 		delete s->snap_spare[d];
 		delete s->level_spare[d];
 	}
+	// buffers that outlive the store (a tape) are freed without its stream
+	s->pool->stream = nullptr;
 	if (s->own_stream) cudaStreamDestroy(s->stream);
 	delete s;
 	return LG_OK;
@@ -887,6 +953,10 @@ uint64_t lg_store_device_bytes(const lg_store* s) {
 		b += c->dels.bytes;
 	}
 	for (const DevBuf& x : s->scratch) b += x.bytes;
+	uint64_t kept = 0;
+	if (cudaMemPoolGetAttribute(s->pool->pool, cudaMemPoolAttrReservedMemCurrent, &kept)
+			== cudaSuccess)
+		b += kept;
 	return b;
 }
 
@@ -1072,7 +1142,7 @@ lg_status lg_snapshot_adjacency(lg_snapshot* sn, int dir, uint64_t* offsets,
 	cudaStream_t st = s->stream;
 	SnapCsr g = sn->view(dir);
 	const uint64_t V = sn->V;
-	DevBuf cnt, off, nb, ei;
+	DevBuf cnt(s->pool), off(s->pool), nb(s->pool), ei(s->pool);
 	LG_TRY(cnt.reserve(V * 4));
 	LG_TRY(off.reserve((V + 1) * 8));
 	live_counts<<<grid_for(V, 256), 256, 0, st>>>(g, cnt.as<uint32_t>());

@@ -167,7 +167,9 @@ extern "C" lg_status lg_triangle_count(lg_snapshot* sn, lg_tc_result* result) {
 	const uint64_t V = sn->V;
 	const uint64_t E = sn->out.n_edges;
 	if (E >= 0xffffffffull) return set_error(LG_ENOTSUP, "more than 2^32-1 live edges");
-	DevBuf rank, keys, tmpk, tmpp, counts, scan_tmp, uniq, flags, off, ctr, adj;
+	DevBuf rank(s->pool), keys(s->pool), tmpk(s->pool), tmpp(s->pool), counts(s->pool),
+			scan_tmp(s->pool), uniq(s->pool), flags(s->pool), off(s->pool), ctr(s->pool),
+			adj(s->pool);
 	LG_TRY(rank.reserve(V * 4));
 	LG_TRY(keys.reserve(std::max<uint64_t>(E, 1) * 8));
 	LG_TRY(ctr.reserve(2 * sizeof(unsigned long long)));
