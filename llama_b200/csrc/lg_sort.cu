@@ -1,14 +1,19 @@
 // lg_sort.cu - device LSD radix sort of 64-bit keys (optional 32-bit
-// payload) and de-duplication, used to flatten and orient snapshots.
+// payload), used to flatten, orient and build snapshots.
 //
-// One pass per 8-bit digit that varies over the input (the varying bits are
-// found first with an OR/AND reduction, so 48-bit keys cost 6 passes):
+// One pass per 8-bit digit that may vary (the caller says which bits, or they
+// are found with an OR/AND reduction; 48-bit keys cost 6 passes):
 //   rs_hist     per-tile digit counts, stored digit-major
 //   scan        exclusive scan of the counts -> scatter bases
-//   rs_scatter  stable scatter: a tile is ranked in 16 rounds of 256 keys;
-//               inside a round, __match_any_sync groups the lanes of a warp
-//               that share a digit and the per-warp counts in shared memory
-//               give the rank across warps, so equal digits keep input order.
+//   rs_scatter  stable scatter: a warp ranks its 512 consecutive keys of the
+//               tile 32 at a time (__match_any_sync groups the lanes that
+//               share a digit, the warp's own counters carry the ranks
+//               forward), one block-wide scan adds the other warps' counts,
+//               and the tile goes through shared memory in digit order, so a
+//               digit's keys leave as one contiguous run.
+// Bound by memory traffic (24 bytes per key and pass): the scatter before it
+// ranked a tile in 16 rounds with three block barriers each and wrote every
+// key straight to its place.
 #include "lg_device.cuh"
 #include "lg_sort.cuh"
 
@@ -49,44 +54,88 @@ rs_hist(const unsigned long long* k, uint64_t n, int shift, uint32_t* counts,
 	counts[(uint64_t)threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
 }
 
+// Shared memory of rs_scatter: the tile in digit order (keys, then payloads).
+constexpr size_t rs_smem(bool pay) { return kRsTile * (pay ? 12 : 8); }
+
+template <bool kPay>
 __global__ void __launch_bounds__(kRsThreads)
 rs_scatter(const unsigned long long* k, const uint32_t* pin, uint64_t n, int shift,
 		const uint32_t* offsets, uint32_t tiles, unsigned long long* kout,
 		uint32_t* pout) {
-	__shared__ uint32_t base[256];
-	__shared__ uint32_t run[256];
-	__shared__ uint32_t wcnt[kRsWarps][256];
-	const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-	base[threadIdx.x] = offsets[(uint64_t)threadIdx.x * tiles + blockIdx.x];
-	run[threadIdx.x] = 0;
-	for (int x = 0; x < kRsWarps; x++) wcnt[x][threadIdx.x] = 0;
-	__syncthreads();
+	extern __shared__ unsigned long long skey[];
+	uint32_t* spay = reinterpret_cast<uint32_t*>(skey + kRsTile);
+	__shared__ uint32_t wcnt[kRsWarps][256];   // per warp: keys of a digit so far
+	__shared__ uint32_t dbase[256];            // digit -> output base - tile position
+	__shared__ uint32_t wsum[kRsWarps];
+	const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
 	const uint64_t tile0 = (uint64_t)blockIdx.x * kRsTile;
+	const uint64_t first = tile0 + w * (32u * kRsItems) + lane;
+	unsigned long long key[kRsItems];
+#pragma unroll
 	for (int r = 0; r < kRsItems; r++) {
-		const uint64_t i = tile0 + (uint64_t)r * kRsThreads + threadIdx.x;
-		const bool valid = i < n;
-		unsigned long long key = valid ? k[i] : 0;
-		uint32_t pay = (valid && pin) ? pin[i] : 0;
-		// invalid lanes take digit 256, which matches no real digit
-		const uint32_t dig = valid ? (uint32_t)((key >> shift) & 0xff) : 256u;
+		const uint64_t i = first + (uint64_t)r * 32u;
+		key[r] = i < n ? k[i] : 0ull;
+	}
+#pragma unroll
+	for (int x = 0; x < kRsWarps; x++) wcnt[x][tid] = 0;
+	const uint32_t goff = offsets[(uint64_t)tid * tiles + blockIdx.x];
+	__syncthreads();
+	uint32_t rank[kRsItems];
+	const uint32_t below = (1u << lane) - 1u;
+#pragma unroll
+	for (int r = 0; r < kRsItems; r++) {
+		const bool valid = first + (uint64_t)r * 32u < n;
+		// lanes past the end take digit 256, which matches no real digit
+		const uint32_t dig = valid ? (uint32_t)((key[r] >> shift) & 0xff) : 256u;
 		const unsigned peers = __match_any_sync(0xffffffffu, dig);
-		const uint32_t wrank = __popc(peers & ((1u << lane) - 1u));
-		if (valid && (32 - __clz(peers)) - 1 == (int)lane) wcnt[w][dig] = __popc(peers);
-		__syncthreads();
-		if (valid) {
-			uint32_t before = run[dig];
-			for (uint32_t x = 0; x < w; x++) before += wcnt[x][dig];
-			const uint32_t pos = base[dig] + before + wrank;
-			kout[pos] = key;
-			if (pout) pout[pos] = pay;
+		const uint32_t before = valid ? wcnt[w][dig] : 0u;
+		__syncwarp();
+		rank[r] = before + __popc(peers & below);
+		if (valid && 31 - __clz(peers) == (int)lane) wcnt[w][dig] = before + __popc(peers);
+		__syncwarp();
+	}
+	__syncthreads();
+	// thread d: digit d's keys per warp -> exclusive over the warps, then the
+	// digits' starts within the tile
+	{
+		uint32_t run = 0;
+#pragma unroll
+		for (int x = 0; x < kRsWarps; x++) {
+			const uint32_t c = wcnt[x][tid];
+			wcnt[x][tid] = run;
+			run += c;
 		}
-		__syncthreads();
-		{
-			uint32_t t = 0;
-			for (int x = 0; x < kRsWarps; x++) { t += wcnt[x][threadIdx.x]; wcnt[x][threadIdx.x] = 0; }
-			run[threadIdx.x] += t;
+		uint32_t inc = run;
+#pragma unroll
+		for (int o = 1; o < 32; o <<= 1) {
+			const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+			if (lane >= (uint32_t)o) inc += y;
 		}
+		if (lane == 31u) wsum[w] = inc;
 		__syncthreads();
+		uint32_t start = inc - run;
+		for (uint32_t x = 0; x < w; x++) start += wsum[x];
+#pragma unroll
+		for (int x = 0; x < kRsWarps; x++) wcnt[x][tid] += start;
+		dbase[tid] = goff - start;
+	}
+	__syncthreads();
+#pragma unroll
+	for (int r = 0; r < kRsItems; r++) {
+		const uint64_t i = first + (uint64_t)r * 32u;
+		if (i < n) {
+			const uint32_t pos = wcnt[w][(key[r] >> shift) & 0xff] + rank[r];
+			skey[pos] = key[r];
+			if (kPay) spay[pos] = pin[i];
+		}
+	}
+	__syncthreads();
+	const uint32_t m = (uint32_t)(n - tile0 < kRsTile ? n - tile0 : kRsTile);
+	for (uint32_t j = tid; j < m; j += kRsThreads) {
+		const unsigned long long x = skey[j];
+		const uint32_t p = dbase[(x >> shift) & 0xff] + j;
+		kout[p] = x;
+		if (kPay) pout[p] = spay[j];
 	}
 }
 
@@ -103,7 +152,7 @@ __global__ void compact_first(const unsigned long long* k, uint64_t n,
 
 lg_status radix_sort_u64(lg_store* s, unsigned long long* keys, uint32_t* payload,
 		uint64_t n, DevBuf& tmp_keys, DevBuf& tmp_pay, DevBuf& counts, DevBuf& scan_tmp,
-		unsigned long long** sorted_keys, uint32_t** sorted_pay) {
+		unsigned long long** sorted_keys, uint32_t** sorted_pay, unsigned long long vary) {
 	cudaStream_t st = s->stream;
 	*sorted_keys = keys;
 	if (sorted_pay) *sorted_pay = payload;
@@ -115,16 +164,22 @@ lg_status radix_sort_u64(lg_store* s, unsigned long long* keys, uint32_t* payloa
 	LG_TRY(counts.reserve(((uint64_t)256 * tiles + 1) * 8 + 16));
 	uint32_t* cnt = counts.as<uint32_t>();
 	uint32_t* off = cnt + (uint64_t)256 * tiles + 1;
-	// which bits vary
-	unsigned long long oa[2] = {0, ~0ull};
-	unsigned long long* d_oa = (unsigned long long*)(counts.as<char>()
-			+ ((uint64_t)256 * tiles + 1) * 8);
-	LG_CUDA(cudaMemcpyAsync(d_oa, oa, 16, cudaMemcpyHostToDevice, st), "h2d");
-	rs_bits<<<592, 256, 0, st>>>(keys, n, d_oa);
-	LG_CUDA(cudaMemcpyAsync(oa, d_oa, 16, cudaMemcpyDeviceToHost, st), "d2h");
-	LG_CUDA(cudaStreamSynchronize(st), "sort bits");
-	s->launches++;
-	const unsigned long long vary = oa[0] ^ oa[1];
+	if (vary == 0) {
+		// which bits vary
+		unsigned long long oa[2] = {0, ~0ull};
+		unsigned long long* d_oa = (unsigned long long*)(counts.as<char>()
+				+ ((uint64_t)256 * tiles + 1) * 8);
+		LG_CUDA(cudaMemcpyAsync(d_oa, oa, 16, cudaMemcpyHostToDevice, st), "h2d");
+		rs_bits<<<592, 256, 0, st>>>(keys, n, d_oa);
+		LG_CUDA(cudaMemcpyAsync(oa, d_oa, 16, cudaMemcpyDeviceToHost, st), "d2h");
+		LG_CUDA(cudaStreamSynchronize(st), "sort bits");
+		s->launches++;
+		vary = oa[0] ^ oa[1];
+	}
+	const size_t smem = rs_smem(payload != nullptr);
+	if (payload)
+		LG_CUDA(cudaFuncSetAttribute(rs_scatter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+				(int)smem), "rs_scatter");
 	unsigned long long* src = keys;
 	unsigned long long* dst = tmp_keys.as<unsigned long long>();
 	uint32_t* psrc = payload;
@@ -133,7 +188,12 @@ lg_status radix_sort_u64(lg_store* s, unsigned long long* keys, uint32_t* payloa
 		if (((vary >> shift) & 0xff) == 0) continue;
 		rs_hist<<<tiles, kRsThreads, 0, st>>>(src, n, shift, cnt, tiles);
 		LG_TRY(exclusive_scan_u32(cnt, off, (uint64_t)256 * tiles, scan_tmp, st, nullptr));
-		rs_scatter<<<tiles, kRsThreads, 0, st>>>(src, psrc, n, shift, off, tiles, dst, pdst);
+		if (payload)
+			rs_scatter<true><<<tiles, kRsThreads, smem, st>>>(src, psrc, n, shift, off, tiles, dst,
+					pdst);
+		else
+			rs_scatter<false><<<tiles, kRsThreads, smem, st>>>(src, nullptr, n, shift, off, tiles,
+					dst, nullptr);
 		LG_CUDA(cudaGetLastError(), "radix sort pass");
 		s->launches += 5;
 		std::swap(src, dst);
