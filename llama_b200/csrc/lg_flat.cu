@@ -188,7 +188,7 @@ SlotSpace slot_space(const lg_snapshot* sn, int dir) {
 	return sp;
 }
 
-lg_status build_flat(lg_snapshot* sn, int dir, FlatCsr& f, bool view) {
+lg_status build_flat(lg_snapshot* sn, int dir, FlatCsr& f, bool view, bool weights) {
 	lg_store* s = sn->store;
 	cudaStream_t st = s->stream;
 	const SlotSpace sp = slot_space(sn, dir);
@@ -197,7 +197,7 @@ lg_status build_flat(lg_snapshot* sn, int dir, FlatCsr& f, bool view) {
 	const DevCsr& csr = dir == 0 ? s->out : s->in;
 	// edge weights are read only along out-edges (SSSP), so only the out
 	// direction carries them into the flat CSR
-	bool weighted = dir == 0;
+	bool weighted = dir == 0 && weights;
 	for (int l = sn->min_level; l <= sn->level && weighted; l++)
 		if (csr.levels[l]->n_fragment_slots > 0 && !csr.levels[l]->w.p) weighted = false;
 

@@ -192,9 +192,10 @@ struct FlatCsr {
 };
 
 // Builds f from direction dir of sn on the store's stream, with the edge
-// weights when every level that holds fragment slots has them, and the
-// fragment view when `view`.  f's buffers are reused (grown) across builds.
-lg_status build_flat(lg_snapshot* sn, int dir, FlatCsr& f, bool view);
+// weights when `weights` and every level that holds fragment slots has them,
+// and the fragment view when `view`.  f's buffers are reused (grown) across
+// builds.
+lg_status build_flat(lg_snapshot* sn, int dir, FlatCsr& f, bool view, bool weights = true);
 
 } // namespace lg
 

@@ -139,17 +139,6 @@ rs_scatter(const unsigned long long* k, const uint32_t* pin, uint64_t n, int shi
 	}
 }
 
-__global__ void mark_first(const unsigned long long* k, uint64_t n, uint32_t* flag) {
-	uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i < n) flag[i] = (i == 0 || k[i] != k[i - 1]) ? 1u : 0u;
-}
-
-__global__ void compact_first(const unsigned long long* k, uint64_t n,
-		const uint32_t* flag, const uint32_t* pos, unsigned long long* out) {
-	uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i < n && flag[i]) out[pos[i]] = k[i];
-}
-
 lg_status radix_sort_u64(lg_store* s, unsigned long long* keys, uint32_t* payload,
 		uint64_t n, DevBuf& tmp_keys, DevBuf& tmp_pay, DevBuf& counts, DevBuf& scan_tmp,
 		unsigned long long** sorted_keys, uint32_t** sorted_pay, unsigned long long vary) {
@@ -201,23 +190,6 @@ lg_status radix_sort_u64(lg_store* s, unsigned long long* keys, uint32_t* payloa
 	}
 	*sorted_keys = src;
 	if (sorted_pay) *sorted_pay = psrc;
-	return LG_OK;
-}
-
-lg_status unique_u64(lg_store* s, const unsigned long long* keys, uint64_t n,
-		unsigned long long* out, DevBuf& flags, DevBuf& scan_tmp, uint64_t* n_out) {
-	cudaStream_t st = s->stream;
-	if (n == 0) { *n_out = 0; return LG_OK; }
-	LG_TRY(flags.reserve((2 * n + 1) * 4));
-	uint32_t* fl = flags.as<uint32_t>();
-	uint32_t* pos = fl + n;
-	mark_first<<<grid_for(n, 256), 256, 0, st>>>(keys, n, fl);
-	uint64_t total = 0;
-	LG_TRY(exclusive_scan_u32(fl, pos, n, scan_tmp, st, &total));
-	compact_first<<<grid_for(n, 256), 256, 0, st>>>(keys, n, fl, pos, out);
-	LG_CUDA(cudaGetLastError(), "unique");
-	s->launches += 5;
-	*n_out = total;
 	return LG_OK;
 }
 

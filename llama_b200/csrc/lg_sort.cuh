@@ -15,11 +15,6 @@ lg_status radix_sort_u64(lg_store* s, unsigned long long* keys, uint32_t* payloa
 		uint64_t n, DevBuf& tmp_keys, DevBuf& tmp_pay, DevBuf& counts, DevBuf& scan_tmp,
 		unsigned long long** sorted_keys, uint32_t** sorted_pay, unsigned long long vary = 0);
 
-// Copy the first of every run of equal keys (sorted input) to `out`; the
-// number kept is returned in *n_out (this synchronises the stream).
-lg_status unique_u64(lg_store* s, const unsigned long long* keys, uint64_t n,
-		unsigned long long* out, DevBuf& flags, DevBuf& scan_tmp, uint64_t* n_out);
-
 } // namespace lg
 
 #endif // LG_SORT_CUH_

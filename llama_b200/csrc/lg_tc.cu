@@ -6,150 +6,418 @@
 // all three undirected edges present, each once.  The reference requires a
 // single level with sorted adjacency (triangle_counting.h:422-425); here the
 // multiversion snapshot is flattened on the device:
-//   1. every live arc u->v (u != v) becomes the undirected edge oriented from
-//      the lower to the higher rank, rank = (out+in degree, id), a total order
-//      that keeps the forward lists of hubs short;
-//   2. the keys (a << 32 | b) are radix sorted and de-duplicated, giving the
-//      forward lists N+(a) sorted by id;
-//   3. every oriented edge (a, b) counts |N+(a) & N+(b)|: each triangle is
-//      seen exactly once, at the edge between its two lowest-ranked vertices.
-//      Short lists are intersected by one lane, long ones by the warp, both
-//      with a binary search per element of the shorter list (merging 32
-//      chunks of similar-length lists was measured slower at R-MAT scale 24:
-//      890 ms against 552 ms for the whole call).
-// The count is an exact integer sum (atomicAdd of per-warp partials).
-#include "lg_expand.cuh"
+//   1. every vertex gets a label, 0 for the highest degree (out + in), equal
+//      degree classes in any order (a class: 1/64 of an octave);
+//   2. every live arc u->v (u != v) becomes the undirected edge oriented from
+//      the larger to the smaller label, a total order that keeps the forward
+//      lists of hubs short and makes their labels small;
+//   3. the keys (a << bits | b) are radix sorted and de-duplicated, giving
+//      the forward lists N+(a), sorted by label;
+//   4. every triangle c < b < a is found at its largest label a: for b in
+//      N+(a), |N+(b) & N+(a)|.  A CTA (or a single warp) holds N+(a) as a
+//      bitmap over the labels below a in shared memory and streams the lists
+//      N+(b) against it.
+//
+// What bounds step 4: one shared-memory probe per streamed id.  The form
+// before it took a binary search per element of the shorter list (log2 of
+// the longer list's uncoalesced loads each): at 700 k vertices and 9.1 M
+// undirected edges 7.3 G search steps, against 1.9 G coalesced ids streamed
+// here.  Because labels follow the degrees, a vertex whose list is long has a
+// small label, so its bitmap is short: 64 Ki labels (8 KB, one warp's own)
+// hold nearly all of the work of that graph.
+// The count is an exact integer sum (atomicAdd of per-warp partials), so the
+// order inside a degree class does not matter.
+#include "lg_flat.cuh"
+#include "lg_queue.cuh"
 #include "lg_sort.cuh"
+
+#include <algorithm>
 
 namespace lg {
 
+typedef unsigned long long u64;
+
+// ---------------------------------------------------------------------------
+// Labels: a counting sort of the vertices by degree class, descending.
+// ---------------------------------------------------------------------------
+
 constexpr int kTcThreads = 256;
+constexpr uint32_t kTcBins = 33u * 64u;     // classes: exponent and 6 mantissa bits
+constexpr uint32_t kTcLabelChunk = 4096;    // vertices per CTA
 
-__device__ __forceinline__ bool rank_less(uint32_t x, uint32_t y, const uint32_t* rk) {
-	uint32_t dx = __ldg(rk + x), dy = __ldg(rk + y);
-	return dx < dy || (dx == dy && x < y);
+__device__ __forceinline__ uint32_t tc_bin(uint32_t deg) {
+	// the float's exponent and top mantissa bits grow with the degree
+	return deg ? (__float_as_uint((float)deg) >> 17) - (127u << 6) : 0u;
 }
 
-__global__ void tc_rank(const uint32_t* out_deg, const uint32_t* in_deg, uint64_t V,
-		uint32_t* rk) {
-	uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (v < V) rk[v] = out_deg[v] + (in_deg ? in_deg[v] : 0u);
+__device__ __forceinline__ uint32_t tc_degree(const uint32_t* out_deg, const uint32_t* in_deg,
+		uint64_t v) {
+	return __ldg(out_deg + v) + (in_deg ? __ldg(in_deg + v) : 0u);
 }
 
-// Every live arc of the out-CSR, over balanced 1024-slot ranges of all
-// vertices' slots (pos = the snapshot's slot prefix), becomes an oriented key;
-// each warp stages its keys in shared memory and appends kTcStage at a time
-// (one counter atomic per batch, not per 32 slots).
-constexpr uint32_t kTcRange = 1024;
-constexpr uint32_t kTcStage = 256;
 __global__ void __launch_bounds__(kTcThreads)
-tc_emit(SnapCsr out, const uint32_t* pos, uint32_t total, const uint32_t* rk,
-		unsigned long long* keys, unsigned long long* n_keys) {
-	__shared__ unsigned long long stage[kTcThreads / 32][kTcStage];
-	unsigned long long* sb = stage[threadIdx.x >> 5];
-	uint32_t ns = 0;                       // staged keys of this warp (warp-uniform)
-	const uint32_t lane = threadIdx.x & 31u;
-	const uint32_t nranges = (total + kTcRange - 1) / kTcRange;
-	const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-	const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-	for (uint32_t r = warp; r < nranges; r += nwarps)
-	range_for_each(out, nullptr, pos, (uint32_t)out.V, total, nranges, kTcRange, r,
-		[&](bool act, uint32_t, uint32_t src, uint32_t nbr, uint32_t, uint32_t) {
-			const bool take = act && nbr != src;
-			unsigned long long key = 0;
-			if (take) {
-				uint32_t a = src, b = nbr;
-				if (rank_less(b, a, rk)) { a = nbr; b = src; }
-				key = ((unsigned long long)a << 32) | b;
-			}
-			const unsigned m = __ballot_sync(0xffffffffu, take);
-			if (m) {
-				if (ns + (uint32_t)__popc(m) > kTcStage) {
-					__syncwarp();
-					unsigned long long base = 0;
-					if (lane == 0) base = atomicAdd(n_keys, (unsigned long long)ns);
-					base = __shfl_sync(0xffffffffu, base, 0);
-					for (uint32_t i = lane; i < ns; i += 32) keys[base + i] = sb[i];
-					__syncwarp();
-					ns = 0;
-				}
-				if (take) sb[ns + __popc(m & ((1u << lane) - 1u))] = key;
-				ns += __popc(m);
-			}
-		});
-	if (ns) {
-		__syncwarp();
-		unsigned long long base = 0;
-		if (lane == 0) base = atomicAdd(n_keys, (unsigned long long)ns);
-		base = __shfl_sync(0xffffffffu, base, 0);
-		for (uint32_t i = lane; i < ns; i += 32) keys[base + i] = sb[i];
+tc_bins(const uint32_t* out_deg, const uint32_t* in_deg, uint64_t V, uint32_t* hist) {
+	__shared__ uint32_t h[kTcBins];
+	for (uint32_t b = threadIdx.x; b < kTcBins; b += kTcThreads) h[b] = 0;
+	__syncthreads();
+	for (uint64_t v = (uint64_t)blockIdx.x * kTcThreads + threadIdx.x; v < V;
+			v += (uint64_t)gridDim.x * kTcThreads)
+		atomicAdd(h + tc_bin(tc_degree(out_deg, in_deg, v)), 1u);
+	__syncthreads();
+	for (uint32_t b = threadIdx.x; b < kTcBins; b += kTcThreads)
+		if (h[b]) atomicAdd(hist + b, h[b]);
+}
+
+// hist[b] <- number of vertices in the classes above b (one CTA).
+__global__ void __launch_bounds__(1024)
+tc_bin_starts(uint32_t* hist) {
+	__shared__ uint32_t wsum[32];
+	const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+	uint32_t carry = 0;
+	for (uint32_t b0 = 0; b0 < kTcBins; b0 += 1024) {
+		const uint32_t i = b0 + threadIdx.x;
+		const uint32_t b = kTcBins - 1u - i;         // highest class first
+		const uint32_t x = i < kTcBins ? hist[b] : 0u;
+		uint32_t inc = x;
+#pragma unroll
+		for (int o = 1; o < 32; o <<= 1) {
+			const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+			if (lane >= (uint32_t)o) inc += y;
+		}
+		if (lane == 31u) wsum[wid] = inc;
+		__syncthreads();
+		uint32_t before = carry, all = 0;
+		for (uint32_t w = 0; w < 32; w++) {
+			if (w < wid) before += wsum[w];
+			all += wsum[w];
+		}
+		if (i < kTcBins) hist[b] = before + inc - x;
+		carry += all;
+		__syncthreads();
 	}
 }
 
-// off[v] = first oriented edge whose source is >= v
-__global__ void tc_offsets(const unsigned long long* keys, uint64_t m, uint64_t V,
-		uint32_t* off) {
-	uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i > m) return;
-	uint64_t a = i < m ? (keys[i] >> 32) : V;
-	int64_t p = i > 0 ? (int64_t)(keys[i - 1] >> 32) : -1;
-	for (int64_t v = p + 1; v <= (int64_t)a && v <= (int64_t)V; v++) off[v] = (uint32_t)i;
+// label[v] from the class's next free place; a CTA takes the places of its
+// vertices with one atomic per class.
+__global__ void __launch_bounds__(kTcThreads)
+tc_labels(const uint32_t* out_deg, const uint32_t* in_deg, uint64_t V, uint32_t* cursor,
+		uint32_t* label) {
+	constexpr int kPer = kTcLabelChunk / kTcThreads;
+	__shared__ uint32_t cnt[kTcBins];
+	for (uint32_t b = threadIdx.x; b < kTcBins; b += kTcThreads) cnt[b] = 0;
+	__syncthreads();
+	uint32_t bin[kPer], at[kPer];
+#pragma unroll
+	for (int j = 0; j < kPer; j++) {
+		const uint64_t v = (uint64_t)blockIdx.x * kTcLabelChunk + j * kTcThreads + threadIdx.x;
+		bin[j] = kTcBins;
+		at[j] = 0;
+		if (v < V) {
+			bin[j] = tc_bin(tc_degree(out_deg, in_deg, v));
+			at[j] = atomicAdd(cnt + bin[j], 1u);
+		}
+	}
+	__syncthreads();
+	for (uint32_t b = threadIdx.x; b < kTcBins; b += kTcThreads)
+		if (cnt[b]) cnt[b] = atomicAdd(cursor + b, cnt[b]);
+	__syncthreads();
+#pragma unroll
+	for (int j = 0; j < kPer; j++) {
+		const uint64_t v = (uint64_t)blockIdx.x * kTcLabelChunk + j * kTcThreads + threadIdx.x;
+		if (v < V) label[v] = cnt[bin[j]] + at[j];
+	}
 }
 
-// adj[i] = target of oriented edge i (the low half of its key): the
-// forward lists as 4-byte ids, half the bytes of the keys.
-__global__ void tc_targets(const unsigned long long* keys, uint64_t m, uint32_t* adj) {
-	for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
-			i += (uint64_t)gridDim.x * blockDim.x)
-		adj[i] = (uint32_t)keys[i];
+// ---------------------------------------------------------------------------
+// Forward lists
+// ---------------------------------------------------------------------------
+
+// Key of every edge of the flat out-CSR, in edge order (lane j of the warp
+// owning tile t takes edges 256 t + 8 j .. + 7): a << bits | b with a > b the
+// labels of its ends.  Self-loops get the key V << bits, which sorts last,
+// and are counted in *loops.
+constexpr int kTcEmitWarps = 8;
+__global__ void __launch_bounds__(kTcEmitWarps * 32)
+tc_emit(const uint32_t* ids, const uint32_t* heads, const uint32_t* nz_rows,
+		const uint32_t* tile_seg, uint32_t E, uint32_t ntiles, const uint32_t* label, int bits,
+		u64 loop_key, u64* keys, u64* loops) {
+	const uint32_t lane = threadIdx.x & 31u;
+	const uint32_t t = blockIdx.x * kTcEmitWarps + (threadIdx.x >> 5);
+	if (t >= ntiles) return;
+	const uint32_t eb = t * kFlatTile + lane * kFlatPerLane;
+	const uint32_t hb = __ldg(reinterpret_cast<const unsigned char*>(heads)
+			+ (size_t)t * (kFlatTile / 8) + lane);
+	uint32_t id[kFlatPerLane];
+#pragma unroll
+	for (int i = 0; i < kFlatPerLane; i++) id[i] = kNoId;
+	if (eb + kFlatPerLane <= E) {
+		const uint4 x = __ldcs(reinterpret_cast<const uint4*>(ids + eb));
+		const uint4 y = __ldcs(reinterpret_cast<const uint4*>(ids + eb + 4));
+		id[0] = x.x; id[1] = x.y; id[2] = x.z; id[3] = x.w;
+		id[4] = y.x; id[5] = y.y; id[6] = y.z; id[7] = y.w;
+	} else {
+#pragma unroll
+		for (int i = 0; i < kFlatPerLane; i++)
+			if (eb + i < E) id[i] = __ldcs(ids + eb + i);
+	}
+	uint32_t ln[kFlatPerLane];
+#pragma unroll
+	for (int i = 0; i < kFlatPerLane; i++) ln[i] = id[i] != kNoId ? __ldg(label + id[i]) : 0u;
+	uint32_t before = __popc(hb);               // heads in the lanes to the left
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1) {
+		const uint32_t q = __shfl_up_sync(0xffffffffu, before, o);
+		if (lane >= (uint32_t)o) before += q;
+	}
+	before -= __popc(hb);
+	uint32_t row = __ldg(tile_seg + t) + before - 1u;   // of the lane's first edge, unless a head
+	uint32_t ls = 0;
+	if (eb < E && !(hb & 1u)) ls = __ldg(label + __ldg(nz_rows + row));
+	uint32_t nl = 0;
+	u64 k[kFlatPerLane];
+#pragma unroll
+	for (int i = 0; i < kFlatPerLane; i++) {
+		if ((hb >> i) & 1u) {
+			row++;
+			ls = __ldg(label + __ldg(nz_rows + row));
+		}
+		const bool loop = ls == ln[i];
+		nl += (id[i] != kNoId && loop) ? 1u : 0u;
+		k[i] = loop ? loop_key : ((u64)max(ls, ln[i]) << bits) | min(ls, ln[i]);
+	}
+	if (eb + kFlatPerLane <= E) {
+#pragma unroll
+		for (int i = 0; i < kFlatPerLane; i += 2)
+			*reinterpret_cast<ulonglong2*>(keys + eb + i) = make_ulonglong2(k[i], k[i + 1]);
+	} else {
+#pragma unroll
+		for (int i = 0; i < kFlatPerLane; i++)
+			if (eb + i < E) keys[eb + i] = k[i];
+	}
+	nl = __reduce_add_sync(0xffffffffu, nl);
+	if (lane == 0 && nl) atomicAdd(loops, (u64)nl);
 }
+
+// The distinct keys in two passes over tiles of kUqTile sorted keys: the
+// number of first occurrences per tile, then (after a scan of those) the
+// lists themselves.  Keys at or above `end` (the self-loops) are left out.
+constexpr int kUqPer = 8;
+constexpr uint32_t kUqTile = (uint32_t)kTcThreads * kUqPer;
+
+__global__ void __launch_bounds__(kTcThreads)
+tc_uniq_count(const u64* keys, uint64_t n, u64 end, uint32_t* tile_cnt) {
+	__shared__ uint32_t s_sum;
+	if (threadIdx.x == 0) s_sum = 0;
+	__syncthreads();
+	const uint64_t base = (uint64_t)blockIdx.x * kUqTile;
+	uint32_t c = 0;
+#pragma unroll
+	for (int j = 0; j < kUqPer; j++) {
+		const uint64_t i = base + (uint64_t)j * kTcThreads + threadIdx.x;
+		if (i < n) {
+			const u64 k = keys[i];
+			c += k < end && (i == 0 || keys[i - 1] != k);
+		}
+	}
+	c = __reduce_add_sync(0xffffffffu, c);
+	if ((threadIdx.x & 31u) == 0 && c) atomicAdd(&s_sum, c);
+	__syncthreads();
+	if (threadIdx.x == 0) tile_cnt[blockIdx.x] = s_sum;
+}
+
+// adj = the targets of the distinct keys; cnt[a] = length of N+(a) (formed as
+// end - start of a's run, each added where the run begins or ends).
+__global__ void __launch_bounds__(kTcThreads)
+tc_uniq_write(const u64* keys, uint64_t n, u64 end, int bits, const uint32_t* tile_pos,
+		uint32_t* adj, uint32_t* cnt) {
+	__shared__ uint32_t wsum[kTcThreads / 32];
+	const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+	const uint64_t base = (uint64_t)blockIdx.x * kUqTile;
+	const u64 low = (1ull << bits) - 1ull;
+	uint32_t run = __ldg(tile_pos + blockIdx.x);
+	for (int j = 0; j < kUqPer; j++) {
+		const uint64_t i = base + (uint64_t)j * kTcThreads + threadIdx.x;
+		u64 k = end, p = end;
+		if (i < n) {
+			k = keys[i];
+			if (i > 0) p = keys[i - 1];
+		}
+		const bool first = k < end && (i == 0 || p != k);
+		const unsigned m = __ballot_sync(0xffffffffu, first);
+		if (lane == 0) wsum[wid] = __popc(m);
+		__syncthreads();
+		uint32_t pos = run, all = 0;
+		for (uint32_t w = 0; w < kTcThreads / 32; w++) {
+			if (w < wid) pos += wsum[w];
+			all += wsum[w];
+		}
+		pos += __popc(m & ((1u << lane) - 1u));
+		if (first) adj[pos] = (uint32_t)(k & low);
+		if (i < n) {
+			// a run of equal a begins at key i (and the run before it ends)
+			const bool begin = k < end && (i == 0 || (p >> bits) != (k >> bits));
+			if (begin) atomicSub(cnt + (k >> bits), pos);
+			if (i > 0 && p < end && (begin || k >= end)) atomicAdd(cnt + (p >> bits), pos);
+			if (i == n - 1 && k < end) atomicAdd(cnt + (k >> bits), pos + (first ? 1u : 0u));
+		}
+		run += all;
+		__syncthreads();
+	}
+}
+
+// ---------------------------------------------------------------------------
+// Counting
+// ---------------------------------------------------------------------------
 
 __device__ __forceinline__ bool bsearch_u32(const uint32_t* base, uint32_t n, uint32_t x) {
 	uint32_t lo = 0, hi = n;
 	while (lo < hi) {
-		uint32_t mid = (lo + hi) >> 1;
-		uint32_t y = __ldg(base + mid);
+		const uint32_t mid = (lo + hi) >> 1;
+		const uint32_t y = __ldg(base + mid);
 		if (y < x) lo = mid + 1; else hi = mid;
 	}
 	return lo < n && __ldg(base + lo) == x;
 }
 
-constexpr uint32_t kTcSmall = 16;   // lists this short are intersected by one lane
+// Vertices by the length la of N+(a) and the label a:
+//   la <= kTcPairs         one thread looks up every pair of the list
+//   a < kTcDomain[c]       list c: bitmap of kTcDomain[c] labels
+//   else                   list 3: a warp looks up every pair
+// A pair (c, b) is looked up by a binary search of c in N+(b): up to eight
+// ids that is 28 searches at most, against eight lists of some 200 ids to
+// stream (the same holds for the first eight ids of a longer list, whose
+// pairs one warp looks up at once).
+constexpr uint32_t kTcPairs = 8;
+constexpr int kTcClasses = 3;
+constexpr uint32_t kTcDomain0 = 1u << 16;     //   8 KB per bitmap: one warp each
+constexpr uint32_t kTcDomain1 = 1u << 18;     //  32 KB: four warps
+constexpr uint32_t kTcDomain2 = 7u << 18;     // 224 KB: a CTA of 32 warps, one per SM
 
 __global__ void __launch_bounds__(kTcThreads)
-tc_count(const unsigned long long* keys, const uint32_t* adj, uint64_t m, const uint32_t* off,
-		unsigned long long* total) {
-	const uint32_t lane = threadIdx.x & 31u;
-	const uint64_t warp = (uint64_t)blockIdx.x * (kTcThreads / 32) + (threadIdx.x >> 5);
-	const uint64_t nwarps = (uint64_t)gridDim.x * (kTcThreads / 32);
-	unsigned long long c = 0;
-	for (uint64_t e0 = warp * 32; e0 < m; e0 += nwarps * 32) {
-		const uint64_t e = e0 + lane;
-		uint32_t sa = 0, la = 0, sb = 0, lb = 0;
-		if (e < m) {
-			const unsigned long long k = keys[e];
-			const uint32_t a = (uint32_t)(k >> 32), b = (uint32_t)k;
-			sa = __ldg(off + a); la = __ldg(off + a + 1) - sa;
-			sb = __ldg(off + b); lb = __ldg(off + b + 1) - sb;
-			if (la > lb) { uint32_t t = sa; sa = sb; sb = t; t = la; la = lb; lb = t; }
-		}
-		// (sa, la) is now the shorter list
-		const bool small = la <= kTcSmall;
-		if (e < m && small)
-			for (uint32_t j = 0; j < la; j++)
-				c += bsearch_u32(adj + sb, lb, __ldg(adj + sa + j));
-		unsigned big = __ballot_sync(0xffffffffu, e < m && !small);
-		while (big) {
-			const int src = __ffs(big) - 1;
-			big &= big - 1;
-			const uint32_t s0 = __shfl_sync(0xffffffffu, sa, src);
-			const uint32_t n0 = __shfl_sync(0xffffffffu, la, src);
-			const uint32_t s1 = __shfl_sync(0xffffffffu, sb, src);
-			const uint32_t n1 = __shfl_sync(0xffffffffu, lb, src);
-			for (uint32_t j = lane; j < n0; j += 32)
-				c += bsearch_u32(adj + s1, n1, __ldg(adj + s0 + j));
+tc_classify(uint32_t V, const uint32_t* off, const uint32_t* adj, uint32_t* lists, u64* ctr,
+		u64* total) {
+	const uint32_t a = blockIdx.x * kTcThreads + threadIdx.x;
+	uint32_t sa = 0, la = 0;
+	if (a < V) {
+		sa = __ldg(off + a);
+		la = __ldg(off + a + 1) - sa;
+	}
+	uint32_t c = 0;
+	if (la >= 2 && la <= kTcPairs) {
+		for (uint32_t j = 1; j < la; j++) {
+			const uint32_t b = __ldg(adj + sa + j);
+			const uint32_t sb = __ldg(off + b), lb = __ldg(off + b + 1) - sb;
+			if (lb == 0) continue;
+			for (uint32_t i = 0; i < j; i++) c += bsearch_u32(adj + sb, lb, __ldg(adj + sa + i));
 		}
 	}
+	c = __reduce_add_sync(0xffffffffu, c);
+	if ((threadIdx.x & 31u) == 0 && c) atomicAdd(total, (u64)c);
+	const bool big = la > kTcPairs;
+	// a CTA's labels lie in one class or two: push only where some may be
+	const uint64_t a0 = (uint64_t)blockIdx.x * kTcThreads, a1 = a0 + kTcThreads;
+	const uint32_t dom[kTcClasses + 2] = {0u, kTcDomain0, kTcDomain1, kTcDomain2, 0xffffffffu};
+#pragma unroll
+	for (int k = 0; k <= kTcClasses; k++) {
+		if (a1 <= dom[k] || a0 >= dom[k + 1]) continue;
+		__syncthreads();
+		block_push<kTcThreads>(big && a >= dom[k] && a < dom[k + 1], a, lists + (size_t)k * V,
+				ctr + k);
+	}
+}
+
+// A CTA of kWarps warps takes the vertices of its list one after the other
+// (from a ticket counter), marks N+(a) in the bitmap and streams N+(b) of
+// every b but the first eight, a list per warp; 128 ids are loaded before any
+// is looked up.
+template <int kWarps>
+__global__ void __launch_bounds__(kWarps * 32)
+tc_bitmap(const uint32_t* list, const u64* n_list, u64* ticket, const uint32_t* off,
+		const uint32_t* adj, uint32_t words, u64* total) {
+	extern __shared__ uint32_t bm[];
+	__shared__ uint32_t s_next;
+	constexpr uint32_t kBatch = kWarps == 1 ? 32u : 8u;   // lists a warp takes at a time
+	constexpr int kAhead = 4;
+	const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5;
+	const uint32_t n = (uint32_t)__ldg(n_list);
+	if (n == 0) return;
+	for (uint32_t w = tid; w < words; w += kWarps * 32) bm[w] = 0;
+	u64 sum = 0;
+	for (;;) {
+		if (tid == 0) s_next = (uint32_t)atomicAdd(ticket, 1ull);
+		__syncthreads();
+		const uint32_t t = s_next;
+		if (t >= n) break;
+		const uint32_t a = __ldg(list + t);
+		const uint32_t sa = __ldg(off + a), la = __ldg(off + a + 1) - sa;
+		for (uint32_t i = tid; i < la; i += kWarps * 32) {
+			const uint32_t x = __ldg(adj + sa + i);
+			atomicOr(bm + (x >> 5), 1u << (x & 31u));
+		}
+		__syncthreads();
+		uint32_t c = 0;
+		if (wid == kWarps - 1 && lane < kTcPairs * (kTcPairs - 1) / 2) {
+			// lane = pair (i, j), i < j, of the first eight
+			uint32_t j = 1, i = lane;
+			while (i >= j) { i -= j; j++; }
+			const uint32_t b = __ldg(adj + sa + j), x = __ldg(adj + sa + i);
+			const uint32_t sb = __ldg(off + b), lb = __ldg(off + b + 1) - sb;
+			c += bsearch_u32(adj + sb, lb, x);
+		}
+		for (uint32_t j0 = kTcPairs + wid * kBatch; j0 < la; j0 += kWarps * kBatch) {
+			const uint32_t nb = min(kBatch, la - j0);
+			uint32_t s = 0, e = 0;
+			if (lane < nb) {
+				const uint32_t b = __ldg(adj + sa + j0 + lane);
+				s = __ldg(off + b);
+				e = __ldg(off + b + 1);
+			}
+			for (uint32_t q = 0; q < nb; q++) {
+				const uint32_t sb = __shfl_sync(0xffffffffu, s, q);
+				const uint32_t eb = __shfl_sync(0xffffffffu, e, q);
+				for (uint32_t p = sb; p < eb; p += 32u * kAhead) {
+					uint32_t x[kAhead];
+#pragma unroll
+					for (int u = 0; u < kAhead; u++) {
+						const uint32_t k = p + u * 32u + lane;
+						x[u] = k < eb ? __ldg(adj + k) : kNoId;
+					}
+#pragma unroll
+					for (int u = 0; u < kAhead; u++)
+						if (x[u] != kNoId) c += (bm[x[u] >> 5] >> (x[u] & 31u)) & 1u;
+				}
+			}
+		}
+		sum += c;
+		__syncthreads();
+		for (uint32_t i = tid; i < la; i += kWarps * 32) bm[__ldg(adj + sa + i) >> 5] = 0;
+	}
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+	if (lane == 0 && sum) atomicAdd(total, sum);
+}
+
+// The vertices whose label no bitmap holds: a warp each, the searches of one
+// b's pairs 32 at a time.
+__global__ void __launch_bounds__(kTcThreads)
+tc_search(const uint32_t* list, const u64* n_list, const uint32_t* off, const uint32_t* adj,
+		u64* total) {
+	const uint32_t lane = threadIdx.x & 31u;
+	const uint32_t nwarps = gridDim.x * (kTcThreads / 32);
+	const uint32_t n = (uint32_t)__ldg(n_list);
+	u64 c = 0;
+	for (uint32_t t = blockIdx.x * (kTcThreads / 32) + (threadIdx.x >> 5); t < n; t += nwarps) {
+		const uint32_t a = __ldg(list + t);
+		const uint32_t sa = __ldg(off + a), la = __ldg(off + a + 1) - sa;
+		for (uint32_t j = 1; j < la; j++) {
+			const uint32_t b = __ldg(adj + sa + j);
+			const uint32_t sb = __ldg(off + b), lb = __ldg(off + b + 1) - sb;
+			if (lb == 0) continue;
+			for (uint32_t i = lane; i < j; i += 32)
+				c += bsearch_u32(adj + sb, lb, __ldg(adj + sa + i));
+		}
+	}
+#pragma unroll
 	for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
 	if (lane == 0 && c) atomicAdd(total, c);
 }
@@ -158,6 +426,29 @@ tc_count(const unsigned long long* keys, const uint32_t* adj, uint64_t m, const 
 
 using namespace lg;
 
+namespace {
+
+// One bitmap class: kWarps warps per CTA, as many CTAs as are resident.
+template <int kWarps>
+lg_status launch_bitmap(lg_store* s, int sms, uint32_t domain, const uint32_t* list, u64* n_list,
+		u64* ticket, const uint32_t* off, const uint32_t* adj, u64* total) {
+	const uint32_t words = (domain + 31u) / 32u;
+	const size_t smem = (size_t)words * 4;
+	LG_CUDA(cudaFuncSetAttribute(tc_bitmap<kWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+			(int)smem), "tc_bitmap");
+	int per_sm = 0;
+	LG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tc_bitmap<kWarps>, kWarps * 32,
+			smem), "tc_bitmap");
+	if (per_sm < 1) return set_error(LG_ECUDA, "tc_bitmap does not fit an SM");
+	tc_bitmap<kWarps><<<(unsigned)(sms * per_sm), kWarps * 32, smem, s->stream>>>(list, n_list,
+			ticket, off, adj, words, total);
+	LG_CUDA(cudaGetLastError(), "tc_bitmap");
+	s->launches++;
+	return LG_OK;
+}
+
+} // namespace
+
 extern "C" lg_status lg_triangle_count(lg_snapshot* sn, lg_tc_result* result) {
 	clear_error();
 	if (!sn || !result) return set_error(LG_EINVAL, "null argument");
@@ -165,51 +456,93 @@ extern "C" lg_status lg_triangle_count(lg_snapshot* sn, lg_tc_result* result) {
 	LG_CUDA(cudaSetDevice(s->device), "cudaSetDevice");
 	cudaStream_t st = s->stream;
 	const uint64_t V = sn->V;
-	const uint64_t E = sn->out.n_edges;
-	if (E >= 0xffffffffull) return set_error(LG_ENOTSUP, "more than 2^32-1 live edges");
-	DevBuf rank(s->pool), keys(s->pool), tmpk(s->pool), tmpp(s->pool), counts(s->pool),
-			scan_tmp(s->pool), uniq(s->pool), flags(s->pool), off(s->pool), ctr(s->pool),
-			adj(s->pool);
-	LG_TRY(rank.reserve(V * 4));
-	LG_TRY(keys.reserve(std::max<uint64_t>(E, 1) * 8));
-	LG_TRY(ctr.reserve(2 * sizeof(unsigned long long)));
-	LG_CUDA(cudaMemsetAsync(ctr.p, 0, 2 * sizeof(unsigned long long), st), "memset");
-	tc_rank<<<grid_for(V, 256), 256, 0, st>>>(sn->out.deg.as<uint32_t>(),
-			sn->in.present ? sn->in.deg.as<uint32_t>() : nullptr, V, rank.as<uint32_t>());
-	const SnapCsr out = sn->view(0);
+	if (sn->out.n_edges >= 0xffffffffull)
+		return set_error(LG_ENOTSUP, "more than 2^32-1 live edges");
+	result->triangles = 0;
+	result->undirected_edges = 0;
+	result->arcs = 0;
+	// the live arcs: the snapshot's flat out-CSR, or one built for the call
+	const FlatCsr* f = sn->flat[0];
+	if (!f) {
+		if (!s->flat_scratch) s->flat_scratch = new FlatCsr;
+		LG_TRY(build_flat(sn, 0, *s->flat_scratch, false, false));
+		f = s->flat_scratch;
+	}
+	const uint64_t E = f->E;
+	if (E == 0) return LG_OK;
+	DevBuf label(s->pool), hist(s->pool), keys(s->pool), tmpk(s->pool), tmpp(s->pool),
+			counts(s->pool), scan_tmp(s->pool), tiles(s->pool), off(s->pool), ctr(s->pool),
+			adj(s->pool), lists(s->pool);
 	int sms = 148;
 	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
-	tc_emit<<<(unsigned)sms * 8u, kTcThreads, 0, st>>>(out, sn->out.slot_off.as<uint32_t>(),
-			(uint32_t)sn->out.n_frag_slots, rank.as<uint32_t>(), keys.as<unsigned long long>(),
-			ctr.as<unsigned long long>());
+	// ctr: [0..3] class sizes, [4..6] tickets, [7] self-loops, [8] triangles
+	LG_TRY(ctr.reserve(9 * sizeof(u64)));
+	u64* cd = ctr.as<u64>();
+	LG_CUDA(cudaMemsetAsync(cd, 0, 9 * sizeof(u64), st), "memset");
+	const uint32_t* odeg = sn->out.deg.as<uint32_t>();
+	const uint32_t* ideg = sn->in.present ? sn->in.deg.as<uint32_t>() : nullptr;
+	LG_TRY(label.reserve(V * 4));
+	LG_TRY(hist.reserve(kTcBins * 4));
+	LG_CUDA(cudaMemsetAsync(hist.p, 0, kTcBins * 4, st), "memset");
+	tc_bins<<<std::min(grid_for(V, kTcLabelChunk), (unsigned)sms * 4u), kTcThreads, 0, st>>>(odeg,
+			ideg, V, hist.as<uint32_t>());
+	tc_bin_starts<<<1, 1024, 0, st>>>(hist.as<uint32_t>());
+	tc_labels<<<grid_for(V, kTcLabelChunk), kTcThreads, 0, st>>>(odeg, ideg, V,
+			hist.as<uint32_t>(), label.as<uint32_t>());
+	// keys a << bits | b; V itself (the self-loops' a) fits the bits too
+	int bits = 1;
+	while ((V >> bits) != 0) bits++;
+	const u64 loop_key = (u64)V << bits;
+	LG_TRY(keys.reserve(E * 8));
+	tc_emit<<<grid_for(f->ntiles, kTcEmitWarps), kTcEmitWarps * 32, 0, st>>>(f->ids.as<uint32_t>(),
+			f->heads(), f->nz_rows(), f->tile_seg(), (uint32_t)E, f->ntiles, label.as<uint32_t>(),
+			bits, loop_key, keys.as<u64>(), cd + 7);
 	LG_CUDA(cudaGetLastError(), "tc_emit");
-	s->launches += 2;
-	unsigned long long nk = 0;
-	LG_CUDA(cudaMemcpyAsync(&nk, ctr.p, 8, cudaMemcpyDeviceToHost, st), "d2h");
-	LG_CUDA(cudaStreamSynchronize(st), "tc emit");
-	s->d2h_bytes += 8;
-	unsigned long long* sorted = nullptr;
-	LG_TRY(radix_sort_u64(s, keys.as<unsigned long long>(), nullptr, nk, tmpk, tmpp,
-			counts, scan_tmp, &sorted, nullptr));
-	LG_TRY(uniq.reserve(std::max<unsigned long long>(nk, 1) * 8));
+	s->launches += 4;
+	u64* sorted = nullptr;
+	LG_TRY(radix_sort_u64(s, keys.as<u64>(), nullptr, E, tmpk, tmpp, counts, scan_tmp, &sorted,
+			nullptr, bits < 32 ? (1ull << (2 * bits)) - 1ull : ~0ull));
+	const unsigned uq_tiles = grid_for(E, kUqTile);
+	LG_TRY(tiles.reserve((2ull * uq_tiles + 1) * 4));
+	uint32_t* tile_cnt = tiles.as<uint32_t>();
+	uint32_t* tile_pos = tile_cnt + uq_tiles;
+	tc_uniq_count<<<uq_tiles, kTcThreads, 0, st>>>(sorted, E, loop_key, tile_cnt);
+	LG_CUDA(cudaGetLastError(), "tc_uniq_count");
 	uint64_t m = 0;
-	LG_TRY(unique_u64(s, sorted, nk, uniq.as<unsigned long long>(), flags, scan_tmp, &m));
-	LG_TRY(off.reserve((V + 1) * 4));
-	tc_offsets<<<grid_for(m + 1, 256), 256, 0, st>>>(uniq.as<unsigned long long>(), m, V,
-			off.as<uint32_t>());
+	LG_TRY(exclusive_scan_u32(tile_cnt, tile_pos, uq_tiles, scan_tmp, st, &m));
 	LG_TRY(adj.reserve(std::max<uint64_t>(m, 1) * 4));
-	tc_targets<<<(unsigned)sms * 8u, 256, 0, st>>>(uniq.as<unsigned long long>(), m,
-			adj.as<uint32_t>());
-	tc_count<<<(unsigned)sms * 16u, kTcThreads, 0, st>>>(uniq.as<unsigned long long>(),
-			adj.as<uint32_t>(), m, off.as<uint32_t>(), ctr.as<unsigned long long>() + 1);
-	LG_CUDA(cudaGetLastError(), "tc_count");
-	s->launches += 3;
-	unsigned long long t = 0;
-	LG_CUDA(cudaMemcpyAsync(&t, ctr.as<unsigned long long>() + 1, 8, cudaMemcpyDeviceToHost, st), "d2h");
-	LG_CUDA(cudaStreamSynchronize(st), "tc");
-	s->d2h_bytes += 8;
-	result->triangles = (int64_t)t;
+	LG_TRY(off.reserve((2 * V + 1) * 4));
+	uint32_t* fcnt = off.as<uint32_t>();
+	uint32_t* foff = fcnt + V;
+	LG_CUDA(cudaMemsetAsync(fcnt, 0, V * 4, st), "memset");
+	tc_uniq_write<<<uq_tiles, kTcThreads, 0, st>>>(sorted, E, loop_key, bits, tile_pos,
+			adj.as<uint32_t>(), fcnt);
+	LG_CUDA(cudaGetLastError(), "tc_uniq_write");
+	LG_TRY(exclusive_scan_u32(fcnt, foff, V, scan_tmp, st, nullptr));
+	LG_TRY(lists.reserve((kTcClasses + 1) * V * 4));
+	uint32_t* ls = lists.as<uint32_t>();
+	const uint32_t* ad = adj.as<uint32_t>();
+	tc_classify<<<grid_for(V, kTcThreads), kTcThreads, 0, st>>>((uint32_t)V, foff, ad, ls, cd,
+			cd + 8);
+	LG_CUDA(cudaGetLastError(), "tc_classify");
+	s->launches += 9;
+	LG_TRY(launch_bitmap<1>(s, sms, (uint32_t)std::min<uint64_t>(V, kTcDomain0), ls, cd, cd + 4,
+			foff, ad, cd + 8));
+	if (V > kTcDomain0)
+		LG_TRY(launch_bitmap<4>(s, sms, (uint32_t)std::min<uint64_t>(V, kTcDomain1), ls + V, cd + 1,
+				cd + 5, foff, ad, cd + 8));
+	if (V > kTcDomain1)
+		LG_TRY(launch_bitmap<32>(s, sms, (uint32_t)std::min<uint64_t>(V, kTcDomain2), ls + 2 * V,
+				cd + 2, cd + 6, foff, ad, cd + 8));
+	if (V > kTcDomain2) {
+		tc_search<<<(unsigned)sms * 8u, kTcThreads, 0, st>>>(ls + 3 * V, cd + 3, foff, ad, cd + 8);
+		LG_CUDA(cudaGetLastError(), "tc_search");
+		s->launches++;
+	}
+	u64 h[2] = {0, 0};
+	LG_TRY(read_words(s, cd + 7, 2, h));
+	result->triangles = (int64_t)h[1];
 	result->undirected_edges = m;
-	result->arcs = nk;
+	result->arcs = E - h[0];
 	return LG_OK;
 }
