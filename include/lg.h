@@ -496,11 +496,12 @@ lg_status lg_bc_batched(lg_snapshot* snap, const int64_t* sources, int n_sources
 		double* bc);
 
 /* Personalized PageRank for K single-vertex seeds, evaluated on n_snaps
- * snapshots of one store in a single CUDA-graph launch.  The reference has no
- * personalized variant: this is the pull iteration of pagerank_double
- * (benchmark/benchmarks/pagerank.h:120-169) with the uniform teleport
- * (1-d)/N replaced, per column k, by (1-d) on seed k; x0 = e_seed, fixed
- * iteration count, dangling mass dropped.  K is a multiple of 32, <= 256.
+ * snapshots of one store.  The reference has no personalized variant: this is
+ * the pull iteration of pagerank_double (benchmark/benchmarks/pagerank.h:
+ * 120-169) with the uniform teleport (1-d)/N replaced, per column k, by (1-d)
+ * on seed k; x0 = e_seed, fixed iteration count, dangling mass dropped.  Reads
+ * the snapshots' flat in-CSRs; one that is not flat is flattened for the call
+ * in scratch of the store (4 bytes per live edge and 24 per vertex).  K is a multiple of 32, <= 256.
  * out: double[n_snaps][max_nodes][K] (row-major, column k = seed k). */
 lg_status lg_ppr(lg_snapshot* const* snaps, int n_snaps, const int64_t* seeds,
 		int K, int iterations, double damping, double* out);
@@ -546,7 +547,8 @@ lg_status lg_adjoint_free(lg_adjoint* tape);
 /* Personalized PageRank: columns per pass (a multiple of 32; the K columns
  * run in passes of this many, each pass all iterations), default 256. */
 #define LG_TUNE_PPR_KTILE       1
-/* Personalized PageRank: in-CSR slots per warp range, default 2048. */
+/* Personalized PageRank: the most in-edges per warp range (rounded down to a
+ * multiple of 32; smaller graphs take fewer), default 2048. */
 #define LG_TUNE_PPR_RANGE       2
 /* Delta-stepping SSSP: queue slots per warp range, default 1024. */
 #define LG_TUNE_SSSP_RANGE      3
