@@ -298,13 +298,11 @@ extern "C" lg_status lg_bc(lg_snapshot* sn, const int64_t* sources, int n_source
 			LG_CUDA(cudaMemsetAsync(ctr, 0, 2 * sizeof(unsigned long long), st), "memset");
 			uint32_t* nxt = ord + off[k + 1];
 			if (top_down) {
-				list_slots<<<grid_for(n, 256), 256, 0, st>>>(out, ord + b, (uint32_t)n,
-						cnt.as<uint32_t>());
-				LG_TRY(exclusive_scan_u32(cnt.as<uint32_t>(), pos.as<uint32_t>(), n, scan_tmp,
-						st, nullptr));
+				LG_TRY(exclusive_scan_slots(out, ord + b, n, cnt.as<uint32_t>(),
+						pos.as<uint32_t>(), scan_tmp, st, nullptr));
 				bc_top_down<<<grid, kBcThreads, 0, st>>>(out, ord + b, pos.as<uint32_t>(),
 						(uint32_t)n, lv, sg, k, nxt, ctr, outdeg);
-				s->launches += 5;
+				s->launches += 1 + scan_launches(n);
 			} else {
 				bc_bottom_up<<<grid_for(V, kBcThreads), kBcThreads, 0, st>>>(
 						fi->off.as<uint32_t>(), fi->ids.as<uint32_t>(), (uint32_t)V, lv, sg, k,
@@ -327,14 +325,12 @@ extern "C" lg_status lg_bc(lg_snapshot* sn, const int64_t* sources, int n_source
 		const int D = (int)off.size() - 2;           // levels 0..D-1 are non-empty
 		for (int k = D - 2; k >= 1; k--) {
 			const uint64_t b = off[k], n = off[k + 1] - off[k];
-			list_slots<<<grid_for(n, 256), 256, 0, st>>>(out, ord + b, (uint32_t)n,
-					cnt.as<uint32_t>());
-			LG_TRY(exclusive_scan_u32(cnt.as<uint32_t>(), pos.as<uint32_t>(), n, scan_tmp, st,
-					nullptr));
+			LG_TRY(exclusive_scan_slots(out, ord + b, n, cnt.as<uint32_t>(),
+					pos.as<uint32_t>(), scan_tmp, st, nullptr));
 			bc_backward<<<grid, kBcThreads, 0, st>>>(out, ord + b, pos.as<uint32_t>(),
 					(uint32_t)n, lv, sg, dl, k);
 			bc_accumulate<<<grid_for(n, 256), 256, 0, st>>>(ord + b, (uint32_t)n, dl, acc);
-			s->launches += 6;
+			s->launches += 2 + scan_launches(n);
 			LG_CUDA(cudaGetLastError(), "bc_backward");
 		}
 	}

@@ -106,15 +106,6 @@ __device__ __forceinline__ void block_append(const bool (&take)[N], const uint32
 	}
 }
 
-// Fragment slots of every frontier entry (to be scanned into range offsets).
-__global__ void bfs_frontier_slots(SnapCsr out, const uint32_t* queue, uint32_t qlen,
-		uint32_t* cnt) {
-	const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= qlen) return;
-	uint32_t f0;
-	cnt[i] = vertex_slots(out, __ldg(queue + i), &f0);
-}
-
 // Top-down step over the frontier's slot space cut into ranges of at most
 // kBfsRange slots, one warp each (lg_expand.cuh).  ctr[0] = next frontier size,
 // ctr[1] = sum of out-degrees of the next frontier.
@@ -334,10 +325,8 @@ extern "C" lg_status lg_bfs(lg_snapshot* sn, int64_t root, int32_t* levels,
 		LG_CUDA(cudaMemsetAsync(ctr, 0, 2 * sizeof(unsigned long long), st), "memset");
 		if (top_down) {
 			// frontier slot offsets, then one warp per range
-			bfs_frontier_slots<<<grid_for(qlen, 256), 256, 0, st>>>(out, q,
-					(uint32_t)qlen, fcnt);
 			uint64_t total = 0;
-			LG_TRY(exclusive_scan_u32(fcnt, fpos, qlen, sc[7], st, &total));
+			LG_TRY(exclusive_scan_slots(out, q, qlen, fcnt, fpos, sc[7], st, &total));
 			s->d2h_bytes += 8;
 			// ranges of up to kBfsRange slots, shorter (down to 32) when the
 			// frontier is too small to give every resident warp one
@@ -349,7 +338,7 @@ extern "C" lg_status lg_bfs(lg_snapshot* sn, int64_t root, int32_t* levels,
 						out, q, fpos, (uint32_t)qlen, (uint32_t)total, (uint32_t)range, nranges,
 						lvl, nq, ctr, cur);
 			td_steps++;
-			s->launches += 5;
+			s->launches += scan_launches(qlen) + (nranges > 0);
 		} else {
 			LG_CUDA(cudaMemsetAsync(bits, 0, ((V + 31) / 32) * 4, st), "memset");
 			bfs_set_bits<<<grid_for(qlen, 256), 256, 0, st>>>(q, (uint32_t)qlen, bits);

@@ -213,8 +213,7 @@ bfs_levels(SnapCsr out, const uint32_t* nz_rows, const uint32_t* nz_off, uint32_
 #pragma unroll
 				for (int j = 0; j < kLvSmallPer; j++) {
 					const uint32_t i = tid * kLvSmallPer + j;
-					uint32_t f0;
-					kc[j] = i < n ? vertex_slots(out, __ldcg(q + i), &f0) : 0u;
+					kc[j] = i < n ? vertex_slots(out, __ldcg(q + i)) : 0u;
 					sum += kc[j];
 				}
 				if (block_sum<kLvWarps>(sum) >= (1ull << 32)) {
@@ -238,8 +237,7 @@ bfs_levels(SnapCsr out, const uint32_t* nz_rows, const uint32_t* nz_off, uint32_
 				const uint32_t c0 = min(n, blockIdx.x * chunk), c1 = min(n, c0 + chunk);
 				unsigned long long s = 0;
 				for (uint32_t i = c0 + tid; i < c1; i += blockDim.x) {
-					uint32_t f0;
-					const uint32_t k = vertex_slots(out, __ldcg(q + i), &f0);
+					const uint32_t k = vertex_slots(out, __ldcg(q + i));
 					fcnt[i] = k;
 					s += k;
 				}

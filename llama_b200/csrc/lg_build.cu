@@ -311,7 +311,7 @@ static lg_status build_dir(lg_store* s, const DevCsr& csr, int l, uint64_t V,
 				d->ids.as<uint32_t>(), w_in ? d->w.as<uint32_t>() : nullptr);
 	ce = cudaGetLastError();
 	if (ce != cudaSuccess) { delete d; return cuda_status(ce, "bl_place"); }
-	s->launches += 2 + (n > 0) + (nd > 0) + 3 + 1 + 3 + (n > 0);
+	s->launches += 2 + 2 * (n > 0) + (nd > 0) + 2 * scan_launches(V);
 	*out = d;
 	return LG_OK;
 }

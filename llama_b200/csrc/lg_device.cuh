@@ -50,6 +50,7 @@ struct SnapCsr {
 	const LevelTab* lt;         // device copy
 	const uint32_t* deg;        // V
 	uint64_t V;
+	const uint32_t* slot_off;   // V + 1 slot prefix of the vertices, or null
 };
 
 __device__ __forceinline__ uint32_t frag_len(uint2 f) { return f.y >> kLevelBits; }
@@ -62,12 +63,11 @@ __device__ __forceinline__ bool slot_deleted(const LevelTab* lt, uint32_t lv,
 }
 
 // Slots (live or deleted) of vertex v's fragments in this snapshot.
-__device__ __forceinline__ uint32_t vertex_slots(const SnapCsr& g, uint32_t v,
-		uint32_t* f0out) {
+__device__ __forceinline__ uint32_t vertex_slots(const SnapCsr& g, uint32_t v) {
+	if (g.slot_off) return __ldg(g.slot_off + v + 1) - __ldg(g.slot_off + v);
 	uint32_t f0 = __ldg(g.frag_off + v), f1 = __ldg(g.frag_off + v + 1);
 	uint32_t c = 0;
 	for (uint32_t f = f0; f < f1; f++) c += frag_len(g.frags[f]);
-	*f0out = f0;
 	return c;
 }
 
@@ -145,8 +145,9 @@ __device__ __forceinline__ double warp_segsum(double v, uint32_t key, bool* tail
 // (trim_pools).  stream becomes null when the store is destroyed; a buffer
 // that outlives its store is then freed with cudaFree.
 struct CallPool {
-	cudaMemPool_t pool = nullptr;
+	cudaMemPool_t pool = nullptr;      // made on first use
 	cudaStream_t stream = nullptr;
+	int device = 0;
 	CallPool() = default;
 	CallPool(const CallPool&) = delete;
 	CallPool& operator=(const CallPool&) = delete;
@@ -221,6 +222,7 @@ struct SnapDir {
 		s.lt = lt.as<LevelTab>();
 		s.deg = deg.as<uint32_t>();
 		s.V = 0;
+		s.slot_off = slot_off.as<uint32_t>();
 		return s;
 	}
 };
@@ -309,6 +311,18 @@ bool is_device_pointer(const void* p);
 // total does not fit 32 bits.  Runs on `stream`, uses `tmp` as scratch.
 lg_status exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint64_t n,
 		DevBuf& tmp, cudaStream_t stream, uint64_t* total);
+
+// The same for the slot counts of list[0 .. n) (all vertices in order when
+// list is null) in g, which are left in cnt[0 .. n).
+lg_status exclusive_scan_slots(const SnapCsr& g, const uint32_t* list, uint64_t n, uint32_t* cnt,
+		uint32_t* out, DevBuf& tmp, cudaStream_t stream, uint64_t* total);
+
+// Kernels a scan of n counts launches.
+constexpr uint64_t kScanTile = 8192;        // values per CTA
+constexpr uint64_t kScanOwnTiles = 4096;    // tiles whose CTAs add up the sums before theirs
+inline uint64_t scan_launches(uint64_t n) {
+	return n <= kScanTile ? 1 : n <= kScanTile * kScanOwnTiles ? 2 : 3;
+}
 
 // Copy `bytes` of device data to a caller buffer (host or device) on the
 // store's stream, counting host-bound bytes.

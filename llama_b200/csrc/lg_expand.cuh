@@ -185,16 +185,6 @@ __device__ __forceinline__ void range_for_each(const SnapCsr& g, const uint32_t*
 	(void)lane;
 }
 
-// Frontier bookkeeping shared by the list-driven kernels: per-entry slot
-// counts, to be scanned into the `pos` offsets range_for_each expects.
-static __global__ void list_slots(SnapCsr g, const uint32_t* list, uint32_t n,
-		uint32_t* cnt) {
-	const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= n) return;
-	uint32_t f0;
-	cnt[i] = vertex_slots(g, list ? __ldg(list + i) : (uint32_t)i, &f0);
-}
-
 } // namespace lg
 
 #endif // LG_EXPAND_CUH_

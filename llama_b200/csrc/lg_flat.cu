@@ -248,7 +248,7 @@ lg_status build_flat(lg_snapshot* sn, int dir, FlatCsr& f, bool view, bool weigh
 				const_cast<uint32_t*>(f.tile_seg()));
 		LG_CUDA(cudaGetLastError(), "flat_tiles");
 	}
-	s->launches += 3 + 1 + 1 + 3 + 1 + (f.ntiles > 0);
+	s->launches += 2 * scan_launches(V) + 3 + (f.ntiles > 0);
 	if (!view) return LG_OK;
 
 	LG_TRY(f.vfrags.reserve(f.rcap() * sizeof(uint2)));

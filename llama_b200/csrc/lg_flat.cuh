@@ -187,6 +187,7 @@ struct FlatCsr {
 		s.lt = vlt.as<LevelTab>();
 		s.deg = deg;
 		s.V = V;
+		s.slot_off = off.as<uint32_t>();
 		return s;
 	}
 };

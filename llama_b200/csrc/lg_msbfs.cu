@@ -747,8 +747,8 @@ extern "C" lg_status lg_bc_batched(lg_snapshot* sn, const int64_t* sources, int 
 			LG_CUDA(cudaMemsetAsync(lk1 + V, 0, V * sizeof(u64), st), "clear level masks");
 			uint32_t* q = queues.as<uint32_t>() + qb;
 			uint32_t* q2 = queues.as<uint32_t>() + qoff[k + 1];
-			list_slots<<<grid_for(qlen, B), B, 0, st>>>(out, q, (uint32_t)qlen, qcnt);
-			LG_TRY(exclusive_scan_u32(qcnt, qpos, qlen, sc[9], st, nullptr));
+			LG_TRY(exclusive_scan_slots(out, q, qlen, qcnt,
+					qpos, sc[9], st, nullptr));
 			if (top_down && has_in && (double)mf > (double)mu / alpha) top_down = false;
 			else if (!top_down && (double)qlen < (double)V / beta) top_down = true;
 			LG_CUDA(cudaMemsetAsync(ctr, 0, 4 * sizeof(unsigned long long), st), "memset");
@@ -761,7 +761,7 @@ extern "C" lg_status lg_bc_batched(lg_snapshot* sn, const int64_t* sources, int 
 					ms_commit<<<grid_for(nc, kMsThreads * kCommitPer), kMsThreads, 0, st>>>(cand,
 							(uint32_t)nc, k + 1, V, n, nxt,
 							seen, lk1, nullptr, outdeg, q2, ctr);
-				s->launches += 5 + (nc > 0);
+				s->launches += 1 + scan_launches(qlen) + (nc > 0);
 			} else {
 				if (fi) {
 					ms_bottom_up_flat<<<grid_for(V, kMsThreads * kMsVerts), kMsThreads, 0, st>>>(
@@ -776,7 +776,7 @@ extern "C" lg_status lg_bc_batched(lg_snapshot* sn, const int64_t* sources, int 
 				ms_commit<<<grid_for(V, kMsThreads * kCommitPer), kMsThreads, 0, st>>>(nullptr,
 						(uint32_t)V, k + 1, V, n, nxt,
 						seen, lk1, nullptr, outdeg, q2, ctr);
-				s->launches += 5;
+				s->launches += 2 + scan_launches(qlen);
 			}
 			if (!has_in) {
 				// push along the level's out-edges (one atomic per down pair)
@@ -788,12 +788,12 @@ extern "C" lg_status lg_bc_batched(lg_snapshot* sn, const int64_t* sources, int 
 			LG_TRY(read_words(s, ctr, 3, h));
 			if (has_in && h[0] > 0) {
 				// pull into the new level over its in-edges
-				list_slots<<<grid_for(h[0], B), B, 0, st>>>(in, q2, (uint32_t)h[0], qcnt);
-				LG_TRY(exclusive_scan_u32(qcnt, qpos, h[0], sc[9], st, nullptr));
+				LG_TRY(exclusive_scan_slots(in, q2, h[0], qcnt,
+						qpos, sc[9], st, nullptr));
 				bcm_sigma_pull<<<grid, kMsThreads, 0, st>>>(in, q2, qpos, (uint32_t)h[0], lk, lk1,
 						sigma);
 				LG_CUDA(cudaGetLastError(), "bc batched sigma");
-				s->launches += 5;
+				s->launches += 1 + scan_launches(h[0]);
 			}
 			qoff.push_back(qoff[k + 1] + h[0]);
 			mf = h[1];
@@ -807,11 +807,11 @@ extern "C" lg_status lg_bc_batched(lg_snapshot* sn, const int64_t* sources, int 
 			const u64* lk = masks.as<u64>() + (uint64_t)k * V;
 			const uint32_t* q = queues.as<uint32_t>() + qb;
 			if (k < D - 1) {                          // the deepest level has no down edges
-				list_slots<<<grid_for(qlen, B), B, 0, st>>>(out, q, (uint32_t)qlen, qcnt);
-				LG_TRY(exclusive_scan_u32(qcnt, qpos, qlen, sc[9], st, nullptr));
+				LG_TRY(exclusive_scan_slots(out, q, qlen, qcnt,
+						qpos, sc[9], st, nullptr));
 				bcm_delta<<<grid, kMsThreads, 0, st>>>(out, q, qpos, (uint32_t)qlen, lk, lk + V,
 						sigma, delta);
-				s->launches += 5;
+				s->launches += 1 + scan_launches(qlen);
 			}
 			if (k > 1) {                              // level k - 1 multiplies by these
 				bcm_quot<<<grid_for(qlen * 32, B), B, 0, st>>>(q, (uint32_t)qlen, lk, sigma, delta);
@@ -920,8 +920,8 @@ extern "C" lg_status lg_bfs_multi(lg_snapshot* sn, const int64_t* roots, int n_r
 			else if (!top_down && (double)qlen < (double)V / beta) top_down = true;
 			LG_CUDA(cudaMemsetAsync(ctr, 0, 4 * sizeof(unsigned long long), st), "memset");
 			if (top_down) {
-				list_slots<<<grid_for(qlen, B), B, 0, st>>>(out, q, (uint32_t)qlen, qcnt);
-				LG_TRY(exclusive_scan_u32(qcnt, qpos, qlen, sc[8], st, nullptr));
+				LG_TRY(exclusive_scan_slots(out, q, qlen, qcnt,
+						qpos, sc[8], st, nullptr));
 				ms_top_down<<<td_blocks, kMsThreads, 0, st>>>(out, q, qpos, (uint32_t)qlen, cur,
 						seen, nxt, cand, ctr + 3);
 				unsigned long long nc = 0;
@@ -931,7 +931,7 @@ extern "C" lg_status lg_bfs_multi(lg_snapshot* sn, const int64_t* roots, int n_r
 							(uint32_t)nc, depth + 1, V, n, nxt,
 							seen, cur2, plv, outdeg, q2, ctr);
 				td++;
-				s->launches += 5 + (nc > 0);
+				s->launches += 1 + scan_launches(qlen) + (nc > 0);
 			} else {
 				if (fi) {
 					ms_bottom_up_flat<<<grid_for(V, kMsThreads * kMsVerts), kMsThreads, 0, st>>>(

@@ -156,14 +156,14 @@ lg_status run_list_step(lg_store* s, const SnapCsr& g, const uint32_t* list, uin
 		DevBuf& cnt, DevBuf& pos, DevBuf& scan_tmp, unsigned long long* ctr,
 		Launch&& launch, uint64_t* produced) {
 	cudaStream_t st = s->stream;
-	list_slots<<<grid_for(n, 256), 256, 0, st>>>(g, list, n, cnt.as<uint32_t>());
 	uint64_t total = 0;
-	LG_TRY(exclusive_scan_u32(cnt.as<uint32_t>(), pos.as<uint32_t>(), n, scan_tmp, st, &total));
+	LG_TRY(exclusive_scan_slots(g, list, n, cnt.as<uint32_t>(), pos.as<uint32_t>(), scan_tmp, st,
+			&total));
 	LG_CUDA(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), st), "memset");
 	const uint32_t nranges = (uint32_t)((total + kSccRange - 1) / kSccRange);
 	if (nranges) launch(grid_for(nranges, kSccThreads / 32), (uint32_t)total, nranges);
 	LG_CUDA(cudaGetLastError(), "scc step");
-	s->launches += 4 + (nranges ? 1 : 0);
+	s->launches += scan_launches(n) + (nranges ? 1 : 0);
 	unsigned long long h = 0;
 	LG_TRY(read_words(s, ctr, 1, &h));
 	*produced = h;

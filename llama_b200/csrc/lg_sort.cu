@@ -184,7 +184,7 @@ lg_status radix_sort_u64(lg_store* s, unsigned long long* keys, uint32_t* payloa
 			rs_scatter<false><<<tiles, kRsThreads, smem, st>>>(src, nullptr, n, shift, off, tiles,
 					dst, nullptr);
 		LG_CUDA(cudaGetLastError(), "radix sort pass");
-		s->launches += 5;
+		s->launches += 2 + scan_launches((uint64_t)256 * tiles);
 		std::swap(src, dst);
 		std::swap(psrc, pdst);
 	}

@@ -180,6 +180,7 @@ struct lg_sssp_split {
 		c.lt = (heavy ? lt_heavy : lt_light).as<LevelTab>();
 		c.deg = deg;
 		c.V = V;
+		c.slot_off = nullptr;
 		return c;
 	}
 };
@@ -350,12 +351,12 @@ extern "C" lg_status lg_sssp_delta(lg_snapshot* sn, int64_t root, uint32_t delta
 			LG_CUDA(cudaMemcpyAsync(ctr, init, 4 * sizeof(unsigned long long),
 					cudaMemcpyHostToDevice, st), "h2d");
 			s->h2d_bytes += 4 * sizeof(unsigned long long);
-			list_slots<<<grid_for(blen, 256), 256, 0, st>>>(heavy, blist, (uint32_t)blen, qcnt);
-			LG_TRY(exclusive_scan_u32(qcnt, qpos, blen, sc[8], st, nullptr));
+			LG_TRY(exclusive_scan_slots(heavy, blist, blen, qcnt,
+					qpos, sc[8], st, nullptr));
 			sssp_relax<<<relax_blocks, kSsspThreads, 0, st>>>(heavy, blist, qpos, (uint32_t)blen,
 					d, stamp, fstamp, round, epoch, hi, qn, far, ctr, range);
 			LG_CUDA(cudaGetLastError(), "sssp_relax heavy");
-			s->launches += 5;
+			s->launches += 1 + scan_launches(blen);
 			LG_CUDA(cudaMemcpyAsync(h, ctr, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st), "d2h");
 			LG_CUDA(cudaStreamSynchronize(st), "sssp heavy");
 			s->d2h_bytes += 4 * sizeof(unsigned long long);
@@ -411,12 +412,12 @@ extern "C" lg_status lg_sssp_delta(lg_snapshot* sn, int64_t root, uint32_t delta
 					kSsspThreads, 0, st>>>(q, (uint32_t)qlen, bstamp, bid, blist, ctr);
 			s->launches++;
 		}
-		list_slots<<<grid_for(qlen, 256), 256, 0, st>>>(out, q, (uint32_t)qlen, qcnt);
-		LG_TRY(exclusive_scan_u32(qcnt, qpos, qlen, sc[8], st, nullptr));
+		LG_TRY(exclusive_scan_slots(out, q, qlen, qcnt,
+				qpos, sc[8], st, nullptr));
 		sssp_relax<<<relax_blocks, kSsspThreads, 0, st>>>(out, q, qpos, (uint32_t)qlen, d,
 				stamp, fstamp, round, epoch, hi, qn, far, ctr, range);
 		LG_CUDA(cudaGetLastError(), "sssp_relax");
-		s->launches += 5;
+		s->launches += 1 + scan_launches(qlen);
 		LG_CUDA(cudaMemcpyAsync(h, ctr, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st), "d2h");
 		LG_CUDA(cudaStreamSynchronize(st), "sssp relax");
 		s->d2h_bytes += 4 * sizeof(unsigned long long);

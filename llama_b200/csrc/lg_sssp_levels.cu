@@ -77,8 +77,7 @@ __device__ bool list_offsets(const SnapCsr& g, const uint32_t* list, uint32_t n,
 #pragma unroll
 		for (int j = 0; j < kSlSmallPer; j++) {
 			const uint32_t i = tid * kSlSmallPer + j;
-			uint32_t f0;
-			kc[j] = i < n ? vertex_slots(g, __ldcg(list + i), &f0) : 0u;
+			kc[j] = i < n ? vertex_slots(g, __ldcg(list + i)) : 0u;
 			sum += kc[j];
 		}
 		if (block_sum<kSlWarps>(sum) >= (1ull << 32)) {
@@ -103,8 +102,7 @@ __device__ bool list_offsets(const SnapCsr& g, const uint32_t* list, uint32_t n,
 	const uint32_t c0 = min(n, blockIdx.x * chunk), c1 = min(n, c0 + chunk);
 	unsigned long long s = 0;
 	for (uint32_t i = c0 + tid; i < c1; i += blockDim.x) {
-		uint32_t f0;
-		const uint32_t k = vertex_slots(g, __ldcg(list + i), &f0);
+		const uint32_t k = vertex_slots(g, __ldcg(list + i));
 		cnt[i] = k;
 		s += k;
 	}

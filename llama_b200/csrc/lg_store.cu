@@ -51,26 +51,36 @@ CallPool::~CallPool() {
 }
 
 lg_status make_pool(int device, cudaStream_t stream, std::shared_ptr<CallPool>* out) {
-	std::shared_ptr<CallPool> c;
 	try {
-		c = std::make_shared<CallPool>();
+		auto c = std::make_shared<CallPool>();
+		c->device = device;
+		c->stream = stream;
 		std::lock_guard<std::mutex> lk(g_pools_mu);
 		g_pools.push_back(c.get());
+		*out = c;
 	} catch (const std::bad_alloc&) {
 		return set_error(LG_ENOMEM, "host allocation");
 	}
+	return LG_OK;
+}
+
+// The pool itself, made when the first buffer asks for memory.
+static cudaError_t open_pool(CallPool* c) {
+	if (c->pool) return cudaSuccess;
 	cudaMemPoolProps props;
 	std::memset(&props, 0, sizeof(props));
 	props.allocType = cudaMemAllocationTypePinned;
 	props.location.type = cudaMemLocationTypeDevice;
-	props.location.id = device;
-	LG_CUDA(cudaMemPoolCreate(&c->pool, &props), "memory pool");
+	props.location.id = c->device;
+	cudaMemPool_t p = nullptr;
+	cudaError_t e = cudaMemPoolCreate(&p, &props);
+	if (e != cudaSuccess) return e;
 	uint64_t keep = kPoolKeep;
-	LG_CUDA(cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep),
-			"memory pool");
-	c->stream = stream;
-	*out = c;
-	return LG_OK;
+	e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+	if (e != cudaSuccess) { cudaMemPoolDestroy(p); return e; }
+	std::lock_guard<std::mutex> lk(g_pools_mu);       // trim_pools reads it
+	c->pool = p;
+	return cudaSuccess;
 }
 
 // Gives the memory no buffer holds back to the device.
@@ -95,7 +105,9 @@ lg_status DevBuf::reserve(size_t n) {
 	if (n == 0) n = 16;
 	cudaError_t e = cudaSuccess;
 	for (int attempt = 0; attempt < 2; attempt++) {
-		e = from ? cudaMallocFromPoolAsync(&p, n, from->pool, from->stream) : cudaMalloc(&p, n);
+		if (!from) e = cudaMalloc(&p, n);
+		else if ((e = open_pool(from.get())) == cudaSuccess)
+			e = cudaMallocFromPoolAsync(&p, n, from->pool, from->stream);
 		if (e != cudaErrorMemoryAllocation || attempt) break;
 		(void)cudaGetLastError();
 		trim_pools();
@@ -217,13 +229,18 @@ lg_status append_dels(lg_store* s, DevCsr& csr, const uint2* add, size_t n,
 }
 
 // ---------------------------------------------------------------------------
-// Exclusive scan (u32 -> u32): per-tile sums, a single-CTA scan of the tile
-// sums, then per-tile scans with the carried offset.
+// Exclusive scan (u32 -> u32) of an array or of the slot counts of a vertex
+// list.  Up to one tile: one CTA.  Up to kScanOwnTiles tiles: per-tile sums
+// (which also store the counts of a list), then per-tile scans whose CTAs each
+// add up the sums before theirs.  More: a single-CTA scan of the sums between
+// the two.  The traversals scan a frontier per step, so what counts up to some
+// 10^5 entries is the number of launches (2 to 3 us each): a list of 10^4
+// takes 1 or 2 where counting and the three-kernel scan took 4.
 // ---------------------------------------------------------------------------
 
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 8;
-constexpr uint64_t kScanTile = (uint64_t)kScanThreads * kScanItems;
+static_assert((uint64_t)kScanThreads * kScanItems == kScanTile, "values per CTA");
 
 __device__ __forceinline__ uint64_t block_excl_scan(uint64_t x, uint64_t* total) {
 	__shared__ uint64_t warp_sums[32];
@@ -253,12 +270,62 @@ __device__ __forceinline__ uint64_t block_excl_scan(uint64_t x, uint64_t* total)
 	return before + v - x;
 }
 
-__global__ void scan_tile_sums(const uint32_t* in, uint64_t n, uint64_t* sums) {
+struct ScanArray {
+	const uint32_t* a;
+	__device__ __forceinline__ uint32_t operator()(uint64_t i) const { return a[i]; }
+};
+
+struct ScanSlots {
+	SnapCsr g;
+	const uint32_t* list;
+	__device__ __forceinline__ uint32_t operator()(uint64_t i) const {
+		return vertex_slots(g, list ? __ldg(list + i) : (uint32_t)i);
+	}
+};
+
+// One tile (n <= kScanTile): out[0 .. n] and the total in one CTA; cnt, if
+// not null, receives the values.
+template <class In>
+__global__ void __launch_bounds__(kScanThreads)
+scan_one(In in, uint32_t* cnt, uint32_t* out, uint32_t n, uint64_t* grand) {
+	uint32_t x[kScanItems];
+#pragma unroll
+	for (int j = 0; j < kScanItems; j++) {
+		const uint32_t i = j * kScanThreads + threadIdx.x;
+		x[j] = i < n ? in(i) : 0u;
+	}
+	uint64_t carry = 0;
+#pragma unroll
+	for (int j = 0; j < kScanItems; j++) {
+		if (j * kScanThreads >= n) break;                    // block-uniform
+		const uint32_t i = j * kScanThreads + threadIdx.x;
+		uint64_t tot;
+		const uint64_t ex = block_excl_scan(x[j], &tot);
+		if (i < n) {
+			out[i] = (uint32_t)(carry + ex);
+			if (cnt) cnt[i] = x[j];
+		}
+		carry += tot;
+	}
+	if (threadIdx.x == 0) {
+		out[n] = (uint32_t)carry;
+		*grand = carry;
+	}
+}
+
+template <class In>
+__global__ void __launch_bounds__(kScanThreads)
+scan_tile_sums(In in, uint64_t n, uint32_t* cnt, uint64_t* sums) {
 	uint64_t base = (uint64_t)blockIdx.x * kScanTile;
 	uint64_t s = 0;
+#pragma unroll
 	for (int i = 0; i < kScanItems; i++) {
 		uint64_t idx = base + (uint64_t)i * kScanThreads + threadIdx.x;
-		if (idx < n) s += in[idx];
+		if (idx < n) {
+			const uint32_t x = in(idx);
+			if (cnt) cnt[idx] = x;
+			s += x;
+		}
 	}
 	uint64_t tot;
 	block_excl_scan(s, &tot);
@@ -278,9 +345,12 @@ __global__ void scan_sums_single(uint64_t* sums, uint64_t n, uint64_t* grand) {
 }
 
 // A thread scans kScanItems consecutive values; with 16-byte aligned arrays
-// it moves them as two 16-byte vectors each way.
-__global__ void scan_tiles(const uint32_t* in, uint32_t* out, uint64_t n,
-		const uint64_t* sums, const uint64_t* grand) {
+// it moves them as two 16-byte vectors each way.  sums: exclusive prefix of
+// the tiles (kOwn false, *grand the total), or the tiles' sums, of which every
+// CTA adds up those before it and the last one writes *grand.
+template <bool kOwn>
+__global__ void __launch_bounds__(kScanThreads)
+scan_tiles(const uint32_t* in, uint32_t* out, uint64_t n, const uint64_t* sums, uint64_t* grand) {
 	static_assert(kScanItems == 8, "two 16-byte vectors per thread");
 	uint64_t base = (uint64_t)blockIdx.x * kScanTile
 		+ (uint64_t)threadIdx.x * kScanItems;
@@ -301,8 +371,15 @@ __global__ void scan_tiles(const uint32_t* in, uint32_t* out, uint64_t n,
 	uint64_t s = 0;
 #pragma unroll
 	for (int i = 0; i < kScanItems; i++) s += vals[i];
-	uint64_t tot;
-	uint64_t ex = block_excl_scan(s, &tot) + sums[blockIdx.x];
+	uint64_t tot, before;
+	if (kOwn) {
+		uint64_t b = 0;
+		for (uint32_t t = threadIdx.x; t < blockIdx.x; t += kScanThreads) b += sums[t];
+		block_excl_scan(b, &before);
+	} else {
+		before = sums[blockIdx.x];
+	}
+	uint64_t ex = block_excl_scan(s, &tot) + before;
 	uint32_t o[kScanItems];
 #pragma unroll
 	for (int i = 0; i < kScanItems; i++) {
@@ -319,19 +396,33 @@ __global__ void scan_tiles(const uint32_t* in, uint32_t* out, uint64_t n,
 			if (idx < n) out[idx] = o[i];
 		}
 	}
-	if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = (uint32_t)*grand;
+	if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+		if (kOwn) *grand = before + tot;
+		out[n] = (uint32_t)(before + tot);
+	}
 }
 
-lg_status exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint64_t n,
-		DevBuf& tmp, cudaStream_t stream, uint64_t* total) {
+template <class In>
+static lg_status exclusive_scan(const In& in, const uint32_t* arr, uint32_t* cnt, uint32_t* out,
+		uint64_t n, DevBuf& tmp, cudaStream_t stream, uint64_t* total) {
 	uint64_t tiles = (n + kScanTile - 1) / kScanTile;
 	if (tiles == 0) tiles = 1;
 	LG_TRY(tmp.reserve((tiles + 1) * sizeof(uint64_t)));
 	uint64_t* sums = tmp.as<uint64_t>();
-	scan_tile_sums<<<(unsigned)tiles, kScanThreads, 0, stream>>>(in, n, sums);
-	scan_sums_single<<<1, kScanThreads, 0, stream>>>(sums, tiles, sums + tiles);
-	scan_tiles<<<(unsigned)tiles, kScanThreads, 0, stream>>>(in, out, n, sums,
-			sums + tiles);
+	if (tiles == 1) {
+		scan_one<<<1, kScanThreads, 0, stream>>>(in, cnt, out, (uint32_t)n, sums + 1);
+	} else {
+		scan_tile_sums<<<(unsigned)tiles, kScanThreads, 0, stream>>>(in, n, cnt, sums);
+		const uint32_t* vals = cnt ? cnt : arr;
+		if (tiles <= kScanOwnTiles) {
+			scan_tiles<true><<<(unsigned)tiles, kScanThreads, 0, stream>>>(vals, out, n, sums,
+					sums + tiles);
+		} else {
+			scan_sums_single<<<1, kScanThreads, 0, stream>>>(sums, tiles, sums + tiles);
+			scan_tiles<false><<<(unsigned)tiles, kScanThreads, 0, stream>>>(vals, out, n, sums,
+					sums + tiles);
+		}
+	}
 	LG_CUDA(cudaGetLastError(), "scan launch");
 	if (total) {
 		// read through one pinned word per host thread (kept for the
@@ -349,6 +440,16 @@ lg_status exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint64_t n,
 			return set_error(LG_ENOTSUP, "more than 2^32-1 fragments in a snapshot");
 	}
 	return LG_OK;
+}
+
+lg_status exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint64_t n,
+		DevBuf& tmp, cudaStream_t stream, uint64_t* total) {
+	return exclusive_scan(ScanArray{in}, in, nullptr, out, n, tmp, stream, total);
+}
+
+lg_status exclusive_scan_slots(const SnapCsr& g, const uint32_t* list, uint64_t n, uint32_t* cnt,
+		uint32_t* out, DevBuf& tmp, cudaStream_t stream, uint64_t* total) {
+	return exclusive_scan(ScanSlots{g, list}, nullptr, cnt, out, n, tmp, stream, total);
 }
 
 // ---------------------------------------------------------------------------
@@ -631,7 +732,7 @@ static lg_status open_dir(lg_snapshot* sn, DevCsr& csr, SnapDir& d) {
 			cnt.as<uint32_t>(), d.deg.as<uint32_t>(), slots.as<uint32_t>(),
 			nullptr, nullptr);
 	LG_CUDA(cudaGetLastError(), "walk_fragments");
-	s->launches += 5;   // two walks and the three scan kernels
+	s->launches += 2 + scan_launches(V);
 	uint64_t F = 0;
 	LG_TRY(exclusive_scan_u32(cnt.as<uint32_t>(), d.frag_off.as<uint32_t>(), V,
 			scan_tmp, st, &F));
@@ -686,6 +787,7 @@ static lg_status open_dir(lg_snapshot* sn, DevCsr& csr, SnapDir& d) {
 		g.lt = d.lt.as<LevelTab>();
 		g.deg = d.deg.as<uint32_t>();
 		g.V = V;
+		g.slot_off = nullptr;
 		live_counts<<<grid_for(V, B), B, 0, st>>>(g, d.deg.as<uint32_t>());
 		LG_CUDA(cudaGetLastError(), "window degrees");
 		s->launches++;
@@ -707,7 +809,7 @@ static lg_status open_dir(lg_snapshot* sn, DevCsr& csr, SnapDir& d) {
 	}
 	sum_u32<<<592, B, 0, st>>>(d.deg.as<uint32_t>(), V, counters.as<unsigned long long>());
 	LG_CUDA(cudaGetLastError(), "degree sum");
-	s->launches += 4;
+	s->launches += 1 + scan_launches(V);
 	unsigned long long sums[2] = {0, 0};
 	LG_CUDA(cudaMemcpyAsync(sums, counters.p, sizeof(sums), cudaMemcpyDeviceToHost, st), "d2h");
 	LG_CUDA(cudaStreamSynchronize(st), "snapshot sizes");
@@ -954,8 +1056,8 @@ uint64_t lg_store_device_bytes(const lg_store* s) {
 	}
 	for (const DevBuf& x : s->scratch) b += x.bytes;
 	uint64_t kept = 0;
-	if (cudaMemPoolGetAttribute(s->pool->pool, cudaMemPoolAttrReservedMemCurrent, &kept)
-			== cudaSuccess)
+	if (s->pool->pool && cudaMemPoolGetAttribute(s->pool->pool, cudaMemPoolAttrReservedMemCurrent,
+			&kept) == cudaSuccess)
 		b += kept;
 	return b;
 }

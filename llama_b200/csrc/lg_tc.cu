@@ -525,7 +525,7 @@ extern "C" lg_status lg_triangle_count(lg_snapshot* sn, lg_tc_result* result) {
 	tc_classify<<<grid_for(V, kTcThreads), kTcThreads, 0, st>>>((uint32_t)V, foff, ad, ls, cd,
 			cd + 8);
 	LG_CUDA(cudaGetLastError(), "tc_classify");
-	s->launches += 9;
+	s->launches += 3 + scan_launches(uq_tiles) + scan_launches(V);
 	LG_TRY(launch_bitmap<1>(s, sms, (uint32_t)std::min<uint64_t>(V, kTcDomain0), ls, cd, cd + 4,
 			foff, ad, cd + 8));
 	if (V > kTcDomain0)
