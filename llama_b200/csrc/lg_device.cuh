@@ -196,10 +196,15 @@ struct DevCsr {
 
 // Slots per PageRank block; range_lb below is computed for this size.
 constexpr uint32_t kBlockSlots = 1024;
+// Virtual slots a warp of the flatten takes; tile_frag is computed for it.
+constexpr uint32_t kSlotTile = 512;
 
 struct SnapDir {
 	DevBuf frag_off, frags, deg, delbits, lt, slot_off;
 	DevBuf range_lb;               // lower_bound(slot_off, r * kBlockSlots), r = 0..nblocks
+	DevBuf frag_start;             // F + 1 u32: first virtual slot of every fragment
+	DevBuf frag_vert;              // F u32: its vertex
+	DevBuf tile_frag;              // fragment that holds virtual slot t * kSlotTile
 	DevBuf tmp_cnt, tmp_slots, tmp_scan, tmp_words, tmp_sum;   // open-time scratch
 	uint64_t n_frags = 0;
 	uint64_t n_edges = 0;          // live edges (sum of degrees)
@@ -209,10 +214,11 @@ struct SnapDir {
 	bool present = false;
 	// exchange device buffers with o (a closed snapshot's, kept for reuse)
 	void swap_buffers(SnapDir& o) {
-		DevBuf* a[] = {&frag_off, &frags, &deg, &delbits, &lt, &slot_off, &range_lb,
-			&tmp_cnt, &tmp_slots, &tmp_scan, &tmp_words, &tmp_sum};
+		DevBuf* a[] = {&frag_off, &frags, &deg, &delbits, &lt, &slot_off, &range_lb, &frag_start,
+			&frag_vert, &tile_frag, &tmp_cnt, &tmp_slots, &tmp_scan, &tmp_words, &tmp_sum};
 		DevBuf* b[] = {&o.frag_off, &o.frags, &o.deg, &o.delbits, &o.lt, &o.slot_off,
-			&o.range_lb, &o.tmp_cnt, &o.tmp_slots, &o.tmp_scan, &o.tmp_words, &o.tmp_sum};
+			&o.range_lb, &o.frag_start, &o.frag_vert, &o.tile_frag, &o.tmp_cnt, &o.tmp_slots,
+			&o.tmp_scan, &o.tmp_words, &o.tmp_sum};
 		for (size_t i = 0; i < sizeof(a) / sizeof(a[0]); i++) a[i]->swap(*b[i]);
 	}
 	SnapCsr view() const {
@@ -312,6 +318,9 @@ bool is_device_pointer(const void* p);
 lg_status exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint64_t n,
 		DevBuf& tmp, cudaStream_t stream, uint64_t* total);
 
+// The same with 1 in the place of every positive value.
+lg_status exclusive_scan_nonzero(const uint32_t* in, uint32_t* out, uint64_t n, DevBuf& tmp,
+		cudaStream_t stream, uint64_t* total);
 // The same for the slot counts of list[0 .. n) (all vertices in order when
 // list is null) in g, which are left in cnt[0 .. n).
 lg_status exclusive_scan_slots(const SnapCsr& g, const uint32_t* list, uint64_t n, uint32_t* cnt,
@@ -323,6 +332,9 @@ constexpr uint64_t kScanOwnTiles = 4096;    // tiles whose CTAs add up the sums 
 inline uint64_t scan_launches(uint64_t n) {
 	return n <= kScanTile ? 1 : n <= kScanTile * kScanOwnTiles ? 2 : 3;
 }
+
+// out[v] = live slots of v's fragments in direction dir (0 out, 1 in).
+lg_status live_degrees(const lg_snapshot* sn, int dir, uint32_t* out);
 
 // Copy `bytes` of device data to a caller buffer (host or device) on the
 // store's stream, counting host-bound bytes.

@@ -3,12 +3,21 @@
 // Reference: ll_t_flatten (benchmark/tools/flatten.h) merges every level of
 // a LLAMA graph into a single level by iterating each vertex's edges
 // (newest fragment first, deleted edges skipped) on the host.  Here the
-// same order is produced in one balanced pass over the virtual slot space
-// (one CTA per 1024 virtual slots): row starts are the scan of the live
-// degrees, and flat_write writes every live slot's id (and weight) at its
-// block's base (found from the row start of the block's first vertex) + its
-// live rank.  Row bookkeeping for the tile kernels (heads, nz_rows,
-// nz_off, tile_seg) and the optional fragment view follow.
+// same order is produced in one balanced pass over the virtual slot space:
+// row starts are the scan of the live degrees, and each warp of flat_write
+// copies the live slots of kSlotTile consecutive virtual slots to its base.
+// With deletions the bases are the scan of the tiles' live slots (flat_live,
+// which reads the deletion words only); without any, slot and edge positions
+// are the same.  Every vertex's row start is checked against the position its
+// first slot goes to, so a degree that is not the live slot count is found.
+// Row bookkeeping for the tile kernels (heads, nz_rows, nz_off, tile_seg) and
+// the optional fragment view follow.
+//
+// flat_write keeps up to 32 fragments in a warp's lanes: the fragments that
+// begin in a 32-slot chunk are bits of one word, so a slot's fragment is a
+// population count away.  The form before it built a slot-to-fragment table
+// per 1024-slot block in shared memory behind a dozen block barriers: it was
+// bound by those and by its instructions, 2.1 ms at 262 M slots.
 #include "lg_flat.cuh"
 
 #include <algorithm>
@@ -16,152 +25,156 @@
 
 namespace lg {
 
-// Writes the live slots of block r to ids[base ...] in slot order (and their
-// weights to w when non-null).  base = the live slots before the block:
-// off[e] of the entry e that holds the block's first slot, plus e's live
-// slots before it (its deleted slots counted a word at a time).  off is the
-// exclusive scan of the snapshot's live degrees; every entry that starts in
-// the block checks it against its rank in the block, and a mismatch (a
-// degree that is not the live slot count) sets bit 2 of *err.
-__global__ void __launch_bounds__(kMapThreads)
-flat_write(SlotSpace sp, const uint32_t* off, uint32_t E, uint32_t* ids, uint32_t* w,
-		unsigned int* err) {
-	constexpr int kGroups = kMapPerThread * (kMapThreads / 32);
-	__shared__ BlockMap m;
-	__shared__ uint16_t rank[kMapRange];
-	__shared__ uint32_t gpre[kGroups];
-	__shared__ uint32_t dead_w[kMapThreads / 32];
-	const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5;
-	const uint32_t r = blockIdx.x, ra = r * kMapRange, rb = block_end(sp, r);
-	map_block(sp, r, ra, rb, m);
+constexpr int kFwThreads = 256;
+constexpr int kFwWarps = kFwThreads / 32;
+constexpr int kFwAhead = 4;             // 32-slot chunks whose loads are issued together
 
-	// the block's slots: deletion word, id (and weight) loads issued first,
-	// for every slot, so they overlap the count below
-	uint32_t dw[kMapPerThread], id[kMapPerThread], wt[kMapPerThread], mask[kMapPerThread];
-	uint32_t bit[kMapPerThread];
-	bool have[kMapPerThread];
-#pragma unroll
-	for (int u = 0; u < kMapPerThread; u++) {
-		uint32_t lv = 0, idx = 0;
-		have[u] = block_slot(m, ra, rb, u * kMapThreads + tid, &lv, &idx);
-		dw[u] = have[u] ? __ldg(sp.g.lt->del[lv] + (idx >> 5)) : 0u;
-		id[u] = have[u] ? __ldg(sp.g.lt->ids[lv] + idx) : 0u;
-		wt[u] = (have[u] && w) ? __ldg(sp.g.lt->w[lv] + idx) : 0u;
-		bit[u] = idx & 31u;
-	}
+// One direction's fragments in virtual slot order.
+struct FragSpace {
+	const uint2* frags;        // F
+	const uint32_t* start;     // F + 1
+	const uint32_t* vert;      // F
+	const uint32_t* frag_off;  // V + 1
+	const uint32_t* tile_frag;
+	const LevelTab* lt;
+	uint32_t F, total, ntiles;
+};
 
-	// the first entry's slots before ra: its fragments lead ftab
-	const uint32_t e0 = m.eb;
-	uint32_t before = 0, dead = 0;
-	if (m.nf > 0 && m.fstart[0] < ra) {
-		const uint32_t nfe = min(__ldg(sp.g.frag_off + e0 + 1) - __ldg(sp.g.frag_off + e0), m.nf);
-		for (uint32_t i = 0; i < nfe; i++) {
-			const uint32_t s0 = m.fstart[i];
-			if (s0 >= ra) break;
-			const uint2 fr = m.ftab[i];
-			const uint32_t n = min(frag_len(fr), ra - s0);
-			before += n;
-			const uint32_t* d = sp.g.lt->del[frag_level(fr)];
-			const uint32_t a = fr.x, b = fr.x + n;          // slots [a, b)
-			for (uint32_t wd = (a >> 5) + tid; wd <= ((b - 1) >> 5); wd += kMapThreads) {
-				uint32_t x = __ldg(d + wd);
-				if (wd == (a >> 5)) x &= ~0u << (a & 31);
-				if (wd == ((b - 1) >> 5) && (b & 31)) x &= (1u << (b & 31)) - 1u;
-				dead += __popc(x);
-			}
+// live[t] = live slots of tile t.  A warp per tile, a lane per fragment piece:
+// the deletion words of the piece's slots, counted.
+__global__ void __launch_bounds__(kFwThreads)
+flat_live(FragSpace fs, uint32_t* live) {
+	const uint32_t lane = threadIdx.x & 31u;
+	const uint32_t t = blockIdx.x * kFwWarps + (threadIdx.x >> 5);
+	if (t >= fs.ntiles) return;
+	const uint32_t s0 = t * kSlotTile;
+	const uint32_t s1 = fs.total - s0 < kSlotTile ? fs.total : s0 + kSlotTile;
+	const uint32_t f0 = __ldg(fs.tile_frag + t);
+	uint32_t dead = 0;
+	for (uint32_t f = f0 + lane; f < fs.F; f += 32u) {
+		const uint32_t st = __ldg(fs.start + f);
+		if (st >= s1) break;
+		const uint2 fr = fs.frags[f];
+		const uint32_t c0 = max(st, s0), c1 = min(st + frag_len(fr), s1);
+		const uint32_t a = fr.x + (c0 - st), b = fr.x + (c1 - st);      // slots [a, b)
+		const uint32_t* d = fs.lt->del[frag_level(fr)];
+		for (uint32_t w = a >> 5; w <= (b - 1u) >> 5; w++) {
+			uint32_t x = __ldg(d + w);
+			if (w == a >> 5) x &= ~0u << (a & 31u);
+			if (w == (b - 1u) >> 5 && (b & 31u)) x &= (1u << (b & 31u)) - 1u;
+			dead += __popc(x);
 		}
 	}
-#pragma unroll
-	for (int o = 16; o > 0; o >>= 1) dead += __shfl_xor_sync(0xffffffffu, dead, o);
-	if (lane == 0) dead_w[wid] = dead;
+	dead = __reduce_add_sync(0xffffffffu, dead);
+	if (lane == 0) live[t] = s1 - s0 - dead;
+}
 
-#pragma unroll
-	for (int u = 0; u < kMapPerThread; u++)
-		mask[u] = __ballot_sync(0xffffffffu, have[u] && !((dw[u] >> bit[u]) & 1u));
-	// slot order is k = u * kMapThreads + wid * 32 + lane: group u * 4 + wid
-	if (lane == 0) {
-#pragma unroll
-		for (int u = 0; u < kMapPerThread; u++)
-			gpre[u * (kMapThreads / 32) + wid] = __popc(mask[u]);
+// The live slots of tile t to ids[base ...] in slot order (and their weights
+// to w when non-null); base = tile_base[t], or the tile's first slot where
+// nothing is deleted (tile_base null).  off = the row starts the degrees
+// give: a vertex whose first slot goes elsewhere, and a last tile that does
+// not end at off[V], set bit 2 of *err.
+template <bool kWeights>
+__global__ void __launch_bounds__(kFwThreads)
+flat_write(FragSpace fs, const uint32_t* tile_base, const uint32_t* off, uint64_t V, uint32_t E,
+		uint32_t* ids, uint32_t* w, unsigned int* err) {
+	__shared__ LevelTab lt;
+	{
+		const uint64_t* src = reinterpret_cast<const uint64_t*>(fs.lt);
+		uint64_t* dst = reinterpret_cast<uint64_t*>(&lt);
+		for (uint32_t i = threadIdx.x; i < sizeof(LevelTab) / 8; i += kFwThreads)
+			dst[i] = __ldg(src + i);
 	}
 	__syncthreads();
-	if (wid == 0) {
-		const uint32_t c = lane < (uint32_t)kGroups ? gpre[lane] : 0u;
-		uint32_t x = c;
-#pragma unroll
-		for (int o = 1; o < 32; o <<= 1) {
-			const uint32_t t = __shfl_up_sync(0xffffffffu, x, o);
-			if (lane >= (uint32_t)o) x += t;
-		}
-		if (lane < (uint32_t)kGroups) gpre[lane] = x - c;
-	}
-	__syncthreads();
-	uint32_t dead_all = 0;
-#pragma unroll
-	for (int x = 0; x < kMapThreads / 32; x++) dead_all += dead_w[x];
-	const uint32_t base = __ldg(off + e0) + before - dead_all;
-	const uint32_t below = (1u << lane) - 1u;
-#pragma unroll
-	for (int u = 0; u < kMapPerThread; u++) {
-		const uint32_t k = u * kMapThreads + tid;
-		const uint32_t rk = gpre[u * (kMapThreads / 32) + wid] + __popc(mask[u] & below);
-		rank[k] = (uint16_t)rk;
-		if ((mask[u] >> lane) & 1u) {
-			if (base + rk < E) {
-				ids[base + rk] = id[u];
-				if (w) w[base + rk] = wt[u];
-			} else {
-				atomicOr(err, 2u);      // degrees and live slots disagree
-			}
-		}
-	}
-	__syncthreads();
-	// entries starting in the block: their row start must be base + rank
-	const uint32_t e_begin = __ldg(sp.range_lb + r);
-	const uint32_t e_end = r == sp.nranges - 1 ? (uint32_t)sp.g.V : __ldg(sp.range_lb + r + 1);
+	const uint32_t lane = threadIdx.x & 31u;
+	const uint32_t t = blockIdx.x * kFwWarps + (threadIdx.x >> 5);
+	if (t >= fs.ntiles) return;
+	const uint32_t s0 = t * kSlotTile;
+	const uint32_t s1 = fs.total - s0 < kSlotTile ? fs.total : s0 + kSlotTile;
+	uint32_t f = __ldg(fs.tile_frag + t);      // the window's first fragment
+	uint32_t run = tile_base ? __ldg(tile_base + t) : s0;
+	uint32_t start = 0, wend = s0;             // the window covers slots up to wend
+	uint2 fr = make_uint2(0u, 0u);
 	bool bad = false;
-	for (uint32_t e = e_begin + tid; e < e_end; e += kMapThreads) {
-		const uint32_t p = __ldg(sp.pos + e);
-		if (p < rb && p >= ra) bad |= __ldg(off + e) != base + rank[p - ra];
+	const uint32_t upto = 2u << lane;          // bits at or below the lane, + 1
+	for (uint32_t pos = s0; pos < s1;) {
+		const uint32_t full = min(pos + 32u * kFwAhead, s1);
+		if (full > wend) {
+			// load the window that begins with the fragment holding pos
+			if (wend > s0) f += __popc(__ballot_sync(0xffffffffu, start <= pos)) - 1u;
+			const uint32_t k = f + lane;
+			start = k < fs.F ? __ldg(fs.start + k) : 0xffffffffu;
+			fr = k < fs.F ? fs.frags[k] : make_uint2(0u, 0u);
+			const uint32_t after = f + 32u <= fs.F ? __ldg(fs.start + f + 32u) : fs.total;
+			wend = after;
+		}
+		const uint32_t end = min(full, wend);
+		uint32_t id[kFwAhead], dw[kFwAhead], wt[kFwAhead], bit[kFwAhead], own[kFwAhead];
+		bool head[kFwAhead];
+#pragma unroll
+		for (int u = 0; u < kFwAhead; u++) {
+			const uint32_t base = pos + u * 32u;
+			// fragments begun by the chunk's first slot, and those that begin
+			// at a later one
+			const uint32_t rel = start - base;
+			const uint32_t begun = __popc(__ballot_sync(0xffffffffu, start <= base));
+			const uint32_t mask = __reduce_or_sync(0xffffffffu,
+					start > base && rel < 32u ? 1u << rel : 0u);
+			own[u] = begun - 1u + __popc(mask & (upto - 1u));
+			const uint32_t ost = __shfl_sync(0xffffffffu, start, own[u]);
+			const uint32_t oix = __shfl_sync(0xffffffffu, fr.x, own[u]);
+			const uint32_t oy = __shfl_sync(0xffffffffu, fr.y, own[u]);
+			const uint32_t s = base + lane;
+			const uint32_t ix = oix + (s - ost), lv = oy & kLevelMask;
+			const bool in = s < end;
+			head[u] = in && s == ost;
+			bit[u] = ix & 31u;
+			dw[u] = in ? __ldg(lt.del[lv] + (ix >> 5)) : ~0u;
+			id[u] = in ? __ldcs(lt.ids[lv] + ix) : 0u;
+			if (kWeights) wt[u] = in ? __ldcs(lt.w[lv] + ix) : 0u;
+		}
+#pragma unroll
+		for (int u = 0; u < kFwAhead; u++) {
+			const bool live = !((dw[u] >> bit[u]) & 1u);
+			const unsigned m = __ballot_sync(0xffffffffu, live);
+			const uint32_t p = run + __popc(m & ((1u << lane) - 1u));
+			if (live) {
+				if (p < E) {
+					ids[p] = id[u];
+					if (kWeights) w[p] = wt[u];
+				} else {
+					bad = true;               // degrees and live slots disagree
+				}
+			}
+			if (head[u]) {
+				// the first fragment of a vertex: its row starts here
+				const uint32_t k = f + own[u], v = __ldg(fs.vert + k);
+				if (__ldg(fs.frag_off + v) == k) bad |= __ldg(off + v) != p;
+			}
+			run += __popc(m);
+		}
+		pos = end;
 	}
-	if (r == sp.nranges - 1 && tid == kMapThreads - 1) {
-		// the last block ends at the total of the degrees
-		const uint32_t nlive = gpre[kGroups - 1] + __popc(mask[kMapPerThread - 1]);
-		bad |= base + nlive != __ldg(off + sp.g.V);
-	}
+	if (t == fs.ntiles - 1u) bad |= run != __ldg(off + V);
 	if (bad) atomicOr(err, 2u);
 }
 
-__global__ void flat_flags(const uint32_t* off, uint64_t V, uint32_t* flags) {
-	const uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (v >= V) return;
-	flags[v] = __ldg(off + v + 1) > __ldg(off + v);
-}
-
+// Rows with edges (vertex, start, head bit) and, for every tile that begins
+// inside or at the end of a row, the rows begun before it.
 __global__ void flat_rows(const uint32_t* off, const uint32_t* kidx, uint64_t V,
-		uint32_t* nz_rows, uint32_t* nz_off, uint32_t* heads) {
+		uint32_t* nz_rows, uint32_t* nz_off, uint32_t* heads, uint32_t ntiles,
+		uint32_t* tile_seg) {
 	const uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
 	if (v >= V) return;
-	const uint32_t o = __ldg(off + v);
-	if (__ldg(off + v + 1) == o) return;
+	const uint32_t o = __ldg(off + v), e = __ldg(off + v + 1);
+	if (e == o) return;
 	const uint32_t k = __ldg(kidx + v);
 	nz_rows[k] = (uint32_t)v;
 	nz_off[k] = o;
 	atomicOr(heads + (o >> 5), 1u << (o & 31u));
-}
-
-// tile_seg[t] = number of rows beginning before edge t * kFlatTile.
-__global__ void flat_tiles(const uint32_t* nz_off, uint32_t R, uint32_t ntiles,
-		uint32_t* tile_seg) {
-	const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-	if (t >= ntiles) return;
-	const uint32_t x = t * kFlatTile;
-	uint32_t lo = 0, hi = R;
-	while (lo < hi) {
-		const uint32_t mid = (lo + hi) >> 1;
-		if (__ldg(nz_off + mid) < x) lo = mid + 1; else hi = mid;
-	}
-	tile_seg[t] = lo;
+	if (k == 0) tile_seg[0] = 0;
+	for (uint32_t t = o / kFlatTile + 1u; t <= e / kFlatTile && t < ntiles; t++)
+		tile_seg[t] = k + 1u;
 }
 
 // Fragment view: row k of the flat CSR is fragment k, {start, len << 6 | 0};
@@ -188,10 +201,12 @@ SlotSpace slot_space(const lg_snapshot* sn, int dir) {
 	return sp;
 }
 
-lg_status build_flat(lg_snapshot* sn, int dir, FlatCsr& f, bool view, bool weights) {
+// build_flat with rows of deg[v] edges, E in all.  *mismatch (and LG_OK, f
+// unfinished): the live slots are not laid out as those degrees say.
+static lg_status build_rows(lg_snapshot* sn, int dir, FlatCsr& f, bool view, bool weights,
+		const uint32_t* deg, uint64_t E, bool* mismatch) {
 	lg_store* s = sn->store;
 	cudaStream_t st = s->stream;
-	const SlotSpace sp = slot_space(sn, dir);
 	const uint64_t V = sn->V;
 	const unsigned B = 256;
 	const DevCsr& csr = dir == 0 ? s->out : s->in;
@@ -204,9 +219,9 @@ lg_status build_flat(lg_snapshot* sn, int dir, FlatCsr& f, bool view, bool weigh
 	f.V = V;
 	f.has_view = false;
 	f.has_nz_outdeg = false;
-	// row starts from the live degrees; flat_write checks them
+	// row starts from the degrees; flat_write checks them
 	const SnapDir& d = dir == 0 ? sn->out : sn->in;
-	const uint64_t E = d.n_edges;
+	*mismatch = false;
 	if (E > 0xffffffffull - 2 * kFlatTile)
 		return set_error(LG_ENOTSUP, "more than 2^32 - %u live edges in one direction",
 				2 * kFlatTile);
@@ -220,35 +235,57 @@ lg_status build_flat(lg_snapshot* sn, int dir, FlatCsr& f, bool view, bool weigh
 	LG_TRY(f.err.reserve(sizeof(unsigned int)));
 	uint32_t* off = f.off.as<uint32_t>();
 	LG_CUDA(cudaMemsetAsync(f.err.p, 0, sizeof(unsigned int), st), "clear flag");
-	LG_TRY(exclusive_scan_u32(d.deg.as<uint32_t>(), off, V, f.scan_tmp, st, nullptr));
-	flat_write<<<sp.nranges, kMapThreads, 0, st>>>(sp, off, (uint32_t)E, f.ids.as<uint32_t>(),
-			weighted ? f.w.as<uint32_t>() : nullptr, f.err.as<unsigned int>());
-	LG_CUDA(cudaGetLastError(), "flat_write");
+	LG_TRY(exclusive_scan_u32(deg, off, V, f.scan_tmp, st, nullptr));
+	FragSpace fs;
+	fs.frags = d.frags.as<uint2>();
+	fs.start = d.frag_start.as<uint32_t>();
+	fs.vert = d.frag_vert.as<uint32_t>();
+	fs.frag_off = d.frag_off.as<uint32_t>();
+	fs.tile_frag = d.tile_frag.as<uint32_t>();
+	fs.lt = d.lt.as<LevelTab>();
+	fs.F = (uint32_t)d.n_frags;
+	fs.total = (uint32_t)d.n_frag_slots;
+	fs.ntiles = (uint32_t)((d.n_frag_slots + kSlotTile - 1) / kSlotTile);
+	const uint32_t* tile_base = nullptr;
+	if (d.n_dels > 0 && fs.ntiles > 0) {
+		LG_TRY(f.flags.reserve((2ull * fs.ntiles + 1) * sizeof(uint32_t)));
+		uint32_t* live = f.flags.as<uint32_t>();
+		flat_live<<<grid_for(fs.ntiles, kFwWarps), kFwThreads, 0, st>>>(fs, live);
+		LG_CUDA(cudaGetLastError(), "flat_live");
+		LG_TRY(exclusive_scan_u32(live, live + fs.ntiles, fs.ntiles, f.scan_tmp, st, nullptr));
+		tile_base = live + fs.ntiles;
+		s->launches += 1 + scan_launches(fs.ntiles);
+	}
+	if (fs.ntiles > 0) {
+		const unsigned blocks = grid_for(fs.ntiles, kFwWarps);
+		unsigned int* err = f.err.as<unsigned int>();
+		if (weighted)
+			flat_write<true><<<blocks, kFwThreads, 0, st>>>(fs, tile_base, off, V, (uint32_t)E,
+					f.ids.as<uint32_t>(), f.w.as<uint32_t>(), err);
+		else
+			flat_write<false><<<blocks, kFwThreads, 0, st>>>(fs, tile_base, off, V, (uint32_t)E,
+					f.ids.as<uint32_t>(), nullptr, err);
+		LG_CUDA(cudaGetLastError(), "flat_write");
+	}
 	unsigned int err = 0;
 	LG_CUDA(cudaMemcpyAsync(&err, f.err.p, sizeof(err), cudaMemcpyDeviceToHost, st), "d2h");
-	LG_TRY(f.flags.reserve(std::max<uint64_t>(V, 1) * sizeof(uint32_t)));
-	flat_flags<<<grid_for(V, B), B, 0, st>>>(off, V, f.flags.as<uint32_t>());
-	LG_CUDA(cudaGetLastError(), "flat_flags");
 	uint64_t R = 0;
-	LG_TRY(exclusive_scan_u32(f.flags.as<uint32_t>(), f.kidx.as<uint32_t>(), V, f.scan_tmp,
-			st, &R));
+	LG_TRY(exclusive_scan_nonzero(deg, f.kidx.as<uint32_t>(), V, f.scan_tmp, st, &R));
 	// (the scan waited for the stream, so err is in)
-	if (err & 2u)
-		return set_error(LG_EINVAL, "a vertex's degree differs from its live edge count");
+	if ((err & 2u) || (fs.ntiles == 0 && E > 0)) {
+		*mismatch = true;
+		return LG_OK;
+	}
 	f.R = R;
 	const uint64_t head_words = (uint64_t)f.ntiles * kFlatTileWords + 1;
 	LG_TRY(f.rows.reserve((2 * f.rcap() + f.ntiles + head_words) * sizeof(uint32_t)));
 	uint32_t* heads = const_cast<uint32_t*>(f.heads());
 	LG_CUDA(cudaMemsetAsync(heads, 0, head_words * sizeof(uint32_t), st), "clear heads");
 	flat_rows<<<grid_for(V, B), B, 0, st>>>(off, f.kidx.as<uint32_t>(), V,
-			const_cast<uint32_t*>(f.nz_rows()), const_cast<uint32_t*>(f.nz_off()), heads);
+			const_cast<uint32_t*>(f.nz_rows()), const_cast<uint32_t*>(f.nz_off()), heads,
+			f.ntiles, const_cast<uint32_t*>(f.tile_seg()));
 	LG_CUDA(cudaGetLastError(), "flat_rows");
-	if (f.ntiles > 0) {
-		flat_tiles<<<grid_for(f.ntiles, B), B, 0, st>>>(f.nz_off(), (uint32_t)R, f.ntiles,
-				const_cast<uint32_t*>(f.tile_seg()));
-		LG_CUDA(cudaGetLastError(), "flat_tiles");
-	}
-	s->launches += 2 * scan_launches(V) + 3 + (f.ntiles > 0);
+	s->launches += 2 * scan_launches(V) + 1 + (fs.ntiles > 0);
 	if (!view) return LG_OK;
 
 	LG_TRY(f.vfrags.reserve(f.rcap() * sizeof(uint2)));
@@ -275,6 +312,25 @@ lg_status build_flat(lg_snapshot* sn, int dir, FlatCsr& f, bool view, bool weigh
 		return set_error(LG_ENOTSUP, "a vertex has more than %u live edges, the longest "
 				"fragment a flat view can describe", (unsigned)LG_MAX_FRAGMENT_LEN);
 	f.has_view = true;
+	return LG_OK;
+}
+
+lg_status build_flat(lg_snapshot* sn, int dir, FlatCsr& f, bool view, bool weights,
+		bool strict) {
+	const SnapDir& d = dir == 0 ? sn->out : sn->in;
+	bool mismatch = false;
+	LG_TRY(build_rows(sn, dir, f, view, weights, d.deg.as<uint32_t>(), d.n_edges, &mismatch));
+	if (!mismatch) return LG_OK;
+	if (strict)
+		return set_error(LG_EINVAL, "a vertex's degree differs from its live edge count");
+	DevBuf cnt(sn->store->pool), tmp(sn->store->pool);
+	LG_TRY(cnt.reserve((2 * sn->V + 1) * sizeof(uint32_t)));
+	uint32_t* live = cnt.as<uint32_t>();
+	LG_TRY(live_degrees(sn, dir, live));
+	uint64_t E = 0;
+	LG_TRY(exclusive_scan_u32(live, live + sn->V, sn->V, tmp, sn->store->stream, &E));
+	LG_TRY(build_rows(sn, dir, f, view, weights, live, E, &mismatch));
+	if (mismatch) return set_error(LG_ECUDA, "live slots changed while they were flattened");
 	return LG_OK;
 }
 

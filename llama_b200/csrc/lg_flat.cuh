@@ -195,8 +195,11 @@ struct FlatCsr {
 // Builds f from direction dir of sn on the store's stream, with the edge
 // weights when `weights` and every level that holds fragment slots has them,
 // and the fragment view when `view`.  f's buffers are reused (grown) across
-// builds.
-lg_status build_flat(lg_snapshot* sn, int dir, FlatCsr& f, bool view, bool weights = true);
+// builds.  A snapshot whose vertex-table degrees are not its live edge counts
+// fails with LG_EINVAL when `strict`; otherwise its live edges are counted and
+// laid out all the same (for the calls that never read the degrees as sizes).
+lg_status build_flat(lg_snapshot* sn, int dir, FlatCsr& f, bool view, bool weights = true,
+		bool strict = true);
 
 } // namespace lg
 

@@ -380,7 +380,7 @@ extern "C" lg_status lg_ppr(lg_snapshot* const* snaps, int n_snaps, const int64_
 		const FlatCsr* f = sn->flat[1];
 		if (!f) {
 			if (!s->flat_scratch) s->flat_scratch = new FlatCsr;
-			LG_TRY(build_flat(sn, 1, *s->flat_scratch, false));
+			LG_TRY(build_flat(sn, 1, *s->flat_scratch, false, true, false));
 			f = s->flat_scratch;
 		}
 		PprArgs a;

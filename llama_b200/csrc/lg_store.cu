@@ -275,6 +275,12 @@ struct ScanArray {
 	__device__ __forceinline__ uint32_t operator()(uint64_t i) const { return a[i]; }
 };
 
+// 1 for the positive values.
+struct ScanNonzero {
+	const uint32_t* a;
+	__device__ __forceinline__ uint32_t operator()(uint64_t i) const { return a[i] != 0u; }
+};
+
 struct ScanSlots {
 	SnapCsr g;
 	const uint32_t* list;
@@ -348,7 +354,7 @@ __global__ void scan_sums_single(uint64_t* sums, uint64_t n, uint64_t* grand) {
 // it moves them as two 16-byte vectors each way.  sums: exclusive prefix of
 // the tiles (kOwn false, *grand the total), or the tiles' sums, of which every
 // CTA adds up those before it and the last one writes *grand.
-template <bool kOwn>
+template <bool kOwn, bool kNonzero>
 __global__ void __launch_bounds__(kScanThreads)
 scan_tiles(const uint32_t* in, uint32_t* out, uint64_t n, const uint64_t* sums, uint64_t* grand) {
 	static_assert(kScanItems == 8, "two 16-byte vectors per thread");
@@ -370,7 +376,10 @@ scan_tiles(const uint32_t* in, uint32_t* out, uint64_t n, const uint64_t* sums, 
 	}
 	uint64_t s = 0;
 #pragma unroll
-	for (int i = 0; i < kScanItems; i++) s += vals[i];
+	for (int i = 0; i < kScanItems; i++) {
+		if (kNonzero) vals[i] = vals[i] != 0u;
+		s += vals[i];
+	}
 	uint64_t tot, before;
 	if (kOwn) {
 		uint64_t b = 0;
@@ -402,8 +411,10 @@ scan_tiles(const uint32_t* in, uint32_t* out, uint64_t n, const uint64_t* sums, 
 	}
 }
 
-template <class In>
-static lg_status exclusive_scan(const In& in, const uint32_t* arr, uint32_t* cnt, uint32_t* out,
+// Scan of in(0 .. n); vals: where the second pass reads the values again
+// (cnt, if not null; kNonzero: they count as 1 where positive).
+template <bool kNonzero, class In>
+static lg_status exclusive_scan(const In& in, const uint32_t* vals, uint32_t* cnt, uint32_t* out,
 		uint64_t n, DevBuf& tmp, cudaStream_t stream, uint64_t* total) {
 	uint64_t tiles = (n + kScanTile - 1) / kScanTile;
 	if (tiles == 0) tiles = 1;
@@ -413,14 +424,13 @@ static lg_status exclusive_scan(const In& in, const uint32_t* arr, uint32_t* cnt
 		scan_one<<<1, kScanThreads, 0, stream>>>(in, cnt, out, (uint32_t)n, sums + 1);
 	} else {
 		scan_tile_sums<<<(unsigned)tiles, kScanThreads, 0, stream>>>(in, n, cnt, sums);
-		const uint32_t* vals = cnt ? cnt : arr;
 		if (tiles <= kScanOwnTiles) {
-			scan_tiles<true><<<(unsigned)tiles, kScanThreads, 0, stream>>>(vals, out, n, sums,
-					sums + tiles);
+			scan_tiles<true, kNonzero><<<(unsigned)tiles, kScanThreads, 0, stream>>>(vals, out, n,
+					sums, sums + tiles);
 		} else {
 			scan_sums_single<<<1, kScanThreads, 0, stream>>>(sums, tiles, sums + tiles);
-			scan_tiles<false><<<(unsigned)tiles, kScanThreads, 0, stream>>>(vals, out, n, sums,
-					sums + tiles);
+			scan_tiles<false, kNonzero><<<(unsigned)tiles, kScanThreads, 0, stream>>>(vals, out, n,
+					sums, sums + tiles);
 		}
 	}
 	LG_CUDA(cudaGetLastError(), "scan launch");
@@ -444,12 +454,17 @@ static lg_status exclusive_scan(const In& in, const uint32_t* arr, uint32_t* cnt
 
 lg_status exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint64_t n,
 		DevBuf& tmp, cudaStream_t stream, uint64_t* total) {
-	return exclusive_scan(ScanArray{in}, in, nullptr, out, n, tmp, stream, total);
+	return exclusive_scan<false>(ScanArray{in}, in, nullptr, out, n, tmp, stream, total);
+}
+
+lg_status exclusive_scan_nonzero(const uint32_t* in, uint32_t* out, uint64_t n, DevBuf& tmp,
+		cudaStream_t stream, uint64_t* total) {
+	return exclusive_scan<true>(ScanNonzero{in}, in, nullptr, out, n, tmp, stream, total);
 }
 
 lg_status exclusive_scan_slots(const SnapCsr& g, const uint32_t* list, uint64_t n, uint32_t* cnt,
 		uint32_t* out, DevBuf& tmp, cudaStream_t stream, uint64_t* total) {
-	return exclusive_scan(ScanSlots{g, list}, nullptr, cnt, out, n, tmp, stream, total);
+	return exclusive_scan<false>(ScanSlots{g, list}, cnt, cnt, out, n, tmp, stream, total);
 }
 
 // ---------------------------------------------------------------------------
@@ -635,21 +650,40 @@ struct VtTab {
 // fragment of a level below minL, as iter_begin / iter_descend end it under
 // LL_MIN_LEVEL (ll_mlcsr_sp.h:2021-2026, 2107-2110); vertex tables of levels
 // below minL are never read.
+//
+// The filling walk also writes every fragment's first virtual slot and vertex,
+// and the fragment that holds the first slot of each kSlotTile-slot tile.
+struct FragOut {
+	const uint32_t* frag_off;
+	const uint32_t* slot_off;
+	uint2* frags;
+	uint32_t* start;
+	uint32_t* vert;
+	uint32_t* tile_frag;
+};
 template <bool kFill>
 __global__ void walk_fragments(VtTab tab, int L, int minL, uint64_t V, uint32_t* count,
-		uint32_t* deg, uint32_t* slots_per_vertex, const uint32_t* frag_off,
-		uint2* frags) {
+		uint32_t* deg, uint32_t* slots_per_vertex, FragOut fo) {
 	uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
 	if (v >= V) return;
 	lg_vt_entry e = tab.vt[L][v];
 	if (!kFill) deg[v] = e.degree;
 	uint32_t n = 0, slots = 0;
-	uint32_t out = kFill ? frag_off[v] : 0;
+	const uint32_t out = kFill ? fo.frag_off[v] : 0;
+	const uint32_t at = kFill ? fo.slot_off[v] : 0;
 	while (e.adj_list_start != LG_NIL_EDGE && e.level_length != 0) {
 		uint32_t lv = LG_EDGE_LEVEL(e.adj_list_start);
 		if ((int)lv < minL) break;
 		uint32_t ix = (uint32_t)LG_EDGE_INDEX(e.adj_list_start);
-		if (kFill) frags[out + n] = make_uint2(ix, (e.level_length << kLevelBits) | lv);
+		if (kFill) {
+			fo.frags[out + n] = make_uint2(ix, (e.level_length << kLevelBits) | lv);
+			fo.start[out + n] = at + slots;
+			fo.vert[out + n] = (uint32_t)v;
+			const uint32_t end = (at + slots + e.level_length - 1u) / kSlotTile;
+			for (uint32_t t = (uint32_t)(((uint64_t)at + slots + kSlotTile - 1u) / kSlotTile);
+					t <= end; t++)
+				fo.tile_frag[t] = out + n;
+		}
 		n++;
 		slots += e.level_length;
 		if ((int)lv <= minL || v >= tab.max_nodes[lv - 1]) break;
@@ -729,18 +763,29 @@ static lg_status open_dir(lg_snapshot* sn, DevCsr& csr, SnapDir& d) {
 	LG_TRY(d.frag_off.reserve((V + 1) * sizeof(uint32_t)));
 	const unsigned B = 256;
 	walk_fragments<false><<<grid_for(V, B), B, 0, st>>>(tab, L, minL, V,
-			cnt.as<uint32_t>(), d.deg.as<uint32_t>(), slots.as<uint32_t>(),
-			nullptr, nullptr);
+			cnt.as<uint32_t>(), d.deg.as<uint32_t>(), slots.as<uint32_t>(), FragOut{});
 	LG_CUDA(cudaGetLastError(), "walk_fragments");
-	s->launches += 2 + scan_launches(V);
-	uint64_t F = 0;
+	s->launches += 2 + 2 * scan_launches(V);
+	// fragment prefix, and the per-vertex slot prefix (the virtual slot space
+	// the balanced kernels cut into ranges)
+	uint64_t F = 0, total_slots = 0;
+	LG_TRY(d.slot_off.reserve((V + 1) * sizeof(uint32_t)));
 	LG_TRY(exclusive_scan_u32(cnt.as<uint32_t>(), d.frag_off.as<uint32_t>(), V,
 			scan_tmp, st, &F));
+	LG_TRY(exclusive_scan_u32(slots.as<uint32_t>(), d.slot_off.as<uint32_t>(), V,
+			scan_tmp, st, &total_slots));
 	d.n_frags = F;
 	LG_TRY(d.frags.reserve(std::max<uint64_t>(F, 1) * sizeof(uint2)));
-	walk_fragments<true><<<grid_for(V, B), B, 0, st>>>(tab, L, minL, V, nullptr,
-			nullptr, nullptr, d.frag_off.as<uint32_t>(), d.frags.as<uint2>());
+	LG_TRY(d.frag_start.reserve((F + 1) * sizeof(uint32_t)));
+	LG_TRY(d.frag_vert.reserve(std::max<uint64_t>(F, 1) * sizeof(uint32_t)));
+	LG_TRY(d.tile_frag.reserve((total_slots / kSlotTile + 1) * sizeof(uint32_t)));
+	walk_fragments<true><<<grid_for(V, B), B, 0, st>>>(tab, L, minL, V, nullptr, nullptr, nullptr,
+			FragOut{d.frag_off.as<uint32_t>(), d.slot_off.as<uint32_t>(), d.frags.as<uint2>(),
+				d.frag_start.as<uint32_t>(), d.frag_vert.as<uint32_t>(),
+				d.tile_frag.as<uint32_t>()});
 	LG_CUDA(cudaGetLastError(), "walk_fragments fill");
+	LG_CUDA(cudaMemcpyAsync(d.frag_start.as<uint32_t>() + F, d.slot_off.as<uint32_t>() + V,
+			sizeof(uint32_t), cudaMemcpyDeviceToDevice, st), "slot total");
 
 	// deletion bitsets of levels minL..L
 	std::vector<uint64_t> word_off(L + 2, 0);
@@ -793,12 +838,6 @@ static lg_status open_dir(lg_snapshot* sn, DevCsr& csr, SnapDir& d) {
 		s->launches++;
 	}
 
-	// per-vertex slot prefix (the virtual slot space the balanced kernels cut
-	// into ranges) and the live edge count
-	uint64_t total_slots = 0;
-	LG_TRY(d.slot_off.reserve((V + 1) * sizeof(uint32_t)));
-	LG_TRY(exclusive_scan_u32(slots.as<uint32_t>(), d.slot_off.as<uint32_t>(), V,
-			scan_tmp, st, &total_slots));
 	{
 		const uint64_t nb = std::max<uint64_t>(1, (total_slots + kBlockSlots - 1) / kBlockSlots);
 		LG_TRY(d.range_lb.reserve((nb + 1) * sizeof(uint32_t)));
@@ -809,7 +848,7 @@ static lg_status open_dir(lg_snapshot* sn, DevCsr& csr, SnapDir& d) {
 	}
 	sum_u32<<<592, B, 0, st>>>(d.deg.as<uint32_t>(), V, counters.as<unsigned long long>());
 	LG_CUDA(cudaGetLastError(), "degree sum");
-	s->launches += 1 + scan_launches(V);
+	s->launches++;
 	unsigned long long sums[2] = {0, 0};
 	LG_CUDA(cudaMemcpyAsync(sums, counters.p, sizeof(sums), cudaMemcpyDeviceToHost, st), "d2h");
 	LG_CUDA(cudaStreamSynchronize(st), "snapshot sizes");
@@ -837,6 +876,13 @@ __global__ void live_counts(SnapCsr g, uint32_t* out) {
 			c += !slot_deleted(g.lt, lv, fr.x + k);
 	}
 	out[v] = c;
+}
+
+lg_status live_degrees(const lg_snapshot* sn, int dir, uint32_t* out) {
+	live_counts<<<grid_for(sn->V, 256), 256, 0, sn->store->stream>>>(sn->view(dir), out);
+	LG_CUDA(cudaGetLastError(), "live_counts");
+	sn->store->launches++;
+	return LG_OK;
 }
 
 __global__ void write_adjacency(SnapCsr g, const uint32_t* off32,

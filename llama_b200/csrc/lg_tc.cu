@@ -465,7 +465,7 @@ extern "C" lg_status lg_triangle_count(lg_snapshot* sn, lg_tc_result* result) {
 	const FlatCsr* f = sn->flat[0];
 	if (!f) {
 		if (!s->flat_scratch) s->flat_scratch = new FlatCsr;
-		LG_TRY(build_flat(sn, 0, *s->flat_scratch, false, false));
+		LG_TRY(build_flat(sn, 0, *s->flat_scratch, false, false, false));
 		f = s->flat_scratch;
 	}
 	const uint64_t E = f->E;
