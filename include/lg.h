@@ -550,7 +550,8 @@ lg_status lg_adjoint_free(lg_adjoint* tape);
 /* Personalized PageRank: the most in-edges per warp range (rounded down to a
  * multiple of 32; smaller graphs take fewer), default 2048. */
 #define LG_TUNE_PPR_RANGE       2
-/* Delta-stepping SSSP: queue slots per warp range, default 1024. */
+/* Delta-stepping SSSP: queue slots per warp range, default 1024; a sixteenth of
+ * it is the longest row (or piece of one) a warp of the one-launch form takes. */
 #define LG_TUNE_SSSP_RANGE      3
 /* Multi-source BFS and batched BC bottom-up steps: in-degree above which a
  * warp, not a thread, scans a vertex's in-edges, default 512. */
@@ -563,20 +564,21 @@ lg_status lg_adjoint_free(lg_adjoint* tape);
  * (weight < delta) of the near queue and the vertices settled in the bucket
  * relax their heavy edges once when it drains, over a copy of the snapshot's
  * out-CSR split per row (built on the first call for a delta, 8 bytes per
- * live edge, kept with the snapshot); 0 = every round relaxes every edge of
- * the near queue.  Default 0 (measured faster on the R-MAT workloads). */
+ * live edge, kept with the snapshot); 0 (default) = no such copy.  With this
+ * and LG_TUNE_SSSP_LEVELS 0 every step runs in one cooperative launch over the
+ * flat out-CSR (the snapshot's own, or one made for the call), which relaxes
+ * light edges only where a bucket's later rounds are long. */
 #define LG_TUNE_SSSP_SPLIT      6
 /* One-root BFS (lg_bfs) with the snapshot's in-CSR flat (or no in-CSR):
  * 1 = every level in one cooperative launch whose CTAs choose the direction
  * on the device and meet at grid barriers; 0 = a launch sequence per level
  * with the direction chosen on the host.  Default 1. */
 #define LG_TUNE_BFS_LEVELS      7
-/* Delta-stepping SSSP: 1 = all rounds, bucket splits and heavy phases in one
- * cooperative launch whose CTAs apply the host loop's rules on the device
- * and meet at bounded grid barriers; 0 = a launch sequence per step with the
- * host reading the counters back.  Default 0: on the R-MAT workloads the one
- * launch gains 3-8 % with LG_TUNE_SSSP_SPLIT and loses 8 % without (its
- * relaxation loop holds fewer warps per SM than the per-step kernel). */
+/* Delta-stepping SSSP, with the light/heavy split or over the levels: 1 = all
+ * rounds, bucket splits and heavy phases in one cooperative launch whose CTAs
+ * apply the host loop's rules on the device and meet at bounded grid barriers;
+ * 0 (default) = a launch sequence per step with the host reading the counters
+ * back. */
 #define LG_TUNE_SSSP_LEVELS     8
 #define LG_TUNE_COUNT           9
 #define LG_TUNE_MAX_DEVICES     64

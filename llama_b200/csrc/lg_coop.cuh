@@ -107,13 +107,14 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t x, uint32_t* t
 	return before + inc - x;
 }
 
-// Co-resident CTAs of `kernel` at `threads` per CTA on `device` (SMs x CTAs
-// per SM), 0 when the device has no cooperative launch.
-inline int coop_grid_size(const void* kernel, int threads, int device) {
+// Co-resident CTAs of `kernel` at `threads` and `smem` bytes of dynamic shared
+// memory per CTA on `device` (SMs x CTAs per SM), 0 when the device has no
+// cooperative launch.
+inline int coop_grid_size(const void* kernel, int threads, int device, size_t smem = 0) {
 	int coop = 0, sms = 0, per_sm = 0;
 	if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess ||
 			cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
-			cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) !=
+			cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) !=
 					cudaSuccess) {
 		cudaGetLastError();
 		return 0;

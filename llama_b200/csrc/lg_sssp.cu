@@ -18,6 +18,7 @@
 #include "lg_expand.cuh"
 #include "lg_flat.cuh"
 #include "lg_sssp.cuh"
+#include "lg_sssp_flat.h"
 #include "lg_sssp_levels.h"
 #include "lg_tune.h"
 
@@ -260,6 +261,31 @@ extern "C" lg_status lg_sssp_delta(lg_snapshot* sn, int64_t root, uint32_t delta
 	cudaStream_t st = s->stream;
 	const uint64_t V = sn->V;
 	DevBuf* sc = s->scratch;
+	const bool dev_out = is_device_pointer(dist);
+	uint32_t* d = dist;
+	if (!dev_out) { LG_TRY(sc[4].reserve(V * 4)); d = sc[4].as<uint32_t>(); }
+	// every step in one launch over the flat out-CSR, the snapshot's own or
+	// one made for the call, unless a tunable asks for another form
+	const FlatCsr* fo = sn->flat[0];
+	if (!tune_value(s->device, LG_TUNE_SSSP_SPLIT) && !tune_value(s->device, LG_TUNE_SSSP_LEVELS)) {
+		const FlatCsr* f = fo && fo->weighted ? fo : nullptr;
+		if (!f) {
+			if (!s->flat_scratch) s->flat_scratch = new FlatCsr;
+			const lg_status fs = build_flat(sn, 0, *s->flat_scratch, false, true, false);
+			if (fs == LG_OK && s->flat_scratch->weighted) f = s->flat_scratch;
+			else if (fs != LG_OK && fs != LG_ENOMEM && fs != LG_ENOTSUP) return fs;
+			else clear_error();            // the levels are read instead
+		}
+		bool ran = false;
+		if (f) LG_TRY(sssp_flat_run(sn, f, (uint32_t)root, delta, d, result, &ran));
+		if (ran) {
+			if (!dev_out) {
+				LG_TRY(copy_out(s, dist, d, V * 4));
+				LG_CUDA(cudaStreamSynchronize(st), "sssp");
+			}
+			return LG_OK;
+		}
+	}
 	LG_TRY(sc[0].reserve(V * 4));          // near queue
 	LG_TRY(sc[1].reserve(V * 4));          // next near queue
 	LG_TRY(sc[2].reserve(V * 4));          // far pile
@@ -273,9 +299,6 @@ extern "C" lg_status lg_sssp_delta(lg_snapshot* sn, int64_t root, uint32_t delta
 	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
 	const unsigned relax_blocks = (unsigned)sms * kRelaxCtasPerSm;   // persistent, one wave
 	const uint32_t range = (uint32_t)tune_value(s->device, LG_TUNE_SSSP_RANGE);
-	const bool dev_out = is_device_pointer(dist);
-	uint32_t* d = dist;
-	if (!dev_out) { LG_TRY(sc[4].reserve(V * 4)); d = sc[4].as<uint32_t>(); }
 	uint32_t* q = sc[0].as<uint32_t>();
 	uint32_t* qn = sc[1].as<uint32_t>();
 	uint32_t* far = sc[2].as<uint32_t>();
@@ -284,7 +307,6 @@ extern "C" lg_status lg_sssp_delta(lg_snapshot* sn, int64_t root, uint32_t delta
 	uint32_t* fstamp = stamp + V;
 	unsigned long long* ctr = sc[6].as<unsigned long long>();
 	// the one-fragment view of a flattened out-CSR when there is one
-	const FlatCsr* fo = sn->flat[0];
 	SnapCsr out = (fo && fo->has_view && fo->weighted)
 			? fo->view(sn->out.deg.as<uint32_t>()) : sn->view(0);
 	// light / heavy split (LG_TUNE_SSSP_SPLIT): rounds walk the light view,
