@@ -329,10 +329,12 @@ lg_status lg_pagerank_pull(lg_snapshot* snap, int iterations, double damping,
  * Every vertex t with out-degree > 0 adds pr[t] / out_degree(t) to each
  * out-neighbour's next value (an atomic add, as in the reference), then
  * pr'[t] = (1-d)/N + d * next[t].  Reads only the out-CSR, so it also runs on
- * stores kept without reverse edges.  The summation order follows the atomic
- * schedule: results agree with lg_pagerank_pull within FP64 rounding, not bit
- * for bit.  Uses the flat out-CSR after lg_snapshot_flatten(snap, 0).
- * ranks: double[max_nodes]. */
+ * stores kept without reverse edges.  No order of a vertex's terms is
+ * promised: results agree with lg_pagerank_pull within FP64 rounding, not bit
+ * for bit.  Where the iterations are worth it, the live out-edges are
+ * transposed for the call (some 24 bytes per edge while it runs; without that
+ * memory every iteration adds along the out-edges).  Uses the flat out-CSR
+ * after lg_snapshot_flatten(snap, 0).  ranks: double[max_nodes]. */
 lg_status lg_pagerank_push(lg_snapshot* snap, int iterations, double damping,
 		double* ranks);
 

@@ -19,6 +19,7 @@
 // per 1024-slot block in shared memory behind a dozen block barriers: it was
 // bound by those and by its instructions, 2.1 ms at 262 M slots.
 #include "lg_flat.cuh"
+#include "lg_sort.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -201,6 +202,108 @@ SlotSpace slot_space(const lg_snapshot* sn, int dir) {
 	return sp;
 }
 
+lg_status flat_row_index(lg_store* s, FlatCsr& f, const uint32_t* deg) {
+	cudaStream_t st = s->stream;
+	const uint64_t V = f.V;
+	uint64_t R = 0;
+	LG_TRY(f.kidx.reserve((V + 1) * sizeof(uint32_t)));
+	LG_TRY(exclusive_scan_nonzero(deg, f.kidx.as<uint32_t>(), V, f.scan_tmp, st, &R));
+	f.R = R;
+	const uint64_t head_words = (uint64_t)f.ntiles * kFlatTileWords + 1;
+	LG_TRY(f.rows.reserve((2 * f.rcap() + f.ntiles + head_words) * sizeof(uint32_t)));
+	uint32_t* heads = const_cast<uint32_t*>(f.heads());
+	LG_CUDA(cudaMemsetAsync(heads, 0, head_words * sizeof(uint32_t), st), "clear heads");
+	flat_rows<<<grid_for(V, 256), 256, 0, st>>>(f.off.as<uint32_t>(), f.kidx.as<uint32_t>(), V,
+			const_cast<uint32_t*>(f.nz_rows()), const_cast<uint32_t*>(f.nz_off()), heads, f.ntiles,
+			const_cast<uint32_t*>(f.tile_seg()));
+	LG_CUDA(cudaGetLastError(), "flat_rows");
+	s->launches += scan_launches(V) + 1;
+	return LG_OK;
+}
+
+// ---------------------------------------------------------------------------
+// Transpose: every edge as (target << 32 | row), radix sorted by target
+// (stable, so a row's sources stay in order).
+// ---------------------------------------------------------------------------
+
+// Lane j of the warp owning tile t takes edges 256 t + 8 j .. + 7 of `a`.
+__global__ void __launch_bounds__(kFwThreads)
+flat_edge_keys(const uint32_t* ids, const uint32_t* heads, const uint32_t* nz_rows,
+		const uint32_t* tile_seg, uint32_t E, uint32_t ntiles, unsigned long long* keys) {
+	const uint32_t lane = threadIdx.x & 31u;
+	const uint32_t t = blockIdx.x * kFwWarps + (threadIdx.x >> 5);
+	if (t >= ntiles) return;
+	const uint32_t eb = t * kFlatTile + lane * kFlatPerLane;
+	const uint32_t hb = __ldg(reinterpret_cast<const unsigned char*>(heads)
+			+ (size_t)t * (kFlatTile / 8) + lane);
+	uint32_t before = __popc(hb);               // heads in the lanes to the left
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1) {
+		const uint32_t q = __shfl_up_sync(0xffffffffu, before, o);
+		if (lane >= (uint32_t)o) before += q;
+	}
+	before -= __popc(hb);
+	uint32_t row = __ldg(tile_seg + t) + before - 1u;   // of the lane's first edge, unless a head
+	uint32_t v = eb < E && !(hb & 1u) ? __ldg(nz_rows + row) : 0u;
+#pragma unroll
+	for (int i = 0; i < kFlatPerLane; i++) {
+		if ((hb >> i) & 1u) v = __ldg(nz_rows + ++row);
+		if (eb + i < E)
+			keys[eb + i] = ((unsigned long long)__ldcs(ids + eb + i) << 32) | v;
+	}
+}
+
+// ids = the sorted keys' rows; cnt[t] = keys of target t (formed as end -
+// start of its run, each added where the run begins or ends).
+__global__ void flat_from_keys(const unsigned long long* keys, uint32_t E, uint32_t* ids,
+		uint32_t* cnt) {
+	const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+	if (i >= E) return;
+	const unsigned long long k = keys[i];
+	const uint32_t t = (uint32_t)(k >> 32);
+	ids[i] = (uint32_t)k;
+	const uint32_t p = i > 0 ? (uint32_t)(keys[i - 1] >> 32) : kNoId;
+	if (p != t) {
+		atomicSub(cnt + t, (uint32_t)i);
+		if (i > 0) atomicAdd(cnt + p, (uint32_t)i);
+	}
+	if (i == E - 1u) atomicAdd(cnt + t, E);
+}
+
+lg_status flat_transpose(lg_store* s, const FlatCsr& a, FlatCsr& f) {
+	cudaStream_t st = s->stream;
+	const uint64_t V = a.V, E = a.E;
+	f.V = V;
+	f.E = E;
+	f.ntiles = a.ntiles;
+	f.weighted = f.has_view = f.has_nz_outdeg = false;
+	DevBuf keys(s->pool), tmpk(s->pool), tmpp(s->pool), counts(s->pool), cnt(s->pool);
+	LG_TRY(keys.reserve(std::max<uint64_t>(E, 1) * 8));
+	LG_TRY(cnt.reserve(V * 4));
+	LG_TRY(f.ids.reserve(std::max<uint64_t>(E, 1) * 4));
+	LG_TRY(f.off.reserve((V + 1) * 4));
+	LG_CUDA(cudaMemsetAsync(cnt.p, 0, V * 4, st), "clear counts");
+	if (E > 0) {
+		flat_edge_keys<<<grid_for(a.ntiles, kFwWarps), kFwThreads, 0, st>>>(a.ids.as<uint32_t>(),
+				a.heads(), a.nz_rows(), a.tile_seg(), (uint32_t)E, a.ntiles,
+				keys.as<unsigned long long>());
+		LG_CUDA(cudaGetLastError(), "flat_edge_keys");
+		unsigned long long targets = 1;          // the bits targets < V may differ in
+		while (targets < V) targets <<= 1;
+		unsigned long long* sorted = nullptr;
+		LG_TRY(radix_sort_u64(s, keys.as<unsigned long long>(), nullptr, E, tmpk, tmpp, counts,
+				f.scan_tmp, &sorted, nullptr, ((targets - 1) << 32) | (1ull << 32)));
+		flat_from_keys<<<grid_for(E, 256), 256, 0, st>>>(sorted, (uint32_t)E, f.ids.as<uint32_t>(),
+				cnt.as<uint32_t>());
+		LG_CUDA(cudaGetLastError(), "flat_from_keys");
+		s->launches += 2;
+	}
+	LG_TRY(exclusive_scan_u32(cnt.as<uint32_t>(), f.off.as<uint32_t>(), V, f.scan_tmp, st,
+			nullptr));
+	s->launches += scan_launches(V);
+	return flat_row_index(s, f, cnt.as<uint32_t>());
+}
+
 // build_flat with rows of deg[v] edges, E in all.  *mismatch (and LG_OK, f
 // unfinished): the live slots are not laid out as those degrees say.
 static lg_status build_rows(lg_snapshot* sn, int dir, FlatCsr& f, bool view, bool weights,
@@ -269,23 +372,14 @@ static lg_status build_rows(lg_snapshot* sn, int dir, FlatCsr& f, bool view, boo
 	}
 	unsigned int err = 0;
 	LG_CUDA(cudaMemcpyAsync(&err, f.err.p, sizeof(err), cudaMemcpyDeviceToHost, st), "d2h");
-	uint64_t R = 0;
-	LG_TRY(exclusive_scan_nonzero(deg, f.kidx.as<uint32_t>(), V, f.scan_tmp, st, &R));
-	// (the scan waited for the stream, so err is in)
+	s->launches += scan_launches(V) + (fs.ntiles > 0);
+	LG_TRY(flat_row_index(s, f, deg));
+	// (that waited for the stream, so err is in)
 	if ((err & 2u) || (fs.ntiles == 0 && E > 0)) {
 		*mismatch = true;
 		return LG_OK;
 	}
-	f.R = R;
-	const uint64_t head_words = (uint64_t)f.ntiles * kFlatTileWords + 1;
-	LG_TRY(f.rows.reserve((2 * f.rcap() + f.ntiles + head_words) * sizeof(uint32_t)));
-	uint32_t* heads = const_cast<uint32_t*>(f.heads());
-	LG_CUDA(cudaMemsetAsync(heads, 0, head_words * sizeof(uint32_t), st), "clear heads");
-	flat_rows<<<grid_for(V, B), B, 0, st>>>(off, f.kidx.as<uint32_t>(), V,
-			const_cast<uint32_t*>(f.nz_rows()), const_cast<uint32_t*>(f.nz_off()), heads,
-			f.ntiles, const_cast<uint32_t*>(f.tile_seg()));
-	LG_CUDA(cudaGetLastError(), "flat_rows");
-	s->launches += 2 * scan_launches(V) + 1 + (fs.ntiles > 0);
+	const uint64_t R = f.R;
 	if (!view) return LG_OK;
 
 	LG_TRY(f.vfrags.reserve(f.rcap() * sizeof(uint2)));

@@ -160,6 +160,11 @@ __device__ __forceinline__ bool block_slot(const BlockMap& m, uint32_t ra, uint3
 SlotSpace slot_space(const lg_snapshot* sn, int dir);
 
 struct FlatCsr {
+	FlatCsr() = default;
+	// a CSR that lives for one call, in the store's call pool
+	explicit FlatCsr(const std::shared_ptr<CallPool>& p)
+		: off(p), kidx(p), ids(p), w(p), rows(p), flags(p), scan_tmp(p), err(p), vfrags(p),
+		  vdel(p), vlt(p), nz_outdeg(p) {}
 	uint64_t V = 0, E = 0, R = 0;
 	uint32_t ntiles = 0;
 	bool weighted = false;     // w holds the edge weights
@@ -200,6 +205,19 @@ struct FlatCsr {
 // laid out all the same (for the calls that never read the degrees as sizes).
 lg_status build_flat(lg_snapshot* sn, int dir, FlatCsr& f, bool view, bool weights = true,
 		bool strict = true);
+
+// The row bookkeeping of f (kidx, R, rows) from its row starts f.off and the
+// rows' lengths deg[V]; f.V, f.E and f.ntiles are set.  Waits for the stream.
+lg_status flat_row_index(lg_store* s, FlatCsr& f, const uint32_t* deg);
+
+// f = the transpose of flat CSR `a` (row t: the rows of `a` that hold t, in
+// order): ids, off and the row bookkeeping, no weights, no view.
+lg_status flat_transpose(lg_store* s, const FlatCsr& a, FlatCsr& f);
+
+// PageRank of sn over f, its flat in-CSR (lg_pagerank_pull's iterations and
+// output; lg_pagerank.cu).
+lg_status pagerank_over(lg_snapshot* sn, FlatCsr* f, int iterations, double damping,
+		double* ranks);
 
 } // namespace lg
 

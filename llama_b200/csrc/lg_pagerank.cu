@@ -263,30 +263,19 @@ static lg_status check_args(lg_snapshot* sn, int iterations, double damping, dou
 
 using namespace lg;
 
-extern "C" lg_status lg_pagerank_pull(lg_snapshot* sn, int iterations,
-		double damping, double* ranks) {
-	clear_error();
-	LG_TRY(check_args(sn, iterations, damping, ranks));
+namespace lg {
+
+lg_status pagerank_over(lg_snapshot* sn, FlatCsr* f, int iterations, double damping,
+		double* ranks) {
 	lg_store* s = sn->store;
-	LG_CUDA(cudaSetDevice(s->device), "cudaSetDevice");
 	cudaStream_t st = s->stream;
 	const uint64_t V = sn->V;
-	if (V == 0) return LG_OK;
 	const double N = (double)V;
 	const double pr0 = 1.0 / N;
 	const double base = (1.0 - damping) / N;
 	const unsigned B = 256;
 	DevBuf* sc = s->scratch;
 	const uint32_t* outdeg = sn->out.deg.as<uint32_t>();
-
-	// flat in-adjacency: the snapshot's own (lg_snapshot_flatten) or one
-	// built for this call in store scratch
-	FlatCsr* f = sn->flat[1];
-	if (!f) {
-		if (!s->flat_scratch) s->flat_scratch = new FlatCsr;
-		LG_TRY(build_flat(sn, 1, *s->flat_scratch, false));
-		f = s->flat_scratch;
-	}
 	if (!f->has_nz_outdeg) {
 		LG_TRY(f->nz_outdeg.reserve(f->rcap() * sizeof(uint32_t)));
 		if (f->R > 0) {
@@ -355,6 +344,26 @@ extern "C" lg_status lg_pagerank_pull(lg_snapshot* sn, int iterations,
 		LG_CUDA(cudaStreamSynchronize(st), "pagerank");
 	}
 	return LG_OK;
+}
+
+} // namespace lg
+
+extern "C" lg_status lg_pagerank_pull(lg_snapshot* sn, int iterations,
+		double damping, double* ranks) {
+	clear_error();
+	LG_TRY(check_args(sn, iterations, damping, ranks));
+	lg_store* s = sn->store;
+	LG_CUDA(cudaSetDevice(s->device), "cudaSetDevice");
+	if (sn->V == 0) return LG_OK;
+	// flat in-adjacency: the snapshot's own (lg_snapshot_flatten) or one
+	// built for this call in store scratch
+	FlatCsr* f = sn->flat[1];
+	if (!f) {
+		if (!s->flat_scratch) s->flat_scratch = new FlatCsr;
+		LG_TRY(build_flat(sn, 1, *s->flat_scratch, false));
+		f = s->flat_scratch;
+	}
+	return pagerank_over(sn, f, iterations, damping, ranks);
 }
 
 // ---------------------------------------------------------------------------
