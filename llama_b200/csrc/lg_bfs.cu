@@ -9,15 +9,11 @@
 // frontier queue over the out-CSR in balanced slot ranges, bottom-up steps let every
 // unvisited vertex look for a parent among its in-neighbours (in-CSR) in a
 // frontier bitmap that stays resident in L2.
+#include "lg_bfs_levels.h"
 #include "lg_expand.cuh"
 #include "lg_flat.cuh"
 
 namespace lg {
-
-// lg_bfs_levels.cu: the whole BFS in one cooperative launch; *ran = false
-// when it does not apply to the snapshot (nothing launched).
-lg_status bfs_levels_run(lg_snapshot* sn, uint32_t root, int32_t* lvl, lg_bfs_result* result,
-		bool* ran);
 
 constexpr int32_t kUnreached = LG_UNREACHED;
 constexpr int kBfsThreads = 256;

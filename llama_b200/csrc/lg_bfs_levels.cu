@@ -39,6 +39,7 @@
 // read-only path.  Every barrier wait is bounded (lg_coop.cuh: kCoopWaitNs of the global
 // timer); a CTA that gives up sets an error flag, leaves, and the host
 // reports LG_ETIMEOUT.
+#include "lg_bfs_levels.h"
 #include "lg_coop.cuh"
 #include "lg_expand.cuh"
 #include "lg_flat.cuh"
@@ -168,7 +169,14 @@ bfs_levels(SnapCsr out, const uint32_t* nz_rows, const uint32_t* nz_off, uint32_
 		uint32_t* bits = bm(cur % 3);
 		uint32_t* nbits = bm((cur + 1) % 3);
 		uint32_t* clear = bm((cur + 2) % 3);
-		const unsigned long long qlen = __ldcg(now + 0), mf = __ldcg(now + 1);
+		// one warp per CTA reads the counters (read by every thread of the grid,
+		// their sector took some 3 us a level)
+		__shared__ unsigned long long s_ctr[4];
+		__syncthreads();                         // s_ctr free from the last level
+		if (tid < 4) s_ctr[tid] = __ldcg(now + tid);
+		__syncthreads();
+		const unsigned long long qlen = s_ctr[0], mf = s_ctr[1];
+		if (!have_queue) list_len = (long long)s_ctr[3];
 		if (qlen == 0) break;
 		reached += qlen;
 		reach_edges += mf;
@@ -402,8 +410,7 @@ bfs_levels(SnapCsr out, const uint32_t* nz_rows, const uint32_t* nz_off, uint32_
 			have_queue = true;
 			list_len = -1;                 // fcnt / fpos were overwritten
 		} else {
-			have_queue = false;
-			list_len = (long long)__ldcg(nxt + 3);
+			have_queue = false;            // list_len: read with the next level's counters
 			list_in_fcnt = !list_in_fcnt;
 		}
 	}
@@ -429,10 +436,6 @@ int coop_grid(int device) {
 
 } // namespace
 
-// One cooperative launch for the whole BFS from `root` into device array lvl
-// (lg_bfs's contract).  *ran = false, and nothing is launched, when the
-// snapshot's in-CSR is kept but not flat, LG_TUNE_BFS_LEVELS is 0, or the
-// device has no cooperative launch; the caller then runs its per-level loop.
 lg_status bfs_levels_run(lg_snapshot* sn, uint32_t root, int32_t* lvl, lg_bfs_result* result,
 		bool* ran) {
 	*ran = false;
@@ -440,10 +443,19 @@ lg_status bfs_levels_run(lg_snapshot* sn, uint32_t root, int32_t* lvl, lg_bfs_re
 	const FlatCsr* fi = sn->flat[1];
 	if (sn->in.present && !fi) return LG_OK;
 	if (!tune_value(s->device, LG_TUNE_BFS_LEVELS)) return LG_OK;
+	const FlatCsr* fo = sn->flat[0];
+	const uint32_t* outdeg = sn->out.deg.as<uint32_t>();
+	const SnapCsr out = (fo && fo->has_view) ? fo->view(outdeg) : sn->view(0);
+	return bfs_levels_over(s, out, fi, outdeg, sn->out.n_edges, root, lvl, result, ran);
+}
+
+lg_status bfs_levels_over(lg_store* s, SnapCsr out, const FlatCsr* fi, const uint32_t* outdeg,
+		uint64_t n_edges, uint32_t root, int32_t* lvl, lg_bfs_result* result, bool* ran) {
+	*ran = false;
 	const int grid = coop_grid(s->device);
 	if (grid <= 0) return LG_OK;
 	cudaStream_t st = s->stream;
-	const uint64_t V = sn->V;
+	const uint64_t V = out.V;
 	const uint64_t W = (V + 31) / 32;
 	DevBuf* sc = s->scratch;
 	LG_TRY(sc[0].reserve(V * 4));
@@ -454,16 +466,13 @@ lg_status bfs_levels_run(lg_snapshot* sn, uint32_t root, int32_t* lvl, lg_bfs_re
 	LG_TRY(sc[5].reserve(V * 4));
 	LG_TRY(sc[6].reserve((V + 1) * 4));
 	LG_TRY(sc[9].reserve(sizeof(LvCtl) + (size_t)grid * sizeof(unsigned long long)));
-	const FlatCsr* fo = sn->flat[0];
-	SnapCsr out = (fo && fo->has_view) ? fo->view(sn->out.deg.as<uint32_t>()) : sn->view(0);
 	const uint32_t* nz_rows = fi ? fi->nz_rows() : nullptr;
 	const uint32_t* nz_off = fi ? fi->nz_off() : nullptr;
 	uint32_t R = fi ? (uint32_t)fi->R : 0u, E = fi ? (uint32_t)fi->E : 0u;
 	const uint32_t* in_ids = fi ? fi->ids.as<uint32_t>() : nullptr;
-	const uint32_t* outdeg = sn->out.deg.as<uint32_t>();
 	uint32_t V32 = (uint32_t)V;
-	unsigned long long out_edges = sn->out.n_edges;
-	int has_in = sn->in.present ? 1 : 0;
+	unsigned long long out_edges = n_edges;
+	int has_in = fi ? 1 : 0;
 	uint32_t* q0 = sc[0].as<uint32_t>();
 	uint32_t* q1 = sc[1].as<uint32_t>();
 	uint32_t* bits0 = sc[2].as<uint32_t>();
