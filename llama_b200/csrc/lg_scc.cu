@@ -15,10 +15,14 @@
 //      colour, collects exactly that component, labelled with the colour;
 //   3. collected vertices leave the remaining set and 1-2 repeat.
 // Each round removes at least the component of the smallest remaining
-// vertex, and labels do not depend on thread order.
+// vertex, and labels do not depend on thread order.  That is done over flat CSRs
+// after the largest component was found by two searches (lg_scc_flat.cu); the
+// kernels here do it over the levels' fragments where there is no memory for
+// the flat ones.
 #include "lg_device.cuh"
 #include "lg_expand.cuh"
 #include "lg_queue.cuh"
+#include "lg_scc_flat.h"
 
 namespace lg {
 
@@ -177,26 +181,19 @@ lg_status read_ctr(lg_store* s, unsigned long long* ctr, uint64_t* v) {
 	return LG_OK;
 }
 
-} // namespace
-
-extern "C" lg_status lg_scc(lg_snapshot* sn, int64_t* labels, lg_scc_result* result) {
-	clear_error();
-	if (!sn || !labels) return set_error(LG_EINVAL, "null argument");
-	if (!sn->in.present) return set_error(LG_ESTATE, "SCC needs the in-CSR (reverse edges)");
+// Colouring over the levels' fragments, the host reading each step's counts:
+// where there is no memory for flat CSRs, or no cooperative launch.
+lg_status scc_by_colour(lg_snapshot* sn, uint32_t* lab, unsigned long long* ctr,
+		uint64_t* trimmed, uint32_t* rounds_out, int* steps_out) {
 	lg_store* s = sn->store;
-	LG_CUDA(cudaSetDevice(s->device), "cudaSetDevice");
 	cudaStream_t st = s->stream;
 	const uint64_t V = sn->V;
-	DevBuf label(s->pool), color(s->pool), mark(s->pool), stamp(s->pool), rem(s->pool),
-			rem2(s->pool), wl(s->pool), wl2(s->pool), cnt(s->pool), pos(s->pool),
-			scan_tmp(s->pool), ctrb(s->pool), outb(s->pool);
-	for (DevBuf* b : {&label, &color, &mark, &stamp, &rem, &rem2, &wl, &wl2, &cnt})
+	DevBuf color(s->pool), mark(s->pool), stamp(s->pool), rem(s->pool), rem2(s->pool),
+			wl(s->pool), wl2(s->pool), cnt(s->pool), pos(s->pool), scan_tmp(s->pool);
+	for (DevBuf* b : {&color, &mark, &stamp, &rem, &rem2, &wl, &wl2, &cnt})
 		LG_TRY(b->reserve(V * 4));
 	LG_TRY(pos.reserve((V + 1) * 4));
-	LG_TRY(ctrb.reserve(2 * sizeof(unsigned long long)));
-	unsigned long long* ctr = ctrb.as<unsigned long long>();
 	const SnapCsr out = sn->view(0), in = sn->view(1);
-	uint32_t* lab = label.as<uint32_t>();
 	uint32_t* col = color.as<uint32_t>();
 	uint32_t* mk = mark.as<uint32_t>();
 	uint32_t* stp = stamp.as<uint32_t>();
@@ -208,7 +205,7 @@ extern "C" lg_status lg_scc(lg_snapshot* sn, int64_t* labels, lg_scc_result* res
 	s->launches++;
 	uint64_t n_rem = 0;
 	LG_TRY(read_ctr(s, ctr, &n_rem));
-	const uint64_t trimmed = V - n_rem;
+	*trimmed = V - n_rem;
 	uint32_t round = 0, prop_round = 0;
 	int steps = 0;
 	uint32_t* R = rem.as<uint32_t>();
@@ -264,6 +261,58 @@ extern "C" lg_status lg_scc(lg_snapshot* sn, int64_t* labels, lg_scc_result* res
 		n_rem = left;
 		std::swap(R, R2);
 	}
+	*rounds_out = round;
+	*steps_out = steps;
+	return LG_OK;
+}
+
+// Over the snapshot's flat CSRs, or ones made for the call; *ran = false where
+// there is no memory for them or no cooperative launch.
+lg_status scc_over_flat(lg_snapshot* sn, uint32_t* lab, uint64_t* trimmed, uint32_t* rounds,
+		int* steps, bool* ran) {
+	lg_store* s = sn->store;
+	*ran = false;
+	FlatCsr made_out(s->pool), made_in(s->pool);
+	const FlatCsr *fo = sn->flat[0], *fi = sn->flat[1];
+	lg_status st = LG_OK;
+	if (!fo) {
+		st = build_flat(sn, 0, made_out, false, false, false);
+		fo = &made_out;
+	}
+	if (st == LG_OK && !fi) {
+		st = build_flat(sn, 1, made_in, false, false, false);
+		fi = &made_in;
+	}
+	if (st == LG_OK) st = scc_flat_run(sn, fo, fi, lab, trimmed, rounds, steps, ran);
+	if (st == LG_ENOMEM || st == LG_ENOTSUP) {
+		clear_error();
+		*ran = false;
+		return LG_OK;
+	}
+	return st;
+}
+
+} // namespace
+
+extern "C" lg_status lg_scc(lg_snapshot* sn, int64_t* labels, lg_scc_result* result) {
+	clear_error();
+	if (!sn || !labels) return set_error(LG_EINVAL, "null argument");
+	if (!sn->in.present) return set_error(LG_ESTATE, "SCC needs the in-CSR (reverse edges)");
+	lg_store* s = sn->store;
+	LG_CUDA(cudaSetDevice(s->device), "cudaSetDevice");
+	cudaStream_t st = s->stream;
+	const uint64_t V = sn->V;
+	DevBuf label(s->pool), ctrb(s->pool), outb(s->pool);
+	LG_TRY(label.reserve(V * 4));
+	LG_TRY(ctrb.reserve(2 * sizeof(unsigned long long)));
+	unsigned long long* ctr = ctrb.as<unsigned long long>();
+	uint32_t* lab = label.as<uint32_t>();
+	uint64_t trimmed = 0;
+	uint32_t round = 0;
+	int steps = 0;
+	bool ran = false;
+	LG_TRY(scc_over_flat(sn, lab, &trimmed, &round, &steps, &ran));
+	if (!ran) LG_TRY(scc_by_colour(sn, lab, ctr, &trimmed, &round, &steps));
 	const bool dev_out = is_device_pointer(labels);
 	long long* o = (long long*)labels;
 	if (!dev_out) { LG_TRY(outb.reserve(V * 8)); o = outb.as<long long>(); }
