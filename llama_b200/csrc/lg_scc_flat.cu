@@ -23,6 +23,7 @@
 #include "lg_scc_flat.h"
 #include "lg_tune.h"
 
+#include <cstddef>
 #include <mutex>
 
 namespace lg {
@@ -434,7 +435,7 @@ lg_status scc_flat_run(lg_snapshot* sn, const FlatCsr* fo, const FlatCsr* fi, ui
 			dim3(kSrThreads), kargs, 0, st), "scc_rest");
 	s->launches += 3;
 	u64 o[6];
-	static_assert(sizeof(CoopBar) == 16, "two words after the results");
+	static_assert(offsetof(SrCtl, bar) == offsetof(SrCtl, out) + 32, "two words after the results");
 	LG_TRY(read_words(s, ctl->out, 6, o));
 	const unsigned err = (unsigned)o[5];               // the barrier's error word
 	if (err & 1u) return set_error(LG_ETIMEOUT, "scc: a grid barrier wait ran out");

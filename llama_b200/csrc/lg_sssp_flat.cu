@@ -45,6 +45,7 @@
 #include "lg_tune.h"
 
 #include <algorithm>
+#include <cstddef>
 #include <mutex>
 
 namespace lg {
@@ -552,7 +553,7 @@ lg_status sssp_flat_run(lg_snapshot* sn, const FlatCsr* f, uint32_t root, uint32
 			dim3(kSfThreads), kargs, sizeof(SfShared), st), "sssp_flat");
 	s->launches++;
 	unsigned long long h[8];
-	static_assert(sizeof(CoopBar) == 16, "two words after the results");
+	static_assert(offsetof(SfCtl, bar) == offsetof(SfCtl, out) + 48, "two words after the results");
 	LG_TRY(read_words(s, ctl->out, 8, h));
 	const unsigned int err = (unsigned int)h[7];      // the barrier's error word
 	if (err & 1u) return set_error(LG_ETIMEOUT, "sssp: a grid barrier wait ran out");
