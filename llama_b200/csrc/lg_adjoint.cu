@@ -28,10 +28,14 @@
 // nothing once it is below tol, and the host reads the residuals of a chunk
 // while the next one runs.  The result is the one the stop-at-first-
 // residual-below-tol loop gives, with no synchronisation per iteration.
+#include "lg_flat_run.cuh"
 #include "lg_flat_sweep.cuh"
 #include "lg_tune.h"
 
 #include <cmath>
+#include <cstddef>
+#include <cstring>
+#include <mutex>
 
 namespace lg {
 
@@ -111,6 +115,105 @@ __global__ void aff_empty_rows(const uint32_t* off, uint64_t V, const double* ba
 #pragma unroll
 	for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
 	if ((threadIdx.x & 31u) == 0 && r != 0.0) atomicAdd(resid0, r);
+}
+
+// The same iterations inside one cooperative launch (lg_flat_run.cuh).
+struct AffRunOp {
+	static constexpr bool kResidual = true;
+	const uint32_t* nz_rows;
+	const double* w;
+	const double* base;
+	const double* x;           // rewritten between iterations: plain loads
+	double* y;
+	double d;
+	uint32_t E;
+	__device__ __forceinline__ void values(uint32_t eb, const uint32_t (&id)[kFlatPerLane],
+			double (&v)[kFlatPerLane]) const {
+		double wv[kFlatPerLane];
+		if (eb + kFlatPerLane <= E) {
+			asm("ld.global.cs.v4.f64 {%0, %1, %2, %3}, [%4];"
+				: "=d"(wv[0]), "=d"(wv[1]), "=d"(wv[2]), "=d"(wv[3]) : "l"(w + eb));
+			asm("ld.global.cs.v4.f64 {%0, %1, %2, %3}, [%4];"
+				: "=d"(wv[4]), "=d"(wv[5]), "=d"(wv[6]), "=d"(wv[7]) : "l"(w + eb + 4));
+		} else {
+#pragma unroll
+			for (int i = 0; i < kFlatPerLane; i++) wv[i] = eb + i < E ? __ldcs(w + eb + i) : 0.0;
+		}
+#pragma unroll
+		for (int i = 0; i < kFlatPerLane; i++)
+			v[i] = id[i] != kNoId ? __dmul_rn(wv[i], x[id[i]]) : 0.0;
+	}
+	struct Row { uint32_t v; double base; };
+	__device__ __forceinline__ Row row(uint32_t k) const {
+		const uint32_t v = __ldg(nz_rows + k);
+		return Row{v, __ldg(base + v)};
+	}
+	__device__ __forceinline__ double old(const Row& r) const { return x[r.v]; }
+	__device__ __forceinline__ double finish(const Row& r, double s, double xv) const {
+		const double yv = __dadd_rn(r.base, __dmul_rn(d, s));
+		y[r.v] = yv;
+		return fabs(yv - xv);
+	}
+};
+
+struct AffRunArgs {
+	FlatTiles a;
+	const uint32_t* off;
+	const uint32_t* nz_rows;
+	const double* w;
+	const double* base;
+	double* xa;                // the start; results of even iteration counts
+	double* xb;
+	double* totals;            // max_iter residuals, zero
+	double d, tol;
+	uint32_t V;
+	int max_iter;
+};
+
+__global__ void __launch_bounds__(kRunThreads, 1)
+aff_run(AffRunArgs g, RunCtl* c) {
+	extern __shared__ __align__(16) unsigned char run_smem[];
+	RunShared& sh = *reinterpret_cast<RunShared*>(run_smem);
+	const uint32_t gtid = blockIdx.x * kRunThreads + threadIdx.x;
+	const uint32_t nthreads = gridDim.x * kRunThreads;
+	uint32_t t0, t1;
+	run_share(g.a.ntiles, &t0, &t1);
+	const uint32_t seg = t0 < t1 ? __ldg(g.a.tile_seg + t0) : 0u;
+	AffRunOp op;
+	op.nz_rows = g.nz_rows;
+	op.w = g.w;
+	op.base = g.base;
+	op.d = g.d;
+	op.E = g.a.E;
+	AffRunOp::Row cross = {};
+	double resid = 0.0;
+	int it = 0;
+	for (; it < g.max_iter; it++) {
+		op.x = (it & 1) ? g.xb : g.xa;
+		op.y = (it & 1) ? g.xa : g.xb;
+		double extra = 0.0;
+		if (it < 2) {
+			// rows without edges: y = base in every iteration, written into
+			// both vectors; the first step's change counts
+			for (uint64_t v = gtid; v < g.V; v += nthreads)
+				if (__ldg(g.off + v + 1) == __ldg(g.off + v)) {
+					const double b = __ldg(g.base + v);
+					if (it == 0) extra += fabs(b - op.x[v]);
+					op.y[v] = b;
+				}
+		}
+		if (!run_iteration(g.a, op, c, sh, t0, t1, seg, extra, it & 1, it == 0, cross,
+				g.totals + it, &resid))
+			return;
+		if (resid < g.tol) {
+			it++;
+			break;
+		}
+	}
+	if (gtid == 0) {
+		c->iters = (uint32_t)it;
+		c->resid = resid;
+	}
 }
 
 // --- per-snapshot maps ----------------------------------------------------
@@ -235,7 +338,7 @@ struct lg_adjoint_maps {
 	DevBuf src;            // E u32: source of each out-adjacency position
 	uint64_t E = 0;
 	// solve buffers, reused by every call on the snapshot
-	DevBuf xa, xb, base, win, carries, resid, stage_w, stage_v, stage_g;
+	DevBuf xa, xb, base, win, carries, resid, run, stage_w, stage_v, stage_g;
 	double* resid_host = nullptr;          // pinned, 2 * kChunk
 	cudaEvent_t chunk_done[2] = {nullptr, nullptr};
 	~lg_adjoint_maps() {
@@ -332,6 +435,24 @@ lg_status ensure_maps(lg_snapshot* sn) {
 	return LG_OK;
 }
 
+std::mutex g_run_mu;
+int g_run[LG_TUNE_MAX_DEVICES];           // co-resident CTAs of aff_run + 1, 0 = not probed
+
+int aff_run_resident(int device) {
+	std::lock_guard<std::mutex> lk(g_run_mu);
+	if (device < 0 || device >= LG_TUNE_MAX_DEVICES) return 0;
+	if (!g_run[device]) {
+		int n = 0;
+		if (cudaFuncSetAttribute(aff_run, cudaFuncAttributeMaxDynamicSharedMemorySize,
+				(int)sizeof(RunShared)) == cudaSuccess)
+			n = coop_grid_size((const void*)aff_run, kRunThreads, device, sizeof(RunShared));
+		else
+			cudaGetLastError();
+		g_run[device] = n + 1;
+	}
+	return g_run[device] - 1;
+}
+
 // Iterate y = base + d * (weighted pull of x) over the flat CSR f until
 // sum |y - x| < tol (at most max_iter iterations); m->xa holds the start on
 // entry.  *out points at the result (m->xa or m->xb) on return.
@@ -348,6 +469,42 @@ lg_status fixed_point(lg_snapshot* sn, const FlatCsr& f, const double* w, const 
 	double* resid = m->resid.as<double>();
 	LG_CUDA(cudaMemsetAsync(resid, 0, (size_t)max_iter * sizeof(double), st), "memset");
 	const FlatTiles a = flat_tiles(f, m->carries.as<double>());
+	const uint32_t* off = f.off.as<uint32_t>();
+	const int ctas = (int)tune_value(s->device, LG_TUNE_PR_CTAS_PER_SM);
+	const int resident = ctas > 0 ? 0 : aff_run_resident(s->device);
+	if (resident > 0) {
+		// every iteration in one launch
+		LG_TRY(m->run.reserve(sizeof(RunCtl)));
+		RunCtl* ctl = m->run.as<RunCtl>();
+		LG_CUDA(cudaMemsetAsync(&ctl->bar, 0, sizeof(RunCtl) - offsetof(RunCtl, bar), st), "memset");
+		AffRunArgs g;
+		g.a = a;
+		g.off = off;
+		g.nz_rows = f.nz_rows();
+		g.w = w;
+		g.base = base;
+		g.xa = A;
+		g.xb = B;
+		g.totals = resid;
+		g.d = d;
+		g.tol = tol;
+		g.V = (uint32_t)V;
+		g.max_iter = max_iter;
+		void* args[] = {&g, &ctl};
+		LG_CUDA(cudaLaunchCooperativeKernel((const void*)aff_run, dim3(run_ctas(f.ntiles, resident)),
+				dim3(kRunThreads), args, sizeof(RunShared), st), "aff_run");
+		s->launches++;
+		unsigned long long h[4];
+		static_assert(sizeof(CoopBar) == 16 && sizeof(RunCtl) - offsetof(RunCtl, bar) == 32,
+				"barrier, residual, iterations");
+		LG_TRY(read_words(s, (const unsigned long long*)&ctl->bar, 4, h));
+		if ((unsigned)h[1] & 1u)
+			return set_error(LG_ETIMEOUT, "pagerank: a grid barrier wait ran out");
+		memcpy(resid_out, &h[2], sizeof(double));
+		*iters = (int)(uint32_t)h[3];
+		*out = (*iters & 1) ? B : A;
+		return LG_OK;
+	}
 	AffOp op;
 	op.nz_rows = f.nz_rows();
 	op.w = w;
@@ -355,8 +512,6 @@ lg_status fixed_point(lg_snapshot* sn, const FlatCsr& f, const double* w, const 
 	op.d = d;
 	op.tol = tol;
 	op.E = (uint32_t)f.E;
-	const uint32_t* off = f.off.as<uint32_t>();
-	const int ctas = (int)tune_value(s->device, LG_TUNE_PR_CTAS_PER_SM);
 	int sms = 148;
 	if (ctas > 0) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
 	aff_empty_rows<<<grid_for(V, 256), 256, 0, st>>>(off, V, base, A, B, resid);

@@ -1,0 +1,94 @@
+"""Iterations inside one launch (PageRank over small in-CSRs, the weighted fixed
+point) at the edges of tiles, warp runs and CTAs, with rows over many of them,
+against a plain FP64 evaluation and the launch-per-iteration form
+(LG_TUNE_PR_CTAS_PER_SM = 4)."""
+import numpy as np
+import pytest
+
+from llama_b200 import Store
+from llama_b200.graph import tune_reset, tune_set
+from tests._util import max_rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def _edges(V, n, hub, seed):
+    rng = np.random.default_rng(seed)
+    k = rng.choice(V * V, n, replace=False) if n else np.zeros(0, np.int64)
+    s, d = k // V, k % V
+    if hub:                                      # rows of thousands, first, last and between
+        for h, m in ((0, V), (V // 2, V // 3), (V - 1, V)):
+            s, d = np.concatenate([s, np.arange(m)]), np.concatenate([d, np.full(m, h)])
+    k = np.unique(s * V + d)
+    return k // V, k % V
+
+
+CASES = [(3, 0, False), (3, 1, False), (40, 255, False), (40, 256, False), (40, 257, False),
+         (600, 8191, False), (600, 8193, False), (9000, 5000, True), (70000, 300000, True),
+         (150000, 2500000, False)]
+
+
+@pytest.mark.parametrize("V,n,hub", CASES)
+def test_pagerank(V, n, hub):
+    s, d = _edges(V, n, hub, n + V)
+    deg = np.bincount(s, minlength=V).astype(np.float64)
+    with Store() as st:
+        st.build_level(V, s, d)
+        with st.snapshot() as sn:
+            for it in (1, 2, 3, 8):
+                x = np.full(V, 1.0 / V)
+                for _ in range(it):
+                    y = np.divide(x, deg, out=np.zeros(V), where=deg > 0)
+                    x = 0.15 / V + 0.85 * np.bincount(d, y[s], V)
+                got = sn.pagerank_pull(it)
+                assert max_rel_err(got, x) <= 1e-12
+                assert np.array_equal(sn.pagerank_pull(it), got)
+                tune_set(0, "pr_ctas_per_sm", 4)
+                try:
+                    assert max_rel_err(sn.pagerank_pull(it), got) <= 1e-12
+                finally:
+                    tune_reset(0)
+
+
+def test_pagerank_device_output_and_sync():
+    import torch
+    s, d = _edges(600, 8193, False, 1)
+    with Store() as st:
+        st.build_level(600, s, d)
+        with st.snapshot() as sn:
+            want = sn.pagerank_pull(7)
+            out = torch.empty(600, dtype=torch.float64, device="cuda")
+            for _ in range(3):
+                sn.pagerank_pull(7, out=out)
+                sn.pagerank_pull(7, out=out)
+                st.sync()
+                assert np.array_equal(out.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("V,n,hub", CASES)
+def test_fixed_point_and_gradient(V, n, hub):
+    s, d = _edges(V, n, hub, n + V + 1)
+    rng = np.random.default_rng(2)
+    deg = np.bincount(s, minlength=V)
+    w = rng.uniform(0.5, 1.0, len(s)) / np.maximum(deg[s], 1)      # edges in (s, d) order
+    v, g = rng.random(V) / V, rng.standard_normal(V) / V
+    with Store() as st:
+        st.build_level(V, s, d)
+        with st.snapshot() as sn:
+            x, tape, r = sn.pagerank_fwd(w, v, tol=1e-13)
+            dw, dv, rb = tape.backward(g)
+            tape.close()
+            # the fixed points' own equations, and the gradients' definition
+            assert np.abs(0.15 * v + 0.85 * np.bincount(d, w * x[s], V) - x).sum() <= 1e-13
+            lam = dv / 0.15
+            assert np.abs(g + 0.85 * np.bincount(s, w * lam[d], V) - lam).sum() <= 2e-13
+            assert np.allclose(dw, 0.85 * lam[d] * x[s], rtol=1e-12, atol=0)
+            tune_set(0, "pr_ctas_per_sm", 4)
+            try:
+                x2, _, r2 = sn.pagerank_fwd(w, v, tol=1e-13, keep_tape=False)
+            finally:
+                tune_reset(0)
+            assert np.abs(x2 - x).sum() <= 2e-13 and abs(r.iterations - r2.iterations) <= 1
+            x3, _, r3 = sn.pagerank_fwd(w, v, tol=1e-300, max_iter=3, keep_tape=False)
+            # (without a path of three edges the residual is 0 before)
+            assert r3.iterations == 3 if n > 1 else r3.iterations <= 3
