@@ -265,6 +265,10 @@ struct lg_store {
 	lg::SnapDir* snap_spare[2] = {nullptr, nullptr};
 	lg::DevLevel* level_spare[2] = {nullptr, nullptr};
 	lg::DevBuf build_tmp[12];   // lg_store_build_level temporaries
+	// control block of one-launch PageRank; run_pending: its error word has not
+	// been read since the last such launch
+	lg::DevBuf run_ctl;
+	bool run_pending = false;
 	int min_level = 0;          // levels below are aged out (lg_store_set_min_level)
 	// LG_OUTPUT_ASYNC: results staged in out_stage[i] and copied to host on
 	// copy_stream; stage_done[i] marks the end of slot i's last copy
@@ -335,6 +339,10 @@ inline uint64_t scan_launches(uint64_t n) {
 
 // out[v] = live slots of v's fragments in direction dir (0 out, 1 in).
 lg_status live_degrees(const lg_snapshot* sn, int dir, uint32_t* out);
+
+// Waits for the store's stream; LG_ETIMEOUT if a one-launch PageRank since the
+// last call gave up a barrier wait (lg_pagerank.cu).
+lg_status finish_run(lg_store* s);
 
 // Copy `bytes` of device data to a caller buffer (host or device) on the
 // store's stream, counting host-bound bytes.

@@ -32,9 +32,11 @@
 // lg_pagerank_pull_noalloc cannot hold the E-sized flat array, so it walks
 // the fragments directly every iteration (pr_pull_step, one CTA per 1024
 // virtual slots, values staged in shared memory).
+#include "lg_flat_run.cuh"
 #include "lg_flat_sweep.cuh"
 #include "lg_tune.h"
 
+#include <cstddef>
 #include <mutex>
 
 namespace lg {
@@ -98,6 +100,91 @@ pr_flat_loop(FlatTiles a, PrOp op) {
 __global__ void __launch_bounds__(kFixupThreads)
 pr_flat_fixup(FlatTiles a, PrOp op) {
 	flat_sweep_fixup_body(a, op);
+}
+
+// The same iterations inside one cooperative launch (lg_flat_run.cuh), the
+// start vectors and the rows without in-edges included.
+struct PrRunOp {
+	static constexpr bool kResidual = false;
+	const uint32_t* nz_rows;
+	const uint32_t* outdeg;
+	const double* contrib;     // rewritten between iterations: plain loads
+	double* contrib_next;
+	double* pr_out;            // written when non-null (last iteration)
+	double base;
+	double d;
+	__device__ __forceinline__ void values(uint32_t, const uint32_t (&id)[kFlatPerLane],
+			double (&x)[kFlatPerLane]) const {
+#pragma unroll
+		for (int i = 0; i < kFlatPerLane; i++) x[i] = id[i] != kNoId ? contrib[id[i]] : 0.0;
+	}
+	struct Row { uint32_t v, dg; };
+	__device__ __forceinline__ Row row(uint32_t k) const {
+		const uint32_t v = __ldg(nz_rows + k);
+		return Row{v, __ldg(outdeg + v)};
+	}
+	__device__ __forceinline__ double old(const Row&) const { return 0.0; }
+	__device__ __forceinline__ double finish(const Row& r, double s, double) const {
+		const double pr = __dadd_rn(base, __dmul_rn(d, s));
+		contrib_next[r.v] = r.dg ? pr / (double)r.dg : 0.0;
+		if (pr_out) pr_out[r.v] = pr;
+		return 0.0;
+	}
+};
+
+struct PrRunArgs {
+	FlatTiles a;
+	const uint32_t* off;
+	const uint32_t* nz_rows;
+	const uint32_t* outdeg;
+	double* c0;
+	double* c1;
+	double* pr_out;
+	double base, d, pr0;
+	uint32_t V;
+	int iterations;            // at least 1
+};
+
+__global__ void __launch_bounds__(kRunThreads, 1)
+pr_run(PrRunArgs g, RunCtl* c) {
+	extern __shared__ __align__(16) unsigned char run_smem[];
+	RunShared& sh = *reinterpret_cast<RunShared*>(run_smem);
+	const uint32_t gtid = blockIdx.x * kRunThreads + threadIdx.x;
+	const uint32_t nthreads = gridDim.x * kRunThreads;
+	uint32_t t0, t1;
+	run_share(g.a.ntiles, &t0, &t1);
+	const uint32_t seg = t0 < t1 ? __ldg(g.a.tile_seg + t0) : 0u;
+	PrRunOp op;
+	op.nz_rows = g.nz_rows;
+	op.outdeg = g.outdeg;
+	op.base = g.base;
+	op.d = g.d;
+	for (uint64_t v = gtid; v < g.V; v += nthreads) {
+		const uint32_t dg = __ldg(g.outdeg + v);
+		g.c0[v] = dg ? g.pr0 / (double)dg : 0.0;
+		if (__ldg(g.off + v + 1) == __ldg(g.off + v)) {
+			g.c1[v] = dg ? g.base / (double)dg : 0.0;
+			g.pr_out[v] = g.base;
+		}
+	}
+	if (!grid_barrier(&c->bar)) return;
+	PrRunOp::Row cross = {};
+	double resid;
+	for (int it = 0; it < g.iterations; it++) {
+		op.contrib = (it & 1) ? g.c1 : g.c0;
+		op.contrib_next = (it & 1) ? g.c0 : g.c1;
+		op.pr_out = it == g.iterations - 1 ? g.pr_out : nullptr;
+		if (it == 1)
+			// c0 still holds pr0 / out_degree for vertices without in-edges
+			for (uint64_t v = gtid; v < g.V; v += nthreads)
+				if (__ldg(g.off + v + 1) == __ldg(g.off + v)) {
+					const uint32_t dg = __ldg(g.outdeg + v);
+					g.c0[v] = dg ? g.base / (double)dg : 0.0;
+				}
+		if (!run_iteration(g.a, op, c, sh, t0, t1, seg, 0.0, it & 1, it == 0, cross, nullptr,
+				&resid))
+			return;
+	}
 }
 
 // nz_outdeg[k] = out-degree of row k's vertex (rows read it in order).
@@ -265,6 +352,47 @@ using namespace lg;
 
 namespace lg {
 
+// Largest in-CSR (in 256-edge tiles) whose iterations run in one launch: an
+// iteration then costs a barrier and some loads, 4 to 6 us, against two launches
+// of 5 us each.  Three programs' calls in turn, result on the device, 10 to 15
+// iterations: 20 k edges (80 tiles) 144 -> 75 us, 140 k (550) 197 -> 109, but
+// 420 k (1640) 194 -> 221 and 840 k 202 -> 244, because launches of several
+// streams overlap and whole-GPU ones do not.  (A single program's gain goes on
+// to some 4000 tiles, 406 -> 289 us at 560 k edges.)
+constexpr uint32_t kPrRunTiles = 1024;
+
+static std::mutex g_run_mu;
+static int g_run[LG_TUNE_MAX_DEVICES];    // co-resident CTAs of pr_run + 1, 0 = not probed
+
+static int pr_run_resident(int device) {
+	std::lock_guard<std::mutex> lk(g_run_mu);
+	if (device < 0 || device >= LG_TUNE_MAX_DEVICES) return 0;
+	if (!g_run[device]) {
+		int n = 0;
+		if (cudaFuncSetAttribute(pr_run, cudaFuncAttributeMaxDynamicSharedMemorySize,
+				(int)sizeof(RunShared)) == cudaSuccess)
+			n = coop_grid_size((const void*)pr_run, kRunThreads, device, sizeof(RunShared));
+		else
+			cudaGetLastError();
+		g_run[device] = n + 1;
+	}
+	return g_run[device] - 1;
+}
+
+lg_status finish_run(lg_store* s) {
+	if (!s->run_pending) {
+		LG_CUDA(cudaStreamSynchronize(s->stream), "sync");
+		return LG_OK;
+	}
+	unsigned long long h[2];
+	static_assert(sizeof(CoopBar) == 16, "two words");
+	LG_TRY(read_words(s, (const unsigned long long*)&s->run_ctl.as<RunCtl>()->bar, 2, h));
+	s->run_pending = false;
+	if ((unsigned)h[1] & 1u)
+		return set_error(LG_ETIMEOUT, "pagerank: a grid barrier wait ran out");
+	return LG_OK;
+}
+
 lg_status pagerank_over(lg_snapshot* sn, FlatCsr* f, int iterations, double damping,
 		double* ranks) {
 	lg_store* s = sn->store;
@@ -276,6 +404,52 @@ lg_status pagerank_over(lg_snapshot* sn, FlatCsr* f, int iterations, double damp
 	const unsigned B = 256;
 	DevBuf* sc = s->scratch;
 	const uint32_t* outdeg = sn->out.deg.as<uint32_t>();
+	const uint32_t ntiles = f->ntiles;
+	const uint32_t* flat_off = f->off.as<uint32_t>();
+
+	LG_TRY(sc[0].reserve(V * sizeof(double)));
+	LG_TRY(sc[1].reserve(V * sizeof(double)));
+	LG_TRY(sc[2].reserve(2ull * std::max<uint32_t>(ntiles, 1) * sizeof(double)));
+	const FlatTiles a = flat_tiles(*f, sc[2].as<double>());
+	const bool dev_out = is_device_pointer(ranks);
+	double* pr_buf = ranks;
+	if (!dev_out) {
+		LG_TRY(sc[4].reserve(V * sizeof(double)));
+		pr_buf = sc[4].as<double>();
+	}
+	double* c0 = sc[0].as<double>();
+	double* c1 = sc[1].as<double>();
+	const int ctas = (int)tune_value(s->device, LG_TUNE_PR_CTAS_PER_SM);
+	const int resident = ctas > 0 || iterations == 0 || ntiles > kPrRunTiles ? 0
+			: pr_run_resident(s->device);
+	if (resident > 0) {
+		LG_TRY(s->run_ctl.reserve(sizeof(RunCtl)));
+		RunCtl* ctl = s->run_ctl.as<RunCtl>();
+		// the error word stays set until it has been reported
+		LG_CUDA(cudaMemsetAsync(&ctl->bar, 0, s->run_pending ? offsetof(CoopBar, err)
+				: sizeof(CoopBar), st), "memset");
+		PrRunArgs g;
+		g.a = a;
+		g.off = flat_off;
+		g.nz_rows = f->nz_rows();
+		g.outdeg = outdeg;
+		g.c0 = c0;
+		g.c1 = c1;
+		g.pr_out = pr_buf;
+		g.base = base;
+		g.d = damping;
+		g.pr0 = pr0;
+		g.V = (uint32_t)V;
+		g.iterations = iterations;
+		void* args[] = {&g, &ctl};
+		LG_CUDA(cudaLaunchCooperativeKernel((const void*)pr_run, dim3(run_ctas(ntiles, resident)),
+				dim3(kRunThreads), args, sizeof(RunShared), st), "pr_run");
+		s->launches++;
+		s->run_pending = true;
+		if (dev_out) return LG_OK;               // lg_store_sync reports a barrier that gave up
+		LG_TRY(copy_out(s, ranks, pr_buf, V * sizeof(double)));
+		return finish_run(s);
+	}
 	if (!f->has_nz_outdeg) {
 		LG_TRY(f->nz_outdeg.reserve(f->rcap() * sizeof(uint32_t)));
 		if (f->R > 0) {
@@ -286,32 +460,16 @@ lg_status pagerank_over(lg_snapshot* sn, FlatCsr* f, int iterations, double damp
 		}
 		f->has_nz_outdeg = true;
 	}
-	const uint32_t ntiles = f->ntiles;
-	const uint32_t* flat_off = f->off.as<uint32_t>();
-
-	LG_TRY(sc[0].reserve(V * sizeof(double)));
-	LG_TRY(sc[1].reserve(V * sizeof(double)));
-	LG_TRY(sc[2].reserve(2ull * std::max<uint32_t>(ntiles, 1) * sizeof(double)));
-	const FlatTiles a = flat_tiles(*f, sc[2].as<double>());
 	PrOp op;
 	op.nz_rows = f->nz_rows();
 	op.nz_outdeg = f->nz_outdeg.as<uint32_t>();
 	op.base = base;
 	op.d = damping;
-	const bool dev_out = is_device_pointer(ranks);
-	double* pr_buf = ranks;
-	if (!dev_out) {
-		LG_TRY(sc[4].reserve(V * sizeof(double)));
-		pr_buf = sc[4].as<double>();
-	}
-	double* c0 = sc[0].as<double>();
-	double* c1 = sc[1].as<double>();
 	pr_init<<<grid_for(V, B), B, 0, st>>>(outdeg, V, pr0, c0, iterations == 0 ? pr_buf : nullptr);
 	pr_empty_rows<<<grid_for(V, B), B, 0, st>>>(flat_off, outdeg, V, base, c1, nullptr);
 	LG_CUDA(cudaGetLastError(), "pr_init");
 	s->launches += 2;
 	const unsigned fix_blocks = flat_fixup_blocks(ntiles);   // a thread per tile boundary
-	const int ctas = (int)tune_value(s->device, LG_TUNE_PR_CTAS_PER_SM);
 	const bool occ8 = tune_value(s->device, LG_TUNE_PR_TILE_OCC) == 8;
 	int sms = 148;
 	if (ctas > 0) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);

@@ -1076,8 +1076,7 @@ lg_status lg_store_sync(lg_store* s) {
 			LG_CUDA(cudaStreamWaitEvent(s->stream, s->stage_done[i], 0), "join copies");
 		LG_CUDA(cudaStreamSynchronize(s->copy_stream), "sync copies");
 	}
-	LG_CUDA(cudaStreamSynchronize(s->stream), "sync");
-	return LG_OK;
+	return finish_run(s);
 }
 
 lg_status lg_store_set_output_mode(lg_store* s, int mode) {
