@@ -17,6 +17,9 @@
 // that ppr_fixup adds in range order.  Rows without in-edges hold a constant
 // after the first iteration and are written once.
 //
+// x0 has one non-zero per column, so the first two iterations look a row up in a
+// bitmap of the rows that are not zero before they load it.
+//
 // Bound by the row gathers (E x K x 8 bytes per iteration, mostly from L2 at
 // 100 k vertices x 96 columns).  The form before it walked fragments and added
 // an edge's row before it loaded the next one: one load per lane in flight,
@@ -39,7 +42,9 @@ constexpr int kPprThreads = 256;
 constexpr int kPprWarps = kPprThreads / 32;
 constexpr uint32_t kNoSeed = 0xffffffffu;
 // Edges whose rows a warp loads ahead: about 8 to 32 loads per lane in
-// flight, within the registers of two resident CTAs.
+// flight.  Up to 128 columns the registers are capped for three resident CTAs
+// (96 columns, 3 M edges: 252 -> 207 us an iteration; with 8 edges ahead and
+// two CTAs 237).
 template <int CPL>
 constexpr int kPprAhead = CPL <= 2 ? 8 : 4;
 
@@ -65,6 +70,8 @@ struct PprArgs {
 	uint32_t K;               // row length of y / x / carries
 	uint32_t col0;            // first column of this pass (a K-tile of CPL * 32 columns)
 	uint32_t range;           // edges per warp range, a multiple of 32
+	const uint32_t* bits;     // kSparse: rows of y that are not zero
+	uint32_t* bits_next;      // those of y_next, if wanted
 };
 
 // Row of vertex v (out-degree dg, first seed sf) has the in-sums s.
@@ -72,6 +79,7 @@ template <int CPL>
 __device__ __forceinline__ void ppr_finish(const PprArgs& a, uint32_t v, uint32_t dg, uint32_t sf,
 		const double* s) {
 	const uint32_t lane = threadIdx.x & 31u;
+	bool some = false;
 #pragma unroll
 	for (int i = 0; i < CPL; i++) {
 		const uint32_t c = a.col0 + lane + 32 * i;
@@ -82,7 +90,10 @@ __device__ __forceinline__ void ppr_finish(const PprArgs& a, uint32_t v, uint32_
 		const double x = __dadd_rn(t, __dmul_rn(a.d, s[i]));
 		a.y_next[(uint64_t)v * a.K + c] = dg ? x / (double)dg : 0.0;
 		if (a.x_out) a.x_out[(uint64_t)v * a.K + c] = x;
+		some |= x != 0.0;
 	}
+	if (a.bits_next && __any_sync(0xffffffffu, some) && lane == 0)
+		atomicOr(a.bits_next + (v >> 5), 1u << (v & 31u));
 }
 
 template <int CPL>
@@ -93,8 +104,8 @@ __device__ __forceinline__ void ppr_carry(double* to, const PprArgs& a, uint32_t
 		to[(uint64_t)r * a.K + a.col0 + (threadIdx.x & 31u) + 32 * i] = s[i];
 }
 
-template <int CPL>
-__global__ void __launch_bounds__(kPprThreads, 2)
+template <int CPL, bool kSparse>
+__global__ void __launch_bounds__(kPprThreads, CPL <= 4 ? 3 : 2)
 ppr_step(PprArgs a) {
 	constexpr int U = kPprAhead<CPL>;
 	const uint32_t lane = threadIdx.x & 31u;
@@ -112,6 +123,10 @@ ppr_step(PprArgs a) {
 		const uint32_t n = min(32u, e1 - base);
 		const uint32_t hw = __ldg(a.heads + (base >> 5));
 		const uint32_t id = lane < n ? __ldcs(a.ids + base + lane) : 0u;
+		unsigned want = n == 32u ? ~0u : (1u << n) - 1u;     // edges whose rows are loaded
+		if (kSparse)
+			want = __ballot_sync(0xffffffffu, lane < n
+					&& ((__ldg(a.bits + (id >> 5)) >> (id & 31u)) & 1u));
 		// lane h: vertex, out-degree and seed of the row that h heads of this
 		// word leave open
 		const uint32_t k = next - 1u + lane;
@@ -128,7 +143,7 @@ ppr_step(PprArgs a) {
 				const uint32_t src = __shfl_sync(0xffffffffu, id, g + u);
 				const double* row = a.y + (uint64_t)src * a.K + a.col0 + lane;
 #pragma unroll
-				for (int i = 0; i < CPL; i++) v[u][i] = g + u < n ? __ldg(row + 32 * i) : 0.0;
+				for (int i = 0; i < CPL; i++) v[u][i] = (want >> (g + u)) & 1u ? __ldg(row + 32 * i) : 0.0;
 			}
 #pragma unroll
 			for (int u = 0; u < U; u++) {
@@ -253,6 +268,14 @@ __global__ void ppr_seed_index(const uint2* seed_col, uint32_t n, uint32_t* seed
 	if (i < n && (i == 0 || seed_col[i - 1].x != seed_col[i].x)) seed_first[seed_col[i].x] = i;
 }
 
+// Rows of x0 that are not zero in columns [col0, col1).
+__global__ void ppr_seed_bits(const uint2* seed_col, uint32_t n, uint32_t col0, uint32_t col1,
+		uint32_t* bits) {
+	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (i >= n || seed_col[i].y < col0 || seed_col[i].y >= col1) return;
+	atomicOr(bits + (seed_col[i].x >> 5), 1u << (seed_col[i].x & 31u));
+}
+
 __global__ void ppr_seed_init(const uint2* seed_col, uint32_t n, const uint32_t* outdeg,
 		uint32_t K, double* y) {
 	const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -265,13 +288,15 @@ __global__ void ppr_seed_init(const uint2* seed_col, uint32_t n, const uint32_t*
 // Seeds without in-edges, columns [col0, col1): y = (1-d) / out_degree from
 // the first iteration on (other rows without in-edges stay 0).
 __global__ void ppr_seed_empty(const uint2* seed_col, uint32_t n, const uint32_t* off,
-		const uint32_t* outdeg, double tele, uint32_t K, uint32_t col0, uint32_t col1, double* y) {
+		const uint32_t* outdeg, double tele, uint32_t K, uint32_t col0, uint32_t col1, double* y,
+		uint32_t* bits) {
 	const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
 	const uint32_t v = seed_col[i].x, c = seed_col[i].y;
 	if (c < col0 || c >= col1 || __ldg(off + v + 1) != __ldg(off + v)) return;
 	const uint32_t dg = outdeg[v];
 	y[(uint64_t)v * K + c] = dg ? tele / (double)dg : 0.0;
+	if (bits) atomicOr(bits + (v >> 5), 1u << (v & 31u));
 }
 
 // Result rows of the vertices without in-edges: (1-d) at their own seeds.
@@ -295,7 +320,8 @@ __global__ void ppr_seed_x(const uint2* seed_col, uint32_t n, uint32_t K, double
 
 template <int CPL>
 void launch_ppr_iteration(const PprArgs& a, cudaStream_t st) {
-	ppr_step<CPL><<<grid_for(a.nranges, kPprWarps), kPprThreads, 0, st>>>(a);
+	if (a.bits) ppr_step<CPL, true><<<grid_for(a.nranges, kPprWarps), kPprThreads, 0, st>>>(a);
+	else ppr_step<CPL, false><<<grid_for(a.nranges, kPprWarps), kPprThreads, 0, st>>>(a);
 	if (a.nranges > 1)
 		ppr_fixup<CPL><<<grid_for(a.nranges - 1, kPprWarps), kPprThreads, 0, st>>>(a);
 }
@@ -342,6 +368,10 @@ extern "C" lg_status lg_ppr(lg_snapshot* const* snaps, int n_snaps, const int64_
 	LG_TRY(yb[1].reserve(V * row));
 	LG_TRY(seedb.reserve(K * sizeof(uint2)));
 	LG_TRY(firstb.reserve(V * 4));
+	const uint64_t words = (V + 31) / 32;
+	LG_TRY(s->scratch[7].reserve(2 * words * 4));
+	uint32_t* bits = s->scratch[7].as<uint32_t>();       // rows not zero before the first
+	                                                     // and the second iteration
 	// launch parameters: columns per pass (a multiple of 32 dividing K) and
 	// the most edges per warp range
 	int ktile = (int)tune_value(s->device, LG_TUNE_PPR_KTILE);
@@ -390,8 +420,9 @@ extern "C" lg_status lg_ppr(lg_snapshot* const* snaps, int n_snaps, const int64_
 		a.nz_off = f->nz_off();
 		a.E = (uint32_t)f->E;
 		a.R = (uint32_t)f->R;
-		// about four ranges for each of 32 warps per SM, a multiple of 32 edges
-		const uint64_t even = ((f->E + (uint64_t)sms * 128u - 1) / ((uint64_t)sms * 128u) + 31) & ~31ull;
+		// about four ranges for each of 24 warps per SM, a multiple of 32 edges
+		// (two or one: 0 to 17 % slower, five: 2 %)
+		const uint64_t even = ((f->E + (uint64_t)sms * 96u - 1) / ((uint64_t)sms * 96u) + 31) & ~31ull;
 		a.range = (uint32_t)std::min(max_range, std::max<uint64_t>(even, 32));
 		a.nranges = (uint32_t)((f->E + a.range - 1) / a.range);
 		LG_TRY(segb.reserve(std::max<uint64_t>(a.nranges, 1) * 4));
@@ -419,14 +450,20 @@ extern "C" lg_status lg_ppr(lg_snapshot* const* snaps, int n_snaps, const int64_
 		// column tiles are independent: each runs all iterations on its columns
 		for (int c0 = 0; c0 < K; c0 += ktile) {
 			a.col0 = (uint32_t)c0;
+			LG_CUDA(cudaMemsetAsync(bits, 0, 2 * words * 4, st), "memset");
+			ppr_seed_bits<<<kb, 256, 0, st>>>(seeds_d, (uint32_t)K, (uint32_t)c0,
+					(uint32_t)(c0 + ktile), bits);
+			s->launches++;
 			for (int it = 0; it < iterations; it++) {
+				a.bits = it < 2 ? bits + it * words : nullptr;
+				a.bits_next = it == 0 ? bits + words : nullptr;
 				a.y = yb[it & 1].as<double>();
 				a.y_next = yb[(it + 1) & 1].as<double>();
 				a.x_out = (it == iterations - 1) ? xo : nullptr;
 				if (it < 2) {
 					// it 0: the block written now; it 1: the first one, read by then
 					ppr_seed_empty<<<kb, 256, 0, st>>>(seeds_d, (uint32_t)K, off, outdeg, a.tele,
-							(uint32_t)K, (uint32_t)c0, (uint32_t)(c0 + ktile), a.y_next);
+							(uint32_t)K, (uint32_t)c0, (uint32_t)(c0 + ktile), a.y_next, a.bits_next);
 					s->launches++;
 				}
 				if (a.nranges == 0) continue;
