@@ -54,8 +54,11 @@ __global__ void bl_keys(const uint32_t* a, const uint32_t* b, uint64_t n, uint64
 		unsigned long long* keys, uint32_t* idx, unsigned* err) {
 	const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
-	const uint32_t x = a[i], y = b[i];
-	if (x >= V || y >= V) atomicOr(err, kErrRange);
+	uint32_t x = a[i], y = b[i];
+	if (x >= V || y >= V) {
+		atomicOr(err, kErrRange);
+		x = y = 0;                 // the level is refused; until then ids index arrays
+	}
 	keys[i] = ((unsigned long long)x << 32) | y;
 	if (idx) idx[i] = (uint32_t)i;
 }
@@ -316,6 +319,13 @@ static lg_status build_dir(lg_store* s, const DevCsr& csr, int l, uint64_t V,
 	return LG_OK;
 }
 
+// The bits in which ids below V may differ (never none).
+static unsigned long long id_bits(uint64_t V) {
+	unsigned long long m = 1;
+	while (m < V) m <<= 1;
+	return m > 1 ? m - 1 : 1;
+}
+
 // Sorted (a << 32 | b) keys of n pairs (payload = input index when `perm`)
 // in `keys`; err gets kErrRange / dup_bit.
 static lg_status sorted_keys(lg_store* s, const uint32_t* a, const uint32_t* b, uint64_t n,
@@ -335,7 +345,8 @@ static lg_status sorted_keys(lg_store* s, const uint32_t* a, const uint32_t* b, 
 	unsigned long long* sk = nullptr;
 	uint32_t* sp = nullptr;
 	LG_TRY(radix_sort_u64(s, keys_buf.as<unsigned long long>(),
-			perm ? perm_buf.as<uint32_t>() : nullptr, n, tmp[0], tmp[1], tmp[2], tmp[3], &sk, &sp));
+			perm ? perm_buf.as<uint32_t>() : nullptr, n, tmp[0], tmp[1], tmp[2], tmp[3], &sk, &sp,
+			id_bits(V) << 32 | id_bits(V)));
 	// keep the result in keys_buf / perm_buf (the temporaries are reused)
 	if (sk != keys_buf.as<unsigned long long>())
 		LG_CUDA(cudaMemcpyAsync(keys_buf.p, sk, n * sizeof(unsigned long long),
@@ -418,7 +429,8 @@ extern "C" lg_status lg_store_build_level(lg_store* s, uint64_t max_nodes,
 	LG_TRY(build_dir(s, s->out, l, V, ok, n_new, od, n_del, operm, dw, sc, &lo));
 
 	// in direction: the same edges keyed by target (sources stay sorted
-	// within a target, as make_reverse_edges leaves them)
+	// within a target, as make_reverse_edges leaves them: the keys are in source
+	// order already and the sort is stable, so it takes the targets' bits only)
 	lg_status rs = LG_OK;
 	if (s->reverse) {
 		DevBuf& ik_keys = s->build_tmp[10];
@@ -431,7 +443,7 @@ extern "C" lg_status lg_store_build_level(lg_store* s, uint64_t max_nodes,
 				unsigned long long* sk = nullptr;
 				uint32_t* sp = nullptr;
 				rs = radix_sort_u64(s, ik_keys.as<unsigned long long>(), nullptr, n_new,
-						sc[4], sc[5], sc[6], sc[7], &sk, &sp);
+						sc[4], sc[5], sc[6], sc[7], &sk, &sp, id_bits(V) << 32);
 				ik = sk;
 			}
 		}
@@ -442,7 +454,7 @@ extern "C" lg_status lg_store_build_level(lg_store* s, uint64_t max_nodes,
 				unsigned long long* sk = nullptr;
 				uint32_t* sp = nullptr;
 				rs = radix_sort_u64(s, id_keys.as<unsigned long long>(), nullptr, n_del,
-						sc[8], sc[9], sc[10], sc[2], &sk, &sp);
+						sc[8], sc[9], sc[10], sc[2], &sk, &sp, id_bits(V) << 32);
 				idk = sk;
 			}
 		}

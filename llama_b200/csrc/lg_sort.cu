@@ -44,12 +44,17 @@ rs_hist(const unsigned long long* k, uint64_t n, int shift, uint32_t* counts,
 		uint32_t tiles) {
 	__shared__ uint32_t h[256];
 	h[threadIdx.x] = 0;
-	__syncthreads();
-	const uint64_t base = (uint64_t)blockIdx.x * kRsTile;
+	const uint64_t base = (uint64_t)blockIdx.x * kRsTile + threadIdx.x;
+	uint32_t dig[kRsItems];              // all loads before the first count
+#pragma unroll
 	for (int r = 0; r < kRsItems; r++) {
-		uint64_t i = base + (uint64_t)r * kRsThreads + threadIdx.x;
-		if (i < n) atomicAdd(&h[(k[i] >> shift) & 0xff], 1u);
+		const uint64_t i = base + (uint64_t)r * kRsThreads;
+		dig[r] = i < n ? (uint32_t)(k[i] >> shift) & 0xffu : 256u;
 	}
+	__syncthreads();
+#pragma unroll
+	for (int r = 0; r < kRsItems; r++)
+		if (dig[r] < 256u) atomicAdd(&h[dig[r]], 1u);
 	__syncthreads();
 	counts[(uint64_t)threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
 }
