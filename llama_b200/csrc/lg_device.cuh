@@ -202,10 +202,8 @@ constexpr uint32_t kSlotTile = 512;
 struct SnapDir {
 	DevBuf frag_off, frags, deg, delbits, lt, slot_off;
 	DevBuf range_lb;               // lower_bound(slot_off, r * kBlockSlots), r = 0..nblocks
-	DevBuf frag_start;             // F + 1 u32: first virtual slot of every fragment
-	DevBuf frag_vert;              // F u32: its vertex
-	DevBuf tile_frag;              // fragment that holds virtual slot t * kSlotTile
-	DevBuf tmp_cnt, tmp_slots, tmp_scan, tmp_words, tmp_sum;   // open-time scratch
+	DevBuf frag_aux;               // u32: frag_start, frag_vert, tile_frag below
+	DevBuf tmp_cnt, tmp_slots, tmp_scan, tmp_scan2, tmp_sum;   // open-time scratch
 	uint64_t n_frags = 0;
 	uint64_t n_edges = 0;          // live edges (sum of degrees)
 	uint64_t n_slots = 0;          // slots of levels 0..L
@@ -214,13 +212,18 @@ struct SnapDir {
 	bool present = false;
 	// exchange device buffers with o (a closed snapshot's, kept for reuse)
 	void swap_buffers(SnapDir& o) {
-		DevBuf* a[] = {&frag_off, &frags, &deg, &delbits, &lt, &slot_off, &range_lb, &frag_start,
-			&frag_vert, &tile_frag, &tmp_cnt, &tmp_slots, &tmp_scan, &tmp_words, &tmp_sum};
+		DevBuf* a[] = {&frag_off, &frags, &deg, &delbits, &lt, &slot_off, &range_lb, &frag_aux,
+			&tmp_cnt, &tmp_slots, &tmp_scan, &tmp_scan2, &tmp_sum};
 		DevBuf* b[] = {&o.frag_off, &o.frags, &o.deg, &o.delbits, &o.lt, &o.slot_off,
-			&o.range_lb, &o.frag_start, &o.frag_vert, &o.tile_frag, &o.tmp_cnt, &o.tmp_slots,
-			&o.tmp_scan, &o.tmp_words, &o.tmp_sum};
+			&o.range_lb, &o.frag_aux, &o.tmp_cnt, &o.tmp_slots, &o.tmp_scan, &o.tmp_scan2,
+			&o.tmp_sum};
 		for (size_t i = 0; i < sizeof(a) / sizeof(a[0]); i++) a[i]->swap(*b[i]);
 	}
+	// first virtual slot of every fragment (n_frags + 1), its vertex, and the
+	// fragment that holds virtual slot t * kSlotTile
+	uint32_t* frag_start() const { return frag_aux.as<uint32_t>(); }
+	uint32_t* frag_vert() const { return frag_start() + n_frags + 1; }
+	uint32_t* tile_frag() const { return frag_vert() + n_frags; }
 	SnapCsr view() const {
 		SnapCsr s;
 		s.frag_off = frag_off.as<uint32_t>();

@@ -341,10 +341,10 @@ static lg_status build_rows(lg_snapshot* sn, int dir, FlatCsr& f, bool view, boo
 	LG_TRY(exclusive_scan_u32(deg, off, V, f.scan_tmp, st, nullptr));
 	FragSpace fs;
 	fs.frags = d.frags.as<uint2>();
-	fs.start = d.frag_start.as<uint32_t>();
-	fs.vert = d.frag_vert.as<uint32_t>();
+	fs.start = d.frag_start();
+	fs.vert = d.frag_vert();
 	fs.frag_off = d.frag_off.as<uint32_t>();
-	fs.tile_frag = d.tile_frag.as<uint32_t>();
+	fs.tile_frag = d.tile_frag();
 	fs.lt = d.lt.as<LevelTab>();
 	fs.F = (uint32_t)d.n_frags;
 	fs.total = (uint32_t)d.n_frag_slots;

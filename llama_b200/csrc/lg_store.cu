@@ -415,7 +415,8 @@ scan_tiles(const uint32_t* in, uint32_t* out, uint64_t n, const uint64_t* sums, 
 // (cnt, if not null; kNonzero: they count as 1 where positive).
 template <bool kNonzero, class In>
 static lg_status exclusive_scan(const In& in, const uint32_t* vals, uint32_t* cnt, uint32_t* out,
-		uint64_t n, DevBuf& tmp, cudaStream_t stream, uint64_t* total) {
+		uint64_t n, DevBuf& tmp, cudaStream_t stream, uint64_t* total,
+		const uint64_t** dev_total = nullptr) {
 	uint64_t tiles = (n + kScanTile - 1) / kScanTile;
 	if (tiles == 0) tiles = 1;
 	LG_TRY(tmp.reserve((tiles + 1) * sizeof(uint64_t)));
@@ -434,6 +435,7 @@ static lg_status exclusive_scan(const In& in, const uint32_t* vals, uint32_t* cn
 		}
 	}
 	LG_CUDA(cudaGetLastError(), "scan launch");
+	if (dev_total) *dev_total = sums + tiles;
 	if (total) {
 		// read through one pinned word per host thread (kept for the
 		// thread's life): per-level loops read a total every step
@@ -455,6 +457,12 @@ static lg_status exclusive_scan(const In& in, const uint32_t* vals, uint32_t* cn
 lg_status exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint64_t n,
 		DevBuf& tmp, cudaStream_t stream, uint64_t* total) {
 	return exclusive_scan<false>(ScanArray{in}, in, nullptr, out, n, tmp, stream, total);
+}
+
+// The total is left at *dev_total (in tmp).
+static lg_status exclusive_scan_u32_dev(const uint32_t* in, uint32_t* out, uint64_t n, DevBuf& tmp,
+		cudaStream_t stream, const uint64_t** dev_total) {
+	return exclusive_scan<false>(ScanArray{in}, in, nullptr, out, n, tmp, stream, nullptr, dev_total);
 }
 
 lg_status exclusive_scan_nonzero(const uint32_t* in, uint32_t* out, uint64_t n, DevBuf& tmp,
@@ -652,7 +660,8 @@ struct VtTab {
 // below minL are never read.
 //
 // The filling walk also writes every fragment's first virtual slot and vertex,
-// and the fragment that holds the first slot of each kSlotTile-slot tile.
+// the fragment that holds the first slot of each kSlotTile-slot tile, and the
+// entry bounds of every kBlockSlots-slot block.
 struct FragOut {
 	const uint32_t* frag_off;
 	const uint32_t* slot_off;
@@ -660,6 +669,8 @@ struct FragOut {
 	uint32_t* start;
 	uint32_t* vert;
 	uint32_t* tile_frag;
+	uint32_t* range_lb;          // lb[r] = first vertex with slot_off >= r * kBlockSlots
+	uint32_t nb;                 // r = 0 .. nb
 };
 template <bool kFill>
 __global__ void walk_fragments(VtTab tab, int L, int minL, uint64_t V, uint32_t* count,
@@ -689,7 +700,17 @@ __global__ void walk_fragments(VtTab tab, int L, int minL, uint64_t V, uint32_t*
 		if ((int)lv <= minL || v >= tab.max_nodes[lv - 1]) break;
 		e = tab.vt[lv - 1][v];
 	}
-	if (!kFill) { count[v] = n; slots_per_vertex[v] = slots; }
+	if (!kFill) {
+		count[v] = n;
+		slots_per_vertex[v] = slots;
+		return;
+	}
+	const uint32_t last = (uint32_t)(((uint64_t)at + slots) / kBlockSlots);
+	if (v == 0) fo.range_lb[0] = 0;
+	for (uint32_t r = at / kBlockSlots + 1u; r <= last && r <= fo.nb; r++)
+		fo.range_lb[r] = (uint32_t)v + 1u;
+	if (v == V - 1)
+		for (uint32_t r = last + 1u; r <= fo.nb; r++) fo.range_lb[r] = (uint32_t)V;
 }
 
 __global__ void live_counts(SnapCsr g, uint32_t* out);
@@ -716,76 +737,85 @@ __global__ void mark_deletions(const uint2* dels, uint64_t n, int L, int minL,
 	if ((threadIdx.x & 31u) == 0 && c) atomicAdd(count, c);
 }
 
-// lb[r] = first vertex e with pos[e] >= r * kBlockSlots (pos has V + 1
-// entries), for r = 0..nb: the entry bounds of every PageRank block.
-__global__ void block_lower_bounds(const uint32_t* pos, uint64_t V, uint64_t nb,
-		uint32_t* lb) {
-	const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (r > nb) return;
-	const uint64_t x = r * kBlockSlots;
-	uint64_t lo = 0, hi = V;                     // answer in [lo, hi]
-	while (lo < hi) {
-		const uint64_t mid = (lo + hi) >> 1;
-		if (pos[mid] < x) lo = mid + 1; else hi = mid;
-	}
-	lb[r] = (uint32_t)lo;
-}
-
 __global__ void sum_u32(const uint32_t* x, uint64_t n, unsigned long long* out) {
 	unsigned long long s = 0;
 	for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
 			i += (uint64_t)gridDim.x * blockDim.x)
 		s += x[i];
-	for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-	if ((threadIdx.x & 31) == 0) atomicAdd(out, s);
+	uint64_t tot;
+	block_excl_scan(s, &tot);
+	if (threadIdx.x == 0 && tot) atomicAdd(out, (unsigned long long)tot);
 }
 
-static lg_status open_dir(lg_snapshot* sn, DevCsr& csr, SnapDir& d) {
-	lg_store* s = sn->store;
-	const int L = sn->level;
-	SnapDir*& spare = s->snap_spare[&csr == &s->out ? 0 : 1];
-	if (spare) d.swap_buffers(*spare);       // a closed snapshot's device buffers
-	const int minL = sn->min_level;
-	const uint64_t V = csr.levels[L]->max_nodes;
-	cudaStream_t st = s->stream;
+// Opening a direction takes three parts, with one wait for both directions
+// after each of the first two; `w` are four of the store's pinned words.
+
+static VtTab vt_tab(const lg_snapshot* sn, const DevCsr& csr) {
 	VtTab tab;
 	std::memset(&tab, 0, sizeof(tab));
-	for (int l = minL; l <= L; l++) {
+	for (int l = sn->min_level; l <= sn->level; l++) {
 		tab.vt[l] = csr.levels[l]->vt.as<lg_vt_entry>();
 		tab.max_nodes[l] = csr.levels[l]->max_nodes;
 	}
-	DevBuf& cnt = d.tmp_cnt;
-	DevBuf& slots = d.tmp_slots;
-	DevBuf& scan_tmp = d.tmp_scan;
-	LG_TRY(cnt.reserve(V * sizeof(uint32_t)));
-	LG_TRY(slots.reserve(V * sizeof(uint32_t)));
+	return tab;
+}
+
+// Fragment and slot counts per vertex and their prefixes; w[0], w[1] = totals.
+static lg_status open_count(lg_snapshot* sn, DevCsr& csr, SnapDir& d, unsigned long long* w) {
+	lg_store* s = sn->store;
+	SnapDir*& spare = s->snap_spare[&csr == &s->out ? 0 : 1];
+	if (spare) d.swap_buffers(*spare);       // a closed snapshot's device buffers
+	const uint64_t V = sn->V;
+	cudaStream_t st = s->stream;
+	LG_TRY(d.tmp_cnt.reserve(V * sizeof(uint32_t)));
+	LG_TRY(d.tmp_slots.reserve(V * sizeof(uint32_t)));
 	LG_TRY(d.deg.reserve(V * sizeof(uint32_t)));
 	LG_TRY(d.frag_off.reserve((V + 1) * sizeof(uint32_t)));
-	const unsigned B = 256;
-	walk_fragments<false><<<grid_for(V, B), B, 0, st>>>(tab, L, minL, V,
-			cnt.as<uint32_t>(), d.deg.as<uint32_t>(), slots.as<uint32_t>(), FragOut{});
+	LG_TRY(d.slot_off.reserve((V + 1) * sizeof(uint32_t)));
+	uint32_t* cnt = d.tmp_cnt.as<uint32_t>();
+	uint32_t* slots = d.tmp_slots.as<uint32_t>();
+	walk_fragments<false><<<grid_for(V, 256), 256, 0, st>>>(vt_tab(sn, csr), sn->level,
+			sn->min_level, V, cnt, d.deg.as<uint32_t>(), slots, FragOut{});
 	LG_CUDA(cudaGetLastError(), "walk_fragments");
-	s->launches += 2 + 2 * scan_launches(V);
 	// fragment prefix, and the per-vertex slot prefix (the virtual slot space
 	// the balanced kernels cut into ranges)
-	uint64_t F = 0, total_slots = 0;
-	LG_TRY(d.slot_off.reserve((V + 1) * sizeof(uint32_t)));
-	LG_TRY(exclusive_scan_u32(cnt.as<uint32_t>(), d.frag_off.as<uint32_t>(), V,
-			scan_tmp, st, &F));
-	LG_TRY(exclusive_scan_u32(slots.as<uint32_t>(), d.slot_off.as<uint32_t>(), V,
-			scan_tmp, st, &total_slots));
+	const uint64_t *f = nullptr, *n = nullptr;
+	LG_TRY(exclusive_scan_u32_dev(cnt, d.frag_off.as<uint32_t>(), V, d.tmp_scan, st, &f));
+	LG_TRY(exclusive_scan_u32_dev(slots, d.slot_off.as<uint32_t>(), V, d.tmp_scan2, st, &n));
+	LG_CUDA(cudaMemcpyAsync(w, f, 8, cudaMemcpyDeviceToHost, st), "scan total");
+	LG_CUDA(cudaMemcpyAsync(w + 1, n, 8, cudaMemcpyDeviceToHost, st), "scan total");
+	s->launches += 1 + 2 * scan_launches(V);
+	s->d2h_bytes += 16;
+	return LG_OK;
+}
+
+// Fragments, deletion bitsets and degrees; w[2] = live edges, w[3] = deletion
+// marks visible.
+static lg_status open_fill(lg_snapshot* sn, DevCsr& csr, SnapDir& d, unsigned long long* w) {
+	lg_store* s = sn->store;
+	const int L = sn->level, minL = sn->min_level;
+	const uint64_t V = sn->V;
+	cudaStream_t st = s->stream;
+	const unsigned B = 256;
+	const uint64_t F = w[0], total_slots = w[1];
+	if (F > 0xffffffffull || total_slots > 0xffffffffull)
+		return set_error(LG_ENOTSUP, "more than 2^32-1 fragments in a snapshot");
 	d.n_frags = F;
+	d.n_frag_slots = total_slots;
+	const uint64_t nb = std::max<uint64_t>(1, (total_slots + kBlockSlots - 1) / kBlockSlots);
+	const uint64_t tiles = total_slots / kSlotTile + 1;
+	// fragments' starts (F + 1) and vertices (F), tiles' fragments
 	LG_TRY(d.frags.reserve(std::max<uint64_t>(F, 1) * sizeof(uint2)));
-	LG_TRY(d.frag_start.reserve((F + 1) * sizeof(uint32_t)));
-	LG_TRY(d.frag_vert.reserve(std::max<uint64_t>(F, 1) * sizeof(uint32_t)));
-	LG_TRY(d.tile_frag.reserve((total_slots / kSlotTile + 1) * sizeof(uint32_t)));
-	walk_fragments<true><<<grid_for(V, B), B, 0, st>>>(tab, L, minL, V, nullptr, nullptr, nullptr,
-			FragOut{d.frag_off.as<uint32_t>(), d.slot_off.as<uint32_t>(), d.frags.as<uint2>(),
-				d.frag_start.as<uint32_t>(), d.frag_vert.as<uint32_t>(),
-				d.tile_frag.as<uint32_t>()});
+	LG_TRY(d.frag_aux.reserve((2 * F + 1 + tiles) * sizeof(uint32_t)));
+	LG_TRY(d.range_lb.reserve((nb + 1) * sizeof(uint32_t)));
+	walk_fragments<true><<<grid_for(V, B), B, 0, st>>>(vt_tab(sn, csr), L, minL, V, nullptr,
+			nullptr, nullptr, FragOut{d.frag_off.as<uint32_t>(), d.slot_off.as<uint32_t>(),
+				d.frags.as<uint2>(), d.frag_start(), d.frag_vert(), d.tile_frag(),
+				d.range_lb.as<uint32_t>(), (uint32_t)nb});
 	LG_CUDA(cudaGetLastError(), "walk_fragments fill");
-	LG_CUDA(cudaMemcpyAsync(d.frag_start.as<uint32_t>() + F, d.slot_off.as<uint32_t>() + V,
-			sizeof(uint32_t), cudaMemcpyDeviceToDevice, st), "slot total");
+	LG_CUDA(cudaMemcpyAsync(d.frag_start() + F, d.slot_off.as<uint32_t>() + V, sizeof(uint32_t),
+			cudaMemcpyDeviceToDevice, st), "slot total");
+	s->launches++;
 
 	// deletion bitsets of levels minL..L
 	std::vector<uint64_t> word_off(L + 2, 0);
@@ -809,55 +839,55 @@ static lg_status open_dir(lg_snapshot* sn, DevCsr& csr, SnapDir& d) {
 	LG_TRY(counters.reserve(2 * sizeof(unsigned long long)));
 	LG_CUDA(cudaMemsetAsync(counters.p, 0, 2 * sizeof(unsigned long long), st), "memset");
 	if (csr.n_dels_dev > 0) {
-		DevBuf& words = d.tmp_words;
-		LG_TRY(words.reserve(sizeof(uint32_t*) * LG_MAX_LEVELS));
-		LG_CUDA(cudaMemcpyAsync(words.p, lt.del, sizeof(lt.del),
-				cudaMemcpyHostToDevice, st), "deletion table");
 		int sms = 148;
 		cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
 		const unsigned mark_blocks = std::min<unsigned>(grid_for(csr.n_dels_dev, B),
 				(unsigned)sms * 8u);
 		mark_deletions<<<mark_blocks, B, 0, st>>>(
 				csr.dels.as<uint2>(), csr.n_dels_dev, L, minL,
-				(uint32_t* const*)words.p, counters.as<unsigned long long>() + 1);
+				const_cast<uint32_t* const*>(d.lt.as<LevelTab>()->del),
+				counters.as<unsigned long long>() + 1);
 		LG_CUDA(cudaGetLastError(), "mark_deletions");
 		s->launches++;
 	}
 	if (minL > 0) {
 		// the vertex table's degree counts edges of every level: in a window
 		// the degree is the number of live slots the chain covers
-		SnapCsr g;
-		g.frag_off = d.frag_off.as<uint32_t>();
-		g.frags = d.frags.as<uint2>();
-		g.lt = d.lt.as<LevelTab>();
-		g.deg = d.deg.as<uint32_t>();
+		SnapCsr g = d.view();
 		g.V = V;
-		g.slot_off = nullptr;
 		live_counts<<<grid_for(V, B), B, 0, st>>>(g, d.deg.as<uint32_t>());
 		LG_CUDA(cudaGetLastError(), "window degrees");
 		s->launches++;
 	}
-
-	{
-		const uint64_t nb = std::max<uint64_t>(1, (total_slots + kBlockSlots - 1) / kBlockSlots);
-		LG_TRY(d.range_lb.reserve((nb + 1) * sizeof(uint32_t)));
-		block_lower_bounds<<<grid_for(nb + 1, B), B, 0, st>>>(d.slot_off.as<uint32_t>(), V,
-				nb, d.range_lb.as<uint32_t>());
-		LG_CUDA(cudaGetLastError(), "block_lower_bounds");
-		s->launches++;
-	}
-	sum_u32<<<592, B, 0, st>>>(d.deg.as<uint32_t>(), V, counters.as<unsigned long long>());
+	sum_u32<<<std::min<unsigned>(grid_for(V, B), 592u), B, 0, st>>>(d.deg.as<uint32_t>(), V,
+			counters.as<unsigned long long>());
 	LG_CUDA(cudaGetLastError(), "degree sum");
 	s->launches++;
-	unsigned long long sums[2] = {0, 0};
-	LG_CUDA(cudaMemcpyAsync(sums, counters.p, sizeof(sums), cudaMemcpyDeviceToHost, st), "d2h");
-	LG_CUDA(cudaStreamSynchronize(st), "snapshot sizes");
-	d.n_edges = sums[0];
-	d.n_frag_slots = total_slots;
+	LG_CUDA(cudaMemcpyAsync(w + 2, counters.p, 16, cudaMemcpyDeviceToHost, st), "d2h");
+	s->d2h_bytes += 16;
+	return LG_OK;
+}
+
+static void open_done(lg_snapshot* sn, DevCsr& csr, SnapDir& d, const unsigned long long* w) {
+	d.n_edges = w[2];
 	d.n_slots = 0;
-	for (int l = minL; l <= L; l++) d.n_slots += csr.levels[l]->n_slots;
-	d.n_dels = sums[1];
+	for (int l = sn->min_level; l <= sn->level; l++) d.n_slots += csr.levels[l]->n_slots;
+	d.n_dels = w[3];
 	d.present = true;
+}
+
+static lg_status open_dirs(lg_snapshot* sn) {
+	lg_store* s = sn->store;
+	unsigned long long* w = nullptr;
+	LG_TRY(host_words(s, &w));
+	LG_TRY(open_count(sn, s->out, sn->out, w));
+	if (s->reverse) LG_TRY(open_count(sn, s->in, sn->in, w + 4));
+	LG_CUDA(cudaStreamSynchronize(s->stream), "snapshot sizes");
+	LG_TRY(open_fill(sn, s->out, sn->out, w));
+	if (s->reverse) LG_TRY(open_fill(sn, s->in, sn->in, w + 4));
+	LG_CUDA(cudaStreamSynchronize(s->stream), "snapshot sizes");
+	open_done(sn, s->out, sn->out, w);
+	if (s->reverse) open_done(sn, s->in, sn->in, w + 4);
 	return LG_OK;
 }
 
@@ -1174,8 +1204,7 @@ lg_status lg_snapshot_open_window(lg_store* s, int level, int min_level,
 	sn->level = level;
 	sn->min_level = min_level;
 	sn->V = s->out.levels[level]->max_nodes;
-	lg_status st = open_dir(sn, s->out, sn->out);
-	if (!st && s->reverse) st = open_dir(sn, s->in, sn->in);
+	const lg_status st = open_dirs(sn);
 	if (st) { cudaStreamSynchronize(s->stream); delete sn; return st; }
 	s->open_snapshots++;
 	*out = sn;
