@@ -542,9 +542,10 @@ lg_status lg_adjoint_free(lg_adjoint* tape);
  * rejected with LG_EINVAL; every value gives the same results, only the
  * speed changes.
  * ------------------------------------------------------------------------- */
-/* Flat-CSR sweeps (PageRank pull, the adjoint's solves): resident CTAs (of
- * 8 warps) per SM of a persistent sweep, each warp looping over 256-edge
- * tiles; 0 = one CTA per 4 tiles, each warp one tile. */
+/* PageRank pull over more than 2^18 in-edges (smaller graphs run all iterations
+ * in one launch): resident CTAs (of 8 warps) per SM of a persistent sweep, each
+ * warp looping over 256-edge tiles; 0 = one CTA per 4 tiles, each warp one
+ * tile. */
 #define LG_TUNE_PR_CTAS_PER_SM  0
 /* Personalized PageRank: columns per pass (a multiple of 32; the K columns
  * run in passes of this many, each pass all iterations), default 256. */

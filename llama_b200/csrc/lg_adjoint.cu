@@ -20,16 +20,15 @@
 // backward sweep reads the weights as given and the forward gathers them
 // once per call into in-edge order.
 //
-// Both sweeps are the flat sweep of lg_flat_sweep.cuh with an affine op:
-// y[v] = base[v] + d * sum over v's edges k of w[k] * x[nbr(k)], and the
-// residual sum |y - x| accumulated per iteration in device memory.  The
-// host does not wait for every iteration: it issues iterations in chunks,
-// every launch first reads the previous iteration's residual and does
-// nothing once it is below tol, and the host reads the residuals of a chunk
-// while the next one runs.  The result is the one the stop-at-first-
-// residual-below-tol loop gives, with no synchronisation per iteration.
+// Both solves run every iteration inside one cooperative launch
+// (lg_flat_run.cuh) with an affine op: y[v] = base[v] + d * sum over v's edges
+// k of w[k] * x[nbr(k)].  The residual sum |y - x| of an iteration is added up
+// on the device before the iteration's barrier, so every CTA stops at the first
+// one below tol, with no launch or wait per iteration.  Bound by the gathers of
+// x and the weights' 8 bytes an edge above some 10^6 edges (15 M edges: 89 us an
+// iteration against 158 us for a launch per iteration at 16.8 M), by the barrier
+// and the loads around it below (30 k edges: 7 us against 14).
 #include "lg_flat_run.cuh"
-#include "lg_flat_sweep.cuh"
 #include "lg_tune.h"
 
 #include <cmath>
@@ -40,84 +39,8 @@
 namespace lg {
 
 constexpr uint32_t kNoPos = 0xffffffffu;
-constexpr int kChunk = 16;            // iterations issued between residual reads
 
-// One iteration of y = base + d * (weighted pull of x) over a flat CSR.
-struct AffOp {
-	static constexpr bool kResidual = true;
-	const uint32_t* nz_rows;   // R
-	const double* w;           // E, in the flat CSR's edge order
-	const double* x;
-	const double* base;
-	double* y;
-	double* resid;             // this iteration's sum |y - x|
-	const double* prev;        // the previous iteration's, null for the first
-	double d, tol;
-	uint32_t E;
-	__device__ __forceinline__ bool skip() const { return prev && __ldcg(prev) < tol; }
-	__device__ __forceinline__ void values(uint32_t eb, const uint32_t (&id)[kFlatPerLane],
-			double (&v)[kFlatPerLane]) const {
-		double wv[kFlatPerLane];
-		if (eb + kFlatPerLane <= E) {
-			// two 32-byte loads (eb is a multiple of 8), streamed
-			asm("ld.global.cs.v4.f64 {%0, %1, %2, %3}, [%4];"
-				: "=d"(wv[0]), "=d"(wv[1]), "=d"(wv[2]), "=d"(wv[3]) : "l"(w + eb));
-			asm("ld.global.cs.v4.f64 {%0, %1, %2, %3}, [%4];"
-				: "=d"(wv[4]), "=d"(wv[5]), "=d"(wv[6]), "=d"(wv[7]) : "l"(w + eb + 4));
-		} else {
-#pragma unroll
-			for (int i = 0; i < kFlatPerLane; i++) wv[i] = eb + i < E ? __ldcs(w + eb + i) : 0.0;
-		}
-#pragma unroll
-		for (int i = 0; i < kFlatPerLane; i++)
-			v[i] = id[i] != kNoId ? __dmul_rn(wv[i], __ldg(x + id[i])) : 0.0;
-	}
-	__device__ __forceinline__ double finish(uint32_t k, double s) const {
-		const uint32_t v = __ldg(nz_rows + k);
-		const double yv = __dadd_rn(__ldg(base + v), __dmul_rn(d, s));
-		y[v] = yv;
-		return fabs(yv - __ldg(x + v));
-	}
-	__device__ __forceinline__ void residual(double r) const { atomicAdd(resid, r); }
-};
-
-__global__ void __launch_bounds__(kFlatWarps * 32)
-aff_flat_step(FlatTiles a, AffOp op) {
-	__shared__ double rowsum[kFlatWarps][kFlatTile];
-	flat_sweep_tile(a, op, rowsum);
-}
-
-template <int kMinBlocks>
-__global__ void __launch_bounds__(kFlatLoopWarps * 32, kMinBlocks)
-aff_flat_loop(FlatTiles a, AffOp op) {
-	__shared__ double rowsum[kFlatLoopWarps][kFlatTile];
-	flat_sweep_loop(a, op, rowsum);
-}
-
-__global__ void __launch_bounds__(kFixupThreads)
-aff_flat_fixup(FlatTiles a, AffOp op) {
-	flat_sweep_fixup_body(a, op);
-}
-
-// Rows without edges: y[v] = base[v] in every iteration.  Written into y
-// with their first-iteration residual |base - x0| added to resid0, or (resid0
-// null) just written.
-__global__ void aff_empty_rows(const uint32_t* off, uint64_t V, const double* base,
-		const double* x0, double* y, double* resid0) {
-	const uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	double r = 0.0;
-	if (v < V && __ldg(off + v + 1) == __ldg(off + v)) {
-		const double b = __ldg(base + v);
-		y[v] = b;
-		if (resid0) r = fabs(b - __ldg(x0 + v));
-	}
-	if (!resid0) return;
-#pragma unroll
-	for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-	if ((threadIdx.x & 31u) == 0 && r != 0.0) atomicAdd(resid0, r);
-}
-
-// The same iterations inside one cooperative launch (lg_flat_run.cuh).
+// The iterations y = base + d * (weighted pull of x) over a flat CSR.
 struct AffRunOp {
 	static constexpr bool kResidual = true;
 	const uint32_t* nz_rows;
@@ -338,13 +261,7 @@ struct lg_adjoint_maps {
 	DevBuf src;            // E u32: source of each out-adjacency position
 	uint64_t E = 0;
 	// solve buffers, reused by every call on the snapshot
-	DevBuf xa, xb, base, win, carries, resid, run, stage_w, stage_v, stage_g;
-	double* resid_host = nullptr;          // pinned, 2 * kChunk
-	cudaEvent_t chunk_done[2] = {nullptr, nullptr};
-	~lg_adjoint_maps() {
-		if (resid_host) cudaFreeHost(resid_host);
-		for (cudaEvent_t e : chunk_done) if (e) cudaEventDestroy(e);
-	}
+	DevBuf xa, xb, base, win, resid, run, stage_w, stage_v, stage_g;
 };
 
 struct lg_adjoint {
@@ -414,10 +331,6 @@ lg_status build_maps(lg_snapshot* sn, lg_adjoint_maps* m) {
 	if (bad)
 		return set_error(LG_EINVAL, "out- and in-CSR of the snapshot disagree, or a "
 				"fragment is not sorted by neighbour id (code %u)", bad);
-	LG_CUDA(cudaHostAlloc((void**)&m->resid_host, 2 * kChunk * sizeof(double),
-			cudaHostAllocDefault), "cudaHostAlloc");
-	for (cudaEvent_t& e : m->chunk_done)
-		LG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
 	return LG_OK;
 }
 
@@ -464,113 +377,40 @@ lg_status fixed_point(lg_snapshot* sn, const FlatCsr& f, const double* w, const 
 	const uint64_t V = sn->V;
 	double* A = m->xa.as<double>();
 	double* B = m->xb.as<double>();
-	LG_TRY(m->carries.reserve(2ull * std::max<uint32_t>(f.ntiles, 1) * sizeof(double)));
 	LG_TRY(m->resid.reserve((size_t)max_iter * sizeof(double)));
 	double* resid = m->resid.as<double>();
 	LG_CUDA(cudaMemsetAsync(resid, 0, (size_t)max_iter * sizeof(double), st), "memset");
-	const FlatTiles a = flat_tiles(f, m->carries.as<double>());
-	const uint32_t* off = f.off.as<uint32_t>();
-	const int ctas = (int)tune_value(s->device, LG_TUNE_PR_CTAS_PER_SM);
-	const int resident = ctas > 0 ? 0 : aff_run_resident(s->device);
-	if (resident > 0) {
-		// every iteration in one launch
-		LG_TRY(m->run.reserve(sizeof(RunCtl)));
-		RunCtl* ctl = m->run.as<RunCtl>();
-		LG_CUDA(cudaMemsetAsync(&ctl->bar, 0, sizeof(RunCtl) - offsetof(RunCtl, bar), st), "memset");
-		AffRunArgs g;
-		g.a = a;
-		g.off = off;
-		g.nz_rows = f.nz_rows();
-		g.w = w;
-		g.base = base;
-		g.xa = A;
-		g.xb = B;
-		g.totals = resid;
-		g.d = d;
-		g.tol = tol;
-		g.V = (uint32_t)V;
-		g.max_iter = max_iter;
-		void* args[] = {&g, &ctl};
-		LG_CUDA(cudaLaunchCooperativeKernel((const void*)aff_run, dim3(run_ctas(f.ntiles, resident)),
-				dim3(kRunThreads), args, sizeof(RunShared), st), "aff_run");
-		s->launches++;
-		unsigned long long h[4];
-		static_assert(sizeof(CoopBar) == 16 && sizeof(RunCtl) - offsetof(RunCtl, bar) == 32,
-				"barrier, residual, iterations");
-		LG_TRY(read_words(s, (const unsigned long long*)&ctl->bar, 4, h));
-		if ((unsigned)h[1] & 1u)
-			return set_error(LG_ETIMEOUT, "pagerank: a grid barrier wait ran out");
-		memcpy(resid_out, &h[2], sizeof(double));
-		*iters = (int)(uint32_t)h[3];
-		*out = (*iters & 1) ? B : A;
-		return LG_OK;
-	}
-	AffOp op;
-	op.nz_rows = f.nz_rows();
-	op.w = w;
-	op.base = base;
-	op.d = d;
-	op.tol = tol;
-	op.E = (uint32_t)f.E;
-	int sms = 148;
-	if (ctas > 0) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
-	aff_empty_rows<<<grid_for(V, 256), 256, 0, st>>>(off, V, base, A, B, resid);
+	const int resident = aff_run_resident(s->device);
+	if (resident <= 0) return set_error(LG_ENOTSUP, "the device has no cooperative launch");
+	LG_TRY(m->run.reserve(sizeof(RunCtl)));
+	RunCtl* ctl = m->run.as<RunCtl>();
+	LG_CUDA(cudaMemsetAsync(&ctl->bar, 0, sizeof(RunCtl) - offsetof(RunCtl, bar), st), "memset");
+	AffRunArgs g;
+	g.a = flat_tiles(f, nullptr);
+	g.off = f.off.as<uint32_t>();
+	g.nz_rows = f.nz_rows();
+	g.w = w;
+	g.base = base;
+	g.xa = A;
+	g.xb = B;
+	g.totals = resid;
+	g.d = d;
+	g.tol = tol;
+	g.V = (uint32_t)V;
+	g.max_iter = max_iter;
+	void* args[] = {&g, &ctl};
+	LG_CUDA(cudaLaunchCooperativeKernel((const void*)aff_run, dim3(run_ctas(f.ntiles, resident)),
+			dim3(kRunThreads), args, sizeof(RunShared), st), "aff_run");
 	s->launches++;
-	int done = -1;          // iterations after which the residual fell below tol
-	int issued = 0, chunk = 0, prev_first = 0, prev_n = 0;
-	double r = 0.0;
-	// waits for chunk c's residual copy and finds the first one below tol
-	auto check = [&](int c, int first, int cnt) -> lg_status {
-		LG_CUDA(cudaEventSynchronize(m->chunk_done[c & 1]), "adjoint step");
-		const double* h = m->resid_host + (c & 1) * kChunk;
-		for (int k = 0; k < cnt && done < 0; k++) {
-			r = h[k];
-			if (r < tol) done = first + k + 1;
-		}
-		return LG_OK;
-	};
-	while (issued < max_iter && done < 0) {
-		const int n = std::min(kChunk, max_iter - issued);
-		for (int j = 0; j < n; j++) {
-			const int it = issued + j;
-			op.x = (it & 1) ? B : A;
-			op.y = (it & 1) ? A : B;
-			op.resid = resid + it;
-			op.prev = it > 0 ? resid + it - 1 : nullptr;
-			if (f.ntiles > 0) {
-				launch_flat_sweep(a, op, sms, ctas, st, aff_flat_step, aff_flat_loop<4>,
-						aff_flat_loop<6>, aff_flat_loop<8>);
-				s->launches++;
-			}
-			if (f.ntiles > 1) {
-				aff_flat_fixup<<<flat_fixup_blocks(f.ntiles), kFixupThreads, 0, st>>>(a, op);
-				s->launches++;
-			}
-			if (it == 0) {
-				// A is read again by the third iteration: its rows without
-				// edges take their constant value now
-				aff_empty_rows<<<grid_for(V, 256), 256, 0, st>>>(off, V, base, nullptr, A,
-						nullptr);
-				s->launches++;
-			}
-		}
-		LG_CUDA(cudaGetLastError(), "adjoint step");
-		LG_CUDA(cudaMemcpyAsync(m->resid_host + (chunk & 1) * kChunk, resid + issued,
-				n * sizeof(double), cudaMemcpyDeviceToHost, st), "d2h");
-		LG_CUDA(cudaEventRecord(m->chunk_done[chunk & 1], st), "event");
-		s->d2h_bytes += n * sizeof(double);
-		// the previous chunk's residuals are read while this one runs
-		if (chunk > 0) LG_TRY(check(chunk - 1, prev_first, prev_n));
-		prev_first = issued;
-		prev_n = n;
-		issued += n;
-		chunk++;
-	}
-	if (done < 0 && chunk > 0) LG_TRY(check(chunk - 1, prev_first, prev_n));
-	if (done < 0) done = max_iter;
-	*iters = done;
-	*resid_out = r;
-	*out = (done & 1) ? B : A;
+	unsigned long long h[4];
+	static_assert(sizeof(CoopBar) == 16 && sizeof(RunCtl) - offsetof(RunCtl, bar) == 32,
+			"barrier, residual, iterations");
+	LG_TRY(read_words(s, (const unsigned long long*)&ctl->bar, 4, h));
+	if ((unsigned)h[1] & 1u)
+		return set_error(LG_ETIMEOUT, "pagerank: a grid barrier wait ran out");
+	memcpy(resid_out, &h[2], sizeof(double));
+	*iters = (int)(uint32_t)h[3];
+	*out = (*iters & 1) ? B : A;
 	return LG_OK;
 }
 

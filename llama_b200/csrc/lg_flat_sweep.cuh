@@ -1,6 +1,6 @@
 // lg_flat_sweep.cuh - one pass of "row sum of gathered edge values" over a
-// flat CSR (lg_flat.cuh), shared by PageRank (lg_pagerank.cu) and the
-// weighted fixed-point solves of the adjoint PageRank (lg_adjoint.cu).
+// flat CSR (lg_flat.cuh), a launch of its own: PageRank over graphs too large
+// for the one-launch form (lg_flat_run.cuh).
 //
 // flat_sweep_tile gives each warp a tile of kFlatTile consecutive edges, 8 per
 // lane: it issues the tile's id loads and the op's value loads up front,
@@ -14,13 +14,10 @@
 // launch lists and profiles name the computation.
 //
 // An Op supplies
-//   bool   skip() const                      the whole launch is a no-op
 //   void   values(eb, id[8], x[8]) const     the 8 edge values of a lane
 //                                            (id = kNoId past the end)
-//   double finish(k, s) const                row k (index into nz_rows) has
-//                                            sum s; returns its residual term
-//   void   residual(r) const                 one warp's residual total
-//   static constexpr bool kResidual          finish() returns something
+//   void   finish(k, s) const                row k (index into nz_rows) has
+//                                            sum s
 #ifndef LG_FLAT_SWEEP_CUH_
 #define LG_FLAT_SWEEP_CUH_
 
@@ -69,9 +66,9 @@ inline FlatTiles flat_tiles(const FlatCsr& f, double* carries) {
 // open row's total so far.
 //
 // Processes tile t with the calling warp (rs: the warp's kFlatTile doubles
-// of shared memory) and returns the lane's residual terms.
+// of shared memory).
 template <class Op>
-__device__ __forceinline__ double flat_sweep_one(const FlatTiles& a, const Op& op, double* rs,
+__device__ __forceinline__ void flat_sweep_one(const FlatTiles& a, const Op& op, double* rs,
 		uint32_t t) {
 	const uint32_t lane = threadIdx.x & 31u;
 	const uint32_t e0 = t * kFlatTile;
@@ -152,18 +149,7 @@ __device__ __forceinline__ double flat_sweep_one(const FlatTiles& a, const Op& o
 	__syncwarp();
 	const uint32_t done = (H > 0 && !closes) ? H - 1 : H;
 	const uint32_t seg0 = __ldg(a.tile_seg + t);
-	double res = 0.0;
-	for (uint32_t r = lane; r < done; r += 32u) res += op.finish(seg0 + r, rs[r]);
-	return res;
-}
-
-template <class Op>
-__device__ __forceinline__ void flat_sweep_residual(const Op& op, double res) {
-	if (Op::kResidual) {
-#pragma unroll
-		for (int o = 16; o > 0; o >>= 1) res += __shfl_xor_sync(0xffffffffu, res, o);
-		if ((threadIdx.x & 31u) == 0 && res != 0.0) op.residual(res);
-	}
+	for (uint32_t r = lane; r < done; r += 32u) op.finish(seg0 + r, rs[r]);
 }
 
 // Body of a kernel launched with kFlatWarps * 32 threads per CTA and one
@@ -174,8 +160,8 @@ __device__ __forceinline__ void flat_sweep_tile(const FlatTiles& a, const Op& op
 		double (*rowsum)[kFlatTile]) {
 	const uint32_t wid = threadIdx.x >> 5;
 	const uint32_t t = blockIdx.x * kFlatWarps + wid;
-	if (t >= a.ntiles || op.skip()) return;          // whole warps leave together
-	flat_sweep_residual(op, flat_sweep_one(a, op, rowsum[wid], t));
+	if (t >= a.ntiles) return;                       // whole warps leave together
+	flat_sweep_one(a, op, rowsum[wid], t);
 }
 
 // The persistent form: a grid of a few CTAs per SM whose warps loop over the
@@ -185,15 +171,12 @@ __device__ __forceinline__ void flat_sweep_tile(const FlatTiles& a, const Op& op
 template <class Op>
 __device__ __forceinline__ void flat_sweep_loop(const FlatTiles& a, const Op& op,
 		double (*rowsum)[kFlatTile]) {
-	if (op.skip()) return;
 	const uint32_t wid = threadIdx.x >> 5;
 	const uint32_t stride = gridDim.x * kFlatLoopWarps;
-	double res = 0.0;
 	for (uint32_t t = blockIdx.x * kFlatLoopWarps + wid; t < a.ntiles; t += stride) {
-		res += flat_sweep_one(a, op, rowsum[wid], t);
+		flat_sweep_one(a, op, rowsum[wid], t);
 		__syncwarp();                     // rowsum is reused by the next tile
 	}
-	flat_sweep_residual(op, res);
 }
 
 // Rows that cross tile boundaries: boundary t (edge t * kFlatTile) owns the
@@ -203,7 +186,6 @@ __device__ __forceinline__ void flat_sweep_loop(const FlatTiles& a, const Op& op
 // tiles are summed by the whole warp.
 template <class Op>
 __device__ __forceinline__ void flat_sweep_fixup_body(const FlatTiles& a, const Op& op) {
-	if (op.skip()) return;
 	const uint32_t lane = threadIdx.x & 31u;
 	const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 	const uint32_t t = w * 32u + lane + 1u;
@@ -223,11 +205,10 @@ __device__ __forceinline__ void flat_sweep_fixup_body(const FlatTiles& a, const 
 			}
 		}
 	}
-	double res = 0.0;
 	if (own && t1 - t < 4) {
 		double s = __ldcg(a.carry_last + t - 1);
 		for (uint32_t x = t; x <= t1; x++) s += __ldcg(a.carry_first + x);
-		res += op.finish(k, s);
+		op.finish(k, s);
 		own = false;
 	}
 	uint32_t mm = __ballot_sync(0xffffffffu, own);
@@ -241,12 +222,7 @@ __device__ __forceinline__ void flat_sweep_fixup_body(const FlatTiles& a, const 
 		for (uint32_t x = tt + lane; x <= tt1; x += 32u) s += __ldcg(a.carry_first + x);
 #pragma unroll
 		for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-		if (lane == 0) res += op.finish(kk, __ldcg(a.carry_last + tt - 1) + s);
-	}
-	if (Op::kResidual) {
-#pragma unroll
-		for (int o = 16; o > 0; o >>= 1) res += __shfl_xor_sync(0xffffffffu, res, o);
-		if (lane == 0 && res != 0.0) op.residual(res);
+		if (lane == 0) op.finish(kk, __ldcg(a.carry_last + tt - 1) + s);
 	}
 }
 

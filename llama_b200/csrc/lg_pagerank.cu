@@ -51,7 +51,6 @@ constexpr uint32_t kPrLong = 64;       // entries with more slots are reduced by
 // is the gathered contribution of its source; a row's sum s gives
 // pr = (1-d)/N + d*s and the next contribution pr / out_degree.
 struct PrOp {
-	static constexpr bool kResidual = false;
 	const uint32_t* nz_rows;   // R
 	const uint32_t* nz_outdeg; // R: out-degree of nz_rows[k]
 	const double* contrib;
@@ -59,22 +58,19 @@ struct PrOp {
 	double* pr_out;            // written when non-null (last iteration)
 	double base;               // (1 - d) / N
 	double d;
-	__device__ __forceinline__ bool skip() const { return false; }
 	__device__ __forceinline__ void values(uint32_t, const uint32_t (&id)[kFlatPerLane],
 			double (&x)[kFlatPerLane]) const {
 #pragma unroll
 		for (int i = 0; i < kFlatPerLane; i++)
 			x[i] = id[i] != kNoId ? __ldg(contrib + id[i]) : 0.0;
 	}
-	__device__ __forceinline__ double finish(uint32_t k, double s) const {
+	__device__ __forceinline__ void finish(uint32_t k, double s) const {
 		const uint32_t v = __ldg(nz_rows + k);
 		const double pr = __dadd_rn(base, __dmul_rn(d, s));
 		const uint32_t dg = __ldg(nz_outdeg + k);
 		contrib_next[v] = dg ? pr / (double)dg : 0.0;
 		if (pr_out) pr_out[v] = pr;
-		return 0.0;
 	}
-	__device__ __forceinline__ void residual(double) const {}
 };
 
 __global__ void __launch_bounds__(kFlatWarps * 32)
@@ -419,9 +415,7 @@ lg_status pagerank_over(lg_snapshot* sn, FlatCsr* f, int iterations, double damp
 	}
 	double* c0 = sc[0].as<double>();
 	double* c1 = sc[1].as<double>();
-	const int ctas = (int)tune_value(s->device, LG_TUNE_PR_CTAS_PER_SM);
-	const int resident = ctas > 0 || iterations == 0 || ntiles > kPrRunTiles ? 0
-			: pr_run_resident(s->device);
+	const int resident = iterations == 0 || ntiles > kPrRunTiles ? 0 : pr_run_resident(s->device);
 	if (resident > 0) {
 		LG_TRY(s->run_ctl.reserve(sizeof(RunCtl)));
 		RunCtl* ctl = s->run_ctl.as<RunCtl>();
@@ -470,6 +464,7 @@ lg_status pagerank_over(lg_snapshot* sn, FlatCsr* f, int iterations, double damp
 	LG_CUDA(cudaGetLastError(), "pr_init");
 	s->launches += 2;
 	const unsigned fix_blocks = flat_fixup_blocks(ntiles);   // a thread per tile boundary
+	const int ctas = (int)tune_value(s->device, LG_TUNE_PR_CTAS_PER_SM);
 	const bool occ8 = tune_value(s->device, LG_TUNE_PR_TILE_OCC) == 8;
 	int sms = 148;
 	if (ctas > 0) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);

@@ -1,12 +1,10 @@
 """Iterations inside one launch (PageRank over small in-CSRs, the weighted fixed
 point) at the edges of tiles, warp runs and CTAs, with rows over many of them,
-against a plain FP64 evaluation and the launch-per-iteration form
-(LG_TUNE_PR_CTAS_PER_SM = 4)."""
+against a plain FP64 evaluation."""
 import numpy as np
 import pytest
 
 from llama_b200 import Store
-from llama_b200.graph import tune_reset, tune_set
 from tests._util import max_rel_err
 
 pytestmark = pytest.mark.gpu
@@ -43,11 +41,6 @@ def test_pagerank(V, n, hub):
                 got = sn.pagerank_pull(it)
                 assert max_rel_err(got, x) <= 1e-12
                 assert np.array_equal(sn.pagerank_pull(it), got)
-                tune_set(0, "pr_ctas_per_sm", 4)
-                try:
-                    assert max_rel_err(sn.pagerank_pull(it), got) <= 1e-12
-                finally:
-                    tune_reset(0)
 
 
 def test_pagerank_device_output_and_sync():
@@ -83,12 +76,6 @@ def test_fixed_point_and_gradient(V, n, hub):
             lam = dv / 0.15
             assert np.abs(g + 0.85 * np.bincount(s, w * lam[d], V) - lam).sum() <= 2e-13
             assert np.allclose(dw, 0.85 * lam[d] * x[s], rtol=1e-12, atol=0)
-            tune_set(0, "pr_ctas_per_sm", 4)
-            try:
-                x2, _, r2 = sn.pagerank_fwd(w, v, tol=1e-13, keep_tape=False)
-            finally:
-                tune_reset(0)
-            assert np.abs(x2 - x).sum() <= 2e-13 and abs(r.iterations - r2.iterations) <= 1
             x3, _, r3 = sn.pagerank_fwd(w, v, tol=1e-300, max_iter=3, keep_tape=False)
             # (without a path of three edges the residual is 0 before)
             assert r3.iterations == 3 if n > 1 else r3.iterations <= 3
