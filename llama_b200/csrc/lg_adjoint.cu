@@ -141,71 +141,88 @@ aff_run(AffRunArgs g, RunCtl* c) {
 
 // --- per-snapshot maps ----------------------------------------------------
 
-// out_pos[k] for every out-CSR virtual slot k: position of the live edge in
-// the out-adjacency order (kNoPos for deleted slots); also src/dst per
-// position.  One thread per vertex, walking its chain.
-__global__ void adj_out_map(SnapCsr g, const uint32_t* slot_off, const uint64_t* adj_off,
-		uint32_t* out_pos, uint32_t* src, uint32_t* dst, uint32_t* bad) {
-	const uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (v >= g.V) return;
-	const LevelTab* lt = g.lt;
-	uint64_t p = adj_off[v];
-	uint32_t k = slot_off[v];
-	for (uint32_t f = g.frag_off[v]; f < g.frag_off[v + 1]; f++) {
-		const uint2 fr = g.frags[f];
-		const uint32_t lv = frag_level(fr);
-		for (uint32_t i = 0; i < frag_len(fr); i++, k++) {
-			const uint32_t idx = fr.x + i;
-			if (slot_deleted(lt, lv, idx)) { out_pos[k] = kNoPos; continue; }
-			out_pos[k] = (uint32_t)p;
-			src[p] = (uint32_t)v;
-			dst[p] = lt->ids[lv][idx];
-			p++;
-		}
+// row_of[k] = the vertex whose row holds edge k of a flat CSR (lane j of the
+// warp owning tile t: edges 256 t + 8 j .. + 7).
+constexpr int kMapWarps = 8;
+__device__ __forceinline__ void edge_rows(const uint32_t* heads, const uint32_t* nz_rows,
+		const uint32_t* tile_seg, uint32_t E, uint32_t t, uint32_t (&v)[kFlatPerLane]) {
+	const uint32_t lane = threadIdx.x & 31u;
+	const uint32_t eb = t * kFlatTile + lane * kFlatPerLane;
+	const uint32_t hb = __ldg(reinterpret_cast<const unsigned char*>(heads)
+			+ (size_t)t * (kFlatTile / 8) + lane);
+	uint32_t before = __popc(hb);               // heads in the lanes to the left
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1) {
+		const uint32_t q = __shfl_up_sync(0xffffffffu, before, o);
+		if (lane >= (uint32_t)o) before += q;
 	}
-	if (p != adj_off[v + 1]) atomicOr(bad, 1u);
+	before -= __popc(hb);
+	uint32_t row = __ldg(tile_seg + t) + before - 1u;
+	uint32_t x = eb < E && !(hb & 1u) ? __ldg(nz_rows + row) : 0u;
+#pragma unroll
+	for (int i = 0; i < kFlatPerLane; i++) {
+		if ((hb >> i) & 1u) x = __ldg(nz_rows + ++row);
+		v[i] = x;
+	}
 }
 
-// in_pos[q] for every in-CSR virtual slot q of vertex t holding source w:
-// the out-adjacency position of edge (w -> t), found by binary search in
-// w's out-fragments (each sorted by target id).
-__global__ void adj_in_map(SnapCsr in, const uint32_t* in_slot_off, SnapCsr out,
-		const uint32_t* out_slot_off, const uint32_t* out_pos, uint32_t* in_pos,
-		uint32_t* bad) {
-	const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (t >= in.V) return;
-	uint32_t q = in_slot_off[t];
-	for (uint32_t f = in.frag_off[t]; f < in.frag_off[t + 1]; f++) {
-		const uint2 fr = in.frags[f];
-		const uint32_t lv = frag_level(fr);
-		for (uint32_t i = 0; i < frag_len(fr); i++, q++) {
-			const uint32_t idx = fr.x + i;
-			if (slot_deleted(in.lt, lv, idx)) { in_pos[q] = kNoPos; continue; }
-			const uint32_t w = in.lt->ids[lv][idx];
-			uint32_t found = kNoPos, k = out_slot_off[w];
-			for (uint32_t g2 = out.frag_off[w]; g2 < out.frag_off[w + 1] && found == kNoPos; g2++) {
-				const uint2 of = out.frags[g2];
-				const uint32_t* ids = out.lt->ids[frag_level(of)] + of.x;
-				uint32_t lo = 0, hi = frag_len(of);
-				while (lo < hi) {
-					const uint32_t mid = (lo + hi) >> 1;
-					if (ids[mid] < (uint32_t)t) lo = mid + 1; else hi = mid;
-				}
-				// the live copy of (w, t): skip deleted duplicates
-				for (uint32_t j = lo; j < frag_len(of) && ids[j] == (uint32_t)t; j++)
-					if (out_pos[k + j] != kNoPos) { found = out_pos[k + j]; break; }
-				k += frag_len(of);
+__global__ void __launch_bounds__(kMapWarps * 32)
+adj_sources(const uint32_t* heads, const uint32_t* nz_rows, const uint32_t* tile_seg, uint32_t E,
+		uint32_t ntiles, uint32_t* src) {
+	const uint32_t t = blockIdx.x * kMapWarps + (threadIdx.x >> 5);
+	if (t >= ntiles) return;
+	uint32_t v[kFlatPerLane];
+	edge_rows(heads, nz_rows, tile_seg, E, t, v);
+	const uint32_t eb = t * kFlatTile + (threadIdx.x & 31u) * kFlatPerLane;
+#pragma unroll
+	for (int i = 0; i < kFlatPerLane; i++)
+		if (eb + i < E) src[eb + i] = v[i];
+}
+
+// in_pos[k] for every edge k = (w -> t) of the flat in-CSR: its out-adjacency
+// position, found by binary search of t in w's out-fragments (each sorted by
+// target id) and read from out_pos, the out-CSR's virtual slots' positions.
+__global__ void __launch_bounds__(kMapWarps * 32)
+adj_in_map(const uint32_t* ids, const uint32_t* heads, const uint32_t* nz_rows,
+		const uint32_t* tile_seg, uint32_t E, uint32_t ntiles, SnapCsr out,
+		const uint32_t* frag_start, const uint32_t* out_pos, uint32_t* in_pos, uint32_t* bad) {
+	const uint32_t tile = blockIdx.x * kMapWarps + (threadIdx.x >> 5);
+	if (tile >= ntiles) return;
+	uint32_t v[kFlatPerLane];
+	edge_rows(heads, nz_rows, tile_seg, E, tile, v);
+	const uint32_t eb = tile * kFlatTile + (threadIdx.x & 31u) * kFlatPerLane;
+	bool miss = false;
+#pragma unroll
+	for (int i = 0; i < kFlatPerLane; i++) {
+		if (eb + i >= E) break;
+		const uint32_t t = v[i], w = __ldg(ids + eb + i);
+		uint32_t found = kNoPos;
+		const uint32_t f1 = __ldg(out.frag_off + w + 1);
+		for (uint32_t f = __ldg(out.frag_off + w); f < f1 && found == kNoPos; f++) {
+			const uint2 of = out.frags[f];
+			const uint32_t* at = out.lt->ids[frag_level(of)] + of.x;
+			uint32_t lo = 0, hi = frag_len(of);
+			while (lo < hi) {
+				const uint32_t mid = (lo + hi) >> 1;
+				if (__ldg(at + mid) < t) lo = mid + 1; else hi = mid;
 			}
-			in_pos[q] = found;
-			if (found == kNoPos) atomicOr(bad, 1u);
+			// the live copy of (w, t): skip deleted duplicates
+			const uint32_t k = __ldg(frag_start + f);
+			for (uint32_t j = lo; j < frag_len(of) && __ldg(at + j) == t; j++) {
+				const uint32_t p = __ldg(out_pos + k + j);
+				if (p != kNoPos) { found = p; break; }
+			}
 		}
+		in_pos[eb + i] = found;
+		miss |= found == kNoPos;
 	}
+	if (miss) atomicOr(bad, 1u);
 }
 
 __global__ void gather_weights(const uint32_t* map, uint64_t n, const double* w,
 		double* out) {
 	const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i < n) { const uint32_t p = map[i]; out[i] = p == kNoPos ? 0.0 : w[p]; }
+	if (i < n) out[i] = w[map[i]];
 }
 
 __global__ void scale_vec(const double* a, double s, uint64_t n, double* out) {
@@ -217,38 +234,6 @@ __global__ void edge_grad(const uint32_t* src, const uint32_t* dst, uint64_t E, 
 		const double* lam, const double* x, double* out) {
 	const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
 	if (p < E) out[p] = d * (lam[dst[p]] * x[src[p]]);
-}
-
-__global__ void widen_prefix(const uint32_t* p32, uint64_t n, uint64_t* p64) {
-	const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i <= n) p64[i] = p32[i];
-}
-
-// 1 for the virtual in-slots that hold a live edge
-__global__ void live_flags(const uint32_t* pos, uint64_t n, uint32_t* flag) {
-	const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i < n) flag[i] = pos[i] != kNoPos;
-}
-
-// in_pos of the flat in-CSR: the live virtual slots' positions, compacted in
-// slot order (the order in which the flat in-CSR lists them); each one's
-// source must be the flat in-edge's id
-__global__ void compact_in_pos(const uint32_t* pos, const uint32_t* at, uint64_t n,
-		const uint32_t* src, const uint32_t* flat_ids, uint32_t* out, uint32_t* bad) {
-	const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= n) return;
-	const uint32_t p = pos[i];
-	if (p == kNoPos) return;
-	const uint32_t k = at[i];
-	out[k] = p;
-	if (src[p] != __ldg(flat_ids + k)) atomicOr(bad, 2u);
-}
-
-// the flat out-CSR must list the out-edges in out-adjacency order
-__global__ void check_out_order(const uint32_t* dst, const uint32_t* flat_ids, uint64_t E,
-		uint32_t* bad) {
-	const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (p < E && dst[p] != flat_ids[p]) atomicOr(bad, 4u);
 }
 
 } // namespace lg
@@ -277,60 +262,36 @@ namespace {
 lg_status build_maps(lg_snapshot* sn, lg_adjoint_maps* m) {
 	lg_store* s = sn->store;
 	cudaStream_t st = s->stream;
-	const uint64_t V = sn->V;
 	const uint64_t E = m->E;
-	DevBuf out_pos(s->pool), in_pos(s->pool), dst(s->pool), adj_off(s->pool), p32(s->pool),
-			scan_tmp(s->pool), badb(s->pool), flag(s->pool), at(s->pool);
-	LG_TRY(out_pos.reserve(std::max<uint64_t>(sn->out.n_frag_slots, 1) * 4));
-	LG_TRY(in_pos.reserve(std::max<uint64_t>(sn->in.n_frag_slots, 1) * 4));
-	LG_TRY(m->src.reserve(std::max<uint64_t>(E, 1) * 4));
-	LG_TRY(dst.reserve(std::max<uint64_t>(E, 1) * 4));
-	LG_TRY(adj_off.reserve((V + 1) * 8));
-	LG_TRY(p32.reserve((V + 1) * 4));
-	LG_TRY(badb.reserve(4));
-	uint64_t tot = 0;
-	LG_TRY(exclusive_scan_u32(sn->out.deg.as<uint32_t>(), p32.as<uint32_t>(), V, scan_tmp, st,
-			&tot));
-	if (tot != E) return set_error(LG_EINVAL, "out-degrees do not add up to the live edges");
-	LG_CUDA(cudaMemsetAsync(badb.p, 0, 4, st), "memset");
-	widen_prefix<<<grid_for(V + 1, 256), 256, 0, st>>>(p32.as<uint32_t>(), V,
-			adj_off.as<uint64_t>());
-	const SnapCsr out = sn->view(0), in = sn->view(1);
-	adj_out_map<<<grid_for(V, 128), 128, 0, st>>>(out, sn->out.slot_off.as<uint32_t>(),
-			adj_off.as<uint64_t>(), out_pos.as<uint32_t>(), m->src.as<uint32_t>(),
-			dst.as<uint32_t>(), badb.as<uint32_t>());
-	adj_in_map<<<grid_for(V, 128), 128, 0, st>>>(in, sn->in.slot_off.as<uint32_t>(), out,
-			sn->out.slot_off.as<uint32_t>(), out_pos.as<uint32_t>(), in_pos.as<uint32_t>(),
-			badb.as<uint32_t>());
-	LG_CUDA(cudaGetLastError(), "adjoint maps");
-	s->launches += 3;
-	// flat CSRs of both directions; the in-edge map compacted to the flat order
+	// flat CSRs of both directions, the out-edges' sources, and every in-edge's
+	// place among the out-edges
 	LG_TRY(build_flat(sn, 1, m->fin, false));
-	LG_TRY(build_flat(sn, 0, m->fout, false));
+	LG_TRY(build_flat(sn, 0, m->fout, false, false));
 	if (m->fin.E != E || m->fout.E != E)
 		return set_error(LG_EINVAL, "the in- and out-CSR of the snapshot differ in edge count");
-	const uint64_t n = sn->in.n_frag_slots;
-	LG_TRY(flag.reserve(std::max<uint64_t>(n, 1) * 4));
-	LG_TRY(at.reserve((n + 1) * 4));
+	DevBuf out_pos(s->pool), badb(s->pool);
+	LG_TRY(out_pos.reserve(std::max<uint64_t>(sn->out.n_frag_slots, 1) * 4));
+	LG_TRY(m->src.reserve(std::max<uint64_t>(E, 1) * 4));
 	LG_TRY(m->in_pos.reserve(std::max<uint64_t>(E, 1) * 4));
-	live_flags<<<grid_for(n, 256), 256, 0, st>>>(in_pos.as<uint32_t>(), n, flag.as<uint32_t>());
-	LG_CUDA(cudaGetLastError(), "live flags");
-	uint64_t live = 0;
-	LG_TRY(exclusive_scan_u32(flag.as<uint32_t>(), at.as<uint32_t>(), n, scan_tmp, st, &live));
-	if (live != E) return set_error(LG_EINVAL, "in-CSR live slots differ from the edge count");
-	compact_in_pos<<<grid_for(n, 256), 256, 0, st>>>(in_pos.as<uint32_t>(), at.as<uint32_t>(),
-			n, m->src.as<uint32_t>(), m->fin.ids.as<uint32_t>(), m->in_pos.as<uint32_t>(),
-			badb.as<uint32_t>());
-	check_out_order<<<grid_for(E, 256), 256, 0, st>>>(dst.as<uint32_t>(),
-			m->fout.ids.as<uint32_t>(), E, badb.as<uint32_t>());
-	s->launches += 4;
-	uint32_t bad = 0;
-	LG_CUDA(cudaGetLastError(), "adjoint maps");
-	LG_CUDA(cudaMemcpyAsync(&bad, badb.p, 4, cudaMemcpyDeviceToHost, st), "d2h");
-	LG_CUDA(cudaStreamSynchronize(st), "adjoint maps");
+	LG_TRY(badb.reserve(8));
+	LG_CUDA(cudaMemsetAsync(badb.p, 0, 8, st), "memset");
+	LG_TRY(flat_positions(sn, 0, m->fout, out_pos.as<uint32_t>()));
+	if (E > 0) {
+		const FlatCsr &fi = m->fin, &fo = m->fout;
+		adj_sources<<<grid_for(fo.ntiles, kMapWarps), kMapWarps * 32, 0, st>>>(fo.heads(),
+				fo.nz_rows(), fo.tile_seg(), (uint32_t)E, fo.ntiles, m->src.as<uint32_t>());
+		adj_in_map<<<grid_for(fi.ntiles, kMapWarps), kMapWarps * 32, 0, st>>>(
+				fi.ids.as<uint32_t>(), fi.heads(), fi.nz_rows(), fi.tile_seg(), (uint32_t)E,
+				fi.ntiles, sn->view(0), sn->out.frag_start(), out_pos.as<uint32_t>(),
+				m->in_pos.as<uint32_t>(), badb.as<uint32_t>());
+		LG_CUDA(cudaGetLastError(), "adjoint maps");
+		s->launches += 2;
+	}
+	unsigned long long bad = 0;
+	LG_TRY(read_words(s, badb.as<unsigned long long>(), 1, &bad));
 	if (bad)
 		return set_error(LG_EINVAL, "out- and in-CSR of the snapshot disagree, or a "
-				"fragment is not sorted by neighbour id (code %u)", bad);
+				"fragment is not sorted by neighbour id (code %u)", (unsigned)bad);
 	return LG_OK;
 }
 

@@ -75,7 +75,9 @@ flat_live(FragSpace fs, uint32_t* live) {
 // nothing is deleted (tile_base null).  off = the row starts the degrees
 // give: a vertex whose first slot goes elsewhere, and a last tile that does
 // not end at off[V], set bit 2 of *err.
-template <bool kWeights>
+// kPositions: instead of the edges, every virtual slot's edge position goes to
+// ids[slot], kNoId for a deleted slot.
+template <bool kWeights, bool kPositions>
 __global__ void __launch_bounds__(kFwThreads)
 flat_write(FragSpace fs, const uint32_t* tile_base, const uint32_t* off, uint64_t V, uint32_t E,
 		uint32_t* ids, uint32_t* w, unsigned int* err) {
@@ -131,7 +133,7 @@ flat_write(FragSpace fs, const uint32_t* tile_base, const uint32_t* off, uint64_
 			head[u] = in && s == ost;
 			bit[u] = ix & 31u;
 			dw[u] = in ? __ldg(lt.del[lv] + (ix >> 5)) : ~0u;
-			id[u] = in ? __ldcs(lt.ids[lv] + ix) : 0u;
+			if (!kPositions) id[u] = in ? __ldcs(lt.ids[lv] + ix) : 0u;
 			if (kWeights) wt[u] = in ? __ldcs(lt.w[lv] + ix) : 0u;
 		}
 #pragma unroll
@@ -139,6 +141,12 @@ flat_write(FragSpace fs, const uint32_t* tile_base, const uint32_t* off, uint64_
 			const bool live = !((dw[u] >> bit[u]) & 1u);
 			const unsigned m = __ballot_sync(0xffffffffu, live);
 			const uint32_t p = run + __popc(m & ((1u << lane) - 1u));
+			if (kPositions) {
+				const uint32_t slot = pos + u * 32u + lane;
+				if (slot < end) ids[slot] = live ? p : kNoId;
+				run += __popc(m);
+				continue;
+			}
 			if (live) {
 				if (p < E) {
 					ids[p] = id[u];
@@ -156,7 +164,7 @@ flat_write(FragSpace fs, const uint32_t* tile_base, const uint32_t* off, uint64_
 		}
 		pos = end;
 	}
-	if (t == fs.ntiles - 1u) bad |= run != __ldg(off + V);
+	if (!kPositions && t == fs.ntiles - 1u) bad |= run != __ldg(off + V);
 	if (bad) atomicOr(err, 2u);
 }
 
@@ -304,6 +312,20 @@ lg_status flat_transpose(lg_store* s, const FlatCsr& a, FlatCsr& f) {
 	return flat_row_index(s, f, cnt.as<uint32_t>());
 }
 
+static FragSpace frag_space(const SnapDir& d) {
+	FragSpace fs;
+	fs.frags = d.frags.as<uint2>();
+	fs.start = d.frag_start();
+	fs.vert = d.frag_vert();
+	fs.frag_off = d.frag_off.as<uint32_t>();
+	fs.tile_frag = d.tile_frag();
+	fs.lt = d.lt.as<LevelTab>();
+	fs.F = (uint32_t)d.n_frags;
+	fs.total = (uint32_t)d.n_frag_slots;
+	fs.ntiles = (uint32_t)((d.n_frag_slots + kSlotTile - 1) / kSlotTile);
+	return fs;
+}
+
 // build_flat with rows of deg[v] edges, E in all.  *mismatch (and LG_OK, f
 // unfinished): the live slots are not laid out as those degrees say.
 static lg_status build_rows(lg_snapshot* sn, int dir, FlatCsr& f, bool view, bool weights,
@@ -339,16 +361,7 @@ static lg_status build_rows(lg_snapshot* sn, int dir, FlatCsr& f, bool view, boo
 	uint32_t* off = f.off.as<uint32_t>();
 	LG_CUDA(cudaMemsetAsync(f.err.p, 0, sizeof(unsigned int), st), "clear flag");
 	LG_TRY(exclusive_scan_u32(deg, off, V, f.scan_tmp, st, nullptr));
-	FragSpace fs;
-	fs.frags = d.frags.as<uint2>();
-	fs.start = d.frag_start();
-	fs.vert = d.frag_vert();
-	fs.frag_off = d.frag_off.as<uint32_t>();
-	fs.tile_frag = d.tile_frag();
-	fs.lt = d.lt.as<LevelTab>();
-	fs.F = (uint32_t)d.n_frags;
-	fs.total = (uint32_t)d.n_frag_slots;
-	fs.ntiles = (uint32_t)((d.n_frag_slots + kSlotTile - 1) / kSlotTile);
+	const FragSpace fs = frag_space(d);
 	const uint32_t* tile_base = nullptr;
 	if (d.n_dels > 0 && fs.ntiles > 0) {
 		LG_TRY(f.flags.reserve((2ull * fs.ntiles + 1) * sizeof(uint32_t)));
@@ -363,10 +376,10 @@ static lg_status build_rows(lg_snapshot* sn, int dir, FlatCsr& f, bool view, boo
 		const unsigned blocks = grid_for(fs.ntiles, kFwWarps);
 		unsigned int* err = f.err.as<unsigned int>();
 		if (weighted)
-			flat_write<true><<<blocks, kFwThreads, 0, st>>>(fs, tile_base, off, V, (uint32_t)E,
+			flat_write<true, false><<<blocks, kFwThreads, 0, st>>>(fs, tile_base, off, V, (uint32_t)E,
 					f.ids.as<uint32_t>(), f.w.as<uint32_t>(), err);
 		else
-			flat_write<false><<<blocks, kFwThreads, 0, st>>>(fs, tile_base, off, V, (uint32_t)E,
+			flat_write<false, false><<<blocks, kFwThreads, 0, st>>>(fs, tile_base, off, V, (uint32_t)E,
 					f.ids.as<uint32_t>(), nullptr, err);
 		LG_CUDA(cudaGetLastError(), "flat_write");
 	}
@@ -406,6 +419,20 @@ static lg_status build_rows(lg_snapshot* sn, int dir, FlatCsr& f, bool view, boo
 		return set_error(LG_ENOTSUP, "a vertex has more than %u live edges, the longest "
 				"fragment a flat view can describe", (unsigned)LG_MAX_FRAGMENT_LEN);
 	f.has_view = true;
+	return LG_OK;
+}
+
+lg_status flat_positions(lg_snapshot* sn, int dir, const FlatCsr& f, uint32_t* pos) {
+	const SnapDir& d = dir == 0 ? sn->out : sn->in;
+	lg_store* s = sn->store;
+	const FragSpace fs = frag_space(d);
+	if (fs.ntiles == 0) return LG_OK;
+	// (the tiles' bases are left from the flatten, behind their live counts)
+	const uint32_t* tile_base = d.n_dels > 0 ? f.flags.as<uint32_t>() + fs.ntiles : nullptr;
+	flat_write<false, true><<<grid_for(fs.ntiles, kFwWarps), kFwThreads, 0, s->stream>>>(fs,
+			tile_base, nullptr, sn->V, 0, pos, nullptr, nullptr);
+	LG_CUDA(cudaGetLastError(), "flat_positions");
+	s->launches++;
 	return LG_OK;
 }
 

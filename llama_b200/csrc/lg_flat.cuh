@@ -206,6 +206,10 @@ struct FlatCsr {
 lg_status build_flat(lg_snapshot* sn, int dir, FlatCsr& f, bool view, bool weights = true,
 		bool strict = true);
 
+// pos[k] = position in f of virtual slot k of direction dir, kNoId for a
+// deleted one; f is that direction's flat CSR as build_flat left it.
+lg_status flat_positions(lg_snapshot* sn, int dir, const FlatCsr& f, uint32_t* pos);
+
 // The row bookkeeping of f (kidx, R, rows) from its row starts f.off and the
 // rows' lengths deg[V]; f.V, f.E and f.ntiles are set.  Waits for the stream.
 lg_status flat_row_index(lg_store* s, FlatCsr& f, const uint32_t* deg);
