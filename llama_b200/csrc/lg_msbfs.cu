@@ -772,10 +772,10 @@ extern "C" lg_status lg_bc_batched(lg_snapshot* sn, const int64_t* sources, int 
 			LG_CUDA(cudaMemsetAsync(lk1 + V, 0, V * sizeof(u64), st), "clear level masks");
 			uint32_t* q = queues.as<uint32_t>() + qb;
 			uint32_t* q2 = queues.as<uint32_t>() + qoff[k + 1];
-			LG_TRY(exclusive_scan_slots(out, q, qlen, qcnt,
-					qpos, sc[9], st, nullptr));
 			if (top_down && has_in && (double)mf > (double)mu / alpha) top_down = false;
 			else if (!top_down && (double)qlen < (double)V / beta) top_down = true;
+			if (top_down)                             // (also read by the pushed sigma)
+				LG_TRY(exclusive_scan_slots(out, q, qlen, qcnt, qpos, sc[9], st, nullptr));
 			LG_CUDA(cudaMemsetAsync(ctr, 0, 4 * sizeof(unsigned long long), st), "memset");
 			if (top_down) {
 				ms_top_down<<<grid, kMsThreads, 0, st>>>(out, q, qpos, (uint32_t)qlen, lk, seen,
@@ -801,7 +801,7 @@ extern "C" lg_status lg_bc_batched(lg_snapshot* sn, const int64_t* sources, int 
 				ms_commit<<<grid_for(V, kMsThreads * kCommitPer), kMsThreads, 0, st>>>(nullptr,
 						(uint32_t)V, k + 1, V, n, nxt,
 						seen, lk1, nullptr, outdeg, q2, ctr);
-				s->launches += 2 + scan_launches(qlen);
+				s->launches += 2;
 			}
 			if (!has_in) {
 				// push along the level's out-edges (one atomic per down pair)
