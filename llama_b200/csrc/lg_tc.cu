@@ -281,17 +281,23 @@ __device__ __forceinline__ bool bsearch_u32(const uint32_t* base, uint32_t n, ui
 
 // Vertices by the length la of N+(a) and the label a:
 //   la <= kTcPairs         one thread looks up every pair of the list
-//   a < kTcDomain[c]       list c: bitmap of kTcDomain[c] labels
-//   else                   list 3: a warp looks up every pair
+//   a < kTcDomain0         list 0: a warp with a bitmap of kTcDomain0 labels
+//   la <= kTcHashMost      list 1: a warp with a hash table of N+(a)
+//   a < kTcDomain1, 2      list 2, 3: a CTA with a bitmap of so many labels
+//   else                   list 4: a warp looks up every pair
 // A pair (c, b) is looked up by a binary search of c in N+(b): up to eight
 // ids that is 28 searches at most, against eight lists of some 200 ids to
 // stream (the same holds for the first eight ids of a longer list, whose
-// pairs one warp looks up at once).
+// pairs one warp looks up at once).  The hash table costs twice a bitmap's
+// instructions per id, but no barriers between the four warps that would share
+// a larger bitmap: 99 k vertices with 9 to 64 ids took them 842 us.
 constexpr uint32_t kTcPairs = 8;
-constexpr int kTcClasses = 3;
+constexpr int kTcLists = 5;
 constexpr uint32_t kTcDomain0 = 1u << 16;     //   8 KB per bitmap: one warp each
 constexpr uint32_t kTcDomain1 = 1u << 18;     //  32 KB: four warps
 constexpr uint32_t kTcDomain2 = 7u << 18;     // 224 KB: a CTA of 32 warps, one per SM
+constexpr uint32_t kTcHashMost = 64;          // a quarter of the table's slots
+constexpr uint32_t kTcHashBits = 8;
 
 __global__ void __launch_bounds__(kTcThreads)
 tc_classify(uint32_t V, const uint32_t* off, const uint32_t* adj, uint32_t* lists, u64* ctr,
@@ -313,23 +319,121 @@ tc_classify(uint32_t V, const uint32_t* off, const uint32_t* adj, uint32_t* list
 	}
 	c = __reduce_add_sync(0xffffffffu, c);
 	if ((threadIdx.x & 31u) == 0 && c) atomicAdd(total, (u64)c);
-	const bool big = la > kTcPairs;
-	// a CTA's labels lie in one class or two: push only where some may be
-	const uint64_t a0 = (uint64_t)blockIdx.x * kTcThreads, a1 = a0 + kTcThreads;
-	const uint32_t dom[kTcClasses + 2] = {0u, kTcDomain0, kTcDomain1, kTcDomain2, 0xffffffffu};
-#pragma unroll
-	for (int k = 0; k <= kTcClasses; k++) {
-		if (a1 <= dom[k] || a0 >= dom[k + 1]) continue;
-		__syncthreads();
-		block_push<kTcThreads>(big && a >= dom[k] && a < dom[k + 1], a, lists + (size_t)k * V,
-				ctr + k);
+	const int cls = la <= kTcPairs ? -1 : a < kTcDomain0 ? 0 : la <= kTcHashMost ? 1
+			: a < kTcDomain1 ? 2 : a < kTcDomain2 ? 3 : 4;
+	// (a CTA's labels do not straddle a bound between the bitmaps)
+	const uint64_t a0 = (uint64_t)blockIdx.x * kTcThreads;
+	const int wide = a0 < kTcDomain1 ? 2 : a0 < kTcDomain2 ? 3 : 4;
+	if (a0 < kTcDomain0) {
+		block_push<kTcThreads>(cls == 0, a, lists, ctr);
+		return;
 	}
+	block_push<kTcThreads>(cls == 1, a, lists + V, ctr + 1);
+	__syncthreads();
+	block_push<kTcThreads>(cls == wide, a, lists + (size_t)wide * V, ctr + wide);
+}
+
+// Pairs (i, j), i < j, of the first eight ids of N+(a) = adj[sa ...): lane =
+// pair; returns whether the lane's two are adjacent.
+__device__ __forceinline__ uint32_t tc_first_pairs(const uint32_t* off, const uint32_t* adj,
+		uint32_t sa) {
+	const uint32_t lane = threadIdx.x & 31u;
+	if (lane >= kTcPairs * (kTcPairs - 1) / 2) return 0;
+	uint32_t j = 1, i = lane;
+	while (i >= j) { i -= j; j++; }
+	const uint32_t b = __ldg(adj + sa + j), x = __ldg(adj + sa + i);
+	const uint32_t sb = __ldg(off + b), lb = __ldg(off + b + 1) - sb;
+	return bsearch_u32(adj + sb, lb, x);
+}
+
+// Streams N+(b) of the lists j0 .. j0 + nb - 1 of N+(a) (nb <= 32) with the
+// calling warp; in(x) = 1 if x is in N+(a).  128 ids are loaded before any is
+// looked up.
+template <class In>
+__device__ __forceinline__ uint32_t tc_stream(const uint32_t* off, const uint32_t* adj,
+		uint32_t first, uint32_t nb, In&& in) {
+	constexpr int kAhead = 4;
+	const uint32_t lane = threadIdx.x & 31u;
+	uint32_t s = 0, e = 0, c = 0;
+	if (lane < nb) {
+		const uint32_t b = __ldg(adj + first + lane);
+		s = __ldg(off + b);
+		e = __ldg(off + b + 1);
+	}
+	for (uint32_t q = 0; q < nb; q++) {
+		const uint32_t sb = __shfl_sync(0xffffffffu, s, q);
+		const uint32_t eb = __shfl_sync(0xffffffffu, e, q);
+		uint32_t p = sb;
+		for (; p + 32u * kAhead <= eb; p += 32u * kAhead) {
+			uint32_t x[kAhead];
+#pragma unroll
+			for (int u = 0; u < kAhead; u++) x[u] = __ldg(adj + p + u * 32u + lane);
+#pragma unroll
+			for (int u = 0; u < kAhead; u++) c += in(x[u]);
+		}
+		if (p < eb) {
+			uint32_t x[kAhead];
+#pragma unroll
+			for (int u = 0; u < kAhead; u++) {
+				const uint32_t k = p + u * 32u + lane;
+				x[u] = k < eb ? __ldg(adj + k) : kNoId;
+			}
+#pragma unroll
+			for (int u = 0; u < kAhead; u++)
+				if (x[u] != kNoId) c += in(x[u]);
+		}
+	}
+	return c;
+}
+
+// A warp per vertex of its list (taken from a ticket counter): N+(a), at most
+// kTcHashMost ids, in a hash table of 2^kTcHashBits slots (open addressing).
+__global__ void __launch_bounds__(kTcThreads)
+tc_hash(const uint32_t* list, const u64* n_list, u64* ticket, const uint32_t* off,
+		const uint32_t* adj, u64* total) {
+	constexpr uint32_t kSlots = 1u << kTcHashBits;
+	__shared__ uint32_t tab[kTcThreads / 32][kSlots];
+	uint32_t* t = tab[threadIdx.x >> 5];
+	const uint32_t lane = threadIdx.x & 31u;
+	const uint32_t n = (uint32_t)__ldg(n_list);
+	auto slot = [](uint32_t x) { return (x * 2654435769u) >> (32u - kTcHashBits); };
+	u64 sum = 0;
+	for (;;) {
+		uint32_t k = 0;
+		if (lane == 0) k = (uint32_t)atomicAdd(ticket, 1ull);
+		k = __shfl_sync(0xffffffffu, k, 0);
+		if (k >= n) break;
+		const uint32_t a = __ldg(list + k);
+		const uint32_t sa = __ldg(off + a), la = __ldg(off + a + 1) - sa;
+		for (uint32_t i = lane; i < kSlots; i += 32) t[i] = kNoId;
+		__syncwarp();
+		for (uint32_t i = lane; i < la; i += 32) {
+			const uint32_t x = __ldg(adj + sa + i);
+			uint32_t h = slot(x);
+			while (atomicCAS(t + h, kNoId, x) != kNoId) h = (h + 1u) & (kSlots - 1u);
+		}
+		__syncwarp();
+		uint32_t c = tc_first_pairs(off, adj, sa);
+		for (uint32_t j = kTcPairs; j < la; j += 32)
+			c += tc_stream(off, adj, sa + j, min(32u, la - j), [&](uint32_t x) {
+				uint32_t h = slot(x), y = t[h];
+				while (y != x && y != kNoId) {
+					h = (h + 1u) & (kSlots - 1u);
+					y = t[h];
+				}
+				return y == x ? 1u : 0u;
+			});
+		sum += c;
+		__syncwarp();
+	}
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+	if (lane == 0 && sum) atomicAdd(total, sum);
 }
 
 // A CTA of kWarps warps takes the vertices of its list one after the other
 // (from a ticket counter), marks N+(a) in the bitmap and streams N+(b) of
-// every b but the first eight, a list per warp; 128 ids are loaded before any
-// is looked up.
+// every b but the first eight, a list per warp.
 template <int kWarps>
 __global__ void __launch_bounds__(kWarps * 32)
 tc_bitmap(const uint32_t* list, const u64* n_list, u64* ticket, const uint32_t* off,
@@ -337,7 +441,6 @@ tc_bitmap(const uint32_t* list, const u64* n_list, u64* ticket, const uint32_t* 
 	extern __shared__ uint32_t bm[];
 	__shared__ uint32_t s_next;
 	constexpr uint32_t kBatch = kWarps == 1 ? 32u : 8u;   // lists a warp takes at a time
-	constexpr int kAhead = 4;
 	const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5;
 	const uint32_t n = (uint32_t)__ldg(n_list);
 	if (n == 0) return;
@@ -355,39 +458,11 @@ tc_bitmap(const uint32_t* list, const u64* n_list, u64* ticket, const uint32_t* 
 			atomicOr(bm + (x >> 5), 1u << (x & 31u));
 		}
 		__syncthreads();
-		uint32_t c = 0;
-		if (wid == kWarps - 1 && lane < kTcPairs * (kTcPairs - 1) / 2) {
-			// lane = pair (i, j), i < j, of the first eight
-			uint32_t j = 1, i = lane;
-			while (i >= j) { i -= j; j++; }
-			const uint32_t b = __ldg(adj + sa + j), x = __ldg(adj + sa + i);
-			const uint32_t sb = __ldg(off + b), lb = __ldg(off + b + 1) - sb;
-			c += bsearch_u32(adj + sb, lb, x);
-		}
-		for (uint32_t j0 = kTcPairs + wid * kBatch; j0 < la; j0 += kWarps * kBatch) {
-			const uint32_t nb = min(kBatch, la - j0);
-			uint32_t s = 0, e = 0;
-			if (lane < nb) {
-				const uint32_t b = __ldg(adj + sa + j0 + lane);
-				s = __ldg(off + b);
-				e = __ldg(off + b + 1);
-			}
-			for (uint32_t q = 0; q < nb; q++) {
-				const uint32_t sb = __shfl_sync(0xffffffffu, s, q);
-				const uint32_t eb = __shfl_sync(0xffffffffu, e, q);
-				for (uint32_t p = sb; p < eb; p += 32u * kAhead) {
-					uint32_t x[kAhead];
-#pragma unroll
-					for (int u = 0; u < kAhead; u++) {
-						const uint32_t k = p + u * 32u + lane;
-						x[u] = k < eb ? __ldg(adj + k) : kNoId;
-					}
-#pragma unroll
-					for (int u = 0; u < kAhead; u++)
-						if (x[u] != kNoId) c += (bm[x[u] >> 5] >> (x[u] & 31u)) & 1u;
-				}
-			}
-		}
+		uint32_t c = wid == kWarps - 1 ? tc_first_pairs(off, adj, sa) : 0u;
+		for (uint32_t j = kTcPairs + wid * kBatch; j < la; j += kWarps * kBatch)
+			c += tc_stream(off, adj, sa + j, min(kBatch, la - j), [&](uint32_t x) {
+				return (bm[x >> 5] >> (x & 31u)) & 1u;
+			});
 		sum += c;
 		__syncthreads();
 		for (uint32_t i = tid; i < la; i += kWarps * 32) bm[__ldg(adj + sa + i) >> 5] = 0;
@@ -475,10 +550,10 @@ extern "C" lg_status lg_triangle_count(lg_snapshot* sn, lg_tc_result* result) {
 			adj(s->pool), lists(s->pool);
 	int sms = 148;
 	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
-	// ctr: [0..3] class sizes, [4..6] tickets, [7] self-loops, [8] triangles
-	LG_TRY(ctr.reserve(9 * sizeof(u64)));
+	// ctr: [0..4] list sizes, [5..8] tickets, [9] self-loops, [10] triangles
+	LG_TRY(ctr.reserve(11 * sizeof(u64)));
 	u64* cd = ctr.as<u64>();
-	LG_CUDA(cudaMemsetAsync(cd, 0, 9 * sizeof(u64), st), "memset");
+	LG_CUDA(cudaMemsetAsync(cd, 0, 11 * sizeof(u64), st), "memset");
 	const uint32_t* odeg = sn->out.deg.as<uint32_t>();
 	const uint32_t* ideg = sn->in.present ? sn->in.deg.as<uint32_t>() : nullptr;
 	LG_TRY(label.reserve(V * 4));
@@ -496,7 +571,7 @@ extern "C" lg_status lg_triangle_count(lg_snapshot* sn, lg_tc_result* result) {
 	LG_TRY(keys.reserve(E * 8));
 	tc_emit<<<grid_for(f->ntiles, kTcEmitWarps), kTcEmitWarps * 32, 0, st>>>(f->ids.as<uint32_t>(),
 			f->heads(), f->nz_rows(), f->tile_seg(), (uint32_t)E, f->ntiles, label.as<uint32_t>(),
-			bits, loop_key, keys.as<u64>(), cd + 7);
+			bits, loop_key, keys.as<u64>(), cd + 9);
 	LG_CUDA(cudaGetLastError(), "tc_emit");
 	s->launches += 4;
 	u64* sorted = nullptr;
@@ -519,28 +594,33 @@ extern "C" lg_status lg_triangle_count(lg_snapshot* sn, lg_tc_result* result) {
 			adj.as<uint32_t>(), fcnt);
 	LG_CUDA(cudaGetLastError(), "tc_uniq_write");
 	LG_TRY(exclusive_scan_u32(fcnt, foff, V, scan_tmp, st, nullptr));
-	LG_TRY(lists.reserve((kTcClasses + 1) * V * 4));
+	LG_TRY(lists.reserve(kTcLists * V * 4));
 	uint32_t* ls = lists.as<uint32_t>();
 	const uint32_t* ad = adj.as<uint32_t>();
+	u64* found = cd + 10;
 	tc_classify<<<grid_for(V, kTcThreads), kTcThreads, 0, st>>>((uint32_t)V, foff, ad, ls, cd,
-			cd + 8);
+			found);
 	LG_CUDA(cudaGetLastError(), "tc_classify");
 	s->launches += 3 + scan_launches(uq_tiles) + scan_launches(V);
-	LG_TRY(launch_bitmap<1>(s, sms, (uint32_t)std::min<uint64_t>(V, kTcDomain0), ls, cd, cd + 4,
-			foff, ad, cd + 8));
-	if (V > kTcDomain0)
-		LG_TRY(launch_bitmap<4>(s, sms, (uint32_t)std::min<uint64_t>(V, kTcDomain1), ls + V, cd + 1,
-				cd + 5, foff, ad, cd + 8));
+	LG_TRY(launch_bitmap<1>(s, sms, (uint32_t)std::min<uint64_t>(V, kTcDomain0), ls, cd, cd + 5,
+			foff, ad, found));
+	if (V > kTcDomain0) {
+		tc_hash<<<(unsigned)sms * 8u, kTcThreads, 0, st>>>(ls + V, cd + 1, cd + 6, foff, ad, found);
+		LG_CUDA(cudaGetLastError(), "tc_hash");
+		s->launches++;
+		LG_TRY(launch_bitmap<4>(s, sms, (uint32_t)std::min<uint64_t>(V, kTcDomain1), ls + 2 * V,
+				cd + 2, cd + 7, foff, ad, found));
+	}
 	if (V > kTcDomain1)
-		LG_TRY(launch_bitmap<32>(s, sms, (uint32_t)std::min<uint64_t>(V, kTcDomain2), ls + 2 * V,
-				cd + 2, cd + 6, foff, ad, cd + 8));
+		LG_TRY(launch_bitmap<32>(s, sms, (uint32_t)std::min<uint64_t>(V, kTcDomain2), ls + 3 * V,
+				cd + 3, cd + 8, foff, ad, found));
 	if (V > kTcDomain2) {
-		tc_search<<<(unsigned)sms * 8u, kTcThreads, 0, st>>>(ls + 3 * V, cd + 3, foff, ad, cd + 8);
+		tc_search<<<(unsigned)sms * 8u, kTcThreads, 0, st>>>(ls + 4 * V, cd + 4, foff, ad, found);
 		LG_CUDA(cudaGetLastError(), "tc_search");
 		s->launches++;
 	}
 	u64 h[2] = {0, 0};
-	LG_TRY(read_words(s, cd + 7, 2, h));
+	LG_TRY(read_words(s, cd + 9, 2, h));
 	result->triangles = (int64_t)h[1];
 	result->undirected_edges = m;
 	result->arcs = E - h[0];

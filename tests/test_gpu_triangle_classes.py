@@ -1,6 +1,6 @@
 """Triangle counting over graphs that reach each of its ways to intersect:
-pairs of short lists, one-warp, four-warp and whole-SM bitmaps, and the
-searches of labels no bitmap holds.  The graphs are circulants (vertex i joined
+pairs of short lists, one-warp, four-warp and whole-SM bitmaps, hash tables of
+up to 64 ids, and the searches of labels no bitmap holds.  The graphs are circulants (vertex i joined
 to i + 1 .. i + k) under a random renaming, whose triangles are known."""
 import numpy as np
 import pytest
@@ -35,7 +35,8 @@ def _circulant(n, k, seed, wheel):
 
 @pytest.mark.parametrize("n,k,wheel", [
     (9, 2, False), (257, 4, True), (4099, 12, True), (70001, 5, False), (70001, 14, True),
-    (300007, 12, False), (1900003, 10, False)])
+    (300007, 12, False), (1900003, 10, False), (70001, 90, False), (280001, 80, False),
+    (1900003, 70, False)])
 def test_circulants(n, k, wheel):
     s, d, first, tri, edges, arcs, V = _circulant(n, k, 7 + n, wheel)
     with Store(reverse_edges=n % 2 == 0) as st:
