@@ -14,17 +14,20 @@
 //   3. the keys (a << bits | b) are radix sorted and de-duplicated, giving
 //      the forward lists N+(a), sorted by label;
 //   4. every triangle c < b < a is found at its largest label a: for b in
-//      N+(a), |N+(b) & N+(a)|.  A CTA (or a single warp) holds N+(a) as a
-//      bitmap over the labels below a in shared memory and streams the lists
-//      N+(b) against it.
+//      N+(a), |N+(b) & N+(a)|.  A group of warps holds N+(a) in shared memory
+//      (a bitmap over the labels below a, or a hash table) and reads the N+(b)
+//      against it: as rows of bits for the hubs, as ids otherwise.
 //
-// What bounds step 4: one shared-memory probe per streamed id.  The form
-// before it took a binary search per element of the shorter list (log2 of
-// the longer list's uncoalesced loads each): at 700 k vertices and 9.1 M
-// undirected edges 7.3 G search steps, against 1.9 G coalesced ids streamed
-// here.  Because labels follow the degrees, a vertex whose list is long has a
-// small label, so its bitmap is short: 64 Ki labels (8 KB, one warp's own)
-// hold nearly all of the work of that graph.
+// What bounds step 4: the visits.  At 700 k vertices and 10.6 M undirected edges
+// there are some 9 M pairs (a, b) and 1.8 G ids in their lists; a form with a
+// binary search per element of the shorter list took 7.3 G search steps and
+// 5950 us, streaming every id against N+(a) 1430 us (one shared-memory probe
+// per id, its bank conflicts, and one list in flight per warp).  Rows of bits
+// for b < 8 Ki leave 218 M ids and 290 M words, and half a warp per row and a
+// quarter per list some 300 M instructions: 600 us.  Because labels follow the
+// degrees, a vertex whose list is long has a small label, so bitmaps stay
+// short: 64 Ki labels (8 KB, two warps') hold nearly all of the work of
+// that graph.
 // The count is an exact integer sum (atomicAdd of per-warp partials), so the
 // order inside a degree class does not matter.
 #include "lg_flat.cuh"
@@ -281,7 +284,7 @@ __device__ __forceinline__ bool bsearch_u32(const uint32_t* base, uint32_t n, ui
 
 // Vertices by the length la of N+(a) and the label a:
 //   la <= kTcPairs         one thread looks up every pair of the list
-//   a < kTcDomain0         list 0: a warp with a bitmap of kTcDomain0 labels
+//   a < kTcDomain0         list 0: two warps with a bitmap of kTcDomain0 labels
 //   la <= kTcHashMost      list 1: a warp with a hash table of N+(a)
 //   a < kTcDomain1, 2      list 2, 3: a CTA with a bitmap of so many labels
 //   else                   list 4: a warp looks up every pair
@@ -290,7 +293,9 @@ __device__ __forceinline__ bool bsearch_u32(const uint32_t* base, uint32_t n, ui
 // stream (the same holds for the first eight ids of a longer list, whose
 // pairs one warp looks up at once).  The hash table costs twice a bitmap's
 // instructions per id, but no barriers between the four warps that would share
-// a larger bitmap: 99 k vertices with 9 to 64 ids took them 842 us.
+// a larger bitmap: 99 k vertices with 9 to 64 ids took them 842 us against
+// 240.  Two warps per 8 KB bitmap keep 48 resident on an SM (one: 24, 610 us
+// against 476; four: 477, and slower with two rows in flight, 516 against 417).
 constexpr uint32_t kTcPairs = 8;
 constexpr int kTcLists = 5;
 constexpr uint32_t kTcDomain0 = 1u << 16;     //   8 KB per bitmap: one warp each
@@ -346,38 +351,92 @@ __device__ __forceinline__ uint32_t tc_first_pairs(const uint32_t* off, const ui
 	return bsearch_u32(adj + sb, lb, x);
 }
 
-// Streams N+(b) of the lists j0 .. j0 + nb - 1 of N+(a) (nb <= 32) with the
-// calling warp; in(x) = 1 if x is in N+(a).  128 ids are loaded before any is
-// looked up.
-template <class In>
-__device__ __forceinline__ uint32_t tc_stream(const uint32_t* off, const uint32_t* adj,
-		uint32_t first, uint32_t nb, In&& in) {
-	constexpr int kAhead = 4;
+// N+(b) of b < kTcRows as a row of bits, where that is the cheaper form: half
+// a warp takes 2048 labels of a row at a time and a quarter 32 ids of a list,
+// with bank conflicts (so from an eighth of an id per word on; a quarter: 418
+// against 410 us).
+constexpr uint32_t kTcRows = 8192;
+constexpr uint32_t kTcRowWords = kTcRows / 32;
+
+__device__ __forceinline__ bool tc_has_row(uint32_t b, uint32_t lb) {
+	return b < kTcRows && 4u * lb > (b >> 5) + 32u;
+}
+
+// rows[b] <- the bits of N+(b), for every b that has a row: a warp each.
+__global__ void __launch_bounds__(kTcThreads)
+tc_rows(uint32_t n, const uint32_t* off, const uint32_t* adj, uint32_t* rows) {
+	__shared__ uint32_t bits[kTcThreads / 32][kTcRowWords];
+	uint32_t* w = bits[threadIdx.x >> 5];
 	const uint32_t lane = threadIdx.x & 31u;
-	uint32_t s = 0, e = 0, c = 0;
-	if (lane < nb) {
-		const uint32_t b = __ldg(adj + first + lane);
-		s = __ldg(off + b);
-		e = __ldg(off + b + 1);
+	const uint32_t b = blockIdx.x * (kTcThreads / 32) + (threadIdx.x >> 5);
+	if (b >= n) return;
+	const uint32_t sb = __ldg(off + b), lb = __ldg(off + b + 1) - sb;
+	if (!tc_has_row(b, lb)) return;
+	const uint32_t nw = (b + 127u) >> 7 << 2;             // whole 16-byte words
+	for (uint32_t i = lane; i < nw; i += 32) w[i] = 0;
+	__syncwarp();
+	for (uint32_t i = lane; i < lb; i += 32) {
+		const uint32_t x = __ldg(adj + sb + i);
+		atomicOr(w + (x >> 5), 1u << (x & 31u));
 	}
-	for (uint32_t q = 0; q < nb; q++) {
-		const uint32_t sb = __shfl_sync(0xffffffffu, s, q);
-		const uint32_t eb = __shfl_sync(0xffffffffu, e, q);
-		uint32_t p = sb;
-		for (; p + 32u * kAhead <= eb; p += 32u * kAhead) {
-			uint32_t x[kAhead];
+	__syncwarp();
+	uint32_t* row = rows + (size_t)b * kTcRowWords;
+	for (uint32_t i = lane; i < nw; i += 32) row[i] = w[i];
+}
+
+// sum of |N+(b) & N+(a)| over the nb <= 32 ids b of adj[first ...): bm holds the
+// labels below kTcRows of N+(a) as bits, in(x) = 1 if x is in N+(a).  Half a warp
+// takes a row (2048 labels a step), a quarter a list (32 ids a step): most visits
+// end within a step, so it is the instructions per visit and the loads in flight
+// that count (whole warps: 676 us against 610, a row at a time 476 against 417).
+// Neighbouring ids b, alike in their lengths, go to different parts of the warp.
+template <class In>
+__device__ __forceinline__ uint32_t tc_lists(const uint32_t* off, const uint32_t* adj,
+		const uint4* rows, uint32_t first, uint32_t nb, const uint32_t* bm, In&& in) {
+	const uint32_t lane = threadIdx.x & 31u;
+	uint32_t b = 0, s = 0, n = 0, c = 0;
+	if (lane < nb) {
+		b = __ldg(adj + first + lane);
+		s = __ldg(off + b);
+		n = __ldg(off + b + 1) - s;
+	}
+	const bool row = tc_has_row(b, n);
+	uint32_t m = __ballot_sync(0xffffffffu, row) & (0x55555555u << (lane >> 4));
+	while (__any_sync(0xffffffffu, m != 0)) {
+		const uint4* w = (const uint4*)bm;
+		const uint4* p[2];
+		uint32_t len[2];
 #pragma unroll
-			for (int u = 0; u < kAhead; u++) x[u] = __ldg(adj + p + u * 32u + lane);
-#pragma unroll
-			for (int u = 0; u < kAhead; u++) c += in(x[u]);
+		for (int i = 0; i < 2; i++) {
+			const uint32_t q = __shfl_sync(0xffffffffu, b, m ? __ffs(m) - 1 : 0);
+			len[i] = m ? (q + 127u) >> 7 : 0u;
+			p[i] = rows + (size_t)q * (kTcRowWords / 4);
+			m &= m - 1u;
 		}
-		if (p < eb) {
+		for (uint32_t k = lane & 15u; k < max(len[0], len[1]); k += 16) {
+			uint4 x[2];
+#pragma unroll
+			for (int i = 0; i < 2; i++)
+				x[i] = k < len[i] ? __ldg(p[i] + k) : make_uint4(0, 0, 0, 0);
+			const uint4 u = w[k];
+#pragma unroll
+			for (int i = 0; i < 2; i++)
+				c += __popc(x[i].x & u.x) + __popc(x[i].y & u.y) + __popc(x[i].z & u.z)
+						+ __popc(x[i].w & u.w);
+		}
+	}
+	m = __ballot_sync(0xffffffffu, n != 0 && !row) & (0x11111111u << (lane >> 3));
+	while (__any_sync(0xffffffffu, m != 0)) {
+		constexpr int kAhead = 4;
+		const uint32_t q = m ? __ffs(m) - 1 : 0;
+		const uint32_t* p = adj + __shfl_sync(0xffffffffu, s, q);
+		const uint32_t l = __shfl_sync(0xffffffffu, n, q);
+		const uint32_t len = m ? l : 0u;
+		m &= m - 1u;
+		for (uint32_t k = lane & 7u; k < len; k += 8u * kAhead) {
 			uint32_t x[kAhead];
 #pragma unroll
-			for (int u = 0; u < kAhead; u++) {
-				const uint32_t k = p + u * 32u + lane;
-				x[u] = k < eb ? __ldg(adj + k) : kNoId;
-			}
+			for (int u = 0; u < kAhead; u++) x[u] = k + 8u * u < len ? __ldg(p + k + 8u * u) : kNoId;
 #pragma unroll
 			for (int u = 0; u < kAhead; u++)
 				if (x[u] != kNoId) c += in(x[u]);
@@ -390,14 +449,17 @@ __device__ __forceinline__ uint32_t tc_stream(const uint32_t* off, const uint32_
 // kTcHashMost ids, in a hash table of 2^kTcHashBits slots (open addressing).
 __global__ void __launch_bounds__(kTcThreads)
 tc_hash(const uint32_t* list, const u64* n_list, u64* ticket, const uint32_t* off,
-		const uint32_t* adj, u64* total) {
+		const uint32_t* adj, const uint4* rows, u64* total) {
 	constexpr uint32_t kSlots = 1u << kTcHashBits;
 	__shared__ uint32_t tab[kTcThreads / 32][kSlots];
+	__shared__ __align__(16) uint32_t bits[kTcThreads / 32][kTcRowWords];
 	uint32_t* t = tab[threadIdx.x >> 5];
+	uint32_t* bm = bits[threadIdx.x >> 5];
 	const uint32_t lane = threadIdx.x & 31u;
 	const uint32_t n = (uint32_t)__ldg(n_list);
 	auto slot = [](uint32_t x) { return (x * 2654435769u) >> (32u - kTcHashBits); };
 	u64 sum = 0;
+	for (uint32_t i = lane; i < kTcRowWords; i += 32) bm[i] = 0;
 	for (;;) {
 		uint32_t k = 0;
 		if (lane == 0) k = (uint32_t)atomicAdd(ticket, 1ull);
@@ -411,11 +473,12 @@ tc_hash(const uint32_t* list, const u64* n_list, u64* ticket, const uint32_t* of
 			const uint32_t x = __ldg(adj + sa + i);
 			uint32_t h = slot(x);
 			while (atomicCAS(t + h, kNoId, x) != kNoId) h = (h + 1u) & (kSlots - 1u);
+			if (x < kTcRows) atomicOr(bm + (x >> 5), 1u << (x & 31u));
 		}
 		__syncwarp();
 		uint32_t c = tc_first_pairs(off, adj, sa);
 		for (uint32_t j = kTcPairs; j < la; j += 32)
-			c += tc_stream(off, adj, sa + j, min(32u, la - j), [&](uint32_t x) {
+			c += tc_lists(off, adj, rows, sa + j, min(32u, la - j), bm, [&](uint32_t x) {
 				uint32_t h = slot(x), y = t[h];
 				while (y != x && y != kNoId) {
 					h = (h + 1u) & (kSlots - 1u);
@@ -425,6 +488,10 @@ tc_hash(const uint32_t* list, const u64* n_list, u64* ticket, const uint32_t* of
 			});
 		sum += c;
 		__syncwarp();
+		for (uint32_t i = lane; i < la; i += 32) {
+			const uint32_t x = __ldg(adj + sa + i);
+			if (x < kTcRows) bm[x >> 5] = 0;
+		}
 	}
 #pragma unroll
 	for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
@@ -437,10 +504,10 @@ tc_hash(const uint32_t* list, const u64* n_list, u64* ticket, const uint32_t* of
 template <int kWarps>
 __global__ void __launch_bounds__(kWarps * 32)
 tc_bitmap(const uint32_t* list, const u64* n_list, u64* ticket, const uint32_t* off,
-		const uint32_t* adj, uint32_t words, u64* total) {
-	extern __shared__ uint32_t bm[];
+		const uint32_t* adj, const uint4* rows, uint32_t words, u64* total) {
+	extern __shared__ __align__(16) uint32_t bm[];
 	__shared__ uint32_t s_next;
-	constexpr uint32_t kBatch = kWarps == 1 ? 32u : 8u;   // lists a warp takes at a time
+	constexpr uint32_t kBatch = kWarps < 32 ? 16u : 8u;   // lists a warp takes at a time
 	const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5;
 	const uint32_t n = (uint32_t)__ldg(n_list);
 	if (n == 0) return;
@@ -460,7 +527,7 @@ tc_bitmap(const uint32_t* list, const u64* n_list, u64* ticket, const uint32_t* 
 		__syncthreads();
 		uint32_t c = wid == kWarps - 1 ? tc_first_pairs(off, adj, sa) : 0u;
 		for (uint32_t j = kTcPairs + wid * kBatch; j < la; j += kWarps * kBatch)
-			c += tc_stream(off, adj, sa + j, min(kBatch, la - j), [&](uint32_t x) {
+			c += tc_lists(off, adj, rows, sa + j, min(kBatch, la - j), bm, [&](uint32_t x) {
 				return (bm[x >> 5] >> (x & 31u)) & 1u;
 			});
 		sum += c;
@@ -506,8 +573,8 @@ namespace {
 // One bitmap class: kWarps warps per CTA, as many CTAs as are resident.
 template <int kWarps>
 lg_status launch_bitmap(lg_store* s, int sms, uint32_t domain, const uint32_t* list, u64* n_list,
-		u64* ticket, const uint32_t* off, const uint32_t* adj, u64* total) {
-	const uint32_t words = (domain + 31u) / 32u;
+		u64* ticket, const uint32_t* off, const uint32_t* adj, const uint4* rows, u64* total) {
+	const uint32_t words = (domain + 127u) / 128u * 4u;   // rows are read by 16 bytes
 	const size_t smem = (size_t)words * 4;
 	LG_CUDA(cudaFuncSetAttribute(tc_bitmap<kWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 			(int)smem), "tc_bitmap");
@@ -516,7 +583,7 @@ lg_status launch_bitmap(lg_store* s, int sms, uint32_t domain, const uint32_t* l
 			smem), "tc_bitmap");
 	if (per_sm < 1) return set_error(LG_ECUDA, "tc_bitmap does not fit an SM");
 	tc_bitmap<kWarps><<<(unsigned)(sms * per_sm), kWarps * 32, smem, s->stream>>>(list, n_list,
-			ticket, off, adj, words, total);
+			ticket, off, adj, rows, words, total);
 	LG_CUDA(cudaGetLastError(), "tc_bitmap");
 	s->launches++;
 	return LG_OK;
@@ -547,7 +614,7 @@ extern "C" lg_status lg_triangle_count(lg_snapshot* sn, lg_tc_result* result) {
 	if (E == 0) return LG_OK;
 	DevBuf label(s->pool), hist(s->pool), keys(s->pool), tmpk(s->pool), tmpp(s->pool),
 			counts(s->pool), scan_tmp(s->pool), tiles(s->pool), off(s->pool), ctr(s->pool),
-			adj(s->pool), lists(s->pool);
+			adj(s->pool), lists(s->pool), rows(s->pool);
 	int sms = 148;
 	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
 	// ctr: [0..4] list sizes, [5..8] tickets, [9] self-loops, [10] triangles
@@ -601,19 +668,25 @@ extern "C" lg_status lg_triangle_count(lg_snapshot* sn, lg_tc_result* result) {
 	tc_classify<<<grid_for(V, kTcThreads), kTcThreads, 0, st>>>((uint32_t)V, foff, ad, ls, cd,
 			found);
 	LG_CUDA(cudaGetLastError(), "tc_classify");
-	s->launches += 3 + scan_launches(uq_tiles) + scan_launches(V);
-	LG_TRY(launch_bitmap<1>(s, sms, (uint32_t)std::min<uint64_t>(V, kTcDomain0), ls, cd, cd + 5,
-			foff, ad, found));
+	const uint32_t nr = (uint32_t)std::min<uint64_t>(V, kTcRows);
+	LG_TRY(rows.reserve((size_t)nr * kTcRowWords * 4));
+	tc_rows<<<grid_for(nr, kTcThreads / 32), kTcThreads, 0, st>>>(nr, foff, ad,
+			rows.as<uint32_t>());
+	LG_CUDA(cudaGetLastError(), "tc_rows");
+	s->launches += 4 + scan_launches(uq_tiles) + scan_launches(V);
+	LG_TRY(launch_bitmap<2>(s, sms, (uint32_t)std::min<uint64_t>(V, kTcDomain0), ls, cd, cd + 5,
+			foff, ad, rows.as<uint4>(), found));
 	if (V > kTcDomain0) {
-		tc_hash<<<(unsigned)sms * 8u, kTcThreads, 0, st>>>(ls + V, cd + 1, cd + 6, foff, ad, found);
+		tc_hash<<<(unsigned)sms * 8u, kTcThreads, 0, st>>>(ls + V, cd + 1, cd + 6, foff, ad,
+				rows.as<uint4>(), found);
 		LG_CUDA(cudaGetLastError(), "tc_hash");
 		s->launches++;
 		LG_TRY(launch_bitmap<4>(s, sms, (uint32_t)std::min<uint64_t>(V, kTcDomain1), ls + 2 * V,
-				cd + 2, cd + 7, foff, ad, found));
+				cd + 2, cd + 7, foff, ad, rows.as<uint4>(), found));
 	}
 	if (V > kTcDomain1)
 		LG_TRY(launch_bitmap<32>(s, sms, (uint32_t)std::min<uint64_t>(V, kTcDomain2), ls + 3 * V,
-				cd + 3, cd + 8, foff, ad, found));
+				cd + 3, cd + 8, foff, ad, rows.as<uint4>(), found));
 	if (V > kTcDomain2) {
 		tc_search<<<(unsigned)sms * 8u, kTcThreads, 0, st>>>(ls + 4 * V, cd + 4, foff, ad, found);
 		LG_CUDA(cudaGetLastError(), "tc_search");
