@@ -17,7 +17,13 @@
 // begin in a 32-slot chunk are bits of one word, so a slot's fragment is a
 // population count away.  The form before it built a slot-to-fragment table
 // per 1024-slot block in shared memory behind a dozen block barriers: it was
-// bound by those and by its instructions, 2.1 ms at 262 M slots.
+// bound by those and by its instructions, 2.1 ms at 262 M slots.  Now it takes
+// 870 us there, some 70 instructions per 32 slots against 3 GB of traffic.
+// What counts is the chains of loads: the next window is under way with the
+// ids of the present one, and where its rows ought to start is looked up per
+// window, not per row (1055 us), and 48 warps per SM hide the rest (96
+// slots a time and 40 registers; 64: 900 us, 128: 929 with 40 registers, 1155 with
+// 48).
 #include "lg_flat.cuh"
 #include "lg_sort.cuh"
 
@@ -28,7 +34,7 @@ namespace lg {
 
 constexpr int kFwThreads = 256;
 constexpr int kFwWarps = kFwThreads / 32;
-constexpr int kFwAhead = 4;             // 32-slot chunks whose loads are issued together
+constexpr int kFwAhead = 3;             // 32-slot chunks whose loads are issued together
 
 // One direction's fragments in virtual slot order.
 struct FragSpace {
@@ -77,8 +83,8 @@ flat_live(FragSpace fs, uint32_t* live) {
 // not end at off[V], set bit 2 of *err.
 // kPositions: instead of the edges, every virtual slot's edge position goes to
 // ids[slot], kNoId for a deleted slot.
-template <bool kWeights, bool kPositions>
-__global__ void __launch_bounds__(kFwThreads)
+template <bool kWeights, bool kPositions, bool kDels>
+__global__ void __launch_bounds__(kFwThreads, 6)
 flat_write(FragSpace fs, const uint32_t* tile_base, const uint32_t* off, uint64_t V, uint32_t E,
 		uint32_t* ids, uint32_t* w, unsigned int* err) {
 	__shared__ LevelTab lt;
@@ -94,53 +100,74 @@ flat_write(FragSpace fs, const uint32_t* tile_base, const uint32_t* off, uint64_
 	if (t >= fs.ntiles) return;
 	const uint32_t s0 = t * kSlotTile;
 	const uint32_t s1 = fs.total - s0 < kSlotTile ? fs.total : s0 + kSlotTile;
-	uint32_t f = __ldg(fs.tile_frag + t);      // the window's first fragment
-	uint32_t run = tile_base ? __ldg(tile_base + t) : s0;
-	uint32_t start = 0, wend = s0;             // the window covers slots up to wend
+	// The window: fragments f ... f + 31, a lane each, covering slots up to wend.
+	// want = where its vertex's row starts if the fragment is the vertex's
+	// first, kNoId if not.
+	uint32_t f = __ldg(fs.tile_frag + t);
+	uint32_t start = 0xffffffffu, wend = fs.total, vert = 0, want = kNoId;
 	uint2 fr = make_uint2(0u, 0u);
+	auto load_window = [&]() {
+		const uint32_t k = f + lane;
+		start = 0xffffffffu;
+		if (k < fs.F) {
+			start = __ldg(fs.start + k);
+			fr = __ldg(fs.frags + k);
+			if (!kPositions) vert = __ldg(fs.vert + k);
+		}
+		wend = f + 32u <= fs.F ? __ldg(fs.start + f + 32u) : fs.total;
+	};
+	auto load_want = [&]() {
+		want = kNoId;
+		if (kPositions || f + lane >= fs.F) return;
+		const uint32_t first = __ldg(fs.frag_off + vert), o = __ldg(off + vert);
+		if (first == f + lane) want = o;
+	};
+	load_window();
+	load_want();
+	uint32_t run = kDels ? __ldg(tile_base + t) : 0u;
 	bool bad = false;
 	const uint32_t upto = 2u << lane;          // bits at or below the lane, + 1
 	for (uint32_t pos = s0; pos < s1;) {
 		const uint32_t full = min(pos + 32u * kFwAhead, s1);
-		if (full > wend) {
-			// load the window that begins with the fragment holding pos
-			if (wend > s0) f += __popc(__ballot_sync(0xffffffffu, start <= pos)) - 1u;
-			const uint32_t k = f + lane;
-			start = k < fs.F ? __ldg(fs.start + k) : 0xffffffffu;
-			fr = k < fs.F ? fs.frags[k] : make_uint2(0u, 0u);
-			const uint32_t after = f + 32u <= fs.F ? __ldg(fs.start + f + 32u) : fs.total;
-			wend = after;
-		}
 		const uint32_t end = min(full, wend);
-		uint32_t id[kFwAhead], dw[kFwAhead], wt[kFwAhead], bit[kFwAhead], own[kFwAhead];
-		bool head[kFwAhead];
+		uint32_t id[kFwAhead], dw[kFwAhead], wt[kFwAhead], bit[kFwAhead];
+		uint32_t row[kFwAhead];                // where a row that begins at the slot starts
 #pragma unroll
 		for (int u = 0; u < kFwAhead; u++) {
 			const uint32_t base = pos + u * 32u;
-			// fragments begun by the chunk's first slot, and those that begin
-			// at a later one
+			// fragments begun before the chunk, and those that begin in it
 			const uint32_t rel = start - base;
-			const uint32_t begun = __popc(__ballot_sync(0xffffffffu, start <= base));
-			const uint32_t mask = __reduce_or_sync(0xffffffffu,
-					start > base && rel < 32u ? 1u << rel : 0u);
-			own[u] = begun - 1u + __popc(mask & (upto - 1u));
-			const uint32_t ost = __shfl_sync(0xffffffffu, start, own[u]);
-			const uint32_t oix = __shfl_sync(0xffffffffu, fr.x, own[u]);
-			const uint32_t oy = __shfl_sync(0xffffffffu, fr.y, own[u]);
-			const uint32_t s = base + lane;
-			const uint32_t ix = oix + (s - ost), lv = oy & kLevelMask;
-			const bool in = s < end;
-			head[u] = in && s == ost;
+			const uint32_t begun = __popc(__ballot_sync(0xffffffffu, start < base));
+			const uint32_t mask = __reduce_or_sync(0xffffffffu, rel < 32u ? 1u << rel : 0u);
+			const uint32_t own = begun - 1u + __popc(mask & (upto - 1u));
+			const uint32_t ix = __shfl_sync(0xffffffffu, fr.x - start, own) + base + lane;
+			const uint32_t lv = __shfl_sync(0xffffffffu, fr.y, own) & kLevelMask;
+			const bool in = base + lane < end;
 			bit[u] = ix & 31u;
-			dw[u] = in ? __ldg(lt.del[lv] + (ix >> 5)) : ~0u;
+			dw[u] = !in ? ~0u : kDels ? __ldg(lt.del[lv] + (ix >> 5)) : 0u;
 			if (!kPositions) id[u] = in ? __ldcs(lt.ids[lv] + ix) : 0u;
 			if (kWeights) wt[u] = in ? __ldcs(lt.w[lv] + ix) : 0u;
+			if (!kPositions) {
+				row[u] = __shfl_sync(0xffffffffu, want, own);
+				if (!in || !((mask >> lane) & 1u)) row[u] = kNoId;
+			}
+		}
+		// the next window, if the next slots run past this one: under way with
+		// the ids
+		const bool next = end < s1 && min(end + 32u * kFwAhead, s1) > wend;
+		if (next) {
+			f = end == wend ? f + 32u : f + __popc(__ballot_sync(0xffffffffu, start <= end)) - 1u;
+			load_window();
 		}
 #pragma unroll
 		for (int u = 0; u < kFwAhead; u++) {
 			const bool live = !((dw[u] >> bit[u]) & 1u);
-			const unsigned m = __ballot_sync(0xffffffffu, live);
-			const uint32_t p = run + __popc(m & ((1u << lane) - 1u));
+			unsigned m = 0;
+			uint32_t p = pos + u * 32u + lane;
+			if (kDels) {
+				m = __ballot_sync(0xffffffffu, live);
+				p = run + __popc(m & ((1u << lane) - 1u));
+			}
 			if (kPositions) {
 				const uint32_t slot = pos + u * 32u + lane;
 				if (slot < end) ids[slot] = live ? p : kNoId;
@@ -155,16 +182,13 @@ flat_write(FragSpace fs, const uint32_t* tile_base, const uint32_t* off, uint64_
 					bad = true;               // degrees and live slots disagree
 				}
 			}
-			if (head[u]) {
-				// the first fragment of a vertex: its row starts here
-				const uint32_t k = f + own[u], v = __ldg(fs.vert + k);
-				if (__ldg(fs.frag_off + v) == k) bad |= __ldg(off + v) != p;
-			}
+			if (row[u] != kNoId) bad |= row[u] != p;
 			run += __popc(m);
 		}
+		if (next) load_want();
 		pos = end;
 	}
-	if (!kPositions && t == fs.ntiles - 1u) bad |= run != __ldg(off + V);
+	if (!kPositions && t == fs.ntiles - 1u) bad |= (kDels ? run : fs.total) != __ldg(off + V);
 	if (bad) atomicOr(err, 2u);
 }
 
@@ -375,12 +399,11 @@ static lg_status build_rows(lg_snapshot* sn, int dir, FlatCsr& f, bool view, boo
 	if (fs.ntiles > 0) {
 		const unsigned blocks = grid_for(fs.ntiles, kFwWarps);
 		unsigned int* err = f.err.as<unsigned int>();
-		if (weighted)
-			flat_write<true, false><<<blocks, kFwThreads, 0, st>>>(fs, tile_base, off, V, (uint32_t)E,
-					f.ids.as<uint32_t>(), f.w.as<uint32_t>(), err);
-		else
-			flat_write<false, false><<<blocks, kFwThreads, 0, st>>>(fs, tile_base, off, V, (uint32_t)E,
-					f.ids.as<uint32_t>(), nullptr, err);
+		const auto k = weighted ? (tile_base ? flat_write<true, false, true>
+						: flat_write<true, false, false>)
+				: tile_base ? flat_write<false, false, true> : flat_write<false, false, false>;
+		k<<<blocks, kFwThreads, 0, st>>>(fs, tile_base, off, V, (uint32_t)E, f.ids.as<uint32_t>(),
+				weighted ? f.w.as<uint32_t>() : nullptr, err);
 		LG_CUDA(cudaGetLastError(), "flat_write");
 	}
 	unsigned int err = 0;
@@ -429,8 +452,9 @@ lg_status flat_positions(lg_snapshot* sn, int dir, const FlatCsr& f, uint32_t* p
 	if (fs.ntiles == 0) return LG_OK;
 	// (the tiles' bases are left from the flatten, behind their live counts)
 	const uint32_t* tile_base = d.n_dels > 0 ? f.flags.as<uint32_t>() + fs.ntiles : nullptr;
-	flat_write<false, true><<<grid_for(fs.ntiles, kFwWarps), kFwThreads, 0, s->stream>>>(fs,
-			tile_base, nullptr, sn->V, 0, pos, nullptr, nullptr);
+	const auto k = tile_base ? flat_write<false, true, true> : flat_write<false, true, false>;
+	k<<<grid_for(fs.ntiles, kFwWarps), kFwThreads, 0, s->stream>>>(fs, tile_base, nullptr, sn->V, 0,
+			pos, nullptr, nullptr);
 	LG_CUDA(cudaGetLastError(), "flat_positions");
 	s->launches++;
 	return LG_OK;
