@@ -334,10 +334,11 @@ lg_status exclusive_scan_slots(const SnapCsr& g, const uint32_t* list, uint64_t 
 		uint32_t* out, DevBuf& tmp, cudaStream_t stream, uint64_t* total);
 
 // Kernels a scan of n counts launches.
-constexpr uint64_t kScanTile = 8192;        // values per CTA
-constexpr uint64_t kScanOwnTiles = 4096;    // tiles whose CTAs add up the sums before theirs
+constexpr uint64_t kScanOne = 8192;         // values one CTA scans alone
+constexpr uint64_t kScanTile = 4096;        // values per CTA beyond that
+constexpr uint64_t kScanOwnTiles = 8192;    // tiles whose CTAs add up the sums before theirs
 inline uint64_t scan_launches(uint64_t n) {
-	return n <= kScanTile ? 1 : n <= kScanTile * kScanOwnTiles ? 2 : 3;
+	return n <= kScanOne ? 1 : n <= kScanTile * kScanOwnTiles ? 2 : 3;
 }
 
 // out[v] = live slots of v's fragments in direction dir (0 out, 1 in).

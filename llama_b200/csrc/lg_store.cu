@@ -230,17 +230,28 @@ lg_status append_dels(lg_store* s, DevCsr& csr, const uint2* add, size_t n,
 
 // ---------------------------------------------------------------------------
 // Exclusive scan (u32 -> u32) of an array or of the slot counts of a vertex
-// list.  Up to one tile: one CTA.  Up to kScanOwnTiles tiles: per-tile sums
-// (which also store the counts of a list), then per-tile scans whose CTAs each
-// add up the sums before theirs.  More: a single-CTA scan of the sums between
-// the two.  The traversals scan a frontier per step, so what counts up to some
-// 10^5 entries is the number of launches (2 to 3 us each): a list of 10^4
-// takes 1 or 2 where counting and the three-kernel scan took 4.
+// list.  Up to kScanOne values: one CTA.  Up to kScanOwnTiles tiles: per-tile
+// sums (which also store the counts of a list), then per-tile scans whose CTAs
+// each add up the sums before theirs.  More: a single-CTA scan of the sums
+// between the two.  The traversals scan a frontier per step, so what counts up
+// to some 10^5 entries is the number of launches (2 to 3 us each) and the
+// chain of loads and barriers in each: a list of 10^4 takes 1 or 2 where
+// counting and the three-kernel scan took 4.  Values go through shared memory,
+// so a warp's global accesses are consecutive whatever the arrays' alignment,
+// while every thread scans its own kItems consecutive values; one barrier
+// per tile.  Figures: 40 k values 3.5 + 3.9 us (4.4 + 9.3 where a thread's values
+// were loaded straight, vectors only in aligned arrays, and a tile took three
+// block scans of three barriers), 3 M values 5 + 7.5 (7 + 10.4, or 22.7
+// unaligned), the slot counts of 16 k vertices 6.5 us (11.5: one vertex's chain
+// of loads after the other).
 // ---------------------------------------------------------------------------
 
-constexpr int kScanThreads = 1024;
-constexpr int kScanItems = 8;
+constexpr int kScanThreads = 256;
+constexpr int kScanItems = 16;
 static_assert((uint64_t)kScanThreads * kScanItems == kScanTile, "values per CTA");
+constexpr int kOneThreads = 1024;                // the one-CTA form and the scan of the sums
+constexpr int kOneItems = 8;
+static_assert((uint64_t)kOneThreads * kOneItems == kScanOne, "values of the one-CTA form");
 
 __device__ __forceinline__ uint64_t block_excl_scan(uint64_t x, uint64_t* total) {
 	__shared__ uint64_t warp_sums[32];
@@ -270,77 +281,188 @@ __device__ __forceinline__ uint64_t block_excl_scan(uint64_t x, uint64_t* total)
 	return before + v - x;
 }
 
+// What is scanned.  load: x[j] = value i + j * step, 0 from n on; the loads of
+// all N values are issued before any is used.
 struct ScanArray {
 	const uint32_t* a;
-	__device__ __forceinline__ uint32_t operator()(uint64_t i) const { return a[i]; }
+	template <int N>
+	__device__ __forceinline__ void load(uint64_t i, uint32_t step, uint64_t n,
+			uint32_t (&x)[N]) const {
+#pragma unroll
+		for (int j = 0; j < N; j++)
+			x[j] = i + (uint64_t)j * step < n ? a[i + (uint64_t)j * step] : 0u;
+	}
 };
 
 // 1 for the positive values.
 struct ScanNonzero {
 	const uint32_t* a;
-	__device__ __forceinline__ uint32_t operator()(uint64_t i) const { return a[i] != 0u; }
+	template <int N>
+	__device__ __forceinline__ void load(uint64_t i, uint32_t step, uint64_t n,
+			uint32_t (&x)[N]) const {
+		ScanArray{a}.load(i, step, n, x);
+#pragma unroll
+		for (int j = 0; j < N; j++) x[j] = x[j] != 0u;
+	}
 };
 
 struct ScanSlots {
 	SnapCsr g;
 	const uint32_t* list;
-	__device__ __forceinline__ uint32_t operator()(uint64_t i) const {
-		return vertex_slots(g, list ? __ldg(list + i) : (uint32_t)i);
+	template <int N>
+	__device__ __forceinline__ void load(uint64_t i, uint32_t step, uint64_t n,
+			uint32_t (&x)[N]) const {
+		uint32_t v[N], a[N], b[N];
+#pragma unroll
+		for (int j = 0; j < N; j++) {
+			const uint64_t k = i + (uint64_t)j * step;
+			v[j] = k >= n ? kNoId : list ? __ldg(list + k) : (uint32_t)k;
+		}
+		const uint32_t* off = g.slot_off ? g.slot_off : g.frag_off;
+#pragma unroll
+		for (int j = 0; j < N; j++) {
+			a[j] = v[j] != kNoId ? __ldg(off + v[j]) : 0u;
+			b[j] = v[j] != kNoId ? __ldg(off + v[j] + 1) : 0u;
+		}
+#pragma unroll
+		for (int j = 0; j < N; j++) x[j] = g.slot_off ? b[j] - a[j] : 0u;
+		if (g.slot_off) return;
+		for (bool more = true; more;) {                // a fragment of each at a time
+			more = false;
+			uint2 f[N];
+#pragma unroll
+			for (int j = 0; j < N; j++) f[j] = a[j] < b[j] ? __ldg(g.frags + a[j]) : make_uint2(0u, 0u);
+#pragma unroll
+			for (int j = 0; j < N; j++) {
+				x[j] += frag_len(f[j]);
+				if (a[j] < b[j]) a[j]++;
+				more |= a[j] < b[j];
+			}
+		}
 	}
 };
 
-// One tile (n <= kScanTile): out[0 .. n] and the total in one CTA; cnt, if
-// not null, receives the values.
-template <class In>
-__global__ void __launch_bounds__(kScanThreads)
-scan_one(In in, uint32_t* cnt, uint32_t* out, uint32_t n, uint64_t* grand) {
-	uint32_t x[kScanItems];
+// One CTA's tile of kThreads * kItems values.
+template <int kThreads, int kItems>
+struct TileScan {
+	static constexpr int kWarps = kThreads / 32;
+	// a warp's values, one unused word after every kItems (no bank conflicts)
+	uint32_t stage[kWarps][32 * (kItems + 1)];
+	uint64_t sums[kWarps], first[kWarps];
+
+	// x[j] = value warp * 32 * kItems + j * 32 + lane of the tile; add(): the
+	// thread's share of what comes before the tile.  store(i, y) is called with
+	// y = the sum before value i.  Returns (all threads) the sum up to the
+	// tile's end.
+	template <class Add, class Store>
+	__device__ __forceinline__ uint64_t run(const uint32_t (&x)[kItems], Add&& add, Store&& store) {
+		static_assert((kItems & (kItems - 1)) == 0, "stage index");
+		const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+		uint32_t* st = stage[wid];
 #pragma unroll
-	for (int j = 0; j < kScanItems; j++) {
-		const uint32_t i = j * kScanThreads + threadIdx.x;
-		x[j] = i < n ? in(i) : 0u;
-	}
-	uint64_t carry = 0;
-#pragma unroll
-	for (int j = 0; j < kScanItems; j++) {
-		if (j * kScanThreads >= n) break;                    // block-uniform
-		const uint32_t i = j * kScanThreads + threadIdx.x;
-		uint64_t tot;
-		const uint64_t ex = block_excl_scan(x[j], &tot);
-		if (i < n) {
-			out[i] = (uint32_t)(carry + ex);
-			if (cnt) cnt[i] = x[j];
+		for (int j = 0; j < kItems; j++) {
+			const uint32_t i = j * 32u + lane;
+			st[i + i / kItems] = x[j];
 		}
-		carry += tot;
+		uint64_t b = add();
+		__syncwarp();
+		uint32_t y[kItems];
+		uint64_t s = 0;
+#pragma unroll
+		for (int j = 0; j < kItems; j++) {
+			y[j] = st[lane * (kItems + 1) + j];
+			s += y[j];
+		}
+		uint64_t v = s;
+#pragma unroll
+		for (int o = 1; o < 32; o <<= 1) {
+			const uint64_t t = __shfl_up_sync(0xffffffffu, v, o);
+			if (lane >= o) v += t;
+			b += __shfl_xor_sync(0xffffffffu, b, o);
+		}
+		if (lane == 31u) {
+			sums[wid] = v;
+			first[wid] = b;
+		}
+		__syncthreads();
+		// lane w of every warp: the sums of warp w
+		uint64_t at = lane < kWarps ? sums[lane] : 0, all = lane < kWarps ? first[lane] : 0;
+		all += at;
+		if (lane >= wid) at = 0;
+		at += lane < kWarps ? first[lane] : 0;
+#pragma unroll
+		for (int o = 16; o > 0; o >>= 1) {
+			at += __shfl_xor_sync(0xffffffffu, at, o);
+			all += __shfl_xor_sync(0xffffffffu, all, o);
+		}
+		uint64_t ex = at + v - s;
+#pragma unroll
+		for (int j = 0; j < kItems; j++) {
+			const uint32_t c = y[j];
+			st[lane * (kItems + 1) + j] = (uint32_t)ex;
+			ex += c;
+		}
+		__syncwarp();
+#pragma unroll
+		for (int j = 0; j < kItems; j++) {
+			const uint32_t i = j * 32u + lane;
+			store(wid * (32u * kItems) + i, st[i + i / kItems]);
+		}
+		return all;
 	}
+};
+
+// n <= kScanOne: out[0 .. n] and the total in one CTA; cnt, if not null,
+// receives the values.
+template <class In>
+__global__ void __launch_bounds__(kOneThreads)
+scan_one(In in, uint32_t* cnt, uint32_t* out, uint32_t n, uint64_t* grand) {
+	__shared__ TileScan<kOneThreads, kOneItems> ts;
+	const uint32_t first = (threadIdx.x >> 5) * (32u * kOneItems) + (threadIdx.x & 31u);
+	uint32_t x[kOneItems];
+	in.load(first, 32u, n, x);
+	if (cnt) {
+#pragma unroll
+		for (int j = 0; j < kOneItems; j++)
+			if (first + j * 32u < n) cnt[first + j * 32u] = x[j];
+	}
+	const uint64_t tot = ts.run(x, [] { return (uint64_t)0; },
+			[&](uint32_t i, uint32_t y) { if (i < n) out[i] = y; });
 	if (threadIdx.x == 0) {
-		out[n] = (uint32_t)carry;
-		*grand = carry;
+		out[n] = (uint32_t)tot;
+		*grand = tot;
 	}
 }
 
 template <class In>
 __global__ void __launch_bounds__(kScanThreads)
 scan_tile_sums(In in, uint64_t n, uint32_t* cnt, uint64_t* sums) {
-	uint64_t base = (uint64_t)blockIdx.x * kScanTile;
+	__shared__ uint64_t wsum[kScanThreads / 32];
+	const uint64_t base = (uint64_t)blockIdx.x * kScanTile + threadIdx.x;
+	uint32_t x[kScanItems];
+	in.load(base, kScanThreads, n, x);
 	uint64_t s = 0;
 #pragma unroll
 	for (int i = 0; i < kScanItems; i++) {
-		uint64_t idx = base + (uint64_t)i * kScanThreads + threadIdx.x;
-		if (idx < n) {
-			const uint32_t x = in(idx);
-			if (cnt) cnt[idx] = x;
-			s += x;
-		}
+		const uint64_t idx = base + (uint64_t)i * kScanThreads;
+		if (cnt && idx < n) cnt[idx] = x[i];
+		s += x[i];
 	}
-	uint64_t tot;
-	block_excl_scan(s, &tot);
-	if (threadIdx.x == 0) sums[blockIdx.x] = tot;
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+	if ((threadIdx.x & 31u) == 0) wsum[threadIdx.x >> 5] = s;
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		uint64_t tot = 0;
+		for (int w = 0; w < kScanThreads / 32; w++) tot += wsum[w];
+		sums[blockIdx.x] = tot;
+	}
 }
 
-__global__ void scan_sums_single(uint64_t* sums, uint64_t n, uint64_t* grand) {
+__global__ void __launch_bounds__(kOneThreads)
+scan_sums_single(uint64_t* sums, uint64_t n, uint64_t* grand) {
 	uint64_t carry = 0;
-	for (uint64_t b = 0; b < n; b += kScanThreads) {
+	for (uint64_t b = 0; b < n; b += kOneThreads) {
 		uint64_t i = b + threadIdx.x;
 		uint64_t x = i < n ? sums[i] : 0, tot;
 		uint64_t ex = block_excl_scan(x, &tot);
@@ -350,64 +472,35 @@ __global__ void scan_sums_single(uint64_t* sums, uint64_t n, uint64_t* grand) {
 	if (threadIdx.x == 0) *grand = carry;
 }
 
-// A thread scans kScanItems consecutive values; with 16-byte aligned arrays
-// it moves them as two 16-byte vectors each way.  sums: exclusive prefix of
-// the tiles (kOwn false, *grand the total), or the tiles' sums, of which every
-// CTA adds up those before it and the last one writes *grand.
+// sums: exclusive prefix of the tiles (kOwn false, *grand the total), or the
+// tiles' sums, of which every CTA adds up those before it and the last one
+// writes *grand.
 template <bool kOwn, bool kNonzero>
 __global__ void __launch_bounds__(kScanThreads)
 scan_tiles(const uint32_t* in, uint32_t* out, uint64_t n, const uint64_t* sums, uint64_t* grand) {
-	static_assert(kScanItems == 8, "two 16-byte vectors per thread");
-	uint64_t base = (uint64_t)blockIdx.x * kScanTile
-		+ (uint64_t)threadIdx.x * kScanItems;
-	const bool vec = ((((uintptr_t)in) | ((uintptr_t)out)) & 15u) == 0 && base + kScanItems <= n;
-	uint32_t vals[kScanItems];
-	if (vec) {
-		const uint4 a = __ldcs(reinterpret_cast<const uint4*>(in + base));
-		const uint4 b = __ldcs(reinterpret_cast<const uint4*>(in + base + 4));
-		vals[0] = a.x; vals[1] = a.y; vals[2] = a.z; vals[3] = a.w;
-		vals[4] = b.x; vals[5] = b.y; vals[6] = b.z; vals[7] = b.w;
-	} else {
+	__shared__ TileScan<kScanThreads, kScanItems> ts;
+	const uint64_t base = (uint64_t)blockIdx.x * kScanTile;
+	const uint64_t first = base + (threadIdx.x >> 5) * (32u * kScanItems) + (threadIdx.x & 31u);
+	uint32_t x[kScanItems];
 #pragma unroll
-		for (int i = 0; i < kScanItems; i++) {
-			uint64_t idx = base + i;
-			vals[i] = idx < n ? in[idx] : 0;
-		}
-	}
-	uint64_t s = 0;
+	for (int j = 0; j < kScanItems; j++)
+		x[j] = first + j * 32u < n ? __ldcs(in + first + j * 32u) : 0u;
+	if (kNonzero) {
 #pragma unroll
-	for (int i = 0; i < kScanItems; i++) {
-		if (kNonzero) vals[i] = vals[i] != 0u;
-		s += vals[i];
+		for (int j = 0; j < kScanItems; j++) x[j] = x[j] != 0u;
 	}
-	uint64_t tot, before;
-	if (kOwn) {
+	const uint64_t end = ts.run(x, [&] {
 		uint64_t b = 0;
-		for (uint32_t t = threadIdx.x; t < blockIdx.x; t += kScanThreads) b += sums[t];
-		block_excl_scan(b, &before);
-	} else {
-		before = sums[blockIdx.x];
-	}
-	uint64_t ex = block_excl_scan(s, &tot) + before;
-	uint32_t o[kScanItems];
-#pragma unroll
-	for (int i = 0; i < kScanItems; i++) {
-		o[i] = (uint32_t)ex;
-		ex += vals[i];
-	}
-	if (vec) {
-		reinterpret_cast<uint4*>(out + base)[0] = make_uint4(o[0], o[1], o[2], o[3]);
-		reinterpret_cast<uint4*>(out + base)[1] = make_uint4(o[4], o[5], o[6], o[7]);
-	} else {
-#pragma unroll
-		for (int i = 0; i < kScanItems; i++) {
-			uint64_t idx = base + i;
-			if (idx < n) out[idx] = o[i];
+		if (kOwn) {
+			for (uint32_t t = threadIdx.x; t < blockIdx.x; t += kScanThreads) b += __ldg(sums + t);
+		} else if (threadIdx.x == 0) {
+			b = __ldg(sums + blockIdx.x);
 		}
-	}
+		return b;
+	}, [&](uint32_t i, uint32_t y) { if (base + i < n) out[base + i] = y; });
 	if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
-		if (kOwn) *grand = before + tot;
-		out[n] = (uint32_t)(before + tot);
+		if (kOwn) *grand = end;
+		out[n] = (uint32_t)end;
 	}
 }
 
@@ -417,19 +510,18 @@ template <bool kNonzero, class In>
 static lg_status exclusive_scan(const In& in, const uint32_t* vals, uint32_t* cnt, uint32_t* out,
 		uint64_t n, DevBuf& tmp, cudaStream_t stream, uint64_t* total,
 		const uint64_t** dev_total = nullptr) {
-	uint64_t tiles = (n + kScanTile - 1) / kScanTile;
-	if (tiles == 0) tiles = 1;
+	const uint64_t tiles = n <= kScanOne ? 1 : (n + kScanTile - 1) / kScanTile;
 	LG_TRY(tmp.reserve((tiles + 1) * sizeof(uint64_t)));
 	uint64_t* sums = tmp.as<uint64_t>();
 	if (tiles == 1) {
-		scan_one<<<1, kScanThreads, 0, stream>>>(in, cnt, out, (uint32_t)n, sums + 1);
+		scan_one<<<1, kOneThreads, 0, stream>>>(in, cnt, out, (uint32_t)n, sums + 1);
 	} else {
 		scan_tile_sums<<<(unsigned)tiles, kScanThreads, 0, stream>>>(in, n, cnt, sums);
 		if (tiles <= kScanOwnTiles) {
 			scan_tiles<true, kNonzero><<<(unsigned)tiles, kScanThreads, 0, stream>>>(vals, out, n,
 					sums, sums + tiles);
 		} else {
-			scan_sums_single<<<1, kScanThreads, 0, stream>>>(sums, tiles, sums + tiles);
+			scan_sums_single<<<1, kOneThreads, 0, stream>>>(sums, tiles, sums + tiles);
 			scan_tiles<false, kNonzero><<<(unsigned)tiles, kScanThreads, 0, stream>>>(vals, out, n,
 					sums, sums + tiles);
 		}
