@@ -6,14 +6,17 @@
 //   rs_hist     per-tile digit counts, stored digit-major
 //   scan        exclusive scan of the counts -> scatter bases
 //   rs_scatter  stable scatter: a warp ranks its 512 consecutive keys of the
-//               tile 32 at a time (__match_any_sync groups the lanes that
-//               share a digit, the warp's own counters carry the ranks
-//               forward), one block-wide scan adds the other warps' counts,
-//               and the tile goes through shared memory in digit order, so a
-//               digit's keys leave as one contiguous run.
-// Bound by memory traffic (24 bytes per key and pass): the scatter before it
-// ranked a tile in 16 rounds with three block barriers each and wrote every
-// key straight to its place.
+//               tile 32 at a time (the lanes that share a digit are found with
+//               one match or nine votes, the warp's own counters carry the
+//               ranks forward), one block-wide scan adds the other warps'
+//               counts, and the tile goes through shared memory in digit order,
+//               so a digit's keys leave as one contiguous run.
+// What bounds rs_scatter is finding those lanes: matches alone keep their unit
+// 74 % busy, votes alone the ALU 85 %.  A third of the rounds by match and the
+// rest by votes uses both: 21.6 M keys take 115 us a pass (153 by match, 126 by
+// votes, 120 half and half; the traffic of 16 bytes per key is worth 53).  Keys
+// are read twice instead of held, which makes three CTAs resident of two (160
+// us); four would spill (136).
 #include "lg_device.cuh"
 #include "lg_sort.cuh"
 
@@ -62,8 +65,21 @@ rs_hist(const unsigned long long* k, uint64_t n, int shift, uint32_t* counts,
 // Shared memory of rs_scatter: the tile in digit order (keys, then payloads).
 constexpr size_t rs_smem(bool pay) { return kRsTile * (pay ? 12 : 8); }
 
+// Lanes of the warp that hold the same digit (0 .. 255); a lane past the end
+// (valid false) meets none of the others.
+__device__ __forceinline__ unsigned rs_peers(uint32_t dig, bool valid) {
+	const unsigned in = __ballot_sync(0xffffffffu, valid);
+	unsigned peers = valid ? in : ~in;
+#pragma unroll
+	for (int b = 0; b < 8; b++) {
+		const unsigned m = __ballot_sync(0xffffffffu, (dig >> b) & 1u);
+		peers &= (dig >> b) & 1u ? m : ~m;
+	}
+	return peers;
+}
+
 template <bool kPay>
-__global__ void __launch_bounds__(kRsThreads)
+__global__ void __launch_bounds__(kRsThreads, 3)
 rs_scatter(const unsigned long long* k, const uint32_t* pin, uint64_t n, int shift,
 		const uint32_t* offsets, uint32_t tiles, unsigned long long* kout,
 		uint32_t* pout) {
@@ -75,28 +91,27 @@ rs_scatter(const unsigned long long* k, const uint32_t* pin, uint64_t n, int shi
 	const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
 	const uint64_t tile0 = (uint64_t)blockIdx.x * kRsTile;
 	const uint64_t first = tile0 + w * (32u * kRsItems) + lane;
-	unsigned long long key[kRsItems];
+	uint32_t dig[kRsItems];                    // the digit; then digit << 16 | rank in the warp
 #pragma unroll
 	for (int r = 0; r < kRsItems; r++) {
 		const uint64_t i = first + (uint64_t)r * 32u;
-		key[r] = i < n ? k[i] : 0ull;
+		dig[r] = i < n ? (uint32_t)(k[i] >> shift) & 0xffu : 0u;
 	}
 #pragma unroll
 	for (int x = 0; x < kRsWarps; x++) wcnt[x][tid] = 0;
 	const uint32_t goff = offsets[(uint64_t)tid * tiles + blockIdx.x];
 	__syncthreads();
-	uint32_t rank[kRsItems];
 	const uint32_t below = (1u << lane) - 1u;
 #pragma unroll
 	for (int r = 0; r < kRsItems; r++) {
 		const bool valid = first + (uint64_t)r * 32u < n;
-		// lanes past the end take digit 256, which matches no real digit
-		const uint32_t dig = valid ? (uint32_t)((key[r] >> shift) & 0xff) : 256u;
-		const unsigned peers = __match_any_sync(0xffffffffu, dig);
-		const uint32_t before = valid ? wcnt[w][dig] : 0u;
+		const uint32_t d = dig[r];
+		const unsigned peers = r % 3 == 0 ? __match_any_sync(0xffffffffu, valid ? d : 256u)
+				: rs_peers(d, valid);
+		const uint32_t before = valid ? wcnt[w][d] : 0u;
 		__syncwarp();
-		rank[r] = before + __popc(peers & below);
-		if (valid && 31 - __clz(peers) == (int)lane) wcnt[w][dig] = before + __popc(peers);
+		dig[r] = d << 16 | (before + __popc(peers & below));
+		if (valid && 31 - __clz(peers) == (int)lane) wcnt[w][d] = before + __popc(peers);
 		__syncwarp();
 	}
 	__syncthreads();
@@ -125,13 +140,24 @@ rs_scatter(const unsigned long long* k, const uint32_t* pin, uint64_t n, int shi
 		dbase[tid] = goff - start;
 	}
 	__syncthreads();
+	// the keys again (from L2): held since the first read they were 32 registers
+	constexpr int kHalf = kRsItems / 2;
 #pragma unroll
-	for (int r = 0; r < kRsItems; r++) {
-		const uint64_t i = first + (uint64_t)r * 32u;
-		if (i < n) {
-			const uint32_t pos = wcnt[w][(key[r] >> shift) & 0xff] + rank[r];
-			skey[pos] = key[r];
-			if (kPay) spay[pos] = pin[i];
+	for (int h = 0; h < kRsItems; h += kHalf) {
+		unsigned long long key[kHalf];
+#pragma unroll
+		for (int r = 0; r < kHalf; r++) {
+			const uint64_t i = first + (uint64_t)(h + r) * 32u;
+			key[r] = i < n ? k[i] : 0ull;
+		}
+#pragma unroll
+		for (int r = 0; r < kHalf; r++) {
+			const uint64_t i = first + (uint64_t)(h + r) * 32u;
+			if (i < n) {
+				const uint32_t pos = wcnt[w][dig[h + r] >> 16] + (dig[h + r] & 0xffffu);
+				skey[pos] = key[r];
+				if (kPay) spay[pos] = pin[i];
+			}
 		}
 	}
 	__syncthreads();
