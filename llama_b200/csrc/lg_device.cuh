@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <memory>
 #include <utility>
 #include <vector>
@@ -139,13 +140,17 @@ __device__ __forceinline__ double warp_segsum(double v, uint32_t key, bool* tail
 
 // A store's stream-ordered memory pool for the temporaries of one call.
 // Memory given back to it is handed out again without a driver call that
-// waits for the GPU; up to kPoolKeep bytes stay with the pool between calls,
-// the rest goes back to the device at the next synchronisation, and all of it
-// when the store is destroyed or when any allocation of the process fails
-// (trim_pools).  stream becomes null when the store is destroyed; a buffer
-// that outlives its store is then freed with cudaFree.
+// waits for the GPU.  It holds at most kPoolKeep bytes, which stay with it until
+// the store is destroyed or any allocation of the process fails (trim_pools);
+// what does not fit is allocated and freed with cudaMalloc and cudaFree: mapping
+// pool memory costs 7 to 14 ms per GB, and giving it back as much again, against
+// 1 to 2 ms for cudaMalloc (SCC over 260 M edges in two flat copies of 1.3 GB
+// took 28 ms in a pool that gave back what it held beyond 1 GiB after every
+// call).  stream becomes null when the store is destroyed; a buffer that
+// outlives its store is then freed with cudaFree.
 struct CallPool {
 	cudaMemPool_t pool = nullptr;      // made on first use
+	std::atomic<uint64_t> used{0};     // bytes its buffers hold
 	cudaStream_t stream = nullptr;
 	int device = 0;
 	CallPool() = default;
@@ -162,6 +167,7 @@ lg_status make_pool(int device, cudaStream_t stream, std::shared_ptr<CallPool>* 
 struct DevBuf {
 	void* p = nullptr;
 	size_t bytes = 0;
+	bool pooled = false;               // p is the pool's
 	std::shared_ptr<CallPool> from;
 	DevBuf() = default;
 	explicit DevBuf(const std::shared_ptr<CallPool>& pool) : from(pool) {}
@@ -172,7 +178,12 @@ struct DevBuf {
 	// (Re)allocate to at least n bytes; contents are not preserved.
 	lg_status reserve(size_t n);
 	template <class T> T* as() const { return static_cast<T*>(p); }
-	void swap(DevBuf& o) { std::swap(p, o.p); std::swap(bytes, o.bytes); from.swap(o.from); }
+	void swap(DevBuf& o) {
+		std::swap(p, o.p);
+		std::swap(bytes, o.bytes);
+		std::swap(pooled, o.pooled);
+		from.swap(o.from);
+	}
 };
 
 struct DevLevel {

@@ -92,9 +92,11 @@ static void trim_pools() {
 
 void DevBuf::release() {
 	if (p) {
-		if (from && from->stream) cudaFreeAsync(p, from->stream);
+		if (pooled && from->stream) cudaFreeAsync(p, from->stream);
 		else cudaFree(p);
+		if (pooled) from->used -= bytes;
 	}
+	pooled = false;
 	p = nullptr;
 	bytes = 0;
 }
@@ -104,8 +106,9 @@ lg_status DevBuf::reserve(size_t n) {
 	release();
 	if (n == 0) n = 16;
 	cudaError_t e = cudaSuccess;
+	const bool in_pool = from && from->used + n <= kPoolKeep;
 	for (int attempt = 0; attempt < 2; attempt++) {
-		if (!from) e = cudaMalloc(&p, n);
+		if (!in_pool) e = cudaMalloc(&p, n);
 		else if ((e = open_pool(from.get())) == cudaSuccess)
 			e = cudaMallocFromPoolAsync(&p, n, from->pool, from->stream);
 		if (e != cudaErrorMemoryAllocation || attempt) break;
@@ -115,9 +118,11 @@ lg_status DevBuf::reserve(size_t n) {
 	if (e != cudaSuccess) {
 		p = nullptr;
 		(void)cudaGetLastError();
-		return cuda_status(e, from ? "cudaMallocFromPoolAsync" : "cudaMalloc");
+		return cuda_status(e, in_pool ? "cudaMallocFromPoolAsync" : "cudaMalloc");
 	}
 	bytes = n;
+	pooled = in_pool;
+	if (in_pool) from->used += n;
 	return LG_OK;
 }
 

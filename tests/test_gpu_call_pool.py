@@ -30,6 +30,23 @@ def test_pool_does_not_grow_from_call_to_call():
         assert st.device_bytes == held
 
 
+def test_temporaries_beyond_the_pool():
+    """1.6 GB of temporaries: what the pool cannot hold is given back."""
+    V, n = 40_000_003, 1000
+    ring = (np.arange(n, dtype=np.int64) * 39_999) % V
+    with Store() as st:
+        st.build_level(V, ring.astype(np.uint32), np.roll(ring, -1).astype(np.uint32))
+        with st.snapshot() as sn:
+            before = st.device_bytes
+            want = np.arange(V)
+            want[ring] = ring.min()
+            for _ in range(2):
+                labels, r = sn.scc()
+                assert r.components == V - n + 1
+                assert np.array_equal(labels, want)
+                assert st.device_bytes - before <= (1 << 30) + (64 << 20)
+
+
 def test_tape_freed_after_its_store():
     st = _store()
     sn = st.snapshot()
