@@ -298,7 +298,7 @@ __device__ __forceinline__ bool bsearch_u32(const uint32_t* base, uint32_t n, ui
 // against 476; four: 477, and slower with two rows in flight, 516 against 417).
 constexpr uint32_t kTcPairs = 8;
 constexpr int kTcLists = 5;
-constexpr uint32_t kTcDomain0 = 1u << 16;     //   8 KB per bitmap: one warp each
+constexpr uint32_t kTcDomain0 = 1u << 16;     //   8 KB per bitmap: two warps
 constexpr uint32_t kTcDomain1 = 1u << 18;     //  32 KB: four warps
 constexpr uint32_t kTcDomain2 = 7u << 18;     // 224 KB: a CTA of 32 warps, one per SM
 constexpr uint32_t kTcHashMost = 64;          // a quarter of the table's slots
