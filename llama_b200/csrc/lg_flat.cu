@@ -28,6 +28,7 @@
 #include "lg_sort.cuh"
 
 #include <algorithm>
+#include <climits>
 #include <cstring>
 
 namespace lg {
@@ -69,9 +70,10 @@ flat_live(FragSpace fs, uint32_t* live) {
 		bool more = true;
 #pragma unroll
 		for (int u = 0; u < kFlAhead; u++) {
-			const uint32_t k = f + u * 32u + lane;
-			const uint32_t st = k < fs.F ? __ldg(fs.start + k) : 0xffffffffu;
-			const uint2 fr = k < fs.F ? __ldg(fs.frags + k) : make_uint2(0u, 0u);
+			const uint32_t i = u * 32u + lane, k = f + i;
+			const bool have = i < fs.F - f;              // (f <= F; f + i may wrap)
+			const uint32_t st = have ? __ldg(fs.start + k) : 0xffffffffu;
+			const uint2 fr = have ? __ldg(fs.frags + k) : make_uint2(0u, 0u);
 			const bool in = st < s1;
 			more = in;
 			a[u] = in ? fr.x + (max(st, s0) - st) : 0u;
@@ -121,27 +123,37 @@ flat_write(FragSpace fs, const uint32_t* tile_base, const uint32_t* off, uint64_
 	const uint32_t lane = threadIdx.x & 31u;
 	const uint32_t t = blockIdx.x * kFwWarps + (threadIdx.x >> 5);
 	if (t >= fs.ntiles) return;
+	// Slots are counted from the tile's first, s0: a bound formed from absolute
+	// slots would wrap in the last tiles of a slot space close to 2^32.
 	const uint32_t s0 = t * kSlotTile;
-	const uint32_t s1 = fs.total - s0 < kSlotTile ? fs.total : s0 + kSlotTile;
-	// The window: fragments f ... f + 31, a lane each, covering slots up to wend.
+	const int n = (int)min(fs.total - s0, kSlotTile);
+	// The window: fragments f ... f + 31 (f <= F), a lane each, covering slots up
+	// to wend; start = the fragment's first slot (INT_MAX from the tile's end
+	// on), src = where slot s0 would lie in its level if the fragment held it.
 	// want = where its vertex's row starts if the fragment is the vertex's
 	// first, kNoId if not.
 	uint32_t f = __ldg(fs.tile_frag + t);
-	uint32_t start = 0xffffffffu, wend = fs.total, vert = 0, want = kNoId;
-	uint2 fr = make_uint2(0u, 0u);
+	int start = INT_MAX, wend = n;
+	uint32_t src = 0, level = 0, vert = 0, want = kNoId;
 	auto load_window = [&]() {
-		const uint32_t k = f + lane;
-		start = 0xffffffffu;
-		if (k < fs.F) {
-			start = __ldg(fs.start + k);
-			fr = __ldg(fs.frags + k);
+		start = INT_MAX;
+		if (lane < fs.F - f) {
+			const uint32_t k = f + lane;
+			const uint32_t a = __ldg(fs.start + k);
+			const uint2 fr = __ldg(fs.frags + k);
+			// (a fragment begun before the tile reaches into it, so it began
+			// less than a fragment's longest length before)
+			if (a < s0 || a - s0 < (uint32_t)n) start = (int)(a - s0);
+			src = fr.x + (s0 - a);
+			level = frag_level(fr);
 			if (!kPositions) vert = __ldg(fs.vert + k);
 		}
-		wend = f + 32u <= fs.F ? __ldg(fs.start + f + 32u) : fs.total;
+		wend = n;
+		if (fs.F - f >= 32u) wend = (int)min(__ldg(fs.start + f + 32u) - s0, (uint32_t)n);
 	};
 	auto load_want = [&]() {
 		want = kNoId;
-		if (kPositions || f + lane >= fs.F) return;
+		if (kPositions || lane >= fs.F - f) return;
 		const uint32_t first = __ldg(fs.frag_off + vert), o = __ldg(off + vert);
 		if (first == f + lane) want = o;
 	};
@@ -150,22 +162,21 @@ flat_write(FragSpace fs, const uint32_t* tile_base, const uint32_t* off, uint64_
 	uint32_t run = kDels ? __ldg(tile_base + t) : 0u;
 	bool bad = false;
 	const uint32_t upto = 2u << lane;          // bits at or below the lane, + 1
-	for (uint32_t pos = s0; pos < s1;) {
-		const uint32_t full = min(pos + 32u * kFwAhead, s1);
-		const uint32_t end = min(full, wend);
+	for (int pos = 0; pos < n;) {
+		const int end = min(min(pos + 32 * kFwAhead, n), wend);
 		uint32_t id[kFwAhead], dw[kFwAhead], wt[kFwAhead], bit[kFwAhead];
 		uint32_t row[kFwAhead];                // where a row that begins at the slot starts
 #pragma unroll
 		for (int u = 0; u < kFwAhead; u++) {
-			const uint32_t base = pos + u * 32u;
+			const int base = pos + u * 32;
 			// fragments begun before the chunk, and those that begin in it
-			const uint32_t rel = start - base;
+			const uint32_t rel = (uint32_t)start - (uint32_t)base;
 			const uint32_t begun = __popc(__ballot_sync(0xffffffffu, start < base));
 			const uint32_t mask = __reduce_or_sync(0xffffffffu, rel < 32u ? 1u << rel : 0u);
 			const uint32_t own = begun - 1u + __popc(mask & (upto - 1u));
-			const uint32_t ix = __shfl_sync(0xffffffffu, fr.x - start, own) + base + lane;
-			const uint32_t lv = __shfl_sync(0xffffffffu, fr.y, own) & kLevelMask;
-			const bool in = base + lane < end;
+			const uint32_t ix = __shfl_sync(0xffffffffu, src, own) + (uint32_t)base + lane;
+			const uint32_t lv = __shfl_sync(0xffffffffu, level, own);
+			const bool in = base + (int)lane < end;
 			bit[u] = ix & 31u;
 			dw[u] = !in ? ~0u : kDels ? __ldg(lt.del[lv] + (ix >> 5)) : 0u;
 			if (!kPositions) id[u] = in ? __ldcs(lt.ids[lv] + ix) : 0u;
@@ -177,7 +188,7 @@ flat_write(FragSpace fs, const uint32_t* tile_base, const uint32_t* off, uint64_
 		}
 		// the next window, if the next slots run past this one: under way with
 		// the ids
-		const bool next = end < s1 && min(end + 32u * kFwAhead, s1) > wend;
+		const bool next = end < n && min(end + 32 * kFwAhead, n) > wend;
 		if (next) {
 			f = end == wend ? f + 32u : f + __popc(__ballot_sync(0xffffffffu, start <= end)) - 1u;
 			load_window();
@@ -186,14 +197,14 @@ flat_write(FragSpace fs, const uint32_t* tile_base, const uint32_t* off, uint64_
 		for (int u = 0; u < kFwAhead; u++) {
 			const bool live = !((dw[u] >> bit[u]) & 1u);
 			unsigned m = 0;
-			uint32_t p = pos + u * 32u + lane;
+			const uint32_t slot = s0 + (uint32_t)(pos + u * 32) + lane;
+			uint32_t p = slot;
 			if (kDels) {
 				m = __ballot_sync(0xffffffffu, live);
 				p = run + __popc(m & ((1u << lane) - 1u));
 			}
 			if (kPositions) {
-				const uint32_t slot = pos + u * 32u + lane;
-				if (slot < end) ids[slot] = live ? p : kNoId;
+				if (pos + u * 32 + (int)lane < end) ids[slot] = live ? p : kNoId;
 				run += __popc(m);
 				continue;
 			}
