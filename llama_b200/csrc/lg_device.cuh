@@ -365,10 +365,11 @@ lg_status copy_out(lg_store* s, void* dst, const void* src, size_t bytes);
 
 // The store's kHostWords pinned words (allocated on first use), for
 // counters a host loop reads back every step.
-constexpr int kHostWords = 16;
+constexpr int kHostWords = 20;
+constexpr int kReadWords = kHostWords - 8;   // the most read_words copies
 lg_status host_words(lg_store* s, unsigned long long** words);
-// Waits for the store's stream and reads n <= 8 device words into out through
-// pinned words 8..15 (words 0..7 stay with the caller).
+// Waits for the store's stream and reads n <= kReadWords device words into out
+// through the pinned words from 8 on (words 0..7 stay with the caller).
 lg_status read_words(lg_store* s, const unsigned long long* dev, int n, unsigned long long* out);
 
 // A DevLevel for direction dir (0 out, 1 in) of a new level: the store's

@@ -9,10 +9,12 @@
 //      giant component that settles nearly all vertices that have edges both
 //      ways, at about a tenth of the edges read once, where colouring reads
 //      them all several times;
-//   3. what is left by rounds of colouring, every step of every round in one
-//      cooperative launch (scc_rest): the smallest label is pushed along
-//      out-edges to a fixpoint, a backward search within a colour from the
-//      vertices that kept their own collects their components.
+//   3. what is left by rounds of colouring, the steps of all rounds in one
+//      cooperative launch (scc_rest), or several of kCoopRunNs each: the smallest
+//      label is pushed along out-edges to a fixpoint, a backward search within a
+//      colour from the vertices that kept their own collects their components.
+//      (A chain whose ids ascend settles one vertex per round, with as many
+//      steps as it is still long.)
 // Colouring alone, over fragments and with the host reading each step's
 // counts, took 2.9 ms at 3 M vertices / 39 M edges, 1.2 ms of it pushing and
 // 1.0 ms searching through the giant component.
@@ -24,6 +26,7 @@
 #include "lg_tune.h"
 
 #include <cstddef>
+#include <cstring>
 #include <mutex>
 
 namespace lg {
@@ -96,15 +99,25 @@ scc_giant_label(const uint32_t* rem, uint32_t n, const int32_t* fwd, const int32
 	block_push<kListThreads>(keep, v, rem_next, ctr);
 }
 
+// The colouring between two steps, the same in every CTA.
+enum SrPhase : uint32_t { kSrColour, kSrPush, kSrRoots, kSrSearch, kSrCollect };
+struct alignas(16) SrState {
+	u64 n_rem;              // vertices left, listed in rem[rsel]
+	u64 n;                  // a push or search step's, in list[lsel]
+	uint32_t rsel, lsel;
+	uint32_t phase;         // of the next step
+	uint32_t slot;          // its counters
+	uint32_t round, stamp, steps, pad;
+};
+
 struct SrCtl {
-	u64 ctr[3][2];          // per step: [0] appends, [1] row pieces
-	u64 out[4];             // rounds, steps
+	u64 ctr[3][3];          // per step: [0] appends, [1] row pieces, [2] the launch's time is up
+	SrState st;             // where the last launch left off
 	CoopBar bar;            // err bit 2: a count out of range, bit 3: round cap
 };
 
 struct SrArgs {
 	const uint32_t *ooff, *oids, *ioff, *iids;
-	const u64* n_rem;       // vertices left, listed in rem[0]
 	uint32_t V;
 	uint32_t max_pieces;
 	uint32_t* rem[2];
@@ -116,7 +129,8 @@ struct SrArgs {
 struct SrShared {
 	uint32_t sbuf[kSrWarps][kPushBuf];
 	RowWindow win[kSrWarps];
-	u64 got[2];
+	u64 got[3];
+	SrState st;
 };
 
 // A warp's expansion of list vertices: colours pushed along out-edges
@@ -223,124 +237,107 @@ scc_rest(SrArgs a, SrCtl* c) {
 	const uint32_t tid = threadIdx.x, wid = tid >> 5;
 	const uint32_t gtid = blockIdx.x * kSrThreads + tid, nthreads = gridDim.x * kSrThreads;
 	const uint32_t gwarp = wid * gridDim.x + blockIdx.x, nwarps = gridDim.x * kSrWarps;
-	uint32_t slot = 0;
+	const uint64_t t0 = global_ns();
+	if (tid < sizeof(SrState) / 4)
+		reinterpret_cast<uint32_t*>(&sh.st)[tid] =
+				__ldcg(reinterpret_cast<const uint32_t*>(&c->st) + tid);
+	__syncthreads();
+	SrState t = sh.st;
 	// counters rotate over three slots: a step fills cnt() and clears the slot
 	// the next one fills, which was read before the last barrier but one
-	auto cnt = [&]() { return c->ctr[slot]; };
-	auto begin = [&]() {
-		if (gtid < 2) c->ctr[slot == 2u ? 0u : slot + 1u][gtid] = 0;
-	};
+	auto cnt = [&]() { return c->ctr[t.slot]; };
 	auto barrier = [&]() {
+		if (gtid == 0 && global_ns() - t0 > kCoopRunNs) cnt()[2] = 1;
 		if (!grid_barrier(&c->bar)) return false;
-		if (tid < 2) sh.got[tid] = __ldcg(cnt() + tid);
+		if (tid < 3) sh.got[tid] = __ldcg(cnt() + tid);
 		__syncthreads();
 		return true;
 	};
-	auto end = [&]() { slot = slot == 2u ? 0u : slot + 1u; };
 	auto fail = [&](unsigned bit) { if (tid == 0) atomicOr(&c->bar.err, bit); };
+	// the vertices of rem[rsel] that take(v) picks, appended to `to`
+	auto pick = [&](uint32_t* to, auto&& take) {
+		uint32_t nb = 0;
+		for (uint64_t i0 = (uint64_t)gwarp * 32u; i0 < t.n_rem; i0 += (uint64_t)nwarps * 32u) {
+			const uint64_t i = i0 + (tid & 31u);
+			const uint32_t v = i < t.n_rem ? __ldcg(a.rem[t.rsel] + i) : 0u;
+			wq_add(i < t.n_rem && take(v), v, sh.sbuf[wid], nb, to, cnt());
+		}
+		wq_flush(sh.sbuf[wid], nb, to, cnt());
+	};
+	// expands list[lsel][0, n) into the other list; false: leave
+	auto expand = [&](auto&& s) {
+		t.steps++;
+		s.lists(a.list[t.lsel], (uint32_t)t.n, gwarp, nwarps);
+		if (!barrier()) return false;
+		const u64 np = sh.got[1];
+		if (np > a.max_pieces) {
+			fail(4u);
+			return false;
+		}
+		if (np) {
+			s.pieces((uint32_t)np, gwarp, nwarps);
+			if (!barrier()) return false;
+		}
+		t.n = sh.got[0];
+		t.lsel ^= 1u;
+		if (t.n <= a.V) return true;
+		fail(4u);
+		return false;
+	};
 
-	if (tid == 0) sh.got[0] = __ldcg(a.n_rem);
-	__syncthreads();
-	u64 n_rem = sh.got[0];
-	__syncthreads();
-	uint32_t rsel = 0, round = 0, stamp = 0, steps = 0;
-	while (n_rem > 0) {
-		round++;
-		if (round > a.V + 1u) return fail(8u);
-		// colours: the vertices' own; the first list is all of them
-		begin();
-		for (uint64_t i = gtid; i < n_rem; i += nthreads) {
-			const uint32_t v = __ldcg(a.rem[rsel] + i);
-			a.color[v] = v;
-			a.list[0][i] = v;
-		}
-		if (!barrier()) return;
-		end();
-		// expands list[lsel][0, n) until nothing is appended
-		u64 n = n_rem;
-		uint32_t lsel = 0;
-		while (n > 0) {
-			begin();
-			stamp++;
-			steps++;
-			SrStep<true> s(a, stamp, sh.sbuf[wid], a.list[lsel ^ 1u], cnt(), sh.win + wid);
-			s.lists(a.list[lsel], (uint32_t)n, gwarp, nwarps);
+	for (bool up = false; t.n_rem > 0 && !up;) {
+		if (gtid < 3) c->ctr[t.slot == 2u ? 0u : t.slot + 1u][gtid] = 0;
+		if (t.phase == kSrColour) {
+			// colours: the vertices' own; the first list is all of them
+			t.round++;
+			if (t.round > a.V + 1u) return fail(8u);
+			for (uint64_t i = gtid; i < t.n_rem; i += nthreads) {
+				const uint32_t v = __ldcg(a.rem[t.rsel] + i);
+				a.color[v] = v;
+				a.list[0][i] = v;
+			}
 			if (!barrier()) return;
-			const u64 np = sh.got[1];
-			if (np > a.max_pieces) return fail(4u);
-			if (np) {
-				s.pieces((uint32_t)np, gwarp, nwarps);
-				if (!barrier()) return;
-			}
-			n = sh.got[0];
-			if (n > a.V) return fail(4u);
-			lsel ^= 1u;
-			end();
-		}
-		// vertices that kept their own colour begin the backward search
-		begin();
-		{
-			uint32_t nb = 0;
-			for (uint64_t i0 = (uint64_t)gwarp * 32u; i0 < n_rem; i0 += (uint64_t)nwarps * 32u) {
-				const uint64_t i = i0 + (tid & 31u);
-				uint32_t v = 0;
-				bool root = false;
-				if (i < n_rem) {
-					v = __ldcg(a.rem[rsel] + i);
-					root = __ldcg(a.color + v) == v;
-					if (root) a.mark[v] = round;
-				}
-				wq_add(root, v, sh.sbuf[wid], nb, a.list[lsel], cnt());
-			}
-			wq_flush(sh.sbuf[wid], nb, a.list[lsel], cnt());
-		}
-		if (!barrier()) return;
-		n = sh.got[0];
-		end();
-		while (n > 0) {
-			begin();
-			steps++;
-			SrStep<false> s(a, round, sh.sbuf[wid], a.list[lsel ^ 1u], cnt(), sh.win + wid);
-			s.lists(a.list[lsel], (uint32_t)n, gwarp, nwarps);
+			t.n = t.n_rem;
+			t.lsel = 0;
+			t.phase = kSrPush;
+		} else if (t.phase == kSrPush) {
+			t.stamp++;
+			if (!expand(SrStep<true>(a, t.stamp, sh.sbuf[wid], a.list[t.lsel ^ 1u], cnt(),
+					sh.win + wid)))
+				return;
+			if (t.n == 0) t.phase = kSrRoots;
+		} else if (t.phase == kSrRoots) {
+			// vertices that kept their own colour begin the backward search
+			pick(a.list[t.lsel], [&](uint32_t v) {
+				const bool root = __ldcg(a.color + v) == v;
+				if (root) a.mark[v] = t.round;
+				return root;
+			});
 			if (!barrier()) return;
-			const u64 np = sh.got[1];
-			if (np > a.max_pieces) return fail(4u);
-			if (np) {
-				s.pieces((uint32_t)np, gwarp, nwarps);
-				if (!barrier()) return;
-			}
-			n = sh.got[0];
-			if (n > a.V) return fail(4u);
-			lsel ^= 1u;
-			end();
+			t.n = sh.got[0];
+			t.phase = kSrSearch;
+		} else if (t.phase == kSrSearch) {
+			if (!expand(SrStep<false>(a, t.round, sh.sbuf[wid], a.list[t.lsel ^ 1u], cnt(),
+					sh.win + wid)))
+				return;
+			if (t.n == 0) t.phase = kSrCollect;
+		} else {
+			// collected vertices are settled, the others stay for the next round
+			pick(a.rem[t.rsel ^ 1u], [&](uint32_t v) {
+				const bool keep = __ldcg(a.mark + v) != t.round;
+				if (!keep) a.label[v] = __ldcg(a.color + v);
+				return keep;
+			});
+			if (!barrier()) return;
+			if (sh.got[0] >= t.n_rem) return fail(4u);     // a round settles some
+			t.n_rem = sh.got[0];
+			t.rsel ^= 1u;
+			t.phase = kSrColour;
 		}
-		// collected vertices are settled, the others stay for the next round
-		begin();
-		{
-			uint32_t nb = 0;
-			for (uint64_t i0 = (uint64_t)gwarp * 32u; i0 < n_rem; i0 += (uint64_t)nwarps * 32u) {
-				const uint64_t i = i0 + (tid & 31u);
-				uint32_t v = 0;
-				bool keep = false;
-				if (i < n_rem) {
-					v = __ldcg(a.rem[rsel] + i);
-					if (__ldcg(a.mark + v) == round) a.label[v] = __ldcg(a.color + v);
-					else keep = true;
-				}
-				wq_add(keep, v, sh.sbuf[wid], nb, a.rem[rsel ^ 1u], cnt());
-			}
-			wq_flush(sh.sbuf[wid], nb, a.rem[rsel ^ 1u], cnt());
-		}
-		if (!barrier()) return;
-		if (sh.got[0] >= n_rem) return fail(4u);         // a round settles some
-		n_rem = sh.got[0];
-		rsel ^= 1u;
-		end();
+		up = sh.got[2] != 0;
+		t.slot = t.slot == 2u ? 0u : t.slot + 1u;
 	}
-	if (gtid == 0) {
-		c->out[0] = round;
-		c->out[1] = steps;
-	}
+	if (gtid == 0) c->st = t;
 }
 
 std::mutex g_coop_mu;
@@ -388,7 +385,8 @@ lg_status scc_flat_run(lg_snapshot* sn, const FlatCsr* fo, const FlatCsr* fi, ui
 	int32_t* fwd = reinterpret_cast<int32_t*>(a.list[0]);
 	int32_t* bwd = reinterpret_cast<int32_t*>(a.list[1]);
 	SrCtl* ctl = ctrb.as<SrCtl>();
-	u64* ctr = reinterpret_cast<u64*>(ctl + 1);      // [0], [1] trim; [2] left; [3] smallest
+	u64* ctr = reinterpret_cast<u64*>(ctl + 1);      // [0], [1] trim; [3] smallest
+	u64* left = &ctl->st.n_rem;                      // the lists' length after the searches
 	LG_CUDA(cudaMemsetAsync(ctl, 0, sizeof(SrCtl) + 3 * sizeof(u64), st), "clear");
 	LG_CUDA(cudaMemsetAsync(ctr + 3, 0xff, sizeof(u64), st), "clear");
 	const uint32_t* odeg = sn->out.deg.as<uint32_t>();
@@ -423,26 +421,34 @@ lg_status scc_flat_run(lg_snapshot* sn, const FlatCsr* fo, const FlatCsr* fi, ui
 	uint32_t* best = reinterpret_cast<uint32_t*>(ctr + 3);
 	scc_giant_min<<<grid_for(n_rem, B), B, 0, st>>>(a.rem[1], (uint32_t)n_rem, fwd, bwd, best);
 	scc_giant_label<<<grid_for(n_rem, B), B, 0, st>>>(a.rem[1], (uint32_t)n_rem, fwd, bwd, best,
-			label, a.rem[0], ctr + 2);
+			label, a.rem[0], left);
 	LG_CUDA(cudaGetLastError(), "scc_giant");
+	s->launches += 2;
 	// the rest
-	a.n_rem = ctr + 2;
 	a.max_pieces = (uint32_t)(2 * std::max(fo->E, fi->E) / kSrPiece + 1);
 	LG_TRY(pieces.reserve((uint64_t)a.max_pieces * sizeof(uint2)));
 	a.pieces = pieces.as<uint2>();
 	void* kargs[] = {&a, &ctl};
-	LG_CUDA(cudaLaunchCooperativeKernel((const void*)scc_rest, dim3((unsigned)grid),
-			dim3(kSrThreads), kargs, 0, st), "scc_rest");
-	s->launches += 3;
-	u64 o[6];
-	static_assert(offsetof(SrCtl, bar) == offsetof(SrCtl, out) + 32, "two words after the results");
-	LG_TRY(read_words(s, ctl->out, 6, o));
-	const unsigned err = (unsigned)o[5];               // the barrier's error word
-	if (err & 1u) return set_error(LG_ETIMEOUT, "scc: a grid barrier wait ran out");
-	if (err & 4u) return set_error(LG_ECUDA, "scc: a list count out of range");
-	if (err & 8u) return set_error(LG_ETIMEOUT, "SCC did not converge");
-	*rounds = (uint32_t)o[0] + 1u;
-	*steps += (int)o[1];
+	for (;;) {
+		LG_CUDA(cudaLaunchCooperativeKernel((const void*)scc_rest, dim3((unsigned)grid),
+				dim3(kSrThreads), kargs, 0, st), "scc_rest");
+		s->launches++;
+		constexpr int kWords = (int)(sizeof(SrState) / sizeof(u64)) + 2;
+		static_assert(offsetof(SrCtl, bar) == offsetof(SrCtl, st) + sizeof(SrState) &&
+				sizeof(SrState) % sizeof(u64) == 0 && kWords <= kReadWords, "state, then the barrier");
+		u64 o[kWords];
+		LG_TRY(read_words(s, reinterpret_cast<const u64*>(&ctl->st), kWords, o));
+		const unsigned err = (unsigned)o[kWords - 1];  // the barrier's error word
+		if (err & 1u) return set_error(LG_ETIMEOUT, "scc: a grid barrier wait ran out");
+		if (err & 4u) return set_error(LG_ECUDA, "scc: a list count out of range");
+		if (err & 8u) return set_error(LG_ETIMEOUT, "SCC did not converge");
+		SrState t;
+		std::memcpy(&t, o, sizeof(t));
+		if (t.n_rem > 0) continue;
+		*rounds = t.round + 1u;
+		*steps += (int)t.steps;
+		break;
+	}
 	*ran = true;
 	return LG_OK;
 }

@@ -73,3 +73,21 @@ def test_partition(shape):
                 both = (np.bincount(s[live], minlength=V) > 0) & (
                     np.bincount(d[live], minlength=V) > 0)
                 assert r.trimmed == V - both.sum()
+
+
+def test_chain_settles_a_vertex_per_round():
+    """Ids that ascend along a chain: n rounds of up to n steps.  No launch
+    takes them all, so that none holds the GPU for as long as they take: a
+    launch ends after 50 ms, and half a million steps with a barrier each
+    (a microsecond at the least) do not fit into five of them."""
+    V = 1000
+    a = np.arange(V - 1)
+    with Store() as st:
+        st.build_level(V, a, a + 1)
+        with st.snapshot() as sn:
+            sn.flatten(0).flatten(1)
+            before = st.launch_count
+            lab, r = sn.scc()
+            assert np.array_equal(lab, np.arange(V)) and r.components == V
+            assert r.rounds >= V - 4 and r.steps >= (V - 4) ** 2 // 2
+            assert st.launch_count - before > 14         # 10 with one launch of scc_rest
