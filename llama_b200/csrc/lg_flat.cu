@@ -28,7 +28,6 @@
 #include "lg_sort.cuh"
 
 #include <algorithm>
-#include <climits>
 #include <cstring>
 
 namespace lg {
@@ -123,33 +122,25 @@ flat_write(FragSpace fs, const uint32_t* tile_base, const uint32_t* off, uint64_
 	const uint32_t lane = threadIdx.x & 31u;
 	const uint32_t t = blockIdx.x * kFwWarps + (threadIdx.x >> 5);
 	if (t >= fs.ntiles) return;
-	// Slots are counted from the tile's first, s0: a bound formed from absolute
-	// slots would wrap in the last tiles of a slot space close to 2^32.
 	const uint32_t s0 = t * kSlotTile;
-	const int n = (int)min(fs.total - s0, kSlotTile);
+	const uint32_t s1 = fs.total - s0 < kSlotTile ? fs.total : s0 + kSlotTile;
 	// The window: fragments f ... f + 31 (f <= F), a lane each, covering slots up
-	// to wend; start = the fragment's first slot (INT_MAX from the tile's end
-	// on), src = where slot s0 would lie in its level if the fragment held it.
+	// to wend.  Sums of slot or fragment numbers may wrap where there are close to
+	// 2^32 of either: what bounds the loop is compared as distances.
 	// want = where its vertex's row starts if the fragment is the vertex's
 	// first, kNoId if not.
 	uint32_t f = __ldg(fs.tile_frag + t);
-	int start = INT_MAX, wend = n;
-	uint32_t src = 0, level = 0, vert = 0, want = kNoId;
+	uint32_t start = 0xffffffffu, wend = fs.total, vert = 0, want = kNoId;
+	uint2 fr = make_uint2(0u, 0u);
 	auto load_window = [&]() {
-		start = INT_MAX;
+		const uint32_t k = f + lane;
+		start = 0xffffffffu;
 		if (lane < fs.F - f) {
-			const uint32_t k = f + lane;
-			const uint32_t a = __ldg(fs.start + k);
-			const uint2 fr = __ldg(fs.frags + k);
-			// (a fragment begun before the tile reaches into it, so it began
-			// less than a fragment's longest length before)
-			if (a < s0 || a - s0 < (uint32_t)n) start = (int)(a - s0);
-			src = fr.x + (s0 - a);
-			level = frag_level(fr);
+			start = __ldg(fs.start + k);
+			fr = __ldg(fs.frags + k);
 			if (!kPositions) vert = __ldg(fs.vert + k);
 		}
-		wend = n;
-		if (fs.F - f >= 32u) wend = (int)min(__ldg(fs.start + f + 32u) - s0, (uint32_t)n);
+		wend = fs.F - f >= 32u ? __ldg(fs.start + f + 32u) : fs.total;
 	};
 	auto load_want = [&]() {
 		want = kNoId;
@@ -162,21 +153,22 @@ flat_write(FragSpace fs, const uint32_t* tile_base, const uint32_t* off, uint64_
 	uint32_t run = kDels ? __ldg(tile_base + t) : 0u;
 	bool bad = false;
 	const uint32_t upto = 2u << lane;          // bits at or below the lane, + 1
-	for (int pos = 0; pos < n;) {
-		const int end = min(min(pos + 32 * kFwAhead, n), wend);
+	for (uint32_t pos = s0; pos < s1;) {
+		const uint32_t most = min(min(s1, wend) - pos, 32u * kFwAhead);
+		const uint32_t end = pos + most;
 		uint32_t id[kFwAhead], dw[kFwAhead], wt[kFwAhead], bit[kFwAhead];
 		uint32_t row[kFwAhead];                // where a row that begins at the slot starts
 #pragma unroll
 		for (int u = 0; u < kFwAhead; u++) {
-			const int base = pos + u * 32;
+			const uint32_t base = pos + u * 32u;
 			// fragments begun before the chunk, and those that begin in it
-			const uint32_t rel = (uint32_t)start - (uint32_t)base;
+			const uint32_t rel = start - base;
 			const uint32_t begun = __popc(__ballot_sync(0xffffffffu, start < base));
 			const uint32_t mask = __reduce_or_sync(0xffffffffu, rel < 32u ? 1u << rel : 0u);
 			const uint32_t own = begun - 1u + __popc(mask & (upto - 1u));
-			const uint32_t ix = __shfl_sync(0xffffffffu, src, own) + (uint32_t)base + lane;
-			const uint32_t lv = __shfl_sync(0xffffffffu, level, own);
-			const bool in = base + (int)lane < end;
+			const uint32_t ix = __shfl_sync(0xffffffffu, fr.x - start, own) + base + lane;
+			const uint32_t lv = __shfl_sync(0xffffffffu, fr.y, own) & kLevelMask;
+			const bool in = u * 32u + lane < most;
 			bit[u] = ix & 31u;
 			dw[u] = !in ? ~0u : kDels ? __ldg(lt.del[lv] + (ix >> 5)) : 0u;
 			if (!kPositions) id[u] = in ? __ldcs(lt.ids[lv] + ix) : 0u;
@@ -188,7 +180,7 @@ flat_write(FragSpace fs, const uint32_t* tile_base, const uint32_t* off, uint64_
 		}
 		// the next window, if the next slots run past this one: under way with
 		// the ids
-		const bool next = end < n && min(end + 32 * kFwAhead, n) > wend;
+		const bool next = wend < s1 && wend - end < 32u * kFwAhead;
 		if (next) {
 			f = end == wend ? f + 32u : f + __popc(__ballot_sync(0xffffffffu, start <= end)) - 1u;
 			load_window();
@@ -197,14 +189,14 @@ flat_write(FragSpace fs, const uint32_t* tile_base, const uint32_t* off, uint64_
 		for (int u = 0; u < kFwAhead; u++) {
 			const bool live = !((dw[u] >> bit[u]) & 1u);
 			unsigned m = 0;
-			const uint32_t slot = s0 + (uint32_t)(pos + u * 32) + lane;
-			uint32_t p = slot;
+			uint32_t p = pos + u * 32u + lane;
 			if (kDels) {
 				m = __ballot_sync(0xffffffffu, live);
 				p = run + __popc(m & ((1u << lane) - 1u));
 			}
 			if (kPositions) {
-				if (pos + u * 32 + (int)lane < end) ids[slot] = live ? p : kNoId;
+				const uint32_t slot = pos + u * 32u + lane;
+				if (u * 32u + lane < most) ids[slot] = live ? p : kNoId;
 				run += __popc(m);
 				continue;
 			}
