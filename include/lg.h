@@ -386,7 +386,8 @@ lg_status lg_pagerank_gather_pass(lg_snapshot* snap, int passes, double* checksu
  * With the snapshot's in-CSR flat (lg_snapshot_flatten(snap, 1)), or a store
  * without one, the whole traversal is one cooperative launch whose CTAs
  * choose each level's direction on the device and meet at bounded grid
- * barriers (LG_TUNE_BFS_LEVELS; LG_ETIMEOUT if a barrier wait runs out);
+ * barriers (LG_TUNE_BFS_LEVELS; LG_ETIMEOUT if a barrier wait runs out; a
+ * launch ends after 50 ms and another goes on from there);
  * otherwise a launch sequence per level with the direction chosen on the
  * host.  Both make the same choices and give the same result. */
 typedef struct lg_bfs_result {

@@ -1,5 +1,6 @@
 // lg_bfs_levels.cu - a whole direction-optimising BFS in one cooperative
-// launch.
+// launch (on graphs of some 10^4 levels and more in several: one returns after
+// kCoopRunCycles, with the traversal's state in the control block).
 //
 // lg_bfs's step-per-launch loop reads the next frontier's size back to the
 // host after every level to choose the next direction, and a top-down level
@@ -60,14 +61,26 @@ constexpr uint32_t kLvMaxRange = 1024; // top-down slots per warp range
 constexpr int32_t kLvUnreached = LG_UNREACHED;
 constexpr double kAlpha = 14.0, kBeta = 24.0;   // as lg_bfs's host loop
 
+// The traversal's state between two levels, the same in every CTA.
+struct LvState {
+	unsigned long long mu;          // out-edges of the vertices not reached yet
+	unsigned long long reached, reach_edges;
+	long long list_len;             // unfound rows of the last bottom-up level, -1: none
+	int32_t cur, td, bu;            // level, steps top-down and bottom-up
+	int32_t qsel;                   // which of the two queues is current
+	int32_t top_down, have_queue;
+	int32_t list_in_fcnt;           // that list is in fcnt (else in fpos)
+	int32_t done;
+};
+
 // Control block (device memory; bfs_levels_init resets it).
 struct LvCtl {
-	unsigned long long ctr[3][4];   // per level: [0] frontier size, [1] its out-degree
-	                                // sum, [2] queue fill cursor, [3] unfound rows
+	unsigned long long ctr[3][5];   // per level: [0] frontier size, [1] its out-degree
+	                                // sum, [2] queue fill cursor, [3] unfound rows,
+	                                // [4] the launch's time was up before it
 	CoopBar bar;                    // err bit 0: a barrier wait gave up, bit 1: slots
 	                                // above 2^32
-	int32_t levels, td, bu, pad;
-	unsigned long long reached, reach_edges;
+	LvState st;                     // where the last launch left off
 };
 
 // Appends item[j] for every j with take[j] to out at slots taken from *len:
@@ -115,17 +128,21 @@ __device__ __forceinline__ uint32_t lv_range(uint32_t total, uint32_t nwarps) {
 
 // Resets the control block and queues the root; bfs_levels fills the level
 // array and the first two bitmaps itself.
-__global__ void bfs_levels_init(uint32_t root, uint32_t* q0, const uint32_t* outdeg, LvCtl* c) {
+__global__ void bfs_levels_init(uint32_t root, uint32_t* q0, const uint32_t* outdeg,
+		unsigned long long out_edges, LvCtl* c) {
 	if (blockIdx.x == 0 && threadIdx.x == 0) {
 		q0[0] = root;
 		for (int i = 0; i < 3; i++)
-			for (int j = 0; j < 4; j++) c->ctr[i][j] = 0;
+			for (int j = 0; j < 5; j++) c->ctr[i][j] = 0;
 		c->ctr[0][0] = 1;
 		c->ctr[0][1] = __ldg(outdeg + root);
 		c->bar.count = 0;
 		c->bar.err = 0;
-		c->levels = c->td = c->bu = c->pad = 0;
-		c->reached = c->reach_edges = 0;
+		LvState t = {};
+		t.mu = out_edges;
+		t.list_len = -1;
+		t.top_down = t.have_queue = 1;
+		c->st = t;
 	}
 }
 
@@ -133,27 +150,34 @@ __global__ void bfs_levels_init(uint32_t root, uint32_t* q0, const uint32_t* out
 __global__ void __launch_bounds__(kLvThreads, 2)
 bfs_levels(SnapCsr out, const uint32_t* nz_rows, const uint32_t* nz_off, uint32_t R,
 		uint32_t E, const uint32_t* in_ids, const uint32_t* outdeg, uint32_t V,
-		unsigned long long out_edges, int has_in, int32_t* level, uint32_t* q0, uint32_t* q1,
-		uint32_t* bits0, uint32_t* bits1, uint32_t* bits2, uint32_t* fcnt, uint32_t* fpos,
-		unsigned long long* bsum, LvCtl* c) {
+		int has_in, int32_t* level, uint32_t* q0, uint32_t* q1, uint32_t* bits0, uint32_t* bits1,
+		uint32_t* bits2, uint32_t* fcnt, uint32_t* fpos, unsigned long long* bsum, LvCtl* c) {
 	const uint32_t W = (uint32_t)(((uint64_t)V + 31u) / 32u);
 	const uint32_t tid = threadIdx.x, lane = tid & 31u;
 	const uint32_t nthreads = gridDim.x * blockDim.x;
 	const uint32_t gtid = blockIdx.x * blockDim.x + tid;
 	const uint32_t nwarps = nthreads >> 5, gwarp = gtid >> 5;
 	__shared__ uint32_t s_pos[kLvThreads * kLvSmallPer + 1];   // offsets of a small queue
-	uint32_t *q = q0, *nq = q1;
 	auto bm = [&](int i) { return i == 0 ? bits0 : i == 1 ? bits1 : bits2; };
-	// every CTA keeps the same copy of the traversal state
-	unsigned long long mu = out_edges, reached = 0, reach_edges = 0;
-	bool top_down = true, have_queue = true;
-	long long list_len = -1;          // unfound rows of the last bottom-up level, -1: none
-	bool list_in_fcnt = false;        // that list is in fcnt (else in fpos)
-	int32_t td = 0, bu = 0, cur = 0;
-	{
+	const long long t0 = clock64();
+	const uint32_t root = __ldcg(q0);          // (of the first launch)
+	// every CTA keeps the same copy of the traversal's state
+	__shared__ LvState s_st;
+	if (tid < sizeof(LvState) / 4)
+		reinterpret_cast<uint32_t*>(&s_st)[tid] =
+				__ldcg(reinterpret_cast<const uint32_t*>(&c->st) + tid);
+	__syncthreads();
+	unsigned long long mu = s_st.mu, reached = s_st.reached, reach_edges = s_st.reach_edges;
+	bool top_down = s_st.top_down, have_queue = s_st.have_queue;
+	long long list_len = s_st.list_len;
+	bool list_in_fcnt = s_st.list_in_fcnt;
+	int32_t td = s_st.td, bu = s_st.bu, cur = s_st.cur;
+	const int32_t first = cur;
+	uint32_t *q = s_st.qsel ? q1 : q0, *nq = s_st.qsel ? q0 : q1;
+	bool done = false;
+	if (cur == 0) {
 		// levels: 0 at the root, unreached elsewhere; bitmap 0 = {root},
 		// bitmap 1 clear (level 0's next frontier)
-		const uint32_t root = __ldcg(q0);
 		for (uint32_t v = gtid; v < V; v += nthreads) level[v] = v == root ? 0 : kLvUnreached;
 		for (uint32_t w = gtid; w < W; w += nthreads) {
 			bits0[w] = w == (root >> 5) ? 1u << (root & 31u) : 0u;
@@ -171,19 +195,20 @@ bfs_levels(SnapCsr out, const uint32_t* nz_rows, const uint32_t* nz_off, uint32_
 		uint32_t* clear = bm((cur + 2) % 3);
 		// one warp per CTA reads the counters (read by every thread of the grid,
 		// their sector took some 3 us a level)
-		__shared__ unsigned long long s_ctr[4];
+		__shared__ unsigned long long s_ctr[5];
 		__syncthreads();                         // s_ctr free from the last level
-		if (tid < 4) s_ctr[tid] = __ldcg(now + tid);
+		if (tid < 5) s_ctr[tid] = __ldcg(now + tid);
 		__syncthreads();
 		const unsigned long long qlen = s_ctr[0], mf = s_ctr[1];
 		if (!have_queue) list_len = (long long)s_ctr[3];
-		if (qlen == 0) break;
+		done = qlen == 0;
+		if (done || (s_ctr[4] && cur != first)) break;
 		reached += qlen;
 		reach_edges += mf;
 		mu -= min(mu, mf);
 		if (top_down && has_in && (double)mf > (double)mu / kAlpha) top_down = false;
 		else if (!top_down && (double)qlen < (double)V / kBeta) top_down = true;
-		if (blockIdx.x == 0 && tid < 4) c->ctr[(cur + 2) % 3][tid] = 0;
+		if (blockIdx.x == 0 && tid < 5) c->ctr[(cur + 2) % 3][tid] = 0;
 		for (uint32_t w = gtid; w < W; w += nthreads) clear[w] = 0u;
 
 		if (top_down) {
@@ -404,6 +429,7 @@ bfs_levels(SnapCsr out, const uint32_t* nz_rows, const uint32_t* nz_off, uint32_
 			}
 			bu++;
 		}
+		if (gtid == 0 && clock64() - t0 > kCoopRunCycles) nxt[4] = 1;
 		if (!grid_barrier(&c->bar)) return;
 		if (top_down) {
 			uint32_t* t = q; q = nq; nq = t;
@@ -414,12 +440,21 @@ bfs_levels(SnapCsr out, const uint32_t* nz_rows, const uint32_t* nz_off, uint32_
 			list_in_fcnt = !list_in_fcnt;
 		}
 	}
-	if (blockIdx.x == 0 && tid == 0) {
-		c->levels = cur;
-		c->td = td;
-		c->bu = bu;
-		c->reached = reached;
-		c->reach_edges = reach_edges;
+	if (gtid == 0) {
+		LvState t;
+		t.mu = mu;
+		t.reached = reached;
+		t.reach_edges = reach_edges;
+		t.list_len = list_len;
+		t.cur = cur;
+		t.td = td;
+		t.bu = bu;
+		t.qsel = q == q1;
+		t.top_down = top_down;
+		t.have_queue = have_queue;
+		t.list_in_fcnt = list_in_fcnt;
+		t.done = done;
+		c->st = t;
 	}
 }
 
@@ -471,7 +506,6 @@ lg_status bfs_levels_over(lg_store* s, SnapCsr out, const FlatCsr* fi, const uin
 	uint32_t R = fi ? (uint32_t)fi->R : 0u, E = fi ? (uint32_t)fi->E : 0u;
 	const uint32_t* in_ids = fi ? fi->ids.as<uint32_t>() : nullptr;
 	uint32_t V32 = (uint32_t)V;
-	unsigned long long out_edges = n_edges;
 	int has_in = fi ? 1 : 0;
 	uint32_t* q0 = sc[0].as<uint32_t>();
 	uint32_t* q1 = sc[1].as<uint32_t>();
@@ -483,28 +517,30 @@ lg_status bfs_levels_over(lg_store* s, SnapCsr out, const FlatCsr* fi, const uin
 	LvCtl* ctl = sc[9].as<LvCtl>();
 	unsigned long long* bsum = reinterpret_cast<unsigned long long*>(
 			sc[9].as<unsigned char>() + sizeof(LvCtl));
-	bfs_levels_init<<<1, 32, 0, st>>>(root, q0, outdeg, ctl);
+	bfs_levels_init<<<1, 32, 0, st>>>(root, q0, outdeg, n_edges, ctl);
 	LG_CUDA(cudaGetLastError(), "bfs_levels_init");
-	void* args[] = {&out, &nz_rows, &nz_off, &R, &E, &in_ids, &outdeg, &V32, &out_edges,
-			&has_in, &lvl, &q0, &q1, &bits0, &bits1, &bits2, &fcnt, &fpos, &bsum, &ctl};
-	LG_CUDA(cudaLaunchCooperativeKernel((const void*)bfs_levels, dim3((unsigned)grid),
-			dim3(kLvThreads), args, 0, st), "bfs_levels");
-	s->launches += 2;
+	void* args[] = {&out, &nz_rows, &nz_off, &R, &E, &in_ids, &outdeg, &V32, &has_in, &lvl, &q0,
+			&q1, &bits0, &bits1, &bits2, &fcnt, &fpos, &bsum, &ctl};
+	s->launches++;
 	LvCtl h;
-	LG_CUDA(cudaMemcpyAsync(&h, ctl, sizeof(h), cudaMemcpyDeviceToHost, st), "d2h");
-	LG_CUDA(cudaStreamSynchronize(st), "bfs_levels");
-	s->d2h_bytes += sizeof(h);
-	if (h.bar.err & 1u)
-		return set_error(LG_ETIMEOUT, "bfs: a grid barrier wait ran out (%d levels done)",
-				h.levels);
-	if (h.bar.err & 2u)
-		return set_error(LG_ENOTSUP, "bfs: a frontier holds 2^32 or more slots");
+	do {
+		LG_CUDA(cudaLaunchCooperativeKernel((const void*)bfs_levels, dim3((unsigned)grid),
+				dim3(kLvThreads), args, 0, st), "bfs_levels");
+		s->launches++;
+		LG_CUDA(cudaMemcpyAsync(&h, ctl, sizeof(h), cudaMemcpyDeviceToHost, st), "d2h");
+		LG_CUDA(cudaStreamSynchronize(st), "bfs_levels");
+		s->d2h_bytes += sizeof(h);
+		if (h.bar.err & 1u)
+			return set_error(LG_ETIMEOUT, "bfs: a grid barrier wait ran out");
+		if (h.bar.err & 2u)
+			return set_error(LG_ENOTSUP, "bfs: a frontier holds 2^32 or more slots");
+	} while (!h.st.done);
 	if (result) {
-		result->reached = h.reached;
-		result->reach_edges = h.reach_edges;
-		result->max_level = h.levels - 1;
-		result->top_down_steps = h.td;
-		result->bottom_up_steps = h.bu;
+		result->reached = h.st.reached;
+		result->reach_edges = h.st.reach_edges;
+		result->max_level = h.st.cur - 1;
+		result->top_down_steps = h.st.td;
+		result->bottom_up_steps = h.st.bu;
 		result->reserved = 0;
 	}
 	*ran = true;

@@ -19,8 +19,9 @@ struct alignas(16) CoopBar {
 constexpr uint64_t kCoopWaitNs = 1000000000ull;   // a barrier wait gives up after 1 s
 // A kernel whose steps depend on the graph (a chain takes as many as it has
 // vertices, or their square) returns with its state after so long, and the
-// host launches it again: neither the host nor other streams wait longer.
-constexpr uint64_t kCoopRunNs = 50000000ull;
+// host launches it again: neither the host nor other streams wait longer.  In
+// cycles of the SM that looks (50 ms at 2 GHz), a register read.
+constexpr long long kCoopRunCycles = 100000000;
 
 __device__ __forceinline__ uint64_t global_ns() {
 	uint64_t t;

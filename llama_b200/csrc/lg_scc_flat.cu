@@ -10,7 +10,7 @@
 //      ways, at about a tenth of the edges read once, where colouring reads
 //      them all several times;
 //   3. what is left by rounds of colouring, the steps of all rounds in one
-//      cooperative launch (scc_rest), or several of kCoopRunNs each: the smallest
+//      cooperative launch (scc_rest), or several of kCoopRunCycles each: the smallest
 //      label is pushed along out-edges to a fixpoint, a backward search within a
 //      colour from the vertices that kept their own collects their components.
 //      (A chain whose ids ascend settles one vertex per round, with as many
@@ -237,7 +237,7 @@ scc_rest(SrArgs a, SrCtl* c) {
 	const uint32_t tid = threadIdx.x, wid = tid >> 5;
 	const uint32_t gtid = blockIdx.x * kSrThreads + tid, nthreads = gridDim.x * kSrThreads;
 	const uint32_t gwarp = wid * gridDim.x + blockIdx.x, nwarps = gridDim.x * kSrWarps;
-	const uint64_t t0 = global_ns();
+	const long long t0 = clock64();
 	if (tid < sizeof(SrState) / 4)
 		reinterpret_cast<uint32_t*>(&sh.st)[tid] =
 				__ldcg(reinterpret_cast<const uint32_t*>(&c->st) + tid);
@@ -247,7 +247,7 @@ scc_rest(SrArgs a, SrCtl* c) {
 	// the next one fills, which was read before the last barrier but one
 	auto cnt = [&]() { return c->ctr[t.slot]; };
 	auto barrier = [&]() {
-		if (gtid == 0 && global_ns() - t0 > kCoopRunNs) cnt()[2] = 1;
+		if (gtid == 0 && clock64() - t0 > kCoopRunCycles) cnt()[2] = 1;
 		if (!grid_barrier(&c->bar)) return false;
 		if (tid < 3) sh.got[tid] = __ldcg(cnt() + tid);
 		__syncthreads();
