@@ -75,9 +75,9 @@ struct LvState {
 
 // Control block (device memory; bfs_levels_init resets it).
 struct LvCtl {
-	unsigned long long ctr[3][5];   // per level: [0] frontier size, [1] its out-degree
-	                                // sum, [2] queue fill cursor, [3] unfound rows,
-	                                // [4] the launch's time was up before it
+	unsigned long long ctr[3][4];   // per level: [0] frontier size, [1] its out-degree
+	                                // sum (and kCoopTimeUp: before the level), [2] queue
+	                                // fill cursor, [3] unfound rows
 	CoopBar bar;                    // err bit 0: a barrier wait gave up, bit 1: slots
 	                                // above 2^32
 	LvState st;                     // where the last launch left off
@@ -128,21 +128,15 @@ __device__ __forceinline__ uint32_t lv_range(uint32_t total, uint32_t nwarps) {
 
 // Resets the control block and queues the root; bfs_levels fills the level
 // array and the first two bitmaps itself.
-__global__ void bfs_levels_init(uint32_t root, uint32_t* q0, const uint32_t* outdeg,
-		unsigned long long out_edges, LvCtl* c) {
+__global__ void bfs_levels_init(uint32_t root, uint32_t* q0, const uint32_t* outdeg, LvCtl* c) {
 	if (blockIdx.x == 0 && threadIdx.x == 0) {
 		q0[0] = root;
 		for (int i = 0; i < 3; i++)
-			for (int j = 0; j < 5; j++) c->ctr[i][j] = 0;
+			for (int j = 0; j < 4; j++) c->ctr[i][j] = 0;
 		c->ctr[0][0] = 1;
 		c->ctr[0][1] = __ldg(outdeg + root);
 		c->bar.count = 0;
 		c->bar.err = 0;
-		LvState t = {};
-		t.mu = out_edges;
-		t.list_len = -1;
-		t.top_down = t.have_queue = 1;
-		c->st = t;
 	}
 }
 
@@ -150,8 +144,9 @@ __global__ void bfs_levels_init(uint32_t root, uint32_t* q0, const uint32_t* out
 __global__ void __launch_bounds__(kLvThreads, 2)
 bfs_levels(SnapCsr out, const uint32_t* nz_rows, const uint32_t* nz_off, uint32_t R,
 		uint32_t E, const uint32_t* in_ids, const uint32_t* outdeg, uint32_t V,
-		int has_in, int32_t* level, uint32_t* q0, uint32_t* q1, uint32_t* bits0, uint32_t* bits1,
-		uint32_t* bits2, uint32_t* fcnt, uint32_t* fpos, unsigned long long* bsum, LvCtl* c) {
+		unsigned long long out_edges, int has_in, int32_t* level, uint32_t* q0, uint32_t* q1,
+		uint32_t* bits0, uint32_t* bits1, uint32_t* bits2, uint32_t* fcnt, uint32_t* fpos,
+		unsigned long long* bsum, LvCtl* c, int resume) {
 	const uint32_t W = (uint32_t)(((uint64_t)V + 31u) / 32u);
 	const uint32_t tid = threadIdx.x, lane = tid & 31u;
 	const uint32_t nthreads = gridDim.x * blockDim.x;
@@ -160,24 +155,34 @@ bfs_levels(SnapCsr out, const uint32_t* nz_rows, const uint32_t* nz_off, uint32_
 	__shared__ uint32_t s_pos[kLvThreads * kLvSmallPer + 1];   // offsets of a small queue
 	auto bm = [&](int i) { return i == 0 ? bits0 : i == 1 ? bits1 : bits2; };
 	const long long t0 = clock64();
-	const uint32_t root = __ldcg(q0);          // (of the first launch)
 	// every CTA keeps the same copy of the traversal's state
-	__shared__ LvState s_st;
-	if (tid < sizeof(LvState) / 4)
-		reinterpret_cast<uint32_t*>(&s_st)[tid] =
-				__ldcg(reinterpret_cast<const uint32_t*>(&c->st) + tid);
-	__syncthreads();
-	unsigned long long mu = s_st.mu, reached = s_st.reached, reach_edges = s_st.reach_edges;
-	bool top_down = s_st.top_down, have_queue = s_st.have_queue;
-	long long list_len = s_st.list_len;
-	bool list_in_fcnt = s_st.list_in_fcnt;
-	int32_t td = s_st.td, bu = s_st.bu, cur = s_st.cur;
-	const int32_t first = cur;
-	uint32_t *q = s_st.qsel ? q1 : q0, *nq = s_st.qsel ? q0 : q1;
-	bool done = false;
-	if (cur == 0) {
+	unsigned long long mu = out_edges, reached = 0, reach_edges = 0;
+	bool top_down = true, have_queue = true;
+	long long list_len = -1;
+	bool list_in_fcnt = false;
+	int32_t td = 0, bu = 0, cur = 0;
+	uint32_t *q = q0, *nq = q1;
+	if (resume) {
+		__shared__ LvState s_st;
+		if (tid < sizeof(LvState) / 4)
+			reinterpret_cast<uint32_t*>(&s_st)[tid] =
+					__ldcg(reinterpret_cast<const uint32_t*>(&c->st) + tid);
+		__syncthreads();
+		mu = s_st.mu;
+		reached = s_st.reached;
+		reach_edges = s_st.reach_edges;
+		top_down = s_st.top_down;
+		have_queue = s_st.have_queue;
+		list_len = s_st.list_len;
+		list_in_fcnt = s_st.list_in_fcnt;
+		td = s_st.td;
+		bu = s_st.bu;
+		cur = s_st.cur;
+		if (s_st.qsel) { q = q1; nq = q0; }
+	} else {
 		// levels: 0 at the root, unreached elsewhere; bitmap 0 = {root},
 		// bitmap 1 clear (level 0's next frontier)
+		const uint32_t root = __ldcg(q0);
 		for (uint32_t v = gtid; v < V; v += nthreads) level[v] = v == root ? 0 : kLvUnreached;
 		for (uint32_t w = gtid; w < W; w += nthreads) {
 			bits0[w] = w == (root >> 5) ? 1u << (root & 31u) : 0u;
@@ -185,6 +190,8 @@ bfs_levels(SnapCsr out, const uint32_t* nz_rows, const uint32_t* nz_off, uint32_
 		}
 		if (!grid_barrier(&c->bar)) return;
 	}
+	const int32_t first = cur;
+	bool done = false;
 	for (;; cur++) {
 		unsigned long long* now = c->ctr[cur % 3];
 		unsigned long long* nxt = c->ctr[(cur + 1) % 3];
@@ -195,20 +202,20 @@ bfs_levels(SnapCsr out, const uint32_t* nz_rows, const uint32_t* nz_off, uint32_
 		uint32_t* clear = bm((cur + 2) % 3);
 		// one warp per CTA reads the counters (read by every thread of the grid,
 		// their sector took some 3 us a level)
-		__shared__ unsigned long long s_ctr[5];
+		__shared__ unsigned long long s_ctr[4];
 		__syncthreads();                         // s_ctr free from the last level
-		if (tid < 5) s_ctr[tid] = __ldcg(now + tid);
+		if (tid < 4) s_ctr[tid] = __ldcg(now + tid);
 		__syncthreads();
-		const unsigned long long qlen = s_ctr[0], mf = s_ctr[1];
+		const unsigned long long qlen = s_ctr[0], mf = s_ctr[1] & ~kCoopTimeUp;
 		if (!have_queue) list_len = (long long)s_ctr[3];
 		done = qlen == 0;
-		if (done || (s_ctr[4] && cur != first)) break;
+		if (done || (s_ctr[1] >= kCoopTimeUp && cur != first)) break;
 		reached += qlen;
 		reach_edges += mf;
 		mu -= min(mu, mf);
 		if (top_down && has_in && (double)mf > (double)mu / kAlpha) top_down = false;
 		else if (!top_down && (double)qlen < (double)V / kBeta) top_down = true;
-		if (blockIdx.x == 0 && tid < 5) c->ctr[(cur + 2) % 3][tid] = 0;
+		if (blockIdx.x == 0 && tid < 4) c->ctr[(cur + 2) % 3][tid] = 0;
 		for (uint32_t w = gtid; w < W; w += nthreads) clear[w] = 0u;
 
 		if (top_down) {
@@ -429,7 +436,7 @@ bfs_levels(SnapCsr out, const uint32_t* nz_rows, const uint32_t* nz_off, uint32_
 			}
 			bu++;
 		}
-		if (gtid == 0 && clock64() - t0 > kCoopRunCycles) nxt[4] = 1;
+		if (gtid == 0 && clock64() - t0 > kCoopRunCycles) atomicOr(nxt + 1, kCoopTimeUp);
 		if (!grid_barrier(&c->bar)) return;
 		if (top_down) {
 			uint32_t* t = q; q = nq; nq = t;
@@ -506,7 +513,8 @@ lg_status bfs_levels_over(lg_store* s, SnapCsr out, const FlatCsr* fi, const uin
 	uint32_t R = fi ? (uint32_t)fi->R : 0u, E = fi ? (uint32_t)fi->E : 0u;
 	const uint32_t* in_ids = fi ? fi->ids.as<uint32_t>() : nullptr;
 	uint32_t V32 = (uint32_t)V;
-	int has_in = fi ? 1 : 0;
+	unsigned long long out_edges = n_edges;
+	int has_in = fi ? 1 : 0, resume = 0;
 	uint32_t* q0 = sc[0].as<uint32_t>();
 	uint32_t* q1 = sc[1].as<uint32_t>();
 	uint32_t* bits0 = sc[2].as<uint32_t>();
@@ -517,13 +525,13 @@ lg_status bfs_levels_over(lg_store* s, SnapCsr out, const FlatCsr* fi, const uin
 	LvCtl* ctl = sc[9].as<LvCtl>();
 	unsigned long long* bsum = reinterpret_cast<unsigned long long*>(
 			sc[9].as<unsigned char>() + sizeof(LvCtl));
-	bfs_levels_init<<<1, 32, 0, st>>>(root, q0, outdeg, n_edges, ctl);
+	bfs_levels_init<<<1, 32, 0, st>>>(root, q0, outdeg, ctl);
 	LG_CUDA(cudaGetLastError(), "bfs_levels_init");
-	void* args[] = {&out, &nz_rows, &nz_off, &R, &E, &in_ids, &outdeg, &V32, &has_in, &lvl, &q0,
-			&q1, &bits0, &bits1, &bits2, &fcnt, &fpos, &bsum, &ctl};
+	void* args[] = {&out, &nz_rows, &nz_off, &R, &E, &in_ids, &outdeg, &V32, &out_edges,
+			&has_in, &lvl, &q0, &q1, &bits0, &bits1, &bits2, &fcnt, &fpos, &bsum, &ctl, &resume};
 	s->launches++;
 	LvCtl h;
-	do {
+	for (;; resume = 1) {
 		LG_CUDA(cudaLaunchCooperativeKernel((const void*)bfs_levels, dim3((unsigned)grid),
 				dim3(kLvThreads), args, 0, st), "bfs_levels");
 		s->launches++;
@@ -534,7 +542,8 @@ lg_status bfs_levels_over(lg_store* s, SnapCsr out, const FlatCsr* fi, const uin
 			return set_error(LG_ETIMEOUT, "bfs: a grid barrier wait ran out");
 		if (h.bar.err & 2u)
 			return set_error(LG_ENOTSUP, "bfs: a frontier holds 2^32 or more slots");
-	} while (!h.st.done);
+		if (h.st.done) break;
+	}
 	if (result) {
 		result->reached = h.st.reached;
 		result->reach_edges = h.st.reach_edges;

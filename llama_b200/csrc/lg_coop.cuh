@@ -22,6 +22,9 @@ constexpr uint64_t kCoopWaitNs = 1000000000ull;   // a barrier wait gives up aft
 // host launches it again: neither the host nor other streams wait longer.  In
 // cycles of the SM that looks (50 ms at 2 GHz), a register read.
 constexpr long long kCoopRunCycles = 100000000;
+// That the time is up is a bit of one of the step's counters, which every CTA
+// reads after the barrier anyway.
+constexpr unsigned long long kCoopTimeUp = 1ull << 63;
 
 __device__ __forceinline__ uint64_t global_ns() {
 	uint64_t t;

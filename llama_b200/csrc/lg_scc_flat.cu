@@ -111,7 +111,7 @@ struct alignas(16) SrState {
 };
 
 struct SrCtl {
-	u64 ctr[3][3];          // per step: [0] appends, [1] row pieces, [2] the launch's time is up
+	u64 ctr[3][2];          // per step: [0] appends, [1] row pieces (and kCoopTimeUp)
 	SrState st;             // where the last launch left off
 	CoopBar bar;            // err bit 2: a count out of range, bit 3: round cap
 };
@@ -129,7 +129,7 @@ struct SrArgs {
 struct SrShared {
 	uint32_t sbuf[kSrWarps][kPushBuf];
 	RowWindow win[kSrWarps];
-	u64 got[3];
+	u64 got[2];
 	SrState st;
 };
 
@@ -206,7 +206,7 @@ struct SrStep {
 				const uint32_t k = (__shfl_sync(0xffffffffu, len, t) - 1u) / kSrPiece + 1u;
 				u64 p = 0;
 				if (lane == 0) p = atomicAdd(cnt + 1, (u64)k);
-				p = __shfl_sync(0xffffffffu, p, 0);
+				p = __shfl_sync(0xffffffffu, p, 0) & ~kCoopTimeUp;
 				for (uint32_t i = lane; i < k; i += 32u)
 					if (p + i < a.max_pieces) a.pieces[p + i] = make_uint2(bv, bs + i * kSrPiece);
 			}
@@ -247,9 +247,9 @@ scc_rest(SrArgs a, SrCtl* c) {
 	// the next one fills, which was read before the last barrier but one
 	auto cnt = [&]() { return c->ctr[t.slot]; };
 	auto barrier = [&]() {
-		if (gtid == 0 && clock64() - t0 > kCoopRunCycles) cnt()[2] = 1;
+		if (gtid == 0 && clock64() - t0 > kCoopRunCycles) atomicOr(cnt() + 1, kCoopTimeUp);
 		if (!grid_barrier(&c->bar)) return false;
-		if (tid < 3) sh.got[tid] = __ldcg(cnt() + tid);
+		if (tid < 2) sh.got[tid] = __ldcg(cnt() + tid);
 		__syncthreads();
 		return true;
 	};
@@ -269,7 +269,7 @@ scc_rest(SrArgs a, SrCtl* c) {
 		t.steps++;
 		s.lists(a.list[t.lsel], (uint32_t)t.n, gwarp, nwarps);
 		if (!barrier()) return false;
-		const u64 np = sh.got[1];
+		const u64 np = sh.got[1] & ~kCoopTimeUp;
 		if (np > a.max_pieces) {
 			fail(4u);
 			return false;
@@ -286,7 +286,7 @@ scc_rest(SrArgs a, SrCtl* c) {
 	};
 
 	for (bool up = false; t.n_rem > 0 && !up;) {
-		if (gtid < 3) c->ctr[t.slot == 2u ? 0u : t.slot + 1u][gtid] = 0;
+		if (gtid < 2) c->ctr[t.slot == 2u ? 0u : t.slot + 1u][gtid] = 0;
 		if (t.phase == kSrColour) {
 			// colours: the vertices' own; the first list is all of them
 			t.round++;
@@ -334,7 +334,7 @@ scc_rest(SrArgs a, SrCtl* c) {
 			t.rsel ^= 1u;
 			t.phase = kSrColour;
 		}
-		up = sh.got[2] != 0;
+		up = sh.got[1] >= kCoopTimeUp;
 		t.slot = t.slot == 2u ? 0u : t.slot + 1u;
 	}
 	if (gtid == 0) c->st = t;
