@@ -1,5 +1,6 @@
 // lg_sssp_flat.cu - delta-stepping SSSP over the flat out-CSR, every step in
-// one cooperative launch.
+// one cooperative launch (of very many steps in several: one returns after
+// kCoopRunCycles, with the traversal's state in the control block).
 //
 // Buckets and bounds are those of lg_sssp.cu's host loop: the near queue holds
 // vertices whose distance fell below the bucket's bound, the far pile every
@@ -73,14 +74,17 @@ struct SfState {
 	uint32_t light;                // rounds relax light edges only
 	uint32_t jump;                 // the next split goes to mind's bucket
 	uint32_t grid;                 // the next step is for the whole grid
+	uint32_t up;                   // the launch's time is up
 };
 
 struct SfCtl {
 	unsigned long long ctr[3][4];   // per step: [0] near appends, [1] far appends,
 	                                // [2] split: max of ~kept distance, [3] row pieces
-	SfState st;                     // handed over by the CTA that worked alone
-	unsigned long long out[6];      // rounds, buckets, relaxations, reached, out-edges of
-	                                // the reached, largest distance
+	                                // (and kCoopTimeUp)
+	SfState st;                     // handed over by the CTA that worked alone, and to
+	                                // the next launch
+	alignas(16) unsigned long long out[8];   // rounds, buckets, relaxations, reached,
+	                                // out-edges of the reached, largest distance, done
 	CoopBar bar;                    // err bit 2: a count out of range, bit 3: step cap
 };
 
@@ -105,6 +109,7 @@ struct SfShared {                   // dynamic shared memory
 	RowWindow win[kSfWarps];
 	unsigned long long ctr[3][4];   // the lone CTA's counters
 	unsigned long long got[4];      // the last step's counters
+	long long t0;                   // the launch's start (CTA 0)
 	SfState st;
 };
 
@@ -237,7 +242,7 @@ __device__ __noinline__ unsigned long long sf_rows(const SfArgs& a, const SfStep
 			}
 			unsigned long long p = 0;
 			if (lane == 31u) p = atomicAdd(s.cnt + 3, (unsigned long long)inc);
-			p = __shfl_sync(0xffffffffu, p, 31) + inc - k;
+			p = (__shfl_sync(0xffffffffu, p, 31) & ~kCoopTimeUp) + inc - k;
 			if (k <= 32u)
 				for (uint32_t i = 0; i < k; i++)
 					if (p + i < a.max_pieces) a.pieces[p + i] = make_uint2(v, start + i * a.piece);
@@ -326,6 +331,8 @@ __device__ __forceinline__ bool sf_step(const SfArgs& a, SfCtl* c, SfShared& sh,
 	if (tid < 4 && (kSolo || blockIdx.x == 0)) (kSolo ? sh.ctr[slot] : c->ctr[slot])[tid] = 0;
 	// after a barrier every thread finds the step's counters in sh.got
 	auto barrier = [&]() {
+		if (tid == 0 && blockIdx.x == 0 && clock64() - sh.t0 > kCoopRunCycles)
+			atomicOr(cnt + 3, kCoopTimeUp);
 		if (!kSolo && !grid_barrier(&c->bar)) return false;
 		if (kSolo) __syncthreads();
 		if (tid < 4) sh.got[tid] = kSolo ? *(volatile unsigned long long*)(cnt + tid) : __ldcg(cnt + tid);
@@ -351,7 +358,7 @@ __device__ __forceinline__ bool sf_step(const SfArgs& a, SfCtl* c, SfShared& sh,
 		relaxations += sf_rows(a, s, heavy ? nullptr : a.q[t.qsel],
 				heavy ? a.V : (uint32_t)t.qlen, t.lo, gwarp, nwarps);
 		if (!barrier()) return false;
-		const unsigned long long np = count(3);
+		const unsigned long long np = count(3) & ~kCoopTimeUp;
 		if (np > a.max_pieces) {
 			if (tid == 0) atomicOr(&c->bar.err, 4u);
 			return false;
@@ -395,43 +402,58 @@ __device__ __forceinline__ bool sf_step(const SfArgs& a, SfCtl* c, SfShared& sh,
 		t.in_bucket = 0;
 		t.jump = !t.jump && t.qlen == 0 && t.flen > 0;
 	}
+	t.up = count(3) >= kCoopTimeUp;
 	return true;
 }
 
-// One CTA of 1024 per SM: 64 registers.
+// The state in c->st, read by a CTA behind a barrier.
+__device__ __forceinline__ SfState sf_load_state(const SfCtl* c, SfShared& sh) {
+	if (threadIdx.x < sizeof(SfState) / 4)
+		reinterpret_cast<unsigned int*>(&sh.st)[threadIdx.x] =
+				__ldcg(reinterpret_cast<const unsigned int*>(&c->st) + threadIdx.x);
+	__syncthreads();
+	return sh.st;
+}
+
+// One CTA of 1024 per SM: 64 registers.  resume: goes on from c->st, where the
+// last launch's time was up.
 __global__ void __launch_bounds__(kSfThreads, 1)
-sssp_flat(SfArgs a, SfCtl* c) {
+sssp_flat(SfArgs a, SfCtl* c, int resume) {
 	extern __shared__ __align__(16) unsigned char sf_smem[];
 	SfShared& sh = *reinterpret_cast<SfShared*>(sf_smem);
 	const uint32_t tid = threadIdx.x, lane = tid & 31u;
 	const uint32_t gtid = blockIdx.x * kSfThreads + tid;
 	const uint32_t nthreads = gridDim.x * kSfThreads;
-	for (uint64_t v = gtid; v < a.V; v += nthreads) {
-		a.dist[v] = v == a.root ? 0u : kInf;
-		a.stamp[v] = 0xffffffffu;
+	SfState t = {};
+	if (resume) {
+		t = sf_load_state(c, sh);
+		t.up = 0;
+	} else {
+		for (uint64_t v = gtid; v < a.V; v += nthreads) {
+			a.dist[v] = v == a.root ? 0u : kInf;
+			a.stamp[v] = 0xffffffffu;
+		}
+		if (gtid == 0) a.q[0][0] = a.root;
+		t.qlen = 1;
+		t.hi = a.delta;
+		t.buckets = 1;
 	}
-	if (gtid == 0) a.q[0][0] = a.root;
+	// (also: every CTA has read c->st)
 	if (!grid_barrier(&c->bar)) return;
-	SfState t;
-	t.qlen = 1;
-	t.flen = 0;
-	t.lo = 0;
-	t.hi = a.delta;
-	t.step = t.round = t.in_bucket = t.mind = t.qsel = t.fsel = t.light = t.jump = t.grid = 0;
-	t.buckets = 1;
 	unsigned long long relaxations = 0;              // the thread's own
 	const uint64_t step_cap = 4ull * a.V + 64;
 	uint32_t solo_slot = 0;
 	if (tid < 4) sh.ctr[0][tid] = 0;
+	if (tid == 0) sh.t0 = clock64();
 	__syncthreads();
-	while (t.qlen > 0 || t.flen > 0 || t.light) {
+	while ((t.qlen > 0 || t.flen > 0 || t.light) && !t.up) {
 		if (t.round >= step_cap) {
 			if (tid == 0) atomicOr(&c->bar.err, 8u);
 			return;
 		}
 		if (!t.grid && !t.light && t.qlen <= kSoloQueue && t.flen <= kSoloFar) {
 			if (blockIdx.x == 0) {
-				for (uint32_t n = 0; n < kSoloSteps && (t.qlen > 0 || t.flen > 0)
+				for (uint32_t n = 0; n < kSoloSteps && !t.up && (t.qlen > 0 || t.flen > 0)
 						&& t.qlen <= kSoloQueue && t.flen <= kSoloFar; n++) {
 					if (t.qlen > 0) {
 						uint32_t len = 0;
@@ -449,19 +471,20 @@ sssp_flat(SfArgs a, SfCtl* c) {
 				if (tid == 0) c->st = t;
 			}
 			if (!grid_barrier(&c->bar)) return;
-			if (blockIdx.x != 0) {
-				if (tid < sizeof(SfState) / 4)
-					reinterpret_cast<unsigned int*>(&sh.st)[tid] =
-							__ldcg(reinterpret_cast<const unsigned int*>(&c->st) + tid);
-				__syncthreads();
-				t = sh.st;
-			}
+			if (blockIdx.x != 0) t = sf_load_state(c, sh);
 			if (!t.grid) t.grid = t.qlen > 0 || t.flen > 0;   // past a CTA's limits
 			// (nobody rewrites c->st before the grid step's barrier)
 			continue;
 		}
 		t.grid = 0;
 		if (!sf_step<false>(a, c, sh, t, t.step, relaxations)) return;
+	}
+	relaxations = block_sum<kSfWarps>(relaxations);
+	if (tid == 0 && relaxations) atomicAdd(c->out + 2, relaxations);
+	if (t.qlen > 0 || t.flen > 0 || t.light) {       // the time is up
+		// (c->st may still be read after a lone CTA's steps: the same values)
+		if (gtid == 0) c->st = t;
+		return;
 	}
 	// reached vertices, their out-edges, the largest distance
 	unsigned long long cnt = 0, edges = 0, mx = 0;
@@ -475,17 +498,16 @@ sssp_flat(SfArgs a, SfCtl* c) {
 	}
 	cnt = block_sum<kSfWarps>(cnt);
 	edges = block_sum<kSfWarps>(edges);
-	relaxations = block_sum<kSfWarps>(relaxations);
 #pragma unroll
 	for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
 	if (lane == 0 && mx) atomicMax(c->out + 5, mx);
 	if (tid == 0) {
-		if (relaxations) atomicAdd(c->out + 2, relaxations);
 		if (cnt) atomicAdd(c->out + 3, cnt);
 		if (edges) atomicAdd(c->out + 4, edges);
 		if (blockIdx.x == 0) {
 			c->out[0] = t.round;
 			c->out[1] = t.buckets;
+			c->out[6] = 1;
 		}
 	}
 }
@@ -548,17 +570,22 @@ lg_status sssp_flat_run(lg_snapshot* sn, const FlatCsr* f, uint32_t root, uint32
 	a.stamp = sc[5].as<uint32_t>();
 	a.pieces = sc[7].as<uint2>();
 	LG_CUDA(cudaMemsetAsync(ctl, 0, sizeof(SfCtl), st), "clear control block");
-	void* kargs[] = {&a, &ctl};
-	LG_CUDA(cudaLaunchCooperativeKernel((const void*)sssp_flat, dim3((unsigned)grid),
-			dim3(kSfThreads), kargs, sizeof(SfShared), st), "sssp_flat");
-	s->launches++;
-	unsigned long long h[8];
-	static_assert(offsetof(SfCtl, bar) == offsetof(SfCtl, out) + 48, "two words after the results");
-	LG_TRY(read_words(s, ctl->out, 8, h));
-	const unsigned int err = (unsigned int)h[7];      // the barrier's error word
-	if (err & 1u) return set_error(LG_ETIMEOUT, "sssp: a grid barrier wait ran out");
-	if (err & 4u) return set_error(LG_ECUDA, "sssp: a queue count out of range");
-	if (err & 8u) return set_error(LG_ECUDA, "sssp: step cap reached");
+	int resume = 0;
+	void* kargs[] = {&a, &ctl, &resume};
+	unsigned long long h[10];
+	static_assert(offsetof(SfCtl, bar) == offsetof(SfCtl, out) + 64 && 10 <= kReadWords,
+			"two words after the results");
+	for (;; resume = 1) {
+		LG_CUDA(cudaLaunchCooperativeKernel((const void*)sssp_flat, dim3((unsigned)grid),
+				dim3(kSfThreads), kargs, sizeof(SfShared), st), "sssp_flat");
+		s->launches++;
+		LG_TRY(read_words(s, ctl->out, 10, h));
+		const unsigned int err = (unsigned int)h[9];      // the barrier's error word
+		if (err & 1u) return set_error(LG_ETIMEOUT, "sssp: a grid barrier wait ran out");
+		if (err & 4u) return set_error(LG_ECUDA, "sssp: a queue count out of range");
+		if (err & 8u) return set_error(LG_ECUDA, "sssp: step cap reached");
+		if (h[6]) break;
+	}
 	if (result) {
 		result->rounds = (int32_t)h[0];
 		result->buckets = (int32_t)h[1];
