@@ -22,9 +22,10 @@
 //
 // Both solves run every iteration inside one cooperative launch
 // (lg_flat_run.cuh) with an affine op: y[v] = base[v] + d * sum over v's edges
-// k of w[k] * x[nbr(k)].  The residual sum |y - x| of an iteration is added up
-// on the device before the iteration's barrier, so every CTA stops at the first
-// one below tol, with no launch or wait per iteration.  Bound by the gathers of
+// k of w[k] * x[nbr(k)].  The CTAs publish their parts of the residual
+// sum |y - x| before the iteration's barrier and each adds them up in the same
+// order, so every CTA stops at the first one below tol, with no launch or wait
+// per iteration, and calls on the same input give the same bits.  Bound by the gathers of
 // x and the weights' 8 bytes an edge above some 10^6 edges (15 M edges: 89 us an
 // iteration against 158 us for a launch per iteration at 16.8 M), by the barrier
 // and the loads around it below (30 k edges: 7 us against 14).
@@ -87,7 +88,6 @@ struct AffRunArgs {
 	const double* base;
 	double* xa;                // the start; results of even iteration counts
 	double* xb;
-	double* totals;            // max_iter residuals, zero
 	double d, tol;
 	uint32_t V;
 	int max_iter;
@@ -126,7 +126,7 @@ aff_run(AffRunArgs g, RunCtl* c) {
 				}
 		}
 		if (!run_iteration(g.a, op, c, sh, t0, t1, seg, extra, it & 1, it == 0, cross,
-				g.totals + it, &resid))
+				&resid))
 			return;
 		if (resid < g.tol) {
 			it++;
@@ -246,7 +246,7 @@ struct lg_adjoint_maps {
 	DevBuf src;            // E u32: source of each out-adjacency position
 	uint64_t E = 0;
 	// solve buffers, reused by every call on the snapshot
-	DevBuf xa, xb, base, win, resid, run, stage_w, stage_v, stage_g;
+	DevBuf xa, xb, base, win, run, stage_w, stage_v, stage_g;
 };
 
 struct lg_adjoint {
@@ -338,9 +338,6 @@ lg_status fixed_point(lg_snapshot* sn, const FlatCsr& f, const double* w, const 
 	const uint64_t V = sn->V;
 	double* A = m->xa.as<double>();
 	double* B = m->xb.as<double>();
-	LG_TRY(m->resid.reserve((size_t)max_iter * sizeof(double)));
-	double* resid = m->resid.as<double>();
-	LG_CUDA(cudaMemsetAsync(resid, 0, (size_t)max_iter * sizeof(double), st), "memset");
 	const int resident = aff_run_resident(s->device);
 	if (resident <= 0) return set_error(LG_ENOTSUP, "the device has no cooperative launch");
 	LG_TRY(m->run.reserve(sizeof(RunCtl)));
@@ -354,7 +351,6 @@ lg_status fixed_point(lg_snapshot* sn, const FlatCsr& f, const double* w, const 
 	g.base = base;
 	g.xa = A;
 	g.xb = B;
-	g.totals = resid;
 	g.d = d;
 	g.tol = tol;
 	g.V = (uint32_t)V;

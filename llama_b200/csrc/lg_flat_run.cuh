@@ -44,6 +44,7 @@ constexpr int kRunMaxCtas = 256;       // more SMs than any device of this archi
 struct RunEnds {
 	double first[kRunMaxCtas];         // sum of the row begun before, up to its end here
 	double last[kRunMaxCtas];          // sum of the row open at the end, if it began here
+	double resid[kRunMaxCtas];         // residual of the rows that ended here
 	uint32_t row[kRunMaxCtas];         // that row, kNoId if no row begins here
 };
 
@@ -61,7 +62,6 @@ struct RunShared {
 	double cfirst[kRunMaxCtas], clast[kRunMaxCtas];
 	uint32_t crow[kRunMaxCtas];
 	double part[kRunWarps];
-	double total;
 };
 
 // Sum of x over the CTA, the same bits in every thread.
@@ -192,14 +192,13 @@ __device__ __forceinline__ double run_join(const double* first, const double* la
 
 // One iteration by the whole grid: sweep, join, barrier, and the rows that
 // cross CTAs, finished by every CTA alike.  *resid = the iteration's residual
-// (the same in every thread of the grid); `total` is where the CTAs add theirs
-// up (zero before the iteration); first_time: the launch's first iteration,
-// which fills `cross`, the constants of the row the thread finishes.  False
-// once a barrier wait gave up.
+// (the same in every thread of the grid: the CTAs' terms in CTA order);
+// first_time: the launch's first iteration, which fills `cross`, the constants
+// of the row the thread finishes.  False once a barrier wait gave up.
 template <class Op>
 __device__ __forceinline__ bool run_iteration(const FlatTiles& a, const Op& op, RunCtl* c,
 		RunShared& sh, uint32_t t0, uint32_t t1, uint32_t seg, double extra, int parity,
-		bool first_time, typename Op::Row& cross, double* total, double* resid) {
+		bool first_time, typename Op::Row& cross, double* resid) {
 	const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5;
 	double res = extra + run_tiles(a, op, sh, t0, t1, seg);
 	__syncthreads();
@@ -231,29 +230,29 @@ __device__ __forceinline__ bool run_iteration(const FlatTiles& a, const Op& op, 
 	}
 	if (Op::kResidual) {
 		res = run_block_sum(sh, res);
-		if (tid == 0 && res != 0.0) atomicAdd(total, res);
+		if (tid == 0) e.resid[blockIdx.x] = res;
 	}
 	// (no CTA writes the last vector before it has passed the barrier)
 	double was = first_time ? 0.0 : op.old(cross);
 	if (!grid_barrier(&c->bar)) return false;
-	static_assert(kRunMaxCtas <= kRunThreads - 32, "a thread per CTA, and one for the total");
+	static_assert(kRunMaxCtas <= kRunThreads, "a thread per CTA");
+	res = 0.0;
 	if (tid < gridDim.x) {
 		sh.cfirst[tid] = __ldcg(e.first + tid);
 		sh.clast[tid] = __ldcg(e.last + tid);
 		if (first_time) sh.crow[tid] = __ldcg(e.row + tid);
+		if (Op::kResidual) res = __ldcg(e.resid + tid);
 	}
-	if (Op::kResidual && tid == kRunThreads - 1) sh.total = __ldcg(total);
 	__syncthreads();
-	res = 0.0;
 	if (tid < gridDim.x && sh.crow[tid] != kNoId) {
 		if (first_time) {
 			cross = op.row(sh.crow[tid]);
 			was = op.old(cross);
 		}
 		bool closed;                             // (the last one ends with the edges)
-		res = op.finish(cross, run_join(sh.cfirst, sh.clast, sh.crow, tid, gridDim.x, &closed), was);
+		res += op.finish(cross, run_join(sh.cfirst, sh.clast, sh.crow, tid, gridDim.x, &closed), was);
 	}
-	if (Op::kResidual) *resid = sh.total + run_block_sum(sh, res);
+	if (Op::kResidual) *resid = run_block_sum(sh, res);
 	__syncthreads();
 	return true;
 }

@@ -177,7 +177,7 @@ pr_run(PrRunArgs g, RunCtl* c) {
 					const uint32_t dg = __ldg(g.outdeg + v);
 					g.c0[v] = dg ? g.base / (double)dg : 0.0;
 				}
-		if (!run_iteration(g.a, op, c, sh, t0, t1, seg, 0.0, it & 1, it == 0, cross, nullptr,
+		if (!run_iteration(g.a, op, c, sh, t0, t1, seg, 0.0, it & 1, it == 0, cross,
 				&resid))
 			return;
 	}

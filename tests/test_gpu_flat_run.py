@@ -79,3 +79,21 @@ def test_fixed_point_and_gradient(V, n, hub):
             x3, _, r3 = sn.pagerank_fwd(w, v, tol=1e-300, max_iter=3, keep_tape=False)
             # (without a path of three edges the residual is 0 before)
             assert r3.iterations == 3 if n > 1 else r3.iterations <= 3
+
+
+def test_fixed_point_repeats_bit_for_bit():
+    """The residual that ends the iterations is added up in one order too."""
+    V, n = 150000, 2500000
+    s, d = _edges(V, n, False, 5)
+    rng = np.random.default_rng(2)
+    deg = np.bincount(s, minlength=V)
+    w = rng.uniform(0.5, 1.0, len(s)) / np.maximum(deg[s], 1)
+    v = rng.random(V) / V
+    with Store() as st:
+        st.build_level(V, s, d)
+        with st.snapshot() as sn:
+            x, _, r = sn.pagerank_fwd(w, v, tol=1e-9, keep_tape=False)
+            for _ in range(15):
+                x2, _, r2 = sn.pagerank_fwd(w, v, tol=1e-9, keep_tape=False)
+                assert (r2.iterations, r2.residual) == (r.iterations, r.residual)
+                assert np.array_equal(x2, x)
