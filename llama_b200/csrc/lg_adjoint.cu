@@ -90,7 +90,7 @@ struct AffRunArgs {
 	double* xb;
 	double d, tol;
 	uint32_t V;
-	int max_iter;
+	int first, end;            // the launch's iterations: first .. end - 1
 };
 
 __global__ void __launch_bounds__(kRunThreads, 1)
@@ -110,8 +110,8 @@ aff_run(AffRunArgs g, RunCtl* c) {
 	op.E = g.a.E;
 	AffRunOp::Row cross = {};
 	double resid = 0.0;
-	int it = 0;
-	for (; it < g.max_iter; it++) {
+	int it = g.first;
+	for (; it < g.end; it++) {
 		op.x = (it & 1) ? g.xb : g.xa;
 		op.y = (it & 1) ? g.xa : g.xb;
 		double extra = 0.0;
@@ -125,7 +125,7 @@ aff_run(AffRunArgs g, RunCtl* c) {
 					op.y[v] = b;
 				}
 		}
-		if (!run_iteration(g.a, op, c, sh, t0, t1, seg, extra, it & 1, it == 0, cross,
+		if (!run_iteration(g.a, op, c, sh, t0, t1, seg, extra, it & 1, it == g.first, cross,
 				&resid))
 			return;
 		if (resid < g.tol) {
@@ -354,19 +354,26 @@ lg_status fixed_point(lg_snapshot* sn, const FlatCsr& f, const double* w, const 
 	g.d = d;
 	g.tol = tol;
 	g.V = (uint32_t)V;
-	g.max_iter = max_iter;
 	void* args[] = {&g, &ctl};
-	LG_CUDA(cudaLaunchCooperativeKernel((const void*)aff_run, dim3(run_ctas(f.ntiles, resident)),
-			dim3(kRunThreads), args, sizeof(RunShared), st), "aff_run");
-	s->launches++;
 	unsigned long long h[4];
 	static_assert(sizeof(CoopBar) == 16 && sizeof(RunCtl) - offsetof(RunCtl, bar) == 32,
 			"barrier, residual, iterations");
-	LG_TRY(read_words(s, (const unsigned long long*)&ctl->bar, 4, h));
-	if ((unsigned)h[1] & 1u)
-		return set_error(LG_ETIMEOUT, "pagerank: a grid barrier wait ran out");
-	memcpy(resid_out, &h[2], sizeof(double));
-	*iters = (int)(uint32_t)h[3];
+	// (a residual that stays above tol, NaN for instance, takes max_iter
+	// iterations, of which a launch takes as many as run_iterations says)
+	const int most = run_iterations(f.E, V);
+	for (g.first = 0;; g.first = g.end) {
+		g.end = most < max_iter - g.first ? g.first + most : max_iter;
+		LG_CUDA(cudaLaunchCooperativeKernel((const void*)aff_run,
+				dim3(run_ctas(f.ntiles, resident)), dim3(kRunThreads), args, sizeof(RunShared), st),
+				"aff_run");
+		s->launches++;
+		LG_TRY(read_words(s, (const unsigned long long*)&ctl->bar, 4, h));
+		if ((unsigned)h[1] & 1u)
+			return set_error(LG_ETIMEOUT, "pagerank: a grid barrier wait ran out");
+		memcpy(resid_out, &h[2], sizeof(double));
+		*iters = (int)(uint32_t)h[3];
+		if (*resid_out < tol || g.end == max_iter) break;
+	}
 	*out = (*iters & 1) ? B : A;
 	return LG_OK;
 }

@@ -264,6 +264,14 @@ inline unsigned run_ctas(uint32_t ntiles, int resident) {
 	return need < 1u ? 1u : need < most ? need : most;
 }
 
+// Iterations of one launch, so that it ends within some 50 ms: neither the host
+// nor other streams wait longer (7 us an iteration and 6 ps an edge, measured
+// at 30 k and 15 M edges; as much for a vertex).
+inline int run_iterations(uint64_t E, uint64_t V) {
+	const double n = 50000.0 / (7.0 + 6e-6 * ((double)E + (double)V));
+	return n < 1.0 ? 1 : (int)n;
+}
+
 // The calling warp's tiles (warps in CTA order).
 __device__ __forceinline__ void run_share(uint32_t ntiles, uint32_t* t0, uint32_t* t1) {
 	const uint64_t w = (uint64_t)blockIdx.x * kRunWarps + (threadIdx.x >> 5);

@@ -139,6 +139,7 @@ struct PrRunArgs {
 	double base, d, pr0;
 	uint32_t V;
 	int iterations;            // at least 1
+	int first, end;            // the launch's: first .. end - 1
 };
 
 __global__ void __launch_bounds__(kRunThreads, 1)
@@ -155,18 +156,20 @@ pr_run(PrRunArgs g, RunCtl* c) {
 	op.outdeg = g.outdeg;
 	op.base = g.base;
 	op.d = g.d;
-	for (uint64_t v = gtid; v < g.V; v += nthreads) {
-		const uint32_t dg = __ldg(g.outdeg + v);
-		g.c0[v] = dg ? g.pr0 / (double)dg : 0.0;
-		if (__ldg(g.off + v + 1) == __ldg(g.off + v)) {
-			g.c1[v] = dg ? g.base / (double)dg : 0.0;
-			g.pr_out[v] = g.base;
+	if (g.first == 0) {
+		for (uint64_t v = gtid; v < g.V; v += nthreads) {
+			const uint32_t dg = __ldg(g.outdeg + v);
+			g.c0[v] = dg ? g.pr0 / (double)dg : 0.0;
+			if (__ldg(g.off + v + 1) == __ldg(g.off + v)) {
+				g.c1[v] = dg ? g.base / (double)dg : 0.0;
+				g.pr_out[v] = g.base;
+			}
 		}
+		if (!grid_barrier(&c->bar)) return;
 	}
-	if (!grid_barrier(&c->bar)) return;
 	PrRunOp::Row cross = {};
 	double resid;
-	for (int it = 0; it < g.iterations; it++) {
+	for (int it = g.first; it < g.end; it++) {
 		op.contrib = (it & 1) ? g.c1 : g.c0;
 		op.contrib_next = (it & 1) ? g.c0 : g.c1;
 		op.pr_out = it == g.iterations - 1 ? g.pr_out : nullptr;
@@ -177,7 +180,7 @@ pr_run(PrRunArgs g, RunCtl* c) {
 					const uint32_t dg = __ldg(g.outdeg + v);
 					g.c0[v] = dg ? g.base / (double)dg : 0.0;
 				}
-		if (!run_iteration(g.a, op, c, sh, t0, t1, seg, 0.0, it & 1, it == 0, cross,
+		if (!run_iteration(g.a, op, c, sh, t0, t1, seg, 0.0, it & 1, it == g.first, cross,
 				&resid))
 			return;
 	}
@@ -436,10 +439,15 @@ lg_status pagerank_over(lg_snapshot* sn, FlatCsr* f, int iterations, double damp
 		g.V = (uint32_t)V;
 		g.iterations = iterations;
 		void* args[] = {&g, &ctl};
-		LG_CUDA(cudaLaunchCooperativeKernel((const void*)pr_run, dim3(run_ctas(ntiles, resident)),
-				dim3(kRunThreads), args, sizeof(RunShared), st), "pr_run");
-		s->launches++;
-		s->run_pending = true;
+		const int most = run_iterations(f->E, V);
+		for (g.first = 0; g.first < iterations; g.first = g.end) {
+			g.end = most < iterations - g.first ? g.first + most : iterations;
+			LG_CUDA(cudaLaunchCooperativeKernel((const void*)pr_run,
+					dim3(run_ctas(ntiles, resident)), dim3(kRunThreads), args, sizeof(RunShared),
+					st), "pr_run");
+			s->launches++;
+			s->run_pending = true;
+		}
 		if (dev_out) return LG_OK;               // lg_store_sync reports a barrier that gave up
 		LG_TRY(copy_out(s, ranks, pr_buf, V * sizeof(double)));
 		return finish_run(s);

@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from llama_b200 import Store
+from tests._util import max_rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -66,3 +67,63 @@ def test_sssp_long_runs_of_the_whole_grid():
             assert np.array_equal(got, want)
             assert r.reached == (n - 1) * k + 1
             assert st.launch_count - before >= 2
+
+
+def _graph(V, n):
+    rng = np.random.default_rng(V)
+    k = np.unique(np.concatenate([rng.integers(0, V * V, n), np.arange(V) * V]))  # a hub
+    return k // V, k % V
+
+
+@pytest.mark.parametrize("V,n", [(50, 200), (3000, 40000)])
+def test_pagerank_of_very_many_iterations(V, n):
+    """A launch takes some 7000 iterations; damping close to 1, so that every
+    one of them counts."""
+    s, d = _graph(V, n)
+    deg = np.bincount(s, minlength=V).astype(np.float64)
+    x = np.full(V, 1.0 / V)
+    damping = 0.9999
+    with Store() as st:
+        st.build_level(V, s, d)
+        with st.snapshot() as sn:
+            sn.flatten(1)
+            done = 0
+            for it in (7001, 14500):
+                for _ in range(it - done):
+                    y = np.divide(x, deg, out=np.zeros(V), where=deg > 0)
+                    x = (1 - damping) / V + damping * np.bincount(d, y[s], V)
+                done = it
+                before = st.launch_count
+                got = sn.pagerank_pull(it, damping)
+                # an iteration adds V terms at the most, its error shrinks by the
+                # damping at the least: V * 2^-53 / (1 - damping) on either side
+                assert max_rel_err(got, x) <= 2 * V * 2.0 ** -53 * 1e4
+                assert st.launch_count - before >= it // 7143
+
+
+def test_fixed_point_of_very_many_iterations():
+    V, n = 3000, 40000
+    s, d = _graph(V, n)
+    rng = np.random.default_rng(3)
+    deg = np.bincount(s, minlength=V)
+    w = rng.uniform(0.5, 1.0, len(s)) / np.maximum(deg[s], 1)
+    v = rng.random(V) / V
+    damping = 0.9999
+    with Store() as st:
+        st.build_level(V, s, d)
+        with st.snapshot() as sn:
+            sn.pagerank_fwd(w, v, damping, max_iter=1, keep_tape=False)
+            x, done = v.copy(), 0
+            for it in (7001, 14500):
+                for _ in range(it - done):
+                    x = (1 - damping) * v + damping * np.bincount(d, w * x[s], V)
+                done = it
+                got, _, r = sn.pagerank_fwd(w, v, damping, tol=1e-300, max_iter=it,
+                                            keep_tape=False)
+                # (the residual is 0 from where the rounding stands still)
+                assert r.iterations == it or r.residual == 0
+                assert max_rel_err(got, x) <= 2 * V * 2.0 ** -53 * 1e4
+            before = st.launch_count
+            nan, _, r = sn.pagerank_fwd(w * np.nan, v, damping, max_iter=20000, keep_tape=False)
+            assert r.iterations == 20000 and np.isnan(r.residual)
+            assert st.launch_count - before >= 5      # 3 with one launch of the iterations
