@@ -220,6 +220,7 @@ struct SnapDir {
 	uint64_t n_slots = 0;          // slots of levels 0..L
 	uint64_t n_frag_slots = 0;     // slots covered by fragments
 	uint64_t n_dels = 0;           // deletion marks visible at L
+	uint64_t n_bare = 0;           // vertices without a fragment but with a degree
 	bool present = false;
 	// exchange device buffers with o (a closed snapshot's, kept for reuse)
 	void swap_buffers(SnapDir& o) {
@@ -365,11 +366,11 @@ lg_status copy_out(lg_store* s, void* dst, const void* src, size_t bytes);
 
 // The store's kHostWords pinned words (allocated on first use), for
 // counters a host loop reads back every step.
-constexpr int kHostWords = 20;
-constexpr int kReadWords = kHostWords - 8;   // the most read_words copies
+constexpr int kHostWords = 22;
+constexpr int kReadWords = 12;               // the last of them: for read_words
 lg_status host_words(lg_store* s, unsigned long long** words);
 // Waits for the store's stream and reads n <= kReadWords device words into out
-// through the pinned words from 8 on (words 0..7 stay with the caller).
+// through the last kReadWords pinned words (the others stay with the caller).
 lg_status read_words(lg_store* s, const unsigned long long* dev, int n, unsigned long long* out);
 
 // A DevLevel for direction dir (0 out, 1 in) of a new level: the store's

@@ -104,7 +104,8 @@ flat_live(FragSpace fs, uint32_t* live) {
 // to w when non-null); base = tile_base[t], or the tile's first slot where
 // nothing is deleted (tile_base null).  off = the row starts the degrees
 // give: a vertex whose first slot goes elsewhere, and a last tile that does
-// not end at off[V], set bit 2 of *err.
+// not end at off[V], set bit 2 of *err.  (With no degrees at vertices without a
+// fragment, which the snapshot's open looked for, every row is then right.)
 // kPositions: instead of the edges, every virtual slot's edge position goes to
 // ids[slot], kNoId for a deleted slot.
 template <bool kWeights, bool kPositions, bool kDels>
@@ -489,8 +490,12 @@ lg_status flat_positions(lg_snapshot* sn, int dir, const FlatCsr& f, uint32_t* p
 lg_status build_flat(lg_snapshot* sn, int dir, FlatCsr& f, bool view, bool weights,
 		bool strict) {
 	const SnapDir& d = dir == 0 ? sn->out : sn->in;
-	bool mismatch = false;
-	LG_TRY(build_rows(sn, dir, f, view, weights, d.deg.as<uint32_t>(), d.n_edges, &mismatch));
+	// flat_write finds a row that does not start where the degrees say; the rows
+	// of vertices without a fragment it never meets (a surplus there can make up
+	// for a deficit of the vertex before)
+	bool mismatch = d.n_bare > 0;
+	if (!mismatch)
+		LG_TRY(build_rows(sn, dir, f, view, weights, d.deg.as<uint32_t>(), d.n_edges, &mismatch));
 	if (!mismatch) return LG_OK;
 	if (strict)
 		return set_error(LG_EINVAL, "a vertex's degree differs from its live edge count");

@@ -181,7 +181,7 @@ lg_status host_words(lg_store* s, unsigned long long** words) {
 lg_status read_words(lg_store* s, const unsigned long long* dev, int n, unsigned long long* out) {
 	unsigned long long* hw = nullptr;
 	LG_TRY(host_words(s, &hw));
-	hw += 8;
+	hw += kHostWords - kReadWords;
 	LG_CUDA(cudaMemcpyAsync(hw, dev, (size_t)n * sizeof(unsigned long long),
 			cudaMemcpyDeviceToHost, s->stream), "d2h");
 	LG_CUDA(cudaStreamSynchronize(s->stream), "d2h");
@@ -768,6 +768,7 @@ struct FragOut {
 	uint32_t* tile_frag;
 	uint32_t* range_lb;          // lb[r] = first vertex with slot_off >= r * kBlockSlots
 	uint32_t nb;                 // r = 0 .. nb
+	unsigned long long* bare;    // += vertices without a fragment but with a degree
 };
 template <bool kFill>
 __global__ void walk_fragments(VtTab tab, int L, int minL, uint64_t V, uint32_t* count,
@@ -802,6 +803,7 @@ __global__ void walk_fragments(VtTab tab, int L, int minL, uint64_t V, uint32_t*
 		slots_per_vertex[v] = slots;
 		return;
 	}
+	if (n == 0 && tab.vt[L][v].degree != 0) atomicAdd(fo.bare, 1ull);
 	const uint32_t last = (uint32_t)(((uint64_t)at + slots) / kBlockSlots);
 	if (v == 0) fo.range_lb[0] = 0;
 	for (uint32_t r = at / kBlockSlots + 1u; r <= last && r <= fo.nb; r++)
@@ -845,7 +847,7 @@ __global__ void sum_u32(const uint32_t* x, uint64_t n, unsigned long long* out) 
 }
 
 // Opening a direction takes three parts, with one wait for both directions
-// after each of the first two; `w` are four of the store's pinned words.
+// after each of the first two; `w` are five of the store's pinned words.
 
 static VtTab vt_tab(const lg_snapshot* sn, const DevCsr& csr) {
 	VtTab tab;
@@ -887,7 +889,7 @@ static lg_status open_count(lg_snapshot* sn, DevCsr& csr, SnapDir& d, unsigned l
 }
 
 // Fragments, deletion bitsets and degrees; w[2] = live edges, w[3] = deletion
-// marks visible.
+// marks visible, w[4] = vertices without a fragment but with a degree.
 static lg_status open_fill(lg_snapshot* sn, DevCsr& csr, SnapDir& d, unsigned long long* w) {
 	lg_store* s = sn->store;
 	const int L = sn->level, minL = sn->min_level;
@@ -905,10 +907,14 @@ static lg_status open_fill(lg_snapshot* sn, DevCsr& csr, SnapDir& d, unsigned lo
 	LG_TRY(d.frags.reserve(std::max<uint64_t>(F, 1) * sizeof(uint2)));
 	LG_TRY(d.frag_aux.reserve((2 * F + 1 + tiles) * sizeof(uint32_t)));
 	LG_TRY(d.range_lb.reserve((nb + 1) * sizeof(uint32_t)));
+	DevBuf& counters = d.tmp_sum;     // [0] live degree sum, [1] deletions visible at L,
+	                                  // [2] vertices without a fragment but with a degree
+	LG_TRY(counters.reserve(3 * sizeof(unsigned long long)));
+	LG_CUDA(cudaMemsetAsync(counters.p, 0, 3 * sizeof(unsigned long long), st), "memset");
 	walk_fragments<true><<<grid_for(V, B), B, 0, st>>>(vt_tab(sn, csr), L, minL, V, nullptr,
 			nullptr, nullptr, FragOut{d.frag_off.as<uint32_t>(), d.slot_off.as<uint32_t>(),
 				d.frags.as<uint2>(), d.frag_start(), d.frag_vert(), d.tile_frag(),
-				d.range_lb.as<uint32_t>(), (uint32_t)nb});
+				d.range_lb.as<uint32_t>(), (uint32_t)nb, counters.as<unsigned long long>() + 2});
 	LG_CUDA(cudaGetLastError(), "walk_fragments fill");
 	LG_CUDA(cudaMemcpyAsync(d.frag_start() + F, d.slot_off.as<uint32_t>() + V, sizeof(uint32_t),
 			cudaMemcpyDeviceToDevice, st), "slot total");
@@ -932,9 +938,6 @@ static lg_status open_fill(lg_snapshot* sn, DevCsr& csr, SnapDir& d, unsigned lo
 	LG_TRY(d.lt.reserve(sizeof(LevelTab)));
 	LG_CUDA(cudaMemcpyAsync(d.lt.p, &lt, sizeof(lt), cudaMemcpyHostToDevice, st),
 			"level table");
-	DevBuf& counters = d.tmp_sum;     // [0] live degree sum, [1] deletions visible at L
-	LG_TRY(counters.reserve(2 * sizeof(unsigned long long)));
-	LG_CUDA(cudaMemsetAsync(counters.p, 0, 2 * sizeof(unsigned long long), st), "memset");
 	if (csr.n_dels_dev > 0) {
 		int sms = 148;
 		cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
@@ -960,8 +963,8 @@ static lg_status open_fill(lg_snapshot* sn, DevCsr& csr, SnapDir& d, unsigned lo
 			counters.as<unsigned long long>());
 	LG_CUDA(cudaGetLastError(), "degree sum");
 	s->launches++;
-	LG_CUDA(cudaMemcpyAsync(w + 2, counters.p, 16, cudaMemcpyDeviceToHost, st), "d2h");
-	s->d2h_bytes += 16;
+	LG_CUDA(cudaMemcpyAsync(w + 2, counters.p, 24, cudaMemcpyDeviceToHost, st), "d2h");
+	s->d2h_bytes += 24;
 	return LG_OK;
 }
 
@@ -970,6 +973,7 @@ static void open_done(lg_snapshot* sn, DevCsr& csr, SnapDir& d, const unsigned l
 	d.n_slots = 0;
 	for (int l = sn->min_level; l <= sn->level; l++) d.n_slots += csr.levels[l]->n_slots;
 	d.n_dels = w[3];
+	d.n_bare = sn->min_level > 0 ? 0 : w[4];      // (a window's degrees were counted)
 	d.present = true;
 }
 
@@ -978,13 +982,13 @@ static lg_status open_dirs(lg_snapshot* sn) {
 	unsigned long long* w = nullptr;
 	LG_TRY(host_words(s, &w));
 	LG_TRY(open_count(sn, s->out, sn->out, w));
-	if (s->reverse) LG_TRY(open_count(sn, s->in, sn->in, w + 4));
+	if (s->reverse) LG_TRY(open_count(sn, s->in, sn->in, w + 5));
 	LG_CUDA(cudaStreamSynchronize(s->stream), "snapshot sizes");
 	LG_TRY(open_fill(sn, s->out, sn->out, w));
-	if (s->reverse) LG_TRY(open_fill(sn, s->in, sn->in, w + 4));
+	if (s->reverse) LG_TRY(open_fill(sn, s->in, sn->in, w + 5));
 	LG_CUDA(cudaStreamSynchronize(s->stream), "snapshot sizes");
 	open_done(sn, s->out, sn->out, w);
-	if (s->reverse) open_done(sn, s->in, sn->in, w + 4);
+	if (s->reverse) open_done(sn, s->in, sn->in, w + 5);
 	return LG_OK;
 }
 

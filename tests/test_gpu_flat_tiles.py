@@ -100,3 +100,51 @@ def test_wrong_degrees():
                         sn.pagerank_pull(2)
                 else:
                     want = got
+
+
+def _store(V, s, d, w, patch):
+    """A store of one level whose vertex tables (out, in) patch(vt, direction)
+    has changed."""
+    hg = HostGraph(V)
+    hg.add_level(s, d, weights=w)
+    desc = hg.level_desc(0)
+    for dr, c in enumerate((desc.out, desc.in_)):
+        patch(np.ctypeslib.as_array(C.cast(c.vt, C.POINTER(C.c_uint8)),
+                                    ((V + 1) * 16,)).view(VT_DTYPE), dr)
+    st = Store()
+    st.ingest(hg)
+    return st
+
+
+@pytest.mark.parametrize("wrong", ["pair", "pair at the end"])
+def test_degrees_that_make_up_for_each_other(wrong):
+    """A degree too small by what the next vertex, which has no edges, has too
+    much: every other row starts where it should."""
+    V, rng = 300, np.random.default_rng(4)
+    key = rng.choice(V * V, size=4000, replace=False)
+    bare = V - 1 if wrong.endswith("end") else 12           # no edges in or out
+    key = key[(key // V != bare) & (key % V != bare) & (key // V != key % V)]
+    s, d = (key // V).astype(np.uint32), (key % V).astype(np.uint32)
+    w = rng.integers(1, 99, len(s)).astype(np.uint32)
+    seeds = np.arange(32)
+
+    def patch(vt, dr):
+        assert vt["degree"][bare] == 0 and vt["degree"][bare - 1] > 3
+        vt["degree"][bare - 1] -= 2
+        vt["degree"][bare] += 2
+    with _store(V, s, d, w, lambda vt, dr: None) as st, st.snapshot() as sn:
+        want = (sn.triangle_count().triangles, sn.scc()[0], sn.sssp(3, 32)[0])
+        right = ppr([sn], seeds, iterations=1)
+    with _store(V, s, d, w, patch) as st, st.snapshot() as sn:
+        got = (sn.triangle_count().triangles, sn.scc()[0], sn.sssp(3, 32)[0])
+        x = ppr([sn], seeds, iterations=1)
+        out = np.setdiff1d(np.arange(V), d[s == bare - 1])  # the others divide by that degree
+        assert np.array_equal(x[:, out], right[:, out])
+        for a, b in zip(got, want):
+            assert np.array_equal(a, b)
+        with pytest.raises(LgError):
+            sn.flatten(1)
+        with pytest.raises(LgError):
+            sn.pagerank_pull(2)
+        with pytest.raises(LgError):
+            sn.flatten(0)
