@@ -492,8 +492,8 @@ lg_status build_flat(lg_snapshot* sn, int dir, FlatCsr& f, bool view, bool weigh
 	const SnapDir& d = dir == 0 ? sn->out : sn->in;
 	// flat_write finds a row that does not start where the degrees say; the rows
 	// of vertices without a fragment it never meets (a surplus there can make up
-	// for a deficit of the vertex before)
-	bool mismatch = d.n_bare > 0;
+	// for a deficit of the vertex before), and more edges than slots need no look
+	bool mismatch = d.n_bare > 0 || (!strict && d.n_edges > d.n_frag_slots);
 	if (!mismatch)
 		LG_TRY(build_rows(sn, dir, f, view, weights, d.deg.as<uint32_t>(), d.n_edges, &mismatch));
 	if (!mismatch) return LG_OK;

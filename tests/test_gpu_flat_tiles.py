@@ -116,10 +116,11 @@ def _store(V, s, d, w, patch):
     return st
 
 
-@pytest.mark.parametrize("wrong", ["pair", "pair at the end"])
+@pytest.mark.parametrize("wrong", ["pair", "pair at the end", "huge"])
 def test_degrees_that_make_up_for_each_other(wrong):
     """A degree too small by what the next vertex, which has no edges, has too
-    much: every other row starts where it should."""
+    much: every other row starts where it should.  And degrees far above the
+    number of slots."""
     V, rng = 300, np.random.default_rng(4)
     key = rng.choice(V * V, size=4000, replace=False)
     bare = V - 1 if wrong.endswith("end") else 12           # no edges in or out
@@ -129,22 +130,29 @@ def test_degrees_that_make_up_for_each_other(wrong):
     seeds = np.arange(32)
 
     def patch(vt, dr):
-        assert vt["degree"][bare] == 0 and vt["degree"][bare - 1] > 3
-        vt["degree"][bare - 1] -= 2
-        vt["degree"][bare] += 2
+        if wrong == "huge":
+            if dr == 1:
+                vt["degree"][[5, 6, 7]] = 1 << 31
+        else:
+            assert vt["degree"][bare] == 0 and vt["degree"][bare - 1] > 3
+            vt["degree"][bare - 1] -= 2
+            vt["degree"][bare] += 2
     with _store(V, s, d, w, lambda vt, dr: None) as st, st.snapshot() as sn:
         want = (sn.triangle_count().triangles, sn.scc()[0], sn.sssp(3, 32)[0])
         right = ppr([sn], seeds, iterations=1)
     with _store(V, s, d, w, patch) as st, st.snapshot() as sn:
         got = (sn.triangle_count().triangles, sn.scc()[0], sn.sssp(3, 32)[0])
         x = ppr([sn], seeds, iterations=1)
-        out = np.setdiff1d(np.arange(V), d[s == bare - 1])  # the others divide by that degree
-        assert np.array_equal(x[:, out], right[:, out])
+        if wrong != "huge":                                 # (divided by the wrong degree)
+            out = np.setdiff1d(np.arange(V), d[s == bare - 1])
+            x, right = x[:, out], right[:, out]
+        assert np.array_equal(x, right)
         for a, b in zip(got, want):
             assert np.array_equal(a, b)
         with pytest.raises(LgError):
             sn.flatten(1)
         with pytest.raises(LgError):
             sn.pagerank_pull(2)
-        with pytest.raises(LgError):
-            sn.flatten(0)
+        if wrong != "huge":
+            with pytest.raises(LgError):
+                sn.flatten(0)
