@@ -324,7 +324,7 @@ int aff_run_resident(int device) {
 			cudaGetLastError();
 		g_run[device] = n + 1;
 	}
-	return g_run[device] - 1;
+	return coop_allowed(g_run[device] - 1);
 }
 
 // Iterate y = base + d * (weighted pull of x) over the flat CSR f until
@@ -361,11 +361,11 @@ lg_status fixed_point(lg_snapshot* sn, const FlatCsr& f, const double* w, const 
 	// (a residual that stays above tol, NaN for instance, takes max_iter
 	// iterations, of which a launch takes as many as run_iterations says)
 	const int most = run_iterations(f.E, V);
+	unsigned grid = run_ctas(f.ntiles, resident);
 	for (g.first = 0;; g.first = g.end) {
 		g.end = most < max_iter - g.first ? g.first + most : max_iter;
-		LG_CUDA(cudaLaunchCooperativeKernel((const void*)aff_run,
-				dim3(run_ctas(f.ntiles, resident)), dim3(kRunThreads), args, sizeof(RunShared), st),
-				"aff_run");
+		LG_CUDA(coop_launch((const void*)aff_run, &grid, kRunThreads, args, sizeof(RunShared), st,
+				&ctl->bar), "aff_run");
 		s->launches++;
 		LG_TRY(read_words(s, (const unsigned long long*)&ctl->bar, 4, h));
 		if ((unsigned)h[1] & 1u)

@@ -473,7 +473,7 @@ int coop_grid(int device) {
 	if (device < 0 || device >= LG_TUNE_MAX_DEVICES) return 0;
 	if (!g_coop[device])
 		g_coop[device] = 1 + coop_grid_size((const void*)bfs_levels, kLvThreads, device);
-	return g_coop[device] - 1;
+	return coop_allowed(g_coop[device] - 1);
 }
 
 } // namespace
@@ -496,6 +496,7 @@ lg_status bfs_levels_over(lg_store* s, SnapCsr out, const FlatCsr* fi, const uin
 	*ran = false;
 	const int grid = coop_grid(s->device);
 	if (grid <= 0) return LG_OK;
+	unsigned ctas = (unsigned)grid;
 	cudaStream_t st = s->stream;
 	const uint64_t V = out.V;
 	const uint64_t W = (V + 31) / 32;
@@ -532,8 +533,8 @@ lg_status bfs_levels_over(lg_store* s, SnapCsr out, const FlatCsr* fi, const uin
 	s->launches++;
 	LvCtl h;
 	for (;; resume = 1) {
-		LG_CUDA(cudaLaunchCooperativeKernel((const void*)bfs_levels, dim3((unsigned)grid),
-				dim3(kLvThreads), args, 0, st), "bfs_levels");
+		LG_CUDA(coop_launch((const void*)bfs_levels, &ctas, kLvThreads, args, 0, st, &ctl->bar),
+				"bfs_levels");
 		s->launches++;
 		LG_CUDA(cudaMemcpyAsync(&h, ctl, sizeof(h), cudaMemcpyDeviceToHost, st), "d2h");
 		LG_CUDA(cudaStreamSynchronize(st), "bfs_levels");

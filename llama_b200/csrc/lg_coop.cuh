@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "lg_internal.h"
+
 namespace lg {
 
 // Barrier state in device memory; count must be 0 before the launch.
@@ -129,6 +131,26 @@ inline int coop_grid_size(const void* kernel, int threads, int device, size_t sm
 	}
 	return coop && sms > 0 && per_sm > 0 ? sms * per_sm : 0;
 }
+
+// Launches `kernel` on *grid CTAs (a grid of any size gives its result), or,
+// where the caller's share of the GPU holds fewer at once than the device's
+// properties say, on half, a quarter ... as many, which *grid becomes.  bar:
+// the kernel's barrier, whose count is a multiple of the grid's size.
+inline cudaError_t coop_launch(const void* kernel, unsigned* grid, int threads, void** args,
+		size_t smem, cudaStream_t st, CoopBar* bar) {
+	for (;; *grid /= 2u) {
+		const cudaError_t e = *grid > test_limits().ctas ? cudaErrorCooperativeLaunchTooLarge
+				: cudaLaunchCooperativeKernel(kernel, dim3(*grid), dim3((unsigned)threads), args,
+						smem, st);
+		if (e != cudaErrorCooperativeLaunchTooLarge || *grid <= 1u) return e;
+		(void)cudaGetLastError();
+		const cudaError_t me = cudaMemsetAsync(&bar->count, 0, sizeof(bar->count), st);
+		if (me != cudaSuccess) return me;
+	}
+}
+
+// The CTAs that coop_grid_size found, 0 where a test wants no cooperative launch.
+inline int coop_allowed(int grid) { return test_limits().ctas > 0 ? grid : 0; }
 
 } // namespace lg
 

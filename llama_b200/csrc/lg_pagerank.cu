@@ -375,7 +375,7 @@ static int pr_run_resident(int device) {
 			cudaGetLastError();
 		g_run[device] = n + 1;
 	}
-	return g_run[device] - 1;
+	return coop_allowed(g_run[device] - 1);
 }
 
 lg_status finish_run(lg_store* s) {
@@ -440,11 +440,11 @@ lg_status pagerank_over(lg_snapshot* sn, FlatCsr* f, int iterations, double damp
 		g.iterations = iterations;
 		void* args[] = {&g, &ctl};
 		const int most = run_iterations(f->E, V);
+		unsigned grid = run_ctas(ntiles, resident);
 		for (g.first = 0; g.first < iterations; g.first = g.end) {
 			g.end = most < iterations - g.first ? g.first + most : iterations;
-			LG_CUDA(cudaLaunchCooperativeKernel((const void*)pr_run,
-					dim3(run_ctas(ntiles, resident)), dim3(kRunThreads), args, sizeof(RunShared),
-					st), "pr_run");
+			LG_CUDA(coop_launch((const void*)pr_run, &grid, kRunThreads, args, sizeof(RunShared),
+					st, &ctl->bar), "pr_run");
 			s->launches++;
 			s->run_pending = true;
 		}

@@ -348,7 +348,7 @@ int coop_grid(int device) {
 	if (device < 0 || device >= LG_TUNE_MAX_DEVICES) return 0;
 	if (!g_coop[device])
 		g_coop[device] = 1 + coop_grid_size((const void*)scc_rest, kSrThreads, device);
-	return g_coop[device] - 1;
+	return coop_allowed(g_coop[device] - 1);
 }
 
 } // namespace
@@ -359,6 +359,7 @@ lg_status scc_flat_run(lg_snapshot* sn, const FlatCsr* fo, const FlatCsr* fi, ui
 	lg_store* s = sn->store;
 	const int grid = coop_grid(s->device);
 	if (grid <= 0) return LG_OK;
+	unsigned ctas = (unsigned)grid;
 	cudaStream_t st = s->stream;
 	const uint64_t V = sn->V;
 	const unsigned B = kListThreads;
@@ -430,8 +431,8 @@ lg_status scc_flat_run(lg_snapshot* sn, const FlatCsr* fo, const FlatCsr* fi, ui
 	a.pieces = pieces.as<uint2>();
 	void* kargs[] = {&a, &ctl};
 	for (;;) {
-		LG_CUDA(cudaLaunchCooperativeKernel((const void*)scc_rest, dim3((unsigned)grid),
-				dim3(kSrThreads), kargs, 0, st), "scc_rest");
+		LG_CUDA(coop_launch((const void*)scc_rest, &ctas, kSrThreads, kargs, 0, st, &ctl->bar),
+				"scc_rest");
 		s->launches++;
 		constexpr int kWords = (int)(sizeof(SrState) / sizeof(u64)) + 2;
 		static_assert(offsetof(SrCtl, bar) == offsetof(SrCtl, st) + sizeof(SrState) &&

@@ -526,7 +526,7 @@ int coop_grid(int device) {
 	if (!g_coop[device])
 		g_coop[device] = 1 + coop_grid_size((const void*)sssp_flat, kSfThreads, device,
 				sizeof(SfShared));
-	return g_coop[device] - 1;
+	return coop_allowed(g_coop[device] - 1);
 }
 
 } // namespace
@@ -537,6 +537,7 @@ lg_status sssp_flat_run(lg_snapshot* sn, const FlatCsr* f, uint32_t root, uint32
 	lg_store* s = sn->store;
 	const int grid = coop_grid(s->device);
 	if (grid <= 0) return LG_OK;
+	unsigned ctas = (unsigned)grid;
 	cudaStream_t st = s->stream;
 	const uint64_t V = sn->V;
 	DevBuf* sc = s->scratch;
@@ -576,8 +577,8 @@ lg_status sssp_flat_run(lg_snapshot* sn, const FlatCsr* f, uint32_t root, uint32
 	static_assert(offsetof(SfCtl, bar) == offsetof(SfCtl, out) + 64 && 10 <= kReadWords,
 			"two words after the results");
 	for (;; resume = 1) {
-		LG_CUDA(cudaLaunchCooperativeKernel((const void*)sssp_flat, dim3((unsigned)grid),
-				dim3(kSfThreads), kargs, sizeof(SfShared), st), "sssp_flat");
+		LG_CUDA(coop_launch((const void*)sssp_flat, &ctas, kSfThreads, kargs, sizeof(SfShared), st, &ctl->bar),
+				"sssp_flat");
 		s->launches++;
 		LG_TRY(read_words(s, ctl->out, 10, h));
 		const unsigned int err = (unsigned int)h[9];      // the barrier's error word

@@ -275,7 +275,7 @@ int coop_grid(int device) {
 	if (device < 0 || device >= LG_TUNE_MAX_DEVICES) return 0;
 	if (!g_coop[device])
 		g_coop[device] = 1 + coop_grid_size((const void*)sssp_levels, kSlThreads, device);
-	return g_coop[device] - 1;
+	return coop_allowed(g_coop[device] - 1);
 }
 
 } // namespace
@@ -285,6 +285,7 @@ lg_status sssp_levels_run(lg_store* s, const SsspLevelsArgs& args, DevBuf& ctl_b
 	*ran = false;
 	const int grid = coop_grid(s->device);
 	if (grid <= 0) return LG_OK;
+	unsigned ctas = (unsigned)grid;
 	cudaStream_t st = s->stream;
 	LG_TRY(ctl_buf.reserve(sizeof(SlCtl) + (size_t)grid * sizeof(unsigned long long)));
 	SlCtl* ctl = ctl_buf.as<SlCtl>();
@@ -293,8 +294,8 @@ lg_status sssp_levels_run(lg_store* s, const SsspLevelsArgs& args, DevBuf& ctl_b
 	sssp_levels_init<<<1, 32, 0, st>>>(ctl);
 	LG_CUDA(cudaGetLastError(), "sssp_levels_init");
 	void* kargs[] = {&a, &ctl};
-	LG_CUDA(cudaLaunchCooperativeKernel((const void*)sssp_levels, dim3((unsigned)grid),
-			dim3(kSlThreads), kargs, 0, st), "sssp_levels");
+	LG_CUDA(coop_launch((const void*)sssp_levels, &ctas, kSlThreads, kargs, 0, st, &ctl->bar),
+			"sssp_levels");
 	s->launches += 2;
 	SlCtl h;
 	LG_CUDA(cudaMemcpyAsync(&h, ctl, sizeof(h), cudaMemcpyDeviceToHost, st), "d2h");

@@ -31,6 +31,17 @@ lg_status set_error(lg_status st, const char* fmt, ...) {
 
 void clear_error() { t_err[0] = 0; }
 
+TestLimits& test_limits() {
+	static thread_local TestLimits t;
+	return t;
+}
+
+// Negative: no limit.
+extern "C" void lg_test_limits(int64_t alloc, int64_t ctas) {
+	test_limits().alloc = alloc < 0 ? ~0ull : (uint64_t)alloc;
+	test_limits().ctas = ctas < 0 ? INT64_MAX : ctas;
+}
+
 lg_status cuda_status(cudaError_t e, const char* what) {
 	if (e == cudaErrorMemoryAllocation)
 		return set_error(LG_ENOMEM, "%s: %s", what, cudaGetErrorString(e));
@@ -105,6 +116,7 @@ lg_status DevBuf::reserve(size_t n) {
 	if (n <= bytes && p) return LG_OK;
 	release();
 	if (n == 0) n = 16;
+	if (n > test_limits().alloc) return cuda_status(cudaErrorMemoryAllocation, "test limit");
 	cudaError_t e = cudaSuccess;
 	const bool in_pool = from && from->used + n <= kPoolKeep;
 	for (int attempt = 0; attempt < 2; attempt++) {
