@@ -1,10 +1,12 @@
 """Cooperative launches where fewer CTAs fit than the device's properties say (a
-share of the GPU): they take a smaller grid, down to one CTA."""
+share of the GPU): they take a smaller grid, down to one CTA; without any, the
+forms with a launch per step."""
 import numpy as np
 import pytest
 
 from llama_b200 import Store, _lib
 from llama_b200.graph import tune_reset, tune_set
+from tests._util import max_rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -50,3 +52,23 @@ def test_smaller_grids(limit):
                         assert np.abs(a - b).sum() <= 2e-12
                     else:
                         assert np.array_equal(a, b)
+
+
+def test_without_cooperative_launches(limit):
+    V = 9000
+    rng = np.random.default_rng(9)
+    k = np.unique(np.concatenate([rng.integers(0, V * V, 60000), np.arange(V) * V]))
+    s, d = k // V, k % V
+    with Store() as st:
+        st.build_level(V, s, d, rng.integers(1, 50, len(s)))
+        with st.snapshot() as sn:
+            for flat in (False, True):
+                if flat:
+                    sn.flatten(0).flatten(1)
+                limit(-1)
+                want = sn.bfs(1)[0], sn.scc()[0], sn.sssp(1, 16)[0], sn.pagerank_pull(9)
+                limit(0)
+                got = sn.bfs(1)[0], sn.scc()[0], sn.sssp(1, 16)[0], sn.pagerank_pull(9)
+                for a, b in zip(got[:3], want[:3]):
+                    assert np.array_equal(a, b)
+                assert max_rel_err(got[3], want[3]) <= 1e-12
