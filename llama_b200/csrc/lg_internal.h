@@ -17,10 +17,11 @@ void clear_error();
 
 // Limits that a test sets for the calls of its own thread (lg_test_limits, which
 // the public headers leave out), to reach what the library does where the GPU
-// has less to give: the largest device allocation that succeeds, and the CTAs
-// of a cooperative launch that fit on it at once (0: no cooperative launch).
+// has less to give: the device allocations that succeed before one fails
+// (negative: none does), and the CTAs of a cooperative launch that fit on it at
+// once (0: no cooperative launch).
 struct TestLimits {
-	uint64_t alloc = ~0ull;
+	int64_t allocs = -1;
 	int64_t ctas = INT64_MAX;
 };
 TestLimits& test_limits();

@@ -97,13 +97,10 @@ lg_status push_transposed(lg_snapshot* sn, int iterations, double damping, doubl
 		out = &made;
 	}
 	if (st == LG_OK) st = flat_transpose(s, *out, in);
-	if (st == LG_ENOMEM || st == LG_ENOTSUP) {
-		clear_error();
-		return LG_OK;
-	}
-	if (st != LG_OK) return st;
-	LG_TRY(pagerank_over(sn, &in, iterations, damping, ranks));
-	*ran = true;
+	if (st == LG_OK) st = pagerank_over(sn, &in, iterations, damping, ranks);
+	*ran = st == LG_OK;
+	if (st != LG_ENOMEM && st != LG_ENOTSUP) return st;
+	clear_error();
 	return LG_OK;
 }
 

@@ -36,10 +36,13 @@ TestLimits& test_limits() {
 	return t;
 }
 
-// Negative: no limit.
-extern "C" void lg_test_limits(int64_t alloc, int64_t ctas) {
-	test_limits().alloc = alloc < 0 ? ~0ull : (uint64_t)alloc;
+// Negative: no limit.  Returns the allocations left to succeed (negative if one
+// failed or there was no limit).
+extern "C" int64_t lg_test_limits(int64_t allocs, int64_t ctas) {
+	const int64_t left = test_limits().allocs;
+	test_limits().allocs = allocs;
 	test_limits().ctas = ctas < 0 ? INT64_MAX : ctas;
+	return left;
 }
 
 lg_status cuda_status(cudaError_t e, const char* what) {
@@ -116,7 +119,8 @@ lg_status DevBuf::reserve(size_t n) {
 	if (n <= bytes && p) return LG_OK;
 	release();
 	if (n == 0) n = 16;
-	if (n > test_limits().alloc) return cuda_status(cudaErrorMemoryAllocation, "test limit");
+	if (test_limits().allocs >= 0 && test_limits().allocs-- == 0)
+		return cuda_status(cudaErrorMemoryAllocation, "test limit");
 	cudaError_t e = cudaSuccess;
 	const bool in_pool = from && from->used + n <= kPoolKeep;
 	for (int attempt = 0; attempt < 2; attempt++) {

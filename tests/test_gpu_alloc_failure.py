@@ -1,0 +1,64 @@
+"""Device allocations that fail, one after the other: a call returns LG_ENOMEM or,
+where it has a form that needs less, the right result; and runs again after."""
+import numpy as np
+import pytest
+
+from llama_b200 import LgError, Store, _lib
+from tests._util import max_rel_err
+
+pytestmark = pytest.mark.gpu
+
+C = _lib.C
+
+
+@pytest.fixture
+def fail_at():
+    f = _lib.lib.lg_test_limits
+    f.argtypes, f.restype = [C.c_int64, C.c_int64], C.c_int64
+    yield lambda k: f(k, -1)
+    f(-1, -1)
+
+
+def _graph(V, n, seed):
+    rng = np.random.default_rng(seed)
+    k = np.unique(rng.integers(0, V * V, n))
+    return k // V, k % V
+
+
+def _each_failure(fail_at, build, call):
+    """call(snapshot) on a new store with its first, second ... allocation
+    failing, until none does; yields (result or None for LG_ENOMEM)."""
+    for k in range(100):
+        with build() as st, st.snapshot() as sn:
+            fail_at(k)
+            try:
+                got = call(sn)
+            except LgError as e:
+                assert e.status == _lib.LG_ENOMEM, e
+                got = None
+            left = fail_at(-1)
+            again = call(sn)
+            if got is None:
+                got = (None, again)
+            else:
+                got = (got, again)
+            yield got
+            if left >= 0:
+                return
+    raise AssertionError("allocations without end")
+
+
+def test_push_runs_without_the_transpose(fail_at):
+    V = 20000
+    s, d = _graph(V, 800_000, 1)
+
+    def build():
+        st = Store(reverse_edges=False)
+        st.build_level(V, s, d)
+        return st
+    results = list(_each_failure(fail_at, build, lambda sn: sn.pagerank_push(10)))
+    assert len(results) > 15
+    want = results[-1][0]
+    for got, again in results:
+        assert got is not None and max_rel_err(got, want) <= 1e-12
+        assert max_rel_err(again, want) <= 1e-12

@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 @pytest.fixture
 def limit():
     f = _lib.lib.lg_test_limits
-    f.argtypes, f.restype = [_lib.C.c_int64, _lib.C.c_int64], None
+    f.argtypes, f.restype = [_lib.C.c_int64, _lib.C.c_int64], _lib.C.c_int64
     yield lambda ctas: f(-1, ctas)
     f(-1, -1)
     tune_reset(0)
