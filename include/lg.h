@@ -504,7 +504,9 @@ lg_status lg_bc_batched(lg_snapshot* snap, const int64_t* sources, int n_sources
  * 120-169) with the uniform teleport (1-d)/N replaced, per column k, by (1-d)
  * on seed k; x0 = e_seed, fixed iteration count, dangling mass dropped.  Reads
  * the snapshots' flat in-CSRs; one that is not flat is flattened for the call
- * in scratch of the store (4 bytes per live edge and 24 per vertex).  K is a multiple of 32, <= 256.
+ * in scratch of the store (4 bytes per live edge and 24 per vertex), or, without
+ * that memory, read from the levels at a fifth of the speed.  K is a multiple of
+ * 32, <= 256.
  * out: double[n_snaps][max_nodes][K] (row-major, column k = seed k). */
 lg_status lg_ppr(lg_snapshot* const* snaps, int n_snaps, const int64_t* seeds,
 		int K, int iterations, double damping, double* out);

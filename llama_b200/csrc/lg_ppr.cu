@@ -10,7 +10,8 @@
 // (w -> t) reads the contiguous K-wide row of w; lane j of a warp owns columns
 // j, j+32, ...  The iterations run over the snapshot's flat in-CSR
 // (lg_flat.cuh: ids, head bits, rows with in-edges), its own when
-// lg_snapshot_flatten made one, else one built for the call: a warp takes a
+// lg_snapshot_flatten made one, else one built for the call (without memory for
+// it lg_ppr_walk.cu walks the levels): a warp takes a
 // range of consecutive edges, loads the rows of kPprAhead of them before it
 // adds any, and finishes a row where the next head bit stands.  A row over
 // more than one range leaves a partial per range (carry_first, carry_last)
@@ -34,6 +35,7 @@
 // a pass narrower.  LG_TUNE_PPR_RANGE bounds the edges per warp range; smaller
 // graphs get shorter ranges, so that every warp slot of the GPU has a few.
 #include "lg_flat.cuh"
+#include "lg_ppr.h"
 #include "lg_tune.h"
 
 #include <algorithm>
@@ -43,7 +45,6 @@ namespace lg {
 
 constexpr int kPprThreads = 256;
 constexpr int kPprWarps = kPprThreads / 32;
-constexpr uint32_t kNoSeed = 0xffffffffu;
 // Edges whose rows a warp loads ahead: about 8 to 32 loads per lane in
 // flight.  Up to 128 columns the registers are capped for three resident CTAs
 // (96 columns, 3 M edges: 252 -> 207 us an iteration; with 8 edges ahead and
@@ -430,7 +431,22 @@ extern "C" lg_status lg_ppr(lg_snapshot* const* snaps, int n_snaps, const int64_
 		const FlatCsr* f = sn->flat[1];
 		if (!f) {
 			if (!s->flat_scratch) s->flat_scratch = new FlatCsr;
-			LG_TRY(build_flat(sn, 1, *s->flat_scratch, false, true, false));
+			const lg_status fs = build_flat(sn, 1, *s->flat_scratch, false, true, false);
+			if (fs == LG_ENOMEM || fs == LG_ENOTSUP) {
+				// over the levels instead, with what the flat copy took
+				clear_error();
+				LG_CUDA(cudaStreamSynchronize(st), "ppr");
+				delete s->flat_scratch;
+				s->flat_scratch = nullptr;
+				LG_CUDA(cudaMemsetAsync(yb[0].p, 0, V * row, st), "memset");
+				ppr_seed_init<<<kb, 256, 0, st>>>(seeds_d, K, outdeg, K, yb[0].as<double>());
+				s->launches++;
+				LG_TRY(ppr_walk(sn, PprSeeds{firstb.as<uint32_t>(), seeds_d, (uint32_t)K},
+						(uint32_t)K, ktile, iterations, damping, yb[0].as<double>(),
+						yb[1].as<double>(), carry, xo));
+				continue;
+			}
+			LG_TRY(fs);
 			f = s->flat_scratch;
 		}
 		PprArgs a;

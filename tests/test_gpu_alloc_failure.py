@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from llama_b200 import LgError, Store, _lib
+from llama_b200.graph import ppr, tune_reset, tune_set
 from tests._util import max_rel_err
 
 pytestmark = pytest.mark.gpu
@@ -62,3 +63,39 @@ def test_push_runs_without_the_transpose(fail_at):
     for got, again in results:
         assert got is not None and max_rel_err(got, want) <= 1e-12
         assert max_rel_err(again, want) <= 1e-12
+
+
+@pytest.mark.parametrize("K,ktile", [(32, 256), (64, 32), (96, 256), (160, 256), (256, 256)])
+def test_ppr_runs_over_the_levels(fail_at, K, ktile):
+    """Without the flat in-CSR; seeds with and without in-edges, some twice."""
+    V = 4000
+    s, d = _graph(V, 60_000, K)
+    s, d = np.concatenate([s, np.arange(V)]), np.concatenate([d, np.full(V, 7)])  # a hub
+    m = d % 9 != 4                                # vertices without in-edges
+    k = np.unique(s[m] * V + d[m])
+    s, d = k // V, k % V
+    rng = np.random.default_rng(K)
+    seeds = rng.integers(0, V, K)
+    seeds[:8] = [4, 4, 13, 7, 7, 22, 31, 4]
+    late = rng.random(len(k)) < 0.3
+    dead = ~late & (rng.random(len(k)) < 0.1)
+
+    def build():
+        st = Store()
+        st.build_level(V, s[~late], d[~late])
+        st.build_level(V, s[late], d[late], None, s[dead], d[dead])
+        return st
+    tune_set(0, "ppr_ktile", ktile)
+    try:
+        results = list(_each_failure(fail_at, build, lambda sn: ppr([sn], seeds, iterations=6)))
+    finally:
+        tune_reset(0)
+    want = results[-1][0]
+    # the call's own allocations are eight at the most; the others, and there are
+    # some, are the flat in-CSR's
+    none = sum(got is None for got, _ in results)
+    assert none <= 8 and len(results) - none >= 4
+    for got, again in results:
+        # rows of at most 4000 positive terms, six iterations
+        assert got is None or max_rel_err(got, want) <= 6 * 2 * 4000 * 2.0 ** -53
+        assert np.array_equal(again, want)
