@@ -421,7 +421,10 @@ lg_status lg_bfs_multi(lg_snapshot* snap, const int64_t* roots, int n_roots,
  * the uint32 per-slot property ingested with the out-CSR (lg_csr_level.weights)
  * and the algorithm is delta-stepping with bucket width `delta`; distances are
  * exact.  dist: uint32[max_nodes], LG_UNREACHED when unreached.  Weights and
- * path lengths must stay below 2^31 - 2.  result (may be NULL): reached
+ * path lengths must stay below 2^31 - 2.  Reads the snapshot's flat out-CSR; one
+ * that is not flat is flattened for the call in scratch the store keeps (8 bytes
+ * per live edge and 24 per vertex), or its levels are read: without that memory,
+ * and where the snapshot is large and the root reaches few vertices.  result (may be NULL): reached
  * vertices (the reference's finalize() value), sum of their out-degrees,
  * largest finite distance, buckets visited, relaxation rounds, relaxations. */
 typedef struct lg_sssp_result {

@@ -244,6 +244,73 @@ lg_status ensure_split(lg_snapshot* sn, uint32_t delta) {
 	return LG_OK;
 }
 
+// Whether the root reaches few vertices: one CTA's search over the levels'
+// fragments (hops, not distances) comes to its end within kProbeLevels hops,
+// kProbeVerts vertices and kProbeSlots slots of theirs.  *large = 1 if not.  (The
+// vertices found before every thread has seen that they are too many fill at
+// most half of the hash table.)
+//
+// It takes some 20 to 50 us with the wait, and an isolated root 100 us in all
+// instead of a flat copy and 414 us at 45 M slots, 204 at 16 M, 135 at 1.5 M.  From
+// kProbeFrom slots on it is worth that to the calls that reach more (1086 -> 1104 us
+// at 16 M slots; 497 -> 550 at 1.5 M).
+constexpr uint64_t kProbeFrom = 1u << 22;
+constexpr int kProbeLevels = 64;
+constexpr int kProbeThreads = 1024;
+constexpr uint32_t kProbeVerts = 1024, kProbeSlots = 8192, kProbeTab = 4096;
+__global__ void __launch_bounds__(kProbeThreads)
+sssp_probe(SnapCsr out, uint32_t root, unsigned long long* large) {
+	__shared__ uint32_t tab[kProbeTab], queue[kProbeVerts];
+	__shared__ uint32_t s_n, s_slots;
+	const uint32_t tid = threadIdx.x, lane = tid & 31u;
+	auto hash = [](uint32_t v) { return (v * 2654435769u) >> 20; };
+	static_assert(kProbeTab == 1u << 12, "hash");
+	for (uint32_t i = tid; i < kProbeTab; i += kProbeThreads) tab[i] = kNoId;
+	__syncthreads();
+	if (tid == 0) {
+		tab[hash(root)] = queue[0] = root;
+		s_n = 1;
+		s_slots = 0;
+	}
+	__syncthreads();
+	auto too_large = [&]() {
+		return *(volatile uint32_t*)&s_n > kProbeVerts || *(volatile uint32_t*)&s_slots > kProbeSlots;
+	};
+	uint32_t head = 0;
+	uint32_t tail = 1;
+	for (int l = 0; l < kProbeLevels && head < tail; l++) {
+		for (uint32_t i = head + (tid >> 5); i < tail; i += kProbeThreads / 32) {
+			const uint32_t v = queue[i];
+			const uint32_t slots = min(vertex_slots(out, v), kProbeSlots + 1u);
+			if (lane == 0) atomicAdd(&s_slots, slots);
+			__syncwarp();
+			if (__any_sync(0xffffffffu, too_large())) break;
+			const uint32_t f1 = __ldg(out.frag_off + v + 1);
+			for (uint32_t f = __ldg(out.frag_off + v); f < f1; f++) {
+				const uint2 fr = __ldg(out.frags + f);
+				const uint32_t lv = frag_level(fr);
+				for (uint32_t k = lane; k < frag_len(fr) && !too_large(); k += 32u) {
+					if (slot_deleted(out.lt, lv, fr.x + k)) continue;
+					const uint32_t w = __ldg(out.lt->ids[lv] + fr.x + k);
+					uint32_t h = hash(w), y;
+					while ((y = atomicCAS(tab + h, kNoId, w)) != kNoId && y != w)
+						h = (h + 1u) & (kProbeTab - 1u);
+					if (y == w) continue;
+					const uint32_t at = atomicAdd(&s_n, 1u);
+					if (at < kProbeVerts) queue[at] = w;
+				}
+				__syncwarp();
+			}
+		}
+		__syncthreads();
+		if (too_large()) break;
+		head = tail;
+		tail = s_n;
+		__syncthreads();
+	}
+	if (tid == 0) *large = head < tail;
+}
+
 } // namespace
 
 extern "C" lg_status lg_sssp_delta(lg_snapshot* sn, int64_t root, uint32_t delta,
@@ -267,9 +334,21 @@ extern "C" lg_status lg_sssp_delta(lg_snapshot* sn, int64_t root, uint32_t delta
 	// every step in one launch over the flat out-CSR, the snapshot's own or
 	// one made for the call, unless a tunable asks for another form
 	const FlatCsr* fo = sn->flat[0];
+	bool small = false;                      // (and the snapshot is not flat)
 	if (!tune_value(s->device, LG_TUNE_SSSP_SPLIT) && !tune_value(s->device, LG_TUNE_SSSP_LEVELS)) {
 		const FlatCsr* f = fo && fo->weighted ? fo : nullptr;
-		if (!f) {
+		if (!f && sn->out.n_frag_slots >= kProbeFrom) {
+			// a flat copy costs the same whatever the root reaches
+			LG_TRY(sc[6].reserve(8 * sizeof(unsigned long long)));
+			unsigned long long large = 0;
+			sssp_probe<<<1, kProbeThreads, 0, st>>>(sn->view(0), (uint32_t)root,
+					sc[6].as<unsigned long long>());
+			LG_CUDA(cudaGetLastError(), "sssp_probe");
+			s->launches++;
+			LG_TRY(read_words(s, sc[6].as<unsigned long long>(), 1, &large));
+			small = !large;
+		}
+		if (!f && !small) {
 			if (!s->flat_scratch) s->flat_scratch = new FlatCsr;
 			const lg_status fs = build_flat(sn, 0, *s->flat_scratch, false, true, false);
 			if (fs == LG_OK && s->flat_scratch->weighted) f = s->flat_scratch;
@@ -339,9 +418,10 @@ extern "C" lg_status lg_sssp_delta(lg_snapshot* sn, int64_t root, uint32_t delta
 	unsigned long long* h = hw;              // 4 words read back
 	unsigned long long* init = hw + 4;       // 4 words written
 	LG_CUDA(cudaMemsetAsync(ctr, 0, 4 * sizeof(unsigned long long), st), "memset");
-	// the same rounds in one cooperative launch (LG_TUNE_SSSP_LEVELS)
+	// the same rounds in one cooperative launch (LG_TUNE_SSSP_LEVELS, or over so few
+	// vertices that the steps' launches would be what counts)
 	bool one_launch = false;
-	if (tune_value(s->device, LG_TUNE_SSSP_LEVELS)) {
+	if (small || tune_value(s->device, LG_TUNE_SSSP_LEVELS)) {
 		SsspLevelsArgs a;
 		a.out = out;
 		a.heavy = heavy;
