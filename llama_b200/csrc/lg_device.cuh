@@ -134,6 +134,26 @@ __device__ __forceinline__ double warp_segsum(double v, uint32_t key, bool* tail
 	return v;
 }
 
+// table[t] = value for t = a ... b - 1 of every lane (all lanes call): by the lane
+// itself, or by the whole warp where there are many, as the marks of one hub's
+// row among the tiles it covers are.
+constexpr uint32_t kLaneMarks = 32;
+__device__ __forceinline__ void mark_range(uint32_t* table, uint32_t a, uint32_t b,
+		uint32_t value) {
+	const uint32_t n = a < b ? b - a : 0u;
+	if (n <= kLaneMarks)
+		for (uint32_t t = a; t < a + n; t++) table[t] = value;
+	unsigned many = __ballot_sync(0xffffffffu, n > kLaneMarks);
+	while (many) {
+		const int l = __ffs(many) - 1;
+		many &= many - 1u;
+		const uint32_t ta = __shfl_sync(0xffffffffu, a, l);
+		const uint32_t tb = __shfl_sync(0xffffffffu, b, l);
+		const uint32_t x = __shfl_sync(0xffffffffu, value, l);
+		for (uint32_t t = ta + (threadIdx.x & 31u); t < tb; t += 32u) table[t] = x;
+	}
+}
+
 // ---------------------------------------------------------------------------
 // Host-side objects
 // ---------------------------------------------------------------------------

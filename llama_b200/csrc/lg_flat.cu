@@ -225,16 +225,19 @@ __global__ void flat_rows(const uint32_t* off, const uint32_t* kidx, uint64_t V,
 		uint32_t* nz_rows, uint32_t* nz_off, uint32_t* heads, uint32_t ntiles,
 		uint32_t* tile_seg) {
 	const uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (v >= V) return;
-	const uint32_t o = __ldg(off + v), e = __ldg(off + v + 1);
-	if (e == o) return;
-	const uint32_t k = __ldg(kidx + v);
-	nz_rows[k] = (uint32_t)v;
-	nz_off[k] = o;
-	atomicOr(heads + (o >> 5), 1u << (o & 31u));
-	if (k == 0) tile_seg[0] = 0;
-	for (uint32_t t = o / kFlatTile + 1u; t <= e / kFlatTile && t < ntiles; t++)
-		tile_seg[t] = k + 1u;
+	uint32_t o = 0, e = 0, k = 0;
+	if (v < V) {
+		o = __ldg(off + v);
+		e = __ldg(off + v + 1);
+	}
+	if (e != o) {
+		k = __ldg(kidx + v);
+		nz_rows[k] = (uint32_t)v;
+		nz_off[k] = o;
+		atomicOr(heads + (o >> 5), 1u << (o & 31u));
+		if (k == 0) tile_seg[0] = 0;
+	}
+	mark_range(tile_seg, o / kFlatTile + 1u, e != o ? min(e / kFlatTile + 1u, ntiles) : 0u, k + 1u);
 }
 
 // Fragment view: row k of the flat CSR is fragment k, {start, len << 6 | 0};

@@ -785,17 +785,27 @@ struct FragOut {
 	uint32_t* range_lb;          // lb[r] = first vertex with slot_off >= r * kBlockSlots
 	uint32_t nb;                 // r = 0 .. nb
 	unsigned long long* bare;    // += vertices without a fragment but with a degree
+	                             // (null: not a window's, whose degrees are counted)
 };
+// Tiles that begin before slot s.
+__device__ __forceinline__ uint32_t frag_tiles(uint32_t s) {
+	return s / kSlotTile + (s % kSlotTile != 0);
+}
 template <bool kFill>
 __global__ void walk_fragments(VtTab tab, int L, int minL, uint64_t V, uint32_t* count,
 		uint32_t* deg, uint32_t* slots_per_vertex, FragOut fo) {
 	uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (v >= V) return;
-	lg_vt_entry e = tab.vt[L][v];
-	if (!kFill) deg[v] = e.degree;
-	uint32_t n = 0, slots = 0;
-	const uint32_t out = kFill ? fo.frag_off[v] : 0;
-	const uint32_t at = kFill ? fo.slot_off[v] : 0;
+	lg_vt_entry e;
+	e.adj_list_start = LG_NIL_EDGE;
+	uint32_t n = 0, slots = 0, out = 0, at = 0, degree = 0;
+	if (v < V) {
+		e = tab.vt[L][v];
+		degree = e.degree;
+		if (!kFill) deg[v] = degree;
+		if (kFill) out = fo.frag_off[v];
+		if (kFill) at = fo.slot_off[v];
+	}
+	bool lengthy = false;                        // one of the fragments spans many tiles
 	while (e.adj_list_start != LG_NIL_EDGE && e.level_length != 0) {
 		uint32_t lv = LG_EDGE_LEVEL(e.adj_list_start);
 		if ((int)lv < minL) break;
@@ -804,10 +814,10 @@ __global__ void walk_fragments(VtTab tab, int L, int minL, uint64_t V, uint32_t*
 			fo.frags[out + n] = make_uint2(ix, (e.level_length << kLevelBits) | lv);
 			fo.start[out + n] = at + slots;
 			fo.vert[out + n] = (uint32_t)v;
-			const uint32_t end = (at + slots + e.level_length - 1u) / kSlotTile;
-			for (uint32_t t = (uint32_t)(((uint64_t)at + slots + kSlotTile - 1u) / kSlotTile);
-					t <= end; t++)
-				fo.tile_frag[t] = out + n;
+			const uint32_t t0 = frag_tiles(at + slots), t1 = frag_tiles(at + slots + e.level_length);
+			if (t1 - t0 > kLaneMarks) lengthy = true;
+			else
+				for (uint32_t t = t0; t < t1; t++) fo.tile_frag[t] = out + n;
 		}
 		n++;
 		slots += e.level_length;
@@ -815,17 +825,29 @@ __global__ void walk_fragments(VtTab tab, int L, int minL, uint64_t V, uint32_t*
 		e = tab.vt[lv - 1][v];
 	}
 	if (!kFill) {
-		count[v] = n;
-		slots_per_vertex[v] = slots;
+		if (v < V) {
+			count[v] = n;
+			slots_per_vertex[v] = slots;
+		}
 		return;
 	}
-	if (n == 0 && tab.vt[L][v].degree != 0) atomicAdd(fo.bare, 1ull);
+	if (n == 0 && degree != 0 && fo.bare) atomicAdd(fo.bare, 1ull);
 	const uint32_t last = (uint32_t)(((uint64_t)at + slots) / kBlockSlots);
 	if (v == 0) fo.range_lb[0] = 0;
-	for (uint32_t r = at / kBlockSlots + 1u; r <= last && r <= fo.nb; r++)
-		fo.range_lb[r] = (uint32_t)v + 1u;
+	mark_range(fo.range_lb, at / kBlockSlots + 1u, min(last, fo.nb) + 1u, (uint32_t)v + 1u);
 	if (v == V - 1)
 		for (uint32_t r = last + 1u; r <= fo.nb; r++) fo.range_lb[r] = (uint32_t)V;
+	// what the lanes left of the tiles' marks, a fragment of 32 vertices at a time
+	for (uint32_t i = 0; __any_sync(0xffffffffu, lengthy && i < n); i++) {
+		uint32_t t0 = 0, t1 = 0;
+		if (lengthy && i < n) {
+			const uint32_t st = fo.start[out + i];   // (its own store)
+			t0 = frag_tiles(st);
+			t1 = frag_tiles(i + 1 < n ? fo.start[out + i + 1] : at + slots);
+			if (t1 - t0 <= kLaneMarks) t1 = t0;
+		}
+		mark_range(fo.tile_frag, t0, t1, out + i);
+	}
 }
 
 __global__ void live_counts(SnapCsr g, uint32_t* out);
@@ -930,7 +952,8 @@ static lg_status open_fill(lg_snapshot* sn, DevCsr& csr, SnapDir& d, unsigned lo
 	walk_fragments<true><<<grid_for(V, B), B, 0, st>>>(vt_tab(sn, csr), L, minL, V, nullptr,
 			nullptr, nullptr, FragOut{d.frag_off.as<uint32_t>(), d.slot_off.as<uint32_t>(),
 				d.frags.as<uint2>(), d.frag_start(), d.frag_vert(), d.tile_frag(),
-				d.range_lb.as<uint32_t>(), (uint32_t)nb, counters.as<unsigned long long>() + 2});
+				d.range_lb.as<uint32_t>(), (uint32_t)nb,
+				minL > 0 ? nullptr : counters.as<unsigned long long>() + 2});
 	LG_CUDA(cudaGetLastError(), "walk_fragments fill");
 	LG_CUDA(cudaMemcpyAsync(d.frag_start() + F, d.slot_off.as<uint32_t>() + V, sizeof(uint32_t),
 			cudaMemcpyDeviceToDevice, st), "slot total");
@@ -989,7 +1012,7 @@ static void open_done(lg_snapshot* sn, DevCsr& csr, SnapDir& d, const unsigned l
 	d.n_slots = 0;
 	for (int l = sn->min_level; l <= sn->level; l++) d.n_slots += csr.levels[l]->n_slots;
 	d.n_dels = w[3];
-	d.n_bare = sn->min_level > 0 ? 0 : w[4];      // (a window's degrees were counted)
+	d.n_bare = w[4];
 	d.present = true;
 }
 

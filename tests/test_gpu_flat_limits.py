@@ -86,3 +86,43 @@ def test_slots_up_to_the_limit(short_of):
                 y = 0.15 * t + 0.85 * np.bincount(dst, w * y[src], V)
             # sums of at most 500 positive terms, contracting by 0.85 at most
             assert np.max(np.abs(x - y) / y) <= 1e-12
+
+
+@pytest.mark.parametrize("hub", [33 * 512 - 1, 33 * 512, 33 * 512 + 1, 70_001])
+def test_rows_over_many_tiles(hub):
+    """Rows and fragments whose marks among the tiles they cover are shared by a
+    warp: several in one warp, in one level and split over three, both ways."""
+    V = hub + 40
+    rng = np.random.default_rng(hub)
+    src, dst = [], []
+    for v, n in ((0, hub), (3, hub), (4, 5), (17, hub), (V - 1, hub), (40, 17_000 % V)):
+        src.append(np.full(n, v))
+        dst.append(rng.permutation(V)[:n])
+    s, d = np.concatenate(src), np.concatenate(dst)
+    k = np.unique(np.concatenate([s * V + d, d * V + s]))
+    s, d = k // V, k % V
+    lev = rng.integers(0, 3, len(s))
+    lev[(s == 3) | (d == 3)] = 0
+    deg = np.bincount(s, minlength=V).astype(np.float64)
+    x = np.full(V, 1.0 / V)
+    for _ in range(3):
+        x = 0.15 / V + 0.85 * np.bincount(d, (x / np.maximum(deg, 1))[s], V)
+    tol = 3 * 2 * V * 2.0 ** -53                  # three sums of at most V terms
+    with Store() as st:
+        for l in range(3):
+            st.build_level(V, s[lev == l], d[lev == l])
+        with st.snapshot() as sn:
+            off, nbr = sn.adjacency(0)
+            own = np.repeat(np.arange(V), np.diff(off.astype(np.int64)))
+            bfs, labels = sn.bfs(0)[0], sn.scc()[0]
+            w, v = rng.uniform(0.5, 1.0, len(s)), rng.uniform(0.5, 1.0, V)
+            # one iteration: every edge's weight by its place among the out-edges
+            y = 0.15 * v + 0.85 * np.bincount(nbr, w * v[own], V)
+            for flat in (False, True):
+                if flat:
+                    sn.flatten(0).flatten(1)
+                assert np.max(np.abs(sn.pagerank_pull(3) - x) / x) <= tol
+                assert np.array_equal(sn.bfs(0)[0], bfs)
+                assert np.array_equal(sn.scc()[0], labels)
+                got = sn.pagerank_fwd(w, v, 0.85, tol=1e-300, max_iter=1, keep_tape=False)[0]
+                assert np.max(np.abs(got - y) / y) <= tol
