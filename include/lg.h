@@ -320,7 +320,11 @@ lg_status lg_snapshot_is_flat(const lg_snapshot* snap, int dir, int* flat);
  * is dropped.  ranks: double[max_nodes].  Requires the in-CSR.
  * iterations = 0 returns pr0; the reference's do-while loop
  * (pagerank.h:133-178) runs one iteration when max is 0, so a caller that
- * forwards the reference's -n value passes max(n, 1). */
+ * forwards the reference's -n value passes max(n, 1).
+ * Up to 2^18 in-edges all iterations run in one cooperative launch whose CTAs
+ * meet at bounded barriers.  Should a wait run out, the call returns LG_ETIMEOUT,
+ * or, with ranks in device memory, for which it does not wait, the next
+ * lg_store_sync (or such call with ranks on the host) does, and ranks are NaN. */
 lg_status lg_pagerank_pull(lg_snapshot* snap, int iterations, double damping,
 		double* ranks);
 

@@ -18,11 +18,13 @@ void clear_error();
 // Limits that a test sets for the calls of its own thread (lg_test_limits, which
 // the public headers leave out), to reach what the library does where the GPU
 // has less to give: the device allocations that succeed before one fails
-// (negative: none does), and the CTAs of a cooperative launch that fit on it at
-// once (0: no cooperative launch).
+// (negative: none does), the CTAs of a cooperative launch that fit on it at once
+// (0: no cooperative launch), and whether the barriers of a one-launch PageRank
+// give up at once.
 struct TestLimits {
 	int64_t allocs = -1;
 	int64_t ctas = INT64_MAX;
+	bool barrier = false;
 };
 TestLimits& test_limits();
 

@@ -36,6 +36,8 @@
 #include "lg_flat_sweep.cuh"
 #include "lg_tune.h"
 
+#include <math_constants.h>
+
 #include <cstddef>
 #include <mutex>
 
@@ -156,6 +158,11 @@ pr_run(PrRunArgs g, RunCtl* c) {
 	op.outdeg = g.outdeg;
 	op.base = g.base;
 	op.d = g.d;
+	// without the other CTAs there is no result: a caller that waits on a stream
+	// of its own must not take what is there for one
+	auto give_up = [&]() {
+		for (uint64_t v = gtid; v < g.V; v += nthreads) g.pr_out[v] = CUDART_NAN;
+	};
 	if (g.first == 0) {
 		for (uint64_t v = gtid; v < g.V; v += nthreads) {
 			const uint32_t dg = __ldg(g.outdeg + v);
@@ -165,7 +172,7 @@ pr_run(PrRunArgs g, RunCtl* c) {
 				g.pr_out[v] = g.base;
 			}
 		}
-		if (!grid_barrier(&c->bar)) return;
+		if (!grid_barrier(&c->bar)) return give_up();
 	}
 	PrRunOp::Row cross = {};
 	double resid;
@@ -182,7 +189,7 @@ pr_run(PrRunArgs g, RunCtl* c) {
 				}
 		if (!run_iteration(g.a, op, c, sh, t0, t1, seg, 0.0, it & 1, it == g.first, cross,
 				&resid))
-			return;
+			return give_up();
 	}
 }
 
@@ -425,6 +432,8 @@ lg_status pagerank_over(lg_snapshot* sn, FlatCsr* f, int iterations, double damp
 		// the error word stays set until it has been reported
 		LG_CUDA(cudaMemsetAsync(&ctl->bar, 0, s->run_pending ? offsetof(CoopBar, err)
 				: sizeof(CoopBar), st), "memset");
+		if (test_limits().barrier)
+			LG_CUDA(cudaMemsetAsync(&ctl->bar.err, 1, 1, st), "memset");
 		PrRunArgs g;
 		g.a = a;
 		g.off = flat_off;
@@ -448,7 +457,7 @@ lg_status pagerank_over(lg_snapshot* sn, FlatCsr* f, int iterations, double damp
 			s->launches++;
 			s->run_pending = true;
 		}
-		if (dev_out) return LG_OK;               // lg_store_sync reports a barrier that gave up
+		if (dev_out) return LG_OK;               // lg_store_sync reports a wait that ran out
 		LG_TRY(copy_out(s, ranks, pr_buf, V * sizeof(double)));
 		return finish_run(s);
 	}

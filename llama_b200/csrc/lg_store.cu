@@ -36,6 +36,8 @@ TestLimits& test_limits() {
 	return t;
 }
 
+extern "C" void lg_test_barrier(int fails) { test_limits().barrier = fails != 0; }
+
 // Negative: no limit.  Returns the allocations left to succeed (negative if one
 // failed or there was no limit).
 extern "C" int64_t lg_test_limits(int64_t allocs, int64_t ctas) {

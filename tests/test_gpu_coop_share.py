@@ -4,7 +4,7 @@ forms with a launch per step."""
 import numpy as np
 import pytest
 
-from llama_b200 import Store, _lib
+from llama_b200 import LgError, Store, _lib
 from llama_b200.graph import tune_reset, tune_set
 from tests._util import max_rel_err
 
@@ -72,3 +72,37 @@ def test_without_cooperative_launches(limit):
                 for a, b in zip(got[:3], want[:3]):
                     assert np.array_equal(a, b)
                 assert max_rel_err(got[3], want[3]) <= 1e-12
+
+
+def test_a_wait_that_runs_out_is_seen():
+    """PageRank in one launch, its barriers giving up: the call or the next wait
+    says so, and ranks in device memory are not mistaken for a result."""
+    import torch
+    fails = _lib.lib.lg_test_barrier
+    fails.argtypes, fails.restype = [_lib.C.c_int], None
+    V = 3000
+    rng = np.random.default_rng(10)
+    k = np.unique(rng.integers(0, V * V, 30000))
+    with Store() as st:
+        st.build_level(V, k // V, k % V)
+        with st.snapshot() as sn:
+            want = sn.pagerank_pull(5)
+            dev = torch.zeros(V, dtype=torch.float64, device="cuda")
+            try:
+                fails(1)
+                with pytest.raises(LgError) as e:
+                    sn.pagerank_pull(5)
+                assert e.value.status == _lib.LG_ETIMEOUT
+                sn.pagerank_pull(5, out=dev)
+            finally:
+                fails(0)
+            torch.cuda.synchronize()
+            assert torch.isnan(dev).all()
+            with pytest.raises(LgError) as e:
+                st.sync()
+            assert e.value.status == _lib.LG_ETIMEOUT
+            st.sync()                                # said once
+            sn.pagerank_pull(5, out=dev)
+            st.sync()
+            assert np.array_equal(dev.cpu().numpy(), want)
+            assert np.array_equal(sn.pagerank_pull(5), want)
