@@ -219,9 +219,13 @@ lg_status flat_row_index(lg_store* s, FlatCsr& f, const uint32_t* deg);
 lg_status flat_transpose(lg_store* s, const FlatCsr& a, FlatCsr& f);
 
 // PageRank of sn over f, its flat in-CSR (lg_pagerank_pull's iterations and
-// output; lg_pagerank.cu).
+// output; lg_pagerank.cu).  sweeps: a launch per iteration also where the graph
+// is small enough for one launch in all.
 lg_status pagerank_over(lg_snapshot* sn, FlatCsr* f, int iterations, double damping,
-		double* ranks);
+		double* ranks, bool sweeps = false);
+// lg_pagerank_pull over the snapshot's flat in-CSR, or one made for the call.
+lg_status pagerank_pull(lg_snapshot* sn, int iterations, double damping, double* ranks,
+		bool sweeps);
 
 } // namespace lg
 

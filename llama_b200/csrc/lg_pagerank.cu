@@ -400,7 +400,7 @@ lg_status finish_run(lg_store* s) {
 }
 
 lg_status pagerank_over(lg_snapshot* sn, FlatCsr* f, int iterations, double damping,
-		double* ranks) {
+		double* ranks, bool sweeps) {
 	lg_store* s = sn->store;
 	cudaStream_t st = s->stream;
 	const uint64_t V = sn->V;
@@ -425,7 +425,8 @@ lg_status pagerank_over(lg_snapshot* sn, FlatCsr* f, int iterations, double damp
 	}
 	double* c0 = sc[0].as<double>();
 	double* c1 = sc[1].as<double>();
-	const int resident = iterations == 0 || ntiles > kPrRunTiles ? 0 : pr_run_resident(s->device);
+	const int resident = iterations == 0 || ntiles > kPrRunTiles || sweeps ? 0
+			: pr_run_resident(s->device);
 	if (resident > 0) {
 		LG_TRY(s->run_ctl.reserve(sizeof(RunCtl)));
 		RunCtl* ctl = s->run_ctl.as<RunCtl>();
@@ -516,11 +517,8 @@ lg_status pagerank_over(lg_snapshot* sn, FlatCsr* f, int iterations, double damp
 	return LG_OK;
 }
 
-} // namespace lg
-
-extern "C" lg_status lg_pagerank_pull(lg_snapshot* sn, int iterations,
-		double damping, double* ranks) {
-	clear_error();
+lg_status pagerank_pull(lg_snapshot* sn, int iterations, double damping, double* ranks,
+		bool sweeps) {
 	LG_TRY(check_args(sn, iterations, damping, ranks));
 	lg_store* s = sn->store;
 	LG_CUDA(cudaSetDevice(s->device), "cudaSetDevice");
@@ -533,7 +531,15 @@ extern "C" lg_status lg_pagerank_pull(lg_snapshot* sn, int iterations,
 		LG_TRY(build_flat(sn, 1, *s->flat_scratch, false));
 		f = s->flat_scratch;
 	}
-	return pagerank_over(sn, f, iterations, damping, ranks);
+	return pagerank_over(sn, f, iterations, damping, ranks, sweeps);
+}
+
+} // namespace lg
+
+extern "C" lg_status lg_pagerank_pull(lg_snapshot* sn, int iterations,
+		double damping, double* ranks) {
+	clear_error();
+	return pagerank_pull(sn, iterations, damping, ranks, false);
 }
 
 // ---------------------------------------------------------------------------

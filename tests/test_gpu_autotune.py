@@ -96,3 +96,36 @@ def test_autotune_leaves_a_flat_snapshot_flat(store):
     assert set(res) == {"ms_heavy"}
     assert res["ms_heavy"]["ms"][res["ms_heavy"]["chosen"]] == min(res["ms_heavy"]["ms"].values())
     tune_reset(0)
+
+
+def test_sweep_values_give_the_same_results():
+    """PageRank's sweep tunables where sweeps run: above 2^18 in-edges, with hub
+    rows over several tiles."""
+    spec = workloads.rmat_multiversion(scale=16, seed=12, levels=2, level0=0.9, delete=0.01)
+    hg = HostGraph.from_spec(spec)
+    with Store() as st:
+        st.ingest(hg)
+        with st.snapshot() as sn:
+            assert sn.num_edges > 1 << 19 and sn.in_degrees().max() > 2000
+            tune_reset(0)
+            try:
+                ref = sn.pagerank_pull(7, 0.85)
+                for c in (4, 5, 6, 8):
+                    tune_set(0, "pr_ctas_per_sm", c)
+                    assert np.array_equal(sn.pagerank_pull(7, 0.85), ref)
+                tune_reset(0)
+                tune_set(0, "pr_tile_occ", 8)
+                assert np.array_equal(sn.pagerank_pull(7, 0.85), ref)
+            finally:
+                tune_reset(0)
+
+
+def test_autotune_times_the_sweeps_on_small_graphs(store):
+    """Six iterations a call, four calls a value: a launch at least for each."""
+    tune_reset(0)
+    with store.snapshot() as sn:
+        for name, values in (("pr_ctas_per_sm", 4), ("pr_tile_occ", 2)):
+            before = store.launch_count
+            assert len(sn.autotune([name])[name]["ms"]) == values
+            assert store.launch_count - before >= values * 4 * 6
+    tune_reset(0)
