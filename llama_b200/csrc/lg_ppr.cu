@@ -18,13 +18,15 @@
 // that ppr_fixup adds in range order.  Rows without in-edges hold a constant
 // after the first iteration and are written once.
 //
-// x0 has one non-zero per column, so the first two iterations look a row up in a
-// bitmap of the rows that are not zero before they load it.
-//
 // Bound by the row gathers (E x K x 8 bytes per iteration, mostly from L2 at
 // 100 k vertices x 96 columns) and the instructions around them: a group of edges
-// in which no row begins and none is skipped (most groups, rows being longer)
-// is loaded and added without a test per edge, 127 us an iteration against 150.
+// in which no row begins (most groups, rows being longer) is loaded and added
+// without a test per edge: 145 us an iteration at 3.1 M edges (16 TB/s of rows),
+// the mean over three snapshots of 1.5 to 3.1 M edges 122 (150 with the tests).
+// x0 has one non-zero per column, but a bitmap of the rows that are not zero,
+// looked up before the first two iterations load them, gained in the first what
+// it cost in the second (844 us for those of the three snapshots against 862),
+// and the code for it cost the others 8 us of 127.
 // The form before it walked fragments and added an edge's row before it loaded
 // the next one: one load per lane in flight, 2.1 TB/s of rows on a 3 M-arc graph
 // with 96 columns.
@@ -74,8 +76,6 @@ struct PprArgs {
 	uint32_t K;               // row length of y / x / carries
 	uint32_t col0;            // first column of this pass (a K-tile of CPL * 32 columns)
 	uint32_t range;           // edges per warp range, a multiple of 32
-	const uint32_t* bits;     // kSparse: rows of y that are not zero
-	uint32_t* bits_next;      // those of y_next, if wanted
 };
 
 // Row of vertex v (out-degree dg, first seed sf) has the in-sums s.
@@ -83,7 +83,6 @@ template <int CPL>
 __device__ __forceinline__ void ppr_finish(const PprArgs& a, uint32_t v, uint32_t dg, uint32_t sf,
 		const double* s) {
 	const uint32_t lane = threadIdx.x & 31u;
-	bool some = false;
 #pragma unroll
 	for (int i = 0; i < CPL; i++) {
 		const uint32_t c = a.col0 + lane + 32 * i;
@@ -94,10 +93,7 @@ __device__ __forceinline__ void ppr_finish(const PprArgs& a, uint32_t v, uint32_
 		const double x = __dadd_rn(t, __dmul_rn(a.d, s[i]));
 		a.y_next[(uint64_t)v * a.K + c] = dg ? x / (double)dg : 0.0;
 		if (a.x_out) a.x_out[(uint64_t)v * a.K + c] = x;
-		some |= x != 0.0;
 	}
-	if (a.bits_next && __any_sync(0xffffffffu, some) && lane == 0)
-		atomicOr(a.bits_next + (v >> 5), 1u << (v & 31u));
 }
 
 template <int CPL>
@@ -108,7 +104,7 @@ __device__ __forceinline__ void ppr_carry(double* to, const PprArgs& a, uint32_t
 		to[(uint64_t)r * a.K + a.col0 + (threadIdx.x & 31u) + 32 * i] = s[i];
 }
 
-template <int CPL, bool kSparse>
+template <int CPL>
 __global__ void __launch_bounds__(kPprThreads, CPL <= 4 ? 3 : 2)
 ppr_step(PprArgs a) {
 	constexpr int U = kPprAhead<CPL>;
@@ -129,10 +125,6 @@ ppr_step(PprArgs a) {
 		const uint32_t n = min(32u, e1 - base);
 		const uint32_t hw = __ldg(a.heads + (base >> 5));
 		const uint32_t id = lane < n ? __ldcs(a.ids + base + lane) : 0u;
-		unsigned want = n == 32u ? ~0u : (1u << n) - 1u;     // edges whose rows are loaded
-		if (kSparse)
-			want = __ballot_sync(0xffffffffu, lane < n
-					&& ((__ldg(a.bits + (id >> 5)) >> (id & 31u)) & 1u));
 		// lane h: vertex, out-degree and seed of the row that h heads of this
 		// word leave open
 		const uint32_t k = next - 1u + lane;
@@ -144,8 +136,8 @@ ppr_step(PprArgs a) {
 		}
 		for (uint32_t g = 0; g < n; g += U) {
 			double v[U][CPL];
-			const unsigned all = (1u << U) - 1u, sel = (want >> g) & all;
-			const bool whole = !kSparse && sel == all;           // no row to skip
+			const unsigned all = (1u << U) - 1u;
+			const bool whole = g + U <= n;
 #pragma unroll
 			for (int u = 0; u < U; u++) {
 				const uint32_t src = __shfl_sync(0xffffffffu, id, g + u);
@@ -156,7 +148,7 @@ ppr_step(PprArgs a) {
 				} else {
 #pragma unroll
 					for (int i = 0; i < CPL; i++)
-						v[u][i] = (sel >> u) & 1u ? __ldg(row + 32 * i) : 0.0;
+						v[u][i] = g + u < n ? __ldg(row + 32 * i) : 0.0;
 				}
 			}
 			if (((hw >> g) & all) == 0) {                        // no row begins here
@@ -289,14 +281,6 @@ __global__ void ppr_seed_index(const uint2* seed_col, uint32_t n, uint32_t* seed
 	if (i < n && (i == 0 || seed_col[i - 1].x != seed_col[i].x)) seed_first[seed_col[i].x] = i;
 }
 
-// Rows of x0 that are not zero in columns [col0, col1).
-__global__ void ppr_seed_bits(const uint2* seed_col, uint32_t n, uint32_t col0, uint32_t col1,
-		uint32_t* bits) {
-	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= n || seed_col[i].y < col0 || seed_col[i].y >= col1) return;
-	atomicOr(bits + (seed_col[i].x >> 5), 1u << (seed_col[i].x & 31u));
-}
-
 __global__ void ppr_seed_init(const uint2* seed_col, uint32_t n, const uint32_t* outdeg,
 		uint32_t K, double* y) {
 	const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -309,15 +293,13 @@ __global__ void ppr_seed_init(const uint2* seed_col, uint32_t n, const uint32_t*
 // Seeds without in-edges, columns [col0, col1): y = (1-d) / out_degree from
 // the first iteration on (other rows without in-edges stay 0).
 __global__ void ppr_seed_empty(const uint2* seed_col, uint32_t n, const uint32_t* off,
-		const uint32_t* outdeg, double tele, uint32_t K, uint32_t col0, uint32_t col1, double* y,
-		uint32_t* bits) {
+		const uint32_t* outdeg, double tele, uint32_t K, uint32_t col0, uint32_t col1, double* y) {
 	const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
 	const uint32_t v = seed_col[i].x, c = seed_col[i].y;
 	if (c < col0 || c >= col1 || __ldg(off + v + 1) != __ldg(off + v)) return;
 	const uint32_t dg = outdeg[v];
 	y[(uint64_t)v * K + c] = dg ? tele / (double)dg : 0.0;
-	if (bits) atomicOr(bits + (v >> 5), 1u << (v & 31u));
 }
 
 // Result rows of the vertices without in-edges: (1-d) at their own seeds.
@@ -341,8 +323,7 @@ __global__ void ppr_seed_x(const uint2* seed_col, uint32_t n, uint32_t K, double
 
 template <int CPL>
 void launch_ppr_iteration(const PprArgs& a, cudaStream_t st) {
-	if (a.bits) ppr_step<CPL, true><<<grid_for(a.nranges, kPprWarps), kPprThreads, 0, st>>>(a);
-	else ppr_step<CPL, false><<<grid_for(a.nranges, kPprWarps), kPprThreads, 0, st>>>(a);
+	ppr_step<CPL><<<grid_for(a.nranges, kPprWarps), kPprThreads, 0, st>>>(a);
 	if (a.nranges > 1)
 		ppr_fixup<CPL><<<grid_for(a.nranges - 1, kPprWarps), kPprThreads, 0, st>>>(a);
 }
@@ -389,10 +370,6 @@ extern "C" lg_status lg_ppr(lg_snapshot* const* snaps, int n_snaps, const int64_
 	LG_TRY(yb[1].reserve(V * row));
 	LG_TRY(seedb.reserve(K * sizeof(uint2)));
 	LG_TRY(firstb.reserve(V * 4));
-	const uint64_t words = (V + 31) / 32;
-	LG_TRY(s->scratch[7].reserve(2 * words * 4));
-	uint32_t* bits = s->scratch[7].as<uint32_t>();       // rows not zero before the first
-	                                                     // and the second iteration
 	// launch parameters: columns per pass (a multiple of 32 dividing K) and
 	// the most edges per warp range
 	int ktile = (int)tune_value(s->device, LG_TUNE_PPR_KTILE);
@@ -486,20 +463,14 @@ extern "C" lg_status lg_ppr(lg_snapshot* const* snaps, int n_snaps, const int64_
 		// column tiles are independent: each runs all iterations on its columns
 		for (int c0 = 0; c0 < K; c0 += ktile) {
 			a.col0 = (uint32_t)c0;
-			LG_CUDA(cudaMemsetAsync(bits, 0, 2 * words * 4, st), "memset");
-			ppr_seed_bits<<<kb, 256, 0, st>>>(seeds_d, (uint32_t)K, (uint32_t)c0,
-					(uint32_t)(c0 + ktile), bits);
-			s->launches++;
 			for (int it = 0; it < iterations; it++) {
-				a.bits = it < 2 ? bits + it * words : nullptr;
-				a.bits_next = it == 0 ? bits + words : nullptr;
 				a.y = yb[it & 1].as<double>();
 				a.y_next = yb[(it + 1) & 1].as<double>();
 				a.x_out = (it == iterations - 1) ? xo : nullptr;
 				if (it < 2) {
 					// it 0: the block written now; it 1: the first one, read by then
 					ppr_seed_empty<<<kb, 256, 0, st>>>(seeds_d, (uint32_t)K, off, outdeg, a.tele,
-							(uint32_t)K, (uint32_t)c0, (uint32_t)(c0 + ktile), a.y_next, a.bits_next);
+							(uint32_t)K, (uint32_t)c0, (uint32_t)(c0 + ktile), a.y_next);
 					s->launches++;
 				}
 				if (a.nranges == 0) continue;
