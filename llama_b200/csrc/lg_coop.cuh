@@ -1,5 +1,6 @@
-// lg_coop.cuh - building blocks of the one-launch traversals (lg_bfs_levels.cu,
-// lg_sssp_levels.cu): a grid barrier for cooperative launches whose waits
+// lg_coop.cuh - building blocks of the one-launch traversals and iterations
+// (lg_bfs_levels.cu, lg_sssp_flat.cu, lg_sssp_levels.cu, lg_scc_flat.cu,
+// lg_flat_run.cuh): cooperative launches, a grid barrier for them whose waits
 // are bounded by the global timer, and CTA-wide sums and scans.
 #ifndef LG_COOP_CUH_
 #define LG_COOP_CUH_

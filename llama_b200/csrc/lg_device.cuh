@@ -161,7 +161,8 @@ __device__ __forceinline__ void mark_range(uint32_t* table, uint32_t a, uint32_t
 // A store's stream-ordered memory pool for the temporaries of one call.
 // Memory given back to it is handed out again without a driver call that
 // waits for the GPU.  It holds at most kPoolKeep bytes, which stay with it until
-// the store is destroyed or any allocation of the process fails (trim_pools);
+// the store is destroyed or an allocation of this library fails (trim_pools; other
+// allocators of the process cannot ask for them);
 // what does not fit is allocated and freed with cudaMalloc and cudaFree: mapping
 // pool memory costs 7 to 14 ms per GB, and giving it back as much again, against
 // 1 to 2 ms for cudaMalloc (SCC over 260 M edges in two flat copies of 1.3 GB

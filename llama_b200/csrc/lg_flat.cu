@@ -18,7 +18,7 @@
 // population count away.  The form before it built a slot-to-fragment table
 // per 1024-slot block in shared memory behind a dozen block barriers: it was
 // bound by those and by its instructions, 2.1 ms at 262 M slots.  Now it takes
-// 870 us there, some 70 instructions per 32 slots against 3 GB of traffic.
+// 890 us there, some 70 instructions per 32 slots against 3 GB of traffic.
 // What counts is the chains of loads: the next window is under way with the
 // ids of the present one, and where its rows ought to start is looked up per
 // window, not per row (1055 us), and 48 warps per SM hide the rest (96

@@ -67,7 +67,7 @@ __device__ inline void map_block(const SlotSpace& sp, uint32_t r, uint32_t ra, u
 	const uint32_t V = (uint32_t)sp.g.V;
 	if (tid == 0) {
 		// entries of the block: those starting in [ra, rb), plus the one
-		// straddling ra (precomputed lower bounds, see block_lower_bounds)
+		// straddling ra (precomputed lower bounds, walk_fragments)
 		uint32_t eb = __ldg(sp.range_lb + r);
 		if (eb > 0 && (eb == V || __ldg(sp.pos + eb) > ra)) eb--;
 		m.eb = eb;
