@@ -146,7 +146,7 @@ bfs_levels(SnapCsr out, const uint32_t* nz_rows, const uint32_t* nz_off, uint32_
 		uint32_t E, const uint32_t* in_ids, const uint32_t* outdeg, uint32_t V,
 		unsigned long long out_edges, int has_in, int32_t* level, uint32_t* q0, uint32_t* q1,
 		uint32_t* bits0, uint32_t* bits1, uint32_t* bits2, uint32_t* fcnt, uint32_t* fpos,
-		unsigned long long* bsum, LvCtl* c, int resume) {
+		unsigned long long* bsum, LvCtl* c, long long cycles, int resume) {
 	const uint32_t W = (uint32_t)(((uint64_t)V + 31u) / 32u);
 	const uint32_t tid = threadIdx.x, lane = tid & 31u;
 	const uint32_t nthreads = gridDim.x * blockDim.x;
@@ -436,7 +436,7 @@ bfs_levels(SnapCsr out, const uint32_t* nz_rows, const uint32_t* nz_off, uint32_
 			}
 			bu++;
 		}
-		if (gtid == 0 && clock64() - t0 > kCoopRunCycles) atomicOr(nxt + 1, kCoopTimeUp);
+		if (gtid == 0 && clock64() - t0 > cycles) atomicOr(nxt + 1, kCoopTimeUp);
 		if (!grid_barrier(&c->bar)) return;
 		if (top_down) {
 			uint32_t* t = q; q = nq; nq = t;
@@ -516,6 +516,7 @@ lg_status bfs_levels_over(lg_store* s, SnapCsr out, const FlatCsr* fi, const uin
 	uint32_t V32 = (uint32_t)V;
 	unsigned long long out_edges = n_edges;
 	int has_in = fi ? 1 : 0, resume = 0;
+	long long cycles = coop_run_cycles();
 	uint32_t* q0 = sc[0].as<uint32_t>();
 	uint32_t* q1 = sc[1].as<uint32_t>();
 	uint32_t* bits0 = sc[2].as<uint32_t>();
@@ -529,7 +530,8 @@ lg_status bfs_levels_over(lg_store* s, SnapCsr out, const FlatCsr* fi, const uin
 	bfs_levels_init<<<1, 32, 0, st>>>(root, q0, outdeg, ctl);
 	LG_CUDA(cudaGetLastError(), "bfs_levels_init");
 	void* args[] = {&out, &nz_rows, &nz_off, &R, &E, &in_ids, &outdeg, &V32, &out_edges,
-			&has_in, &lvl, &q0, &q1, &bits0, &bits1, &bits2, &fcnt, &fpos, &bsum, &ctl, &resume};
+			&has_in, &lvl, &q0, &q1, &bits0, &bits1, &bits2, &fcnt, &fpos, &bsum, &ctl, &cycles,
+			&resume};
 	s->launches++;
 	LvCtl h;
 	for (;; resume = 1) {

@@ -150,6 +150,9 @@ inline cudaError_t coop_launch(const void* kernel, unsigned* grid, int threads, 
 	}
 }
 
+// Cycles after which a launch's time is up (kCoopRunCycles; a test's: none).
+inline long long coop_run_cycles() { return test_limits().one_step ? -1 : kCoopRunCycles; }
+
 // The CTAs that coop_grid_size found, 0 where a test wants no cooperative launch.
 inline int coop_allowed(int grid) { return test_limits().ctas > 0 ? grid : 0; }
 

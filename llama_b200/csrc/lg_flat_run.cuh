@@ -269,7 +269,7 @@ inline unsigned run_ctas(uint32_t ntiles, int resident) {
 // at 30 k and 15 M edges; as much for a vertex).
 inline int run_iterations(uint64_t E, uint64_t V) {
 	const double n = 50000.0 / (7.0 + 6e-6 * ((double)E + (double)V));
-	return n < 1.0 ? 1 : (int)n;
+	return n < 1.0 || test_limits().one_step ? 1 : (int)n;
 }
 
 // The calling warp's tiles (warps in CTA order).

@@ -19,12 +19,13 @@ void clear_error();
 // the public headers leave out), to reach what the library does where the GPU
 // has less to give: the device allocations that succeed before one fails
 // (negative: none does), the CTAs of a cooperative launch that fit on it at once
-// (0: no cooperative launch), and whether the barriers of a one-launch PageRank
-// give up at once.
+// (0: no cooperative launch), whether the barriers of a one-launch PageRank
+// give up at once, and whether a launch's time is up after its first step.
 struct TestLimits {
 	int64_t allocs = -1;
 	int64_t ctas = INT64_MAX;
 	bool barrier = false;
+	bool one_step = false;
 };
 TestLimits& test_limits();
 

@@ -124,6 +124,7 @@ struct SrArgs {
 	uint32_t* list[2];
 	uint32_t *label, *color, *mark, *stamp;
 	uint2* pieces;          // {vertex, first edge}
+	long long cycles;       // the launch's time
 };
 
 struct SrShared {
@@ -247,7 +248,7 @@ scc_rest(SrArgs a, SrCtl* c) {
 	// the next one fills, which was read before the last barrier but one
 	auto cnt = [&]() { return c->ctr[t.slot]; };
 	auto barrier = [&]() {
-		if (gtid == 0 && clock64() - t0 > kCoopRunCycles) atomicOr(cnt() + 1, kCoopTimeUp);
+		if (gtid == 0 && clock64() - t0 > a.cycles) atomicOr(cnt() + 1, kCoopTimeUp);
 		if (!grid_barrier(&c->bar)) return false;
 		if (tid < 2) sh.got[tid] = __ldcg(cnt() + tid);
 		__syncthreads();
@@ -429,6 +430,7 @@ lg_status scc_flat_run(lg_snapshot* sn, const FlatCsr* fo, const FlatCsr* fi, ui
 	a.max_pieces = (uint32_t)(2 * std::max(fo->E, fi->E) / kSrPiece + 1);
 	LG_TRY(pieces.reserve((uint64_t)a.max_pieces * sizeof(uint2)));
 	a.pieces = pieces.as<uint2>();
+	a.cycles = coop_run_cycles();
 	void* kargs[] = {&a, &ctl};
 	for (;;) {
 		LG_CUDA(coop_launch((const void*)scc_rest, &ctas, kSrThreads, kargs, 0, st, &ctl->bar),

@@ -99,6 +99,7 @@ struct SfArgs {
 	uint32_t* far[2];
 	uint32_t *dist, *stamp;
 	uint2* pieces;                  // {vertex, first edge} of long rows' pieces
+	long long cycles;               // the launch's time
 };
 
 constexpr uint32_t kSfCand = 64;
@@ -331,7 +332,7 @@ __device__ __forceinline__ bool sf_step(const SfArgs& a, SfCtl* c, SfShared& sh,
 	if (tid < 4 && (kSolo || blockIdx.x == 0)) (kSolo ? sh.ctr[slot] : c->ctr[slot])[tid] = 0;
 	// after a barrier every thread finds the step's counters in sh.got
 	auto barrier = [&]() {
-		if (tid == 0 && blockIdx.x == 0 && clock64() - sh.t0 > kCoopRunCycles)
+		if (tid == 0 && blockIdx.x == 0 && clock64() - sh.t0 > a.cycles)
 			atomicOr(cnt + 3, kCoopTimeUp);
 		if (!kSolo && !grid_barrier(&c->bar)) return false;
 		if (kSolo) __syncthreads();
@@ -571,6 +572,7 @@ lg_status sssp_flat_run(lg_snapshot* sn, const FlatCsr* f, uint32_t root, uint32
 	a.stamp = sc[5].as<uint32_t>();
 	a.pieces = sc[7].as<uint2>();
 	LG_CUDA(cudaMemsetAsync(ctl, 0, sizeof(SfCtl), st), "clear control block");
+	a.cycles = coop_run_cycles();
 	int resume = 0;
 	void* kargs[] = {&a, &ctl, &resume};
 	unsigned long long h[10];

@@ -37,6 +37,7 @@ TestLimits& test_limits() {
 }
 
 extern "C" void lg_test_barrier(int fails) { test_limits().barrier = fails != 0; }
+extern "C" void lg_test_one_step(int on) { test_limits().one_step = on != 0; }
 
 // Negative: no limit.  Returns the allocations left to succeed (negative if one
 // failed or there was no limit).

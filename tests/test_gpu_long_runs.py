@@ -5,7 +5,7 @@ takes a microsecond or (there) half of one at the least."""
 import numpy as np
 import pytest
 
-from llama_b200 import Store
+from llama_b200 import Store, _lib
 from tests._util import max_rel_err
 
 pytestmark = pytest.mark.gpu
@@ -127,3 +127,59 @@ def test_fixed_point_of_very_many_iterations():
             nan, _, r = sn.pagerank_fwd(w * np.nan, v, damping, max_iter=20000, keep_tape=False)
             assert r.iterations == 20000 and np.isnan(r.residual)
             assert st.launch_count - before >= 5      # 3 with one launch of the iterations
+
+
+@pytest.fixture
+def one_step():
+    f = _lib.lib.lg_test_one_step
+    f.argtypes, f.restype = [_lib.C.c_int], None
+    yield f
+    f(0)
+
+
+@pytest.mark.parametrize("V,n,hub", [(2000, 9000, False), (60000, 500000, True),
+                                     (300000, 3000000, False)])
+def test_a_launch_for_every_step(one_step, V, n, hub):
+    """State handed from launch to launch at every step there is: top-down and
+    bottom-up levels, buckets, light and heavy phases, colouring, iterations."""
+    rng = np.random.default_rng(V)
+    k = rng.integers(0, V * V, n)
+    if hub:
+        k = np.concatenate([k, np.arange(V), np.arange(V) * V])
+    k = np.unique(k)
+    s, d = k // V, k % V
+    w = rng.uniform(0.5, 1.0, len(s)) / np.bincount(s, minlength=V)[s]
+    v = rng.random(V) / V
+    with Store() as st:
+        st.build_level(V, s, d, rng.integers(1, 200, len(s)))
+        with st.snapshot() as sn:
+            sn.flatten(0).flatten(1)
+
+            def results():
+                out = [x for root in (0, 7) for x in (sn.bfs(root), sn.sssp(root, 40))]
+                out.append(sn.scc())
+                x, tape, r = sn.pagerank_fwd(w, v, max_iter=9)
+                dw, dv, rb = tape.backward(v)
+                tape.close()
+                return out, (x, dw, dv, sn.pagerank_pull(9)), (r, rb)
+
+            def fields(r):
+                # (what a step finds of the improvements of the same step, and so
+                # these, depends on the order of the warps)
+                vary = ("reserved", "rounds", "relaxations", "steps")
+                return [getattr(r, f) for f, _ in type(r)._fields_ if f not in vary]
+            one_step(0)
+            before = st.launch_count
+            out, real, fix = results()
+            few = st.launch_count - before
+            one_step(1)
+            before = st.launch_count
+            out1, real1, fix1 = results()
+            assert st.launch_count - before > few + 40
+            one_step(0)
+            for (a, r), (b, r1) in zip(out, out1):
+                assert np.array_equal(a, b) and fields(r) == fields(r1)
+            for a, b in zip(real, real1):
+                assert np.array_equal(a, b)
+            for r, r1 in zip(fix, fix1):
+                assert fields(r) == fields(r1)
