@@ -74,7 +74,6 @@ struct SfState {
 	uint32_t light;                // rounds relax light edges only
 	uint32_t jump;                 // the next split goes to mind's bucket
 	uint32_t grid;                 // the next step is for the whole grid
-	uint32_t up;                   // the launch's time is up
 };
 
 struct SfCtl {
@@ -83,6 +82,7 @@ struct SfCtl {
 	                                // (and kCoopTimeUp)
 	SfState st;                     // handed over by the CTA that worked alone, and to
 	                                // the next launch
+	uint32_t up;                    // by that CTA: the launch's time is up
 	alignas(16) unsigned long long out[8];   // rounds, buckets, relaxations, reached,
 	                                // out-edges of the reached, largest distance, done
 	CoopBar bar;                    // err bit 2: a count out of range, bit 3: step cap
@@ -111,6 +111,7 @@ struct SfShared {                   // dynamic shared memory
 	unsigned long long ctr[3][4];   // the lone CTA's counters
 	unsigned long long got[4];      // the last step's counters
 	long long t0;                   // the launch's start (CTA 0)
+	uint32_t up;                    // its time is up
 	SfState st;
 };
 
@@ -336,7 +337,12 @@ __device__ __forceinline__ bool sf_step(const SfArgs& a, SfCtl* c, SfShared& sh,
 			atomicOr(cnt + 3, kCoopTimeUp);
 		if (!kSolo && !grid_barrier(&c->bar)) return false;
 		if (kSolo) __syncthreads();
-		if (tid < 4) sh.got[tid] = kSolo ? *(volatile unsigned long long*)(cnt + tid) : __ldcg(cnt + tid);
+		if (tid < 4) {
+			const unsigned long long x = kSolo ? *(volatile unsigned long long*)(cnt + tid)
+					: __ldcg(cnt + tid);
+			sh.got[tid] = x & ~kCoopTimeUp;
+			if (tid == 3) sh.up = x >= kCoopTimeUp;
+		}
 		__syncthreads();
 		return true;
 	};
@@ -359,7 +365,7 @@ __device__ __forceinline__ bool sf_step(const SfArgs& a, SfCtl* c, SfShared& sh,
 		relaxations += sf_rows(a, s, heavy ? nullptr : a.q[t.qsel],
 				heavy ? a.V : (uint32_t)t.qlen, t.lo, gwarp, nwarps);
 		if (!barrier()) return false;
-		const unsigned long long np = count(3) & ~kCoopTimeUp;
+		const unsigned long long np = count(3);
 		if (np > a.max_pieces) {
 			if (tid == 0) atomicOr(&c->bar.err, 4u);
 			return false;
@@ -403,7 +409,6 @@ __device__ __forceinline__ bool sf_step(const SfArgs& a, SfCtl* c, SfShared& sh,
 		t.in_bucket = 0;
 		t.jump = !t.jump && t.qlen == 0 && t.flen > 0;
 	}
-	t.up = count(3) >= kCoopTimeUp;
 	return true;
 }
 
@@ -428,7 +433,6 @@ sssp_flat(SfArgs a, SfCtl* c, int resume) {
 	SfState t = {};
 	if (resume) {
 		t = sf_load_state(c, sh);
-		t.up = 0;
 	} else {
 		for (uint64_t v = gtid; v < a.V; v += nthreads) {
 			a.dist[v] = v == a.root ? 0u : kInf;
@@ -445,16 +449,20 @@ sssp_flat(SfArgs a, SfCtl* c, int resume) {
 	const uint64_t step_cap = 4ull * a.V + 64;
 	uint32_t solo_slot = 0;
 	if (tid < 4) sh.ctr[0][tid] = 0;
-	if (tid == 0) sh.t0 = clock64();
+	if (tid == 0) {
+		sh.t0 = clock64();
+		sh.up = 0;
+	}
 	__syncthreads();
-	while ((t.qlen > 0 || t.flen > 0 || t.light) && !t.up) {
+	// (sh.up changes between barriers only)
+	while ((t.qlen > 0 || t.flen > 0 || t.light) && !sh.up) {
 		if (t.round >= step_cap) {
 			if (tid == 0) atomicOr(&c->bar.err, 8u);
 			return;
 		}
 		if (!t.grid && !t.light && t.qlen <= kSoloQueue && t.flen <= kSoloFar) {
 			if (blockIdx.x == 0) {
-				for (uint32_t n = 0; n < kSoloSteps && !t.up && (t.qlen > 0 || t.flen > 0)
+				for (uint32_t n = 0; n < kSoloSteps && !sh.up && (t.qlen > 0 || t.flen > 0)
 						&& t.qlen <= kSoloQueue && t.flen <= kSoloFar; n++) {
 					if (t.qlen > 0) {
 						uint32_t len = 0;
@@ -469,10 +477,16 @@ sssp_flat(SfArgs a, SfCtl* c, int resume) {
 					}
 					if (!sf_step<true>(a, c, sh, t, solo_slot, relaxations)) return;
 				}
-				if (tid == 0) c->st = t;
+				if (tid == 0) {
+					c->st = t;
+					c->up = sh.up;
+				}
 			}
 			if (!grid_barrier(&c->bar)) return;
-			if (blockIdx.x != 0) t = sf_load_state(c, sh);
+			if (blockIdx.x != 0) {
+				if (tid == 0) sh.up = __ldcg(&c->up);
+				t = sf_load_state(c, sh);            // (synchronises)
+			}
 			if (!t.grid) t.grid = t.qlen > 0 || t.flen > 0;   // past a CTA's limits
 			// (nobody rewrites c->st before the grid step's barrier)
 			continue;
