@@ -21,7 +21,10 @@
 //   - from a bucket's second round on, a long queue relaxes only edges lighter
 //     than delta (a vertex of the first bucket of an R-MAT graph is improved
 //     three times on average), and the heavier edges of the vertices whose
-//     distance ended up in the bucket are relaxed once when it has drained;
+//     distance ended up in the bucket are relaxed once when it has drained (with
+//     no heavier edge anywhere all rounds relax all edges, and that pass over the
+//     rows falls away: delta 1000 with weights below 100 at 16 M edges and 4 M
+//     vertices 1320 -> 1100 us);
 //   - edges that would improve their target are collected per warp and relaxed
 //     32 at a time: few edges of a step do, and waiting for the atomics of each
 //     128 edges doubled the time of the large steps; the next edges' loads are
@@ -72,6 +75,7 @@ struct SfState {
 	uint32_t mind;                 // smallest distance the last split kept
 	uint32_t qsel, fsel;           // which of the two queues / piles is current
 	uint32_t light;                // rounds relax light edges only
+	uint32_t heavy;                // whether there are other edges (SfHeavy)
 	uint32_t jump;                 // the next split goes to mind's bucket
 	uint32_t grid;                 // the next step is for the whole grid
 };
@@ -84,7 +88,8 @@ struct SfCtl {
 	                                // the next launch
 	uint32_t up;                    // by that CTA: the launch's time is up
 	alignas(16) unsigned long long out[8];   // rounds, buckets, relaxations, reached,
-	                                // out-edges of the reached, largest distance, done
+	                                // out-edges of the reached, largest distance, done,
+	                                // an edge of at least delta was found
 	CoopBar bar;                    // err bit 2: a count out of range, bit 3: step cap
 };
 
@@ -93,7 +98,7 @@ struct SfArgs {
 	const uint32_t* ids;
 	const uint32_t* w;
 	const uint32_t* outdeg;
-	uint32_t V, root, delta, piece;
+	uint32_t V, E, root, delta, piece;
 	uint32_t max_pieces, light_min;
 	uint32_t* q[2];
 	uint32_t* far[2];
@@ -112,8 +117,11 @@ struct SfShared {                   // dynamic shared memory
 	unsigned long long got[4];      // the last step's counters
 	long long t0;                   // the launch's start (CTA 0)
 	uint32_t up;                    // its time is up
+	uint32_t heavy;
 	SfState st;
 };
+
+enum SfHeavy : uint32_t { kNotLooked, kSomeHeavy, kNoHeavy };
 
 enum SfEdges : uint32_t { kAllEdges, kLightEdges, kHeavyEdges };
 
@@ -350,7 +358,8 @@ __device__ __forceinline__ bool sf_step(const SfArgs& a, SfCtl* c, SfShared& sh,
 	t.round++;
 	if (t.qlen > 0 || t.light) {
 		const bool heavy = t.qlen == 0;          // the bucket has drained
-		if (!heavy && t.in_bucket > 0 && t.qlen >= a.light_min) t.light = 1;
+		if (!heavy && t.in_bucket > 0 && t.qlen >= a.light_min && t.heavy == kSomeHeavy)
+			t.light = 1;
 		SfStep s;
 		s.round = t.round;
 		s.hi = t.hi;
@@ -412,6 +421,26 @@ __device__ __forceinline__ bool sf_step(const SfArgs& a, SfCtl* c, SfShared& sh,
 	return true;
 }
 
+// Looks for an edge of at least delta, until a CTA has found one (one thread of
+// a CTA says so and asks: all of them at one address took 100 us).  A first look,
+// at a tile per CTA while the distances are filled, usually finds one.
+__device__ __noinline__ void sf_look(const SfArgs& a, SfCtl* c, bool first) {
+	constexpr uint32_t kLook = 8, kTile = kLook * kSfThreads;
+	for (uint64_t b = (uint64_t)blockIdx.x * kTile; b < a.E; b += (uint64_t)gridDim.x * kTile) {
+		uint32_t w = 0;
+#pragma unroll
+		for (uint32_t u = 0; u < kLook; u++) {
+			const uint64_t e = b + u * kSfThreads + threadIdx.x;
+			w = max(w, e < a.E ? __ldg(a.w + e) : 0u);
+		}
+		volatile unsigned long long* some = c->out + 7;
+		const bool others = threadIdx.x == 0 && *some != 0;
+		const bool found = __syncthreads_or(w >= a.delta);
+		if (found && threadIdx.x == 0) *some = 1;
+		if (__syncthreads_or(found || others) || first) break;
+	}
+}
+
 // The state in c->st, read by a CTA behind a barrier.
 __device__ __forceinline__ SfState sf_load_state(const SfCtl* c, SfShared& sh) {
 	if (threadIdx.x < sizeof(SfState) / 4)
@@ -438,6 +467,7 @@ sssp_flat(SfArgs a, SfCtl* c, int resume) {
 			a.dist[v] = v == a.root ? 0u : kInf;
 			a.stamp[v] = 0xffffffffu;
 		}
+		sf_look(a, c, true);
 		if (gtid == 0) a.q[0][0] = a.root;
 		t.qlen = 1;
 		t.hi = a.delta;
@@ -452,8 +482,10 @@ sssp_flat(SfArgs a, SfCtl* c, int resume) {
 	if (tid == 0) {
 		sh.t0 = clock64();
 		sh.up = 0;
+		sh.heavy = __ldcg(c->out + 7) ? kSomeHeavy : kNotLooked;
 	}
 	__syncthreads();
+	if (!resume) t.heavy = sh.heavy;
 	// (sh.up changes between barriers only)
 	while ((t.qlen > 0 || t.flen > 0 || t.light) && !sh.up) {
 		if (t.round >= step_cap) {
@@ -492,6 +524,13 @@ sssp_flat(SfArgs a, SfCtl* c, int resume) {
 			continue;
 		}
 		t.grid = 0;
+		if (t.heavy == kNotLooked && t.in_bucket > 0 && t.qlen >= a.light_min) {
+			sf_look(a, c, false);
+			if (!grid_barrier(&c->bar)) return;
+			if (tid == 0) sh.heavy = __ldcg(c->out + 7) ? kSomeHeavy : kNoHeavy;
+			__syncthreads();
+			t.heavy = sh.heavy;
+		}
 		if (!sf_step<false>(a, c, sh, t, t.step, relaxations)) return;
 	}
 	relaxations = block_sum<kSfWarps>(relaxations);
@@ -576,6 +615,7 @@ lg_status sssp_flat_run(lg_snapshot* sn, const FlatCsr* f, uint32_t root, uint32
 	a.w = f->w.as<uint32_t>();
 	a.outdeg = sn->out.deg.as<uint32_t>();
 	a.V = (uint32_t)V;
+	a.E = (uint32_t)f->E;
 	a.root = root;
 	a.delta = delta;
 	a.q[0] = sc[0].as<uint32_t>();

@@ -80,3 +80,30 @@ def test_single_vertex_and_no_edges():
         with st.snapshot() as sn:
             got, r = sn.sssp(0, 32)
             assert list(got) == [0] and (r.reached, r.reach_edges, r.max_dist) == (1, 0, 0)
+
+
+@pytest.mark.parametrize("heavy", ["none", "last rows", "one", "first rows"])
+def test_few_heavy_edges(heavy):
+    """Edges of at least delta nowhere, or where a first look may not meet them;
+    queues long enough for rounds over the light edges alone."""
+    rng = np.random.default_rng(len(heavy))
+    V = 150000
+    key = np.unique(rng.integers(0, V, 2400000) * V + rng.integers(0, V, 2400000))
+    s, d = key // V, key % V
+    w = rng.integers(1, 31, len(s))
+    delta = 40
+    at = {"none": s < 0, "last rows": s >= V - 300, "first rows": s < 300,
+          "one": np.arange(len(s)) == len(s) - 7}[heavy]
+    w[at] = rng.integers(delta, 4 * delta, at.sum())
+    # long ways round: rows that only heavy edges improve
+    want = dijkstra(csr_matrix((w.astype(np.float64), (s, d)), (V, V)), indices=[0, int(s[-7])])
+    with Store(reverse_edges=False) as st:
+        st.build_level(V, s, d, w)
+        with st.snapshot() as sn:
+            for flat in (False, True):
+                if flat:
+                    sn.flatten(0)
+                for i, root in enumerate((0, int(s[-7]))):
+                    ref = np.where(np.isinf(want[i]), LG_UNREACHED, want[i]).astype(np.uint32)
+                    for dl in (delta, delta + 1, 31, 15):
+                        assert np.array_equal(sn.sssp(root, dl)[0], ref), (root, dl)
