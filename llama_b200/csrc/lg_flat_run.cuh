@@ -38,6 +38,7 @@ namespace lg {
 
 constexpr int kRunThreads = 1024;      // one CTA per SM, 64 registers a thread
 constexpr int kRunWarps = kRunThreads / 32;
+constexpr int kRunRows = 4;
 constexpr int kRunMaxCtas = 256;       // more SMs than any device of this architecture has
 
 // What a CTA publishes of its edges, twice: iterations alternate.
@@ -158,12 +159,22 @@ __device__ __forceinline__ double run_tiles(const FlatTiles& a, const Op& op, Ru
 			if (lane == 0) first = rs[0];
 			before = false;
 		}
-		for (uint32_t r = lane; r < H; r += 32u) {
-			if (r >= 32u) {
-				row = op.row(seg + r - 1u);
-				was = op.old(row);
+		if (lane < H && (lane > 0 || !lead_row)) res += op.finish(row, rs[lane], was);
+		// the rows behind the first 32 (short rows: up to 256 in a tile), the loads
+		// of some of a lane's before the first of them is finished
+		for (uint32_t r0 = 32u; r0 < H; r0 += 32u * kRunRows) {
+			typename Op::Row rw[kRunRows];
+			double old[kRunRows];
+#pragma unroll
+			for (int u = 0; u < kRunRows; u++)
+				rw[u] = op.row(min(seg + r0 + u * 32u + lane - 1u, a.R - 1u));
+#pragma unroll
+			for (int u = 0; u < kRunRows; u++) old[u] = op.old(rw[u]);
+#pragma unroll
+			for (int u = 0; u < kRunRows; u++) {
+				const uint32_t r = r0 + u * 32u + lane;
+				if (r < H) res += op.finish(rw[u], rs[r], old[u]);
 			}
-			if (r > 0 || !lead_row) res += op.finish(row, rs[r], was);
 		}
 		seg += H;
 		__syncwarp();                          // rs is reused by the next tile

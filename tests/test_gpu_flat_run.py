@@ -97,3 +97,30 @@ def test_fixed_point_repeats_bit_for_bit():
                 x2, _, r2 = sn.pagerank_fwd(w, v, tol=1e-300, max_iter=5, keep_tape=False)
                 assert (r2.iterations, r2.residual) == (r.iterations, r.residual)
                 assert np.array_equal(x2, x)
+
+
+@pytest.mark.parametrize("longest", [1, 2, 3, 9])
+def test_short_rows(longest):
+    """From 25 to 256 rows begin in a tile: the counts at which a lane finishes
+    one more, or four more."""
+    rng = np.random.default_rng(longest)
+    V = 30000
+    n = rng.integers(1, longest + 1, V)
+    n[::97] = 0
+    d = np.repeat(np.arange(V), n)
+    s = (d * 7919 + np.concatenate([np.arange(k) for k in n]) * 104729) % V
+    k = np.unique(s * V + d)
+    s, d = k // V, k % V
+    deg = np.bincount(s, minlength=V).astype(np.float64)
+    w = rng.uniform(0.5, 1.0, len(s)) / deg[s]
+    v = rng.random(V) / V
+    with Store() as st:
+        st.build_level(V, s, d)
+        with st.snapshot() as sn:
+            x, y = np.full(V, 1.0 / V), v.copy()
+            for it in (1, 2, 3):
+                x = 0.15 / V + 0.85 * np.bincount(d, (x / np.maximum(deg, 1))[s], V)
+                y = 0.15 * v + 0.85 * np.bincount(d, w * y[s], V)
+                assert max_rel_err(sn.pagerank_pull(it), x) <= 1e-14
+                got, _, r = sn.pagerank_fwd(w, v, tol=1e-300, max_iter=it, keep_tape=False)
+                assert max_rel_err(got, y) <= 1e-14
