@@ -366,6 +366,9 @@ namespace lg {
 // streams overlap and whole-GPU ones do not.  (A single program's gain goes on
 // to some 4000 tiles, 406 -> 289 us at 560 k edges.)
 constexpr uint32_t kPrRunTiles = 1024;
+// Fewest iterations: a cooperative launch takes some 6 us to begin (one iteration
+// of a flattened graph of 2 k to 20 k edges 35 us, 29 in launches).
+constexpr int kPrRunIters = 3;
 
 static std::mutex g_run_mu;
 static int g_run[LG_TUNE_MAX_DEVICES];    // co-resident CTAs of pr_run + 1, 0 = not probed
@@ -425,7 +428,7 @@ lg_status pagerank_over(lg_snapshot* sn, FlatCsr* f, int iterations, double damp
 	}
 	double* c0 = sc[0].as<double>();
 	double* c1 = sc[1].as<double>();
-	const int resident = iterations == 0 || ntiles > kPrRunTiles || sweeps ? 0
+	const int resident = iterations < kPrRunIters || ntiles > kPrRunTiles || sweeps ? 0
 			: pr_run_resident(s->device);
 	if (resident > 0) {
 		LG_TRY(s->run_ctl.reserve(sizeof(RunCtl)));
