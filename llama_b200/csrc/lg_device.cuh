@@ -242,6 +242,7 @@ struct SnapDir {
 	uint64_t n_frag_slots = 0;     // slots covered by fragments
 	uint64_t n_dels = 0;           // deletion marks visible at L
 	uint64_t n_bare = 0;           // vertices without a fragment but with a degree
+	uint64_t max_degree = 0;
 	bool present = false;
 	// exchange device buffers with o (a closed snapshot's, kept for reuse)
 	void swap_buffers(SnapDir& o) {
@@ -387,7 +388,7 @@ lg_status copy_out(lg_store* s, void* dst, const void* src, size_t bytes);
 
 // The store's kHostWords pinned words (allocated on first use), for
 // counters a host loop reads back every step.
-constexpr int kHostWords = 22;
+constexpr int kHostWords = 24;
 constexpr int kReadWords = 12;               // the last of them: for read_words
 lg_status host_words(lg_store* s, unsigned long long** words);
 // Waits for the store's stream and reads n <= kReadWords device words into out

@@ -76,11 +76,24 @@ using namespace lg;
 
 namespace {
 
-// Whether transposing E edges for `iterations` iterations beats pushing: it
-// saves about 32 ps per edge and iteration after the first and costs about as
-// much again per edge, and 0.15 ms of launches and waits.
-bool transpose_pays(int iterations, uint64_t E) {
-	return iterations > 1 && (uint64_t)(iterations - 1) * E > 5000000ull;
+// Whether transposing E edges for `iterations` iterations beats pushing.  Where
+// hubs take a good part of the reductions, these wait for one another: an
+// iteration costs 75 ps per edge at 2 M edges of an R-MAT graph and 35 at 20 M, and
+// transposing saves nearly all of it for about as much again and 0.15 ms of
+// launches and waits (2 M: even at 3 iterations, 16 M: at 2).  Without hubs the
+// reductions are 7 to 25 ps per edge, the cheaper the more edges a vertex has,
+// the sweeps' gathers half of that, and the transpose 45 to 60: even at 6.5
+// iterations for 1 M vertices and 2 M edges, 7.5 for 4 M and 16 M, 9 for 4 M and 32 M,
+// 19 for 0.5 M and 16 M, 8.5 for a grid of 2 M edges.  A hub is told by the largest
+// degree (out-degree where no in-edges are kept): from 0.1 % of the edges in R-MAT
+// graphs, up to 0.025 % in those others.
+bool transpose_pays(const lg_snapshot* sn, int iterations) {
+	const uint64_t E = sn->out.n_edges, V = sn->V;
+	const SnapDir& d = sn->in.present ? sn->in : sn->out;
+	if (iterations < 2) return false;
+	const uint64_t visits = (uint64_t)(iterations - 1) * E;
+	if (d.max_degree >= E / 2048u) return visits > 5000000ull;
+	return visits > 13000000ull && (uint64_t)iterations >= 8u + E / (3u * V);
 }
 
 // The iterations over the transposed out-edges; *ran = false, and nothing is
@@ -118,7 +131,7 @@ extern "C" lg_status lg_pagerank_push(lg_snapshot* sn, int iterations, double da
 	cudaStream_t st = s->stream;
 	const uint64_t V = sn->V;
 	if (V == 0) return LG_OK;
-	if (transpose_pays(iterations, sn->out.n_edges)) {
+	if (transpose_pays(sn, iterations)) {
 		bool ran = false;
 		LG_TRY(push_transposed(sn, iterations, damping, ranks, &ran));
 		if (ran) return LG_OK;

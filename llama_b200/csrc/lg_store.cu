@@ -877,18 +877,26 @@ __global__ void mark_deletions(const uint2* dels, uint64_t n, int L, int minL,
 	if ((threadIdx.x & 31u) == 0 && c) atomicAdd(count, c);
 }
 
-__global__ void sum_u32(const uint32_t* x, uint64_t n, unsigned long long* out) {
+// *sum += the degrees, *most = the largest.
+__global__ void sum_degrees(const uint32_t* x, uint64_t n, unsigned long long* sum,
+		unsigned long long* most) {
 	unsigned long long s = 0;
+	uint32_t m = 0;
 	for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-			i += (uint64_t)gridDim.x * blockDim.x)
+			i += (uint64_t)gridDim.x * blockDim.x) {
 		s += x[i];
+		m = max(m, x[i]);
+	}
 	uint64_t tot;
 	block_excl_scan(s, &tot);
-	if (threadIdx.x == 0 && tot) atomicAdd(out, (unsigned long long)tot);
+	if (threadIdx.x == 0 && tot) atomicAdd(sum, (unsigned long long)tot);
+	m = __reduce_max_sync(0xffffffffu, m);
+	if ((threadIdx.x & 31u) == 0 && m > *(volatile unsigned long long*)most)
+		atomicMax(most, (unsigned long long)m);
 }
 
 // Opening a direction takes three parts, with one wait for both directions
-// after each of the first two; `w` are five of the store's pinned words.
+// after each of the first two; `w` are six of the store's pinned words.
 
 static VtTab vt_tab(const lg_snapshot* sn, const DevCsr& csr) {
 	VtTab tab;
@@ -930,7 +938,8 @@ static lg_status open_count(lg_snapshot* sn, DevCsr& csr, SnapDir& d, unsigned l
 }
 
 // Fragments, deletion bitsets and degrees; w[2] = live edges, w[3] = deletion
-// marks visible, w[4] = vertices without a fragment but with a degree.
+// marks visible, w[4] = vertices without a fragment but with a degree, w[5] = the
+// largest degree.
 static lg_status open_fill(lg_snapshot* sn, DevCsr& csr, SnapDir& d, unsigned long long* w) {
 	lg_store* s = sn->store;
 	const int L = sn->level, minL = sn->min_level;
@@ -949,9 +958,10 @@ static lg_status open_fill(lg_snapshot* sn, DevCsr& csr, SnapDir& d, unsigned lo
 	LG_TRY(d.frag_aux.reserve((2 * F + 1 + tiles) * sizeof(uint32_t)));
 	LG_TRY(d.range_lb.reserve((nb + 1) * sizeof(uint32_t)));
 	DevBuf& counters = d.tmp_sum;     // [0] live degree sum, [1] deletions visible at L,
-	                                  // [2] vertices without a fragment but with a degree
-	LG_TRY(counters.reserve(3 * sizeof(unsigned long long)));
-	LG_CUDA(cudaMemsetAsync(counters.p, 0, 3 * sizeof(unsigned long long), st), "memset");
+	                                  // [2] vertices without a fragment but with a degree,
+	                                  // [3] largest degree
+	LG_TRY(counters.reserve(4 * sizeof(unsigned long long)));
+	LG_CUDA(cudaMemsetAsync(counters.p, 0, 4 * sizeof(unsigned long long), st), "memset");
 	walk_fragments<true><<<grid_for(V, B), B, 0, st>>>(vt_tab(sn, csr), L, minL, V, nullptr,
 			nullptr, nullptr, FragOut{d.frag_off.as<uint32_t>(), d.slot_off.as<uint32_t>(),
 				d.frags.as<uint2>(), d.frag_start(), d.frag_vert(), d.tile_frag(),
@@ -1001,12 +1011,12 @@ static lg_status open_fill(lg_snapshot* sn, DevCsr& csr, SnapDir& d, unsigned lo
 		LG_CUDA(cudaGetLastError(), "window degrees");
 		s->launches++;
 	}
-	sum_u32<<<std::min<unsigned>(grid_for(V, B), 592u), B, 0, st>>>(d.deg.as<uint32_t>(), V,
-			counters.as<unsigned long long>());
+	sum_degrees<<<std::min<unsigned>(grid_for(V, B), 592u), B, 0, st>>>(d.deg.as<uint32_t>(), V,
+			counters.as<unsigned long long>(), counters.as<unsigned long long>() + 3);
 	LG_CUDA(cudaGetLastError(), "degree sum");
 	s->launches++;
-	LG_CUDA(cudaMemcpyAsync(w + 2, counters.p, 24, cudaMemcpyDeviceToHost, st), "d2h");
-	s->d2h_bytes += 24;
+	LG_CUDA(cudaMemcpyAsync(w + 2, counters.p, 32, cudaMemcpyDeviceToHost, st), "d2h");
+	s->d2h_bytes += 32;
 	return LG_OK;
 }
 
@@ -1016,6 +1026,7 @@ static void open_done(lg_snapshot* sn, DevCsr& csr, SnapDir& d, const unsigned l
 	for (int l = sn->min_level; l <= sn->level; l++) d.n_slots += csr.levels[l]->n_slots;
 	d.n_dels = w[3];
 	d.n_bare = w[4];
+	d.max_degree = w[5];
 	d.present = true;
 }
 
@@ -1024,13 +1035,13 @@ static lg_status open_dirs(lg_snapshot* sn) {
 	unsigned long long* w = nullptr;
 	LG_TRY(host_words(s, &w));
 	LG_TRY(open_count(sn, s->out, sn->out, w));
-	if (s->reverse) LG_TRY(open_count(sn, s->in, sn->in, w + 5));
+	if (s->reverse) LG_TRY(open_count(sn, s->in, sn->in, w + 6));
 	LG_CUDA(cudaStreamSynchronize(s->stream), "snapshot sizes");
 	LG_TRY(open_fill(sn, s->out, sn->out, w));
-	if (s->reverse) LG_TRY(open_fill(sn, s->in, sn->in, w + 5));
+	if (s->reverse) LG_TRY(open_fill(sn, s->in, sn->in, w + 6));
 	LG_CUDA(cudaStreamSynchronize(s->stream), "snapshot sizes");
 	open_done(sn, s->out, sn->out, w);
-	if (s->reverse) open_done(sn, s->in, sn->in, w + 5);
+	if (s->reverse) open_done(sn, s->in, sn->in, w + 6);
 	return LG_OK;
 }
 

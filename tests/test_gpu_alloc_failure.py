@@ -52,6 +52,8 @@ def _each_failure(fail_at, build, call):
 def test_push_runs_without_the_transpose(fail_at):
     V = 20000
     s, d = _graph(V, 800_000, 1)
+    k = np.unique(np.concatenate([s * V + d, np.arange(V)]))     # vertex 0 to all: a hub
+    s, d = k // V, k % V
 
     def build():
         st = Store(reverse_edges=False)

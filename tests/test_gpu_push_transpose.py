@@ -41,3 +41,24 @@ def test_push_both_ways(V, n, hub, reverse):
                 for it in (0, 1, 2, 4, 9):      # 5 M edge-iterations lie between
                     got = sn.pagerank_push(it)
                     assert max_rel_err(got, _reference(V, s[live], d[live], it)) <= 1e-12
+
+
+def test_graphs_without_hubs_push_for_longer():
+    """The rule's two lines.  A push takes a launch to begin and two per
+    iteration, the transpose a dozen and some more."""
+    rng = np.random.default_rng(5)
+    V, n = 100_000, 1_000_000
+    k = np.unique(rng.integers(0, V * V, n))
+    hub = np.unique(np.concatenate([k, 3 * V + np.arange(0, V, 50), np.arange(0, V, 50) * V + 3]))
+    for keys, last in ((k, 14), (hub, 5)):
+        s, d = keys // V, keys % V
+        for reverse in (False, True):
+            with Store(reverse_edges=reverse) as st:
+                st.build_level(V, s, d)
+                with st.snapshot() as sn:
+                    for it in (last, last + 1):
+                        before = st.launch_count
+                        got = sn.pagerank_push(it)
+                        pushed = st.launch_count - before == 1 + 2 * it
+                        assert pushed == (it == last)
+                        assert max_rel_err(got, _reference(V, s, d, it)) <= 1e-12
