@@ -250,14 +250,16 @@ lg_status ensure_split(lg_snapshot* sn, uint32_t delta) {
 // vertices found before every thread has seen that they are too many fill at
 // most half of the hash table.)
 //
-// It takes some 20 to 50 us with the wait, and an isolated root 100 us in all
+// It takes some 20 to 30 us with the wait, and an isolated root 100 us in all
 // instead of a flat copy and 414 us at 45 M slots, 204 at 16 M, 135 at 1.5 M.  From
-// kProbeFrom slots on it is worth that to the calls that reach more (1086 -> 1104 us
-// at 16 M slots; 497 -> 550 at 1.5 M).
-constexpr uint64_t kProbeFrom = 1u << 22;
-constexpr int kProbeLevels = 64;
+// kProbeFrom on, the slots and four times the vertices (what the copy's time goes
+// by), it is worth that to the calls that reach more: 1086 -> 1106 us at 16 M slots
+// and 1 M vertices; at 2 M and 1 M it would be 176 -> 211 for a star of 500.  (With
+// 1024 vertices and 8192 slots up to 60 us: 860 -> 930 us at two edges a vertex.)
+constexpr uint64_t kProbeFrom = 1u << 23;
+constexpr int kProbeLevels = 32;
 constexpr int kProbeThreads = 1024;
-constexpr uint32_t kProbeVerts = 1024, kProbeSlots = 8192, kProbeTab = 4096;
+constexpr uint32_t kProbeVerts = 256, kProbeSlots = 2048, kProbeTab = 4096;
 __global__ void __launch_bounds__(kProbeThreads)
 sssp_probe(SnapCsr out, uint32_t root, unsigned long long* large) {
 	__shared__ uint32_t tab[kProbeTab], queue[kProbeVerts];
@@ -337,7 +339,7 @@ extern "C" lg_status lg_sssp_delta(lg_snapshot* sn, int64_t root, uint32_t delta
 	bool small = false;                      // (and the snapshot is not flat)
 	if (!tune_value(s->device, LG_TUNE_SSSP_SPLIT) && !tune_value(s->device, LG_TUNE_SSSP_LEVELS)) {
 		const FlatCsr* f = fo && fo->weighted ? fo : nullptr;
-		if (!f && sn->out.n_frag_slots >= kProbeFrom) {
+		if (!f && sn->out.n_frag_slots + 4u * V >= kProbeFrom) {
 			// a flat copy costs the same whatever the root reaches
 			LG_TRY(sc[6].reserve(8 * sizeof(unsigned long long)));
 			unsigned long long large = 0;

@@ -26,19 +26,19 @@ def test_roots_of_every_reach():
     one = np.zeros(0, int)
     part("alone", 1, one, one)
     part("loop", 1, [0], [0])
-    for n in (30, 64, 65, 200):                  # hops up to the bound and beyond
+    for n in (20, 32, 33, 200):                  # hops up to the bound and beyond
         part(f"path {n}", n, np.arange(n - 1), np.arange(1, n))
-    for n in (1023, 1024, 1025, 5000):           # vertices
+    for n in (255, 256, 257, 1023, 1300, 5000):  # vertices
         part(f"star {n}", n, np.zeros(n - 1, int), np.arange(1, n))
-    for n in (90, 91, 92, 128):                  # slots: n (n - 1)
+    for n in (44, 45, 46, 128):                  # slots: n (n - 1)
         i, j = np.divmod(np.arange(n * n), n)
         part(f"clique {n}", n, i[i != j], j[i != j])
-    a = np.arange(1, 400)                        # a tree, and back edges
-    part("tree", 400, np.concatenate([(a - 1) // 3, a]), np.concatenate([a, a // 2]))
+    a = np.arange(1, 250)                        # a tree, and back edges
+    part("tree", 250, np.concatenate([(a - 1) // 3, a]), np.concatenate([a, a // 2]))
     part("cut", 10, [0, 1, 2], [1, 2, 3])        # 1 -> 2 is deleted later
     part("late", 10, one, one)                   # gets its edge later
     small = np.concatenate([p[0] for p in parts]), np.concatenate([p[1] for p in parts])
-    V = at
+    V = at + 1_000_000                           # (the rule counts vertices too)
     s = np.concatenate([key // big, small[0]])
     d = np.concatenate([key % big, small[1]])
     w = rng.integers(1, 70, len(s))
@@ -64,8 +64,8 @@ def test_roots_of_every_reach():
                 near = got < LG_UNREACHED
                 assert (r.reached, r.reach_edges, r.max_dist) == (
                     near.sum(), deg[near].sum(), got[near].max()), name
-                many = name in ("graph", "path 65", "path 200", "star 1025", "star 5000",
-                                "clique 92", "clique 128", "late")
+                many = name in ("graph", "path 33", "path 200", "star 257", "star 1023",
+                                "star 1300", "star 5000", "clique 46", "clique 128", "late")
                 # the search, init, the two launches of the steps and the sums;
                 # or (the search and) a flat copy
                 assert (st.launch_count - before > 5) == many, name
