@@ -339,10 +339,11 @@ __device__ __forceinline__ bool sf_step(const SfArgs& a, SfCtl* c, SfShared& sh,
 	unsigned long long* cnt = kSolo ? sh.ctr[slot] : c->ctr[slot];
 	slot = slot == 2u ? 0u : slot + 1u;
 	if (tid < 4 && (kSolo || blockIdx.x == 0)) (kSolo ? sh.ctr[slot] : c->ctr[slot])[tid] = 0;
+	// (by a warp that has the fewest rows, beside the others' work)
+	if (tid == kSfThreads - 1 && blockIdx.x == 0 && clock64() - sh.t0 > a.cycles)
+		atomicOr(cnt + 3, kCoopTimeUp);
 	// after a barrier every thread finds the step's counters in sh.got
 	auto barrier = [&]() {
-		if (tid == 0 && blockIdx.x == 0 && clock64() - sh.t0 > a.cycles)
-			atomicOr(cnt + 3, kCoopTimeUp);
 		if (!kSolo && !grid_barrier(&c->bar)) return false;
 		if (kSolo) __syncthreads();
 		if (tid < 4) {
