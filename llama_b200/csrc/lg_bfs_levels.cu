@@ -216,6 +216,9 @@ bfs_levels(SnapCsr out, const uint32_t* nz_rows, const uint32_t* nz_off, uint32_
 		if (top_down && has_in && (double)mf > (double)mu / kAlpha) top_down = false;
 		else if (!top_down && (double)qlen < (double)V / kBeta) top_down = true;
 		if (blockIdx.x == 0 && tid < 4) c->ctr[(cur + 2) % 3][tid] = 0;
+		// (by a warp that has the fewest rows, beside the others' work)
+		if (blockIdx.x == 0 && tid == kLvThreads - 1 && clock64() - t0 > cycles)
+			atomicOr(nxt + 1, kCoopTimeUp);
 		for (uint32_t w = gtid; w < W; w += nthreads) clear[w] = 0u;
 
 		if (top_down) {
@@ -436,7 +439,6 @@ bfs_levels(SnapCsr out, const uint32_t* nz_rows, const uint32_t* nz_off, uint32_
 			}
 			bu++;
 		}
-		if (gtid == 0 && clock64() - t0 > cycles) atomicOr(nxt + 1, kCoopTimeUp);
 		if (!grid_barrier(&c->bar)) return;
 		if (top_down) {
 			uint32_t* t = q; q = nq; nq = t;

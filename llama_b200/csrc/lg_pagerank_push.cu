@@ -86,13 +86,15 @@ namespace {
 // iterations for 1 M vertices and 2 M edges, 7.5 for 4 M and 16 M, 9 for 4 M and 32 M,
 // 19 for 0.5 M and 16 M, 8.5 for a grid of 2 M edges.  A hub is told by the largest
 // degree (out-degree where no in-edges are kept): from 0.1 % of the edges in R-MAT
-// graphs, up to 0.025 % in those others.
+// graphs, up to 0.025 % in those others.  With fewer edges than vertices a warp's
+// range of edges spans so many vertices that pushing takes longer than either (3 M
+// vertices, 0.3 M edges: 700 us an iteration; transposed, 20 take 632).
 bool transpose_pays(const lg_snapshot* sn, int iterations) {
 	const uint64_t E = sn->out.n_edges, V = sn->V;
 	const SnapDir& d = sn->in.present ? sn->in : sn->out;
 	if (iterations < 2) return false;
 	const uint64_t visits = (uint64_t)(iterations - 1) * E;
-	if (d.max_degree >= E / 2048u) return visits > 5000000ull;
+	if (d.max_degree >= E / 2048u || E < V) return visits > 5000000ull;
 	return visits > 13000000ull && (uint64_t)iterations >= 8u + E / (3u * V);
 }
 

@@ -887,12 +887,15 @@ __global__ void sum_degrees(const uint32_t* x, uint64_t n, unsigned long long* s
 		s += x[i];
 		m = max(m, x[i]);
 	}
-	uint64_t tot;
-	block_excl_scan(s, &tot);
-	if (threadIdx.x == 0 && tot) atomicAdd(sum, (unsigned long long)tot);
+	__shared__ uint32_t warp_most[32];
 	m = __reduce_max_sync(0xffffffffu, m);
-	if ((threadIdx.x & 31u) == 0 && m > *(volatile unsigned long long*)most)
-		atomicMax(most, (unsigned long long)m);
+	if ((threadIdx.x & 31u) == 0) warp_most[threadIdx.x >> 5] = m;
+	uint64_t tot;
+	block_excl_scan(s, &tot);                // (synchronises)
+	if (threadIdx.x != 0 || tot == 0) return;
+	for (uint32_t w = 1; w < blockDim.x / 32u; w++) m = max(m, warp_most[w]);
+	atomicAdd(sum, (unsigned long long)tot);
+	atomicMax(most, (unsigned long long)m);
 }
 
 // Opening a direction takes three parts, with one wait for both directions

@@ -62,3 +62,19 @@ def test_graphs_without_hubs_push_for_longer():
                         pushed = st.launch_count - before == 1 + 2 * it
                         assert pushed == (it == last)
                         assert max_rel_err(got, _reference(V, s, d, it)) <= 1e-12
+
+
+def test_fewer_edges_than_vertices():
+    """Transposed from the lower line on, hubs or not."""
+    rng = np.random.default_rng(6)
+    V = 1_500_000
+    k = np.unique(rng.integers(0, V * V, 600_000))
+    s, d = k // V, k % V
+    with Store(reverse_edges=False) as st:
+        st.build_level(V, s, d)
+        with st.snapshot() as sn:
+            for it, push in ((9, True), (10, False)):
+                before = st.launch_count
+                got = sn.pagerank_push(it)
+                assert (st.launch_count - before == 1 + 2 * it) == push
+                assert max_rel_err(got, _reference(V, s, d, it)) <= 1e-12
