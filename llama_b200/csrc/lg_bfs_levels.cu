@@ -46,6 +46,8 @@
 #include "lg_flat.cuh"
 #include "lg_tune.h"
 
+#include <cstddef>
+#include <cstring>
 #include <mutex>
 
 namespace lg {
@@ -535,26 +537,28 @@ lg_status bfs_levels_over(lg_store* s, SnapCsr out, const FlatCsr* fi, const uin
 			&has_in, &lvl, &q0, &q1, &bits0, &bits1, &bits2, &fcnt, &fpos, &bsum, &ctl, &cycles,
 			&resume};
 	s->launches++;
-	LvCtl h;
+	LvState t;
 	for (;; resume = 1) {
 		LG_CUDA(coop_launch((const void*)bfs_levels, &ctas, kLvThreads, args, 0, st, &ctl->bar),
 				"bfs_levels");
 		s->launches++;
-		LG_CUDA(cudaMemcpyAsync(&h, ctl, sizeof(h), cudaMemcpyDeviceToHost, st), "d2h");
-		LG_CUDA(cudaStreamSynchronize(st), "bfs_levels");
-		s->d2h_bytes += sizeof(h);
-		if (h.bar.err & 1u)
-			return set_error(LG_ETIMEOUT, "bfs: a grid barrier wait ran out");
-		if (h.bar.err & 2u)
-			return set_error(LG_ENOTSUP, "bfs: a frontier holds 2^32 or more slots");
-		if (h.st.done) break;
+		constexpr int kWords = 2 + (int)(sizeof(LvState) / 8);
+		static_assert(offsetof(LvCtl, st) == offsetof(LvCtl, bar) + 16 && kWords <= kReadWords,
+				"the barrier, then the state");
+		unsigned long long o[kWords];
+		LG_TRY(read_words(s, reinterpret_cast<const unsigned long long*>(&ctl->bar), kWords, o));
+		const unsigned err = (unsigned)o[1];
+		if (err & 1u) return set_error(LG_ETIMEOUT, "bfs: a grid barrier wait ran out");
+		if (err & 2u) return set_error(LG_ENOTSUP, "bfs: a frontier holds 2^32 or more slots");
+		std::memcpy(&t, o + 2, sizeof(t));
+		if (t.done) break;
 	}
 	if (result) {
-		result->reached = h.st.reached;
-		result->reach_edges = h.st.reach_edges;
-		result->max_level = h.st.cur - 1;
-		result->top_down_steps = h.st.td;
-		result->bottom_up_steps = h.st.bu;
+		result->reached = t.reached;
+		result->reach_edges = t.reach_edges;
+		result->max_level = t.cur - 1;
+		result->top_down_steps = t.td;
+		result->bottom_up_steps = t.bu;
 		result->reserved = 0;
 	}
 	*ran = true;
