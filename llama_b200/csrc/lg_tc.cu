@@ -642,8 +642,21 @@ extern "C" lg_status lg_triangle_count(lg_snapshot* sn, lg_tc_result* result) {
 	LG_CUDA(cudaGetLastError(), "tc_emit");
 	s->launches += 4;
 	u64* sorted = nullptr;
-	LG_TRY(radix_sort_u64(s, keys.as<u64>(), nullptr, E, tmpk, tmpp, counts, scan_tmp, &sorted,
-			nullptr, bits < 32 ? (1ull << (2 * bits)) - 1ull : ~0ull));
+	auto sort = [&]() {
+		return radix_sort_u64(s, keys.as<u64>(), nullptr, E, tmpk, tmpp, counts, scan_tmp, &sorted,
+				nullptr, bits < 32 ? (1ull << (2 * bits)) - 1ull : ~0ull);
+	};
+	lg_status sorted_ok = sort();
+	if (sorted_ok == LG_ENOMEM && f == s->flat_scratch) {
+		// with what the flat copy took: the keys hold the edges now
+		clear_error();
+		LG_CUDA(cudaStreamSynchronize(st), "triangles");
+		f = nullptr;
+		delete s->flat_scratch;
+		s->flat_scratch = nullptr;
+		sorted_ok = sort();
+	}
+	LG_TRY(sorted_ok);
 	const unsigned uq_tiles = grid_for(E, kUqTile);
 	LG_TRY(tiles.reserve((2ull * uq_tiles + 1) * 4));
 	uint32_t* tile_cnt = tiles.as<uint32_t>();

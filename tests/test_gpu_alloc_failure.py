@@ -101,3 +101,19 @@ def test_ppr_runs_over_the_levels(fail_at, K, ktile):
         # rows of at most 4000 positive terms, six iterations
         assert got is None or max_rel_err(got, want) <= 6 * 2 * 4000 * 2.0 ** -53
         assert np.array_equal(again, want)
+
+
+def test_triangles_sort_without_the_flat_copy(fail_at):
+    V = 3000
+    s, d = _graph(V, 90_000, 7)
+
+    def build():
+        st = Store(reverse_edges=False)
+        st.build_level(V, s, d)
+        return st
+    results = list(_each_failure(fail_at, build, lambda sn: sn.triangle_count().triangles))
+    want = results[-1][0]
+    right = [got is not None for got, _ in results]
+    assert all(got in (None, want) and again == want for got, again in results)
+    # two of the sort's at the least: its second array of keys and its counts
+    assert sum(right[:-1]) >= 2 and want > 0
